@@ -73,6 +73,11 @@ inline float rn_reciprocal(float b)
     return best;
 }
 
+// Whether the division-free quotients (and, for the zero point, the 2^23 byte-to-float trick) are exact for a tensor's
+// quantisation parameters; anything else takes the kernels with the IEEE division.
+inline bool ordinary_scale(float s) { return s >= 1e-20f && s <= 1e20f; }
+inline bool ordinary_quant(const b200k_qtensor& t) { return ordinary_scale(t.scale) && t.zero_point > -(1 << 20) && t.zero_point < (1 << 20); }
+
 // The contraction epilogue v = fl(fl(acc * m) + b); q = clamp(zy + round_half_away(fl(v / sy)), lo, hi) without the
 // division unit: with y = RN(1 / sy) from the host, p = fl(v * y) and q = fma(fma(-p, sy, v), y, p) is the correctly
 // rounded quotient (Markstein); it is rounded with the 1.5 * 2^23 constant (halves to even) and only exact halves, or
@@ -290,6 +295,62 @@ __device__ __forceinline__ void requant_fast2(int acc0, int acc1, f32x2 m2, f32x
     r1 = fminf(fmaxf(z1, lo), hi);
 }
 
+
+// zero point + round_half_away(fl(v / sy)) of four values (integer-valued floats, not clamped): Markstein's correctly
+// rounded quotient with inv = RN(1 / sy), the 1.5 * 2^23 constant, roundf for exact halves (see requant_fast; values too
+// large for the constant are far outside every 8-bit range).  One test for the four.
+struct Quant4 {
+    float sy, inv_sy, zy;
+    __device__ __forceinline__ void operator()(f32x2 v01, f32x2 v23, float* z) const
+    {
+        const f32x2 magic2 = pack2(12582912.0f, 12582912.0f), sy2n = pack2(-sy, -sy), inv2 = pack2(inv_sy, inv_sy), zy2 = pack2(zy, zy);
+        const f32x2 p01 = mul2(v01, inv2), p23 = mul2(v23, inv2);
+        const f32x2 q01 = fma2(fma2(p01, sy2n, v01), inv2, p01), q23 = fma2(fma2(p23, sy2n, v23), inv2, p23);
+        f32x2 n01 = sub2(add2(q01, magic2), magic2), n23 = sub2(add2(q23, magic2), magic2);
+        float d[4];
+        unpack2(sub2(q01, n01), d[0], d[1]);
+        unpack2(sub2(q23, n23), d[2], d[3]);
+        if (fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fmaxf(fabsf(d[2]), fabsf(d[3]))) >= 0.5f) {
+            float q[4], n[4];
+            unpack2(q01, q[0], q[1]); unpack2(q23, q[2], q[3]);
+            unpack2(n01, n[0], n[1]); unpack2(n23, n[2], n[3]);
+            #pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (fabsf(d[k]) >= 0.5f) n[k] = roundf(q[k]);
+            n01 = pack2(n[0], n[1]); n23 = pack2(n[2], n[3]);
+        }
+        unpack2(add2(n01, zy2), z[0], z[1]);
+        unpack2(add2(n23, zy2), z[2], z[3]);
+    }
+};
+
+// The four bytes of a word minus the zero point, as float pairs: a byte below 2^23's exponent is the float 2^23 + byte, so
+// one permute per value and one exact subtraction per pair replace extractions, sign extensions and conversions (which
+// share a slow pipe).  flip: 0x80808080 for int8 (re-read as byte + 128), 0 for uint8; off = 2^23 + zero point (+ 128 for
+// int8), twice.
+__device__ __forceinline__ void bytes_minus_zp(uint32_t w, uint32_t flip, f32x2 off2, f32x2& v01, f32x2& v23)
+{
+    w ^= flip;
+    v01 = sub2(pack2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440)), __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7441))), off2);
+    v23 = sub2(pack2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7442)), __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7443))), off2);
+}
+
+// Four integer-valued floats as bytes with the 8-bit type's own saturation (a conversion and a saturating pack per pair)
+__device__ __forceinline__ uint32_t sat_pack4(const float* z, bool s8)
+{
+    int i[4];
+    #pragma unroll
+    for (int k = 0; k < 4; ++k) asm("cvt.rni.s32.f32 %0, %1;" : "=r"(i[k]) : "f"(z[k]));
+    uint32_t hi, out;
+    if (s8) {
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(i[3]), "r"(i[2]), "r"(0));
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(out) : "r"(i[1]), "r"(i[0]), "r"(hi));
+    } else {
+        asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(i[3]), "r"(i[2]), "r"(0));
+        asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(out) : "r"(i[1]), "r"(i[0]), "r"(hi));
+    }
+    return out;
+}
 
 // Addend of the one-FMA requantisation q" = fma(float(acc), m / sy, bq): bq of one (class, column) to within one rounding
 // of its last operation: X = (b - cc m) / sy from error-free
