@@ -105,6 +105,25 @@ __device__ __forceinline__ int dp4a_mixed(uint32_t x, uint32_t w, int acc)
     return d;
 }
 
+// Sixteen bytes from any address, the first n of them (zeros for the rest; n may be <= 0 or > 16): from the aligned words that
+// hold them, of which only those with at least one wanted byte are read.
+__device__ __forceinline__ uint4 load16_any(const uint8_t* p, int n)
+{
+    const int sh = (int)((uintptr_t)p & 3);
+    const uint32_t* q = (const uint32_t*)(p - sh);
+    uint32_t w[5], o[4];
+    const int end = sh + (n < 16 ? n : 16);
+    #pragma unroll
+    for (int i = 0; i < 5; ++i) w[i] = n > 0 && 4 * i < end ? q[i] : 0u;
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t v = __funnelshift_r(w[i], w[i + 1], 8 * sh);
+        const int keep = n - 4 * i;
+        o[i] = keep >= 4 ? v : (keep <= 0 ? 0u : v & (0xffffffffu >> (8 * (4 - keep))));
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // v = float(q - zp) * scale
 __device__ __forceinline__ float dequantize_dev(int q, float scale, int zp)
 {

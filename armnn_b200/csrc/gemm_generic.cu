@@ -2,7 +2,6 @@
 // tensor-core kernel of bmm_mma.cu) and FullyConnected with non-transposed ([K, N]) weights.  16 x 16 output tile per
 // CTA, operands staged through shared memory as zero-point-corrected ints.
 #include <string.h>
-#include <atomic>
 #include "common.cuh"
 
 namespace b200k {
@@ -14,6 +13,8 @@ bool fc_stream_eligible(const b200k_fc_params* p);
 bool bmm_mma_eligible(const b200k_bmm_params* p);
 int launch_bmm_mma(const b200k_bmm_params* p, cudaStream_t stream);
 int launch_fc_stream(const b200k_fc_params* p, cudaStream_t stream);
+bool fc_mma_eligible(const b200k_fc_params* p);
+int launch_fc_mma(const b200k_fc_params* p, cudaStream_t stream);
 
 struct BmmArgs {
     const void* x; const void* y; void* out; int32_t* acc_out;
@@ -87,14 +88,14 @@ extern "C" int b200k_batch_matmul_q8(const b200k_bmm_params* p, void* stream)
     return check_launch("bmm_generic_kernel");
 }
 
-// ---- FullyConnected with [N, K] weights that the tcgen05 kernel cannot take (N not a multiple of 16: classifier heads)
+// ---- FullyConnected with [N, K] weights and at most FC_ROWS rows whose K the weight-streaming kernel cannot take
 //
-// A block owns FC_COLS output columns (one per warp) and FC_ROWS (4, 16 or 32: the smallest that covers M) rows of x, which it stages in shared memory once.
+// A block owns FC_COLS output columns (one per warp) and all rows of x, which it stages in shared memory once.
 // A warp streams its weight row through registers 16 bytes per lane at a time and multiplies it with every staged row
 // (dp4a); the per-lane partial sums of the FC_ROWS rows are then reduced across the warp so that lane r ends up with
 // row r, applies the zero-point terms  sum (x - zx)(w - zw) = sum x w - zw sum x - zx sum w + K zx zw  and the
 // requantisation, and stores one byte.
-constexpr int FC_COLS = 8, FC_KT = 2048;              // rows per block: 4, 16 or 32 (template parameter)
+constexpr int FC_COLS = 8, FC_KT = 2048, FC_ROWS = 4;
 
 struct FcRowsArgs {
     const uint8_t* x; const uint8_t* w; const int32_t* bias; uint8_t* y; int32_t* acc_out;
@@ -105,7 +106,7 @@ struct FcRowsArgs {
     float inv_sy, lo, hi;
 };
 
-template <bool XU, bool WU, int FC_ROWS>
+template <bool XU, bool WU>
 __global__ void __launch_bounds__(32 * FC_COLS) fc_rows_kernel(const FcRowsArgs a)
 {
     pdl_enter();
@@ -212,30 +213,10 @@ static int launch_fc_rows(const b200k_fc_params* p, cudaStream_t stream)
     a.hi = fminf(a.rq.thi, (float)a.rq.chi);
     const int kt = p->k < FC_KT ? p->k : FC_KT;
     const bool xu = p->x.dtype == B200K_U8, wu = p->w.dtype == B200K_U8;
-    #define B200K_FC_ROWS(XU, WU, RB)                                                                                  \
-        do {                                                                                                           \
-            /* the opt-in is per device: one flag per device index */                                                  \
-            static std::atomic<bool> configured[64];                                                                   \
-            int dev_ = 0;                                                                                              \
-            if (cudaGetDevice(&dev_) != cudaSuccess || dev_ < 0 || dev_ >= 64) dev_ = 0;                               \
-            if (!configured[dev_].load(std::memory_order_acquire)) {                                                   \
-                B200K_CUDA(cudaFuncSetAttribute(fc_rows_kernel<XU, WU, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                RB * FC_KT));                                                          \
-                configured[dev_].store(true, std::memory_order_release);                                               \
-            }                                                                                                          \
-            const dim3 grid(div_up(p->n, FC_COLS), div_up(p->m, RB), 1);                                               \
-            launch_pdl(fc_rows_kernel<XU, WU, RB>, grid, dim3(32 * FC_COLS), (size_t)RB * kt, stream, a);              \
-        } while (0)
-    #define B200K_FC_TYPES(RB)                                                                                         \
-        do {                                                                                                           \
-            if (xu) { if (wu) B200K_FC_ROWS(true, true, RB); else B200K_FC_ROWS(true, false, RB); }                    \
-            else    { if (wu) B200K_FC_ROWS(false, true, RB); else B200K_FC_ROWS(false, false, RB); }                  \
-        } while (0)
-    if (p->m <= 4)       B200K_FC_TYPES(4);
-    else if (p->m <= 16) B200K_FC_TYPES(16);
-    else                 B200K_FC_TYPES(32);
-    #undef B200K_FC_TYPES
-    #undef B200K_FC_ROWS
+    const dim3 grid(div_up(p->n, FC_COLS), div_up(p->m, FC_ROWS), 1);
+    auto go = [&](auto kern) { launch_pdl(kern, grid, dim3(32 * FC_COLS), (size_t)FC_ROWS * kt, stream, a); };
+    if (xu) { if (wu) go(fc_rows_kernel<true, true>); else go(fc_rows_kernel<true, false>); }
+    else    { if (wu) go(fc_rows_kernel<false, true>); else go(fc_rows_kernel<false, false>); }
     return check_launch("fc_rows_kernel");
 }
 
@@ -252,12 +233,13 @@ extern "C" int b200k_fully_connected_q8(const b200k_fc_params* p, void* stream)
         c.kh = c.kw = 1; c.stride_h = c.stride_w = 1; c.dil_h = c.dil_w = 1;
         c.clamp_lo = p->clamp_lo; c.clamp_hi = p->clamp_hi; c.acc_out = p->acc_out; c.algo = p->algo;
         c.packed = p->packed;
-        // the tcgen05 kernel when it can take the shape; otherwise the row kernel; the CUDA-core convolution for the rest
-        // (a few rows are a weight-streaming problem: the row kernel spreads the columns over every SM, whereas the
-        // tensor-core kernel would give each 64-column tile's whole K loop to one CTA)
+        // (a few rows are a weight-streaming problem: the first two kernels spread the columns over every SM, whereas the
+        // tcgen05 kernel would give each 64-column tile's whole K loop to one CTA)
         // at most 16 rows: nothing but a read of the weights, which the streaming kernel spreads over every SM
         if (p->algo == 0 && fc_stream_eligible(p)) return launch_fc_stream(p, (cudaStream_t)stream);
-        if (p->algo == 0 && fc_rows_eligible(p) && (p->m <= 4 || !conv_tc_eligible(&c))) return launch_fc_rows(p, (cudaStream_t)stream);
+        if (p->algo == 0 && fc_rows_eligible(p) && p->m <= FC_ROWS) return launch_fc_rows(p, (cudaStream_t)stream);
+        // the tcgen05 kernel when it can take the shape, mma.sync for the odd ones
+        if (p->algo == 0 && !conv_tc_eligible(&c) && fc_mma_eligible(p)) return launch_fc_mma(p, (cudaStream_t)stream);
         return conv2d_dispatch(&c, (cudaStream_t)stream);
     }
     B200K_REQUIRE(p->x.data && p->w.data && p->y.data, B200K_E_INVALID, "fully_connected_q8: null tensor pointer");

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from cases import F32, S8, U8, SimpleCase, _abi, _rand, qt, qt_out, run_case
-from q8util import activation_clamp, diff_stats
+from q8util import activation_clamp, diff_stats, random_fc_case
 
 pytestmark = pytest.mark.gpu
 
@@ -160,7 +160,16 @@ def mean(seed, n, h, w, c, dtype):
 MEAN_CASES = {"f32_1x1_c1": lambda: mean(1, 2, 1, 1, 1, F32), "f32_28x28_c33": lambda: mean(2, 2, 28, 28, 33, F32), "s8_128_pixels_c132": lambda: mean(3, 2, 8, 16, 132, S8),
               "u8_129_pixels_c5": lambda: mean(4, 1, 3, 43, 5, U8)}
 
-EXACT = {"f32": F32_CASES, "eltwise": ELTWISE_CASES, "resize": RESIZE_CASES, "arg": ARG_CASES, "mean": MEAN_CASES}
+U8_HEAD = dict(x_dtype=U8, w_dtype=U8, y_dtype=U8, per_axis=False, x_q=(0.03, 119))
+FC_CASES = {
+    # 32 x 32 tiles with remainders; K below a slice, beyond one pass, odd and at odd addresses; every signedness
+    "m5_k1_n1": lambda: random_fc_case(1, 5, 1, 1), "m33_k31_n33": lambda: random_fc_case(2, 33, 31, 33),
+    "m200_k1280_n1001_u8": lambda: random_fc_case(3, 200, 1280, 1001, **U8_HEAD), "m32_k2049_n40": lambda: random_fc_case(4, 32, 2049, 40),
+    "m64_k4101_n65_u8": lambda: random_fc_case(5, 64, 4101, 65, **U8_HEAD), "m17_k130_n2033_u8x": lambda: random_fc_case(6, 17, 130, 2033, x_dtype=U8, y_dtype=U8, x_q=(0.03, 100)),
+    "m6_k2080_n31_u8w": lambda: random_fc_case(7, 6, 2080, 31, w_dtype=U8, per_axis=False), "m1_k451_n77": lambda: random_fc_case(8, 1, 451, 77),
+}
+
+EXACT = {"fc": FC_CASES, "f32": F32_CASES, "eltwise": ELTWISE_CASES, "resize": RESIZE_CASES, "arg": ARG_CASES, "mean": MEAN_CASES}
 ROUNDED = {"softmax": SOFTMAX_CASES}
 
 
