@@ -169,7 +169,30 @@ FC_CASES = {
     "m6_k2080_n31_u8w": lambda: random_fc_case(7, 6, 2080, 31, w_dtype=U8, per_axis=False), "m1_k451_n77": lambda: random_fc_case(8, 1, 451, 77),
 }
 
-EXACT = {"fc": FC_CASES, "f32": F32_CASES, "eltwise": ELTWISE_CASES, "resize": RESIZE_CASES, "arg": ARG_CASES, "mean": MEAN_CASES}
+
+def bmm(seed, batch, m, k, n, tx, ty, xt=S8, yt=S8, ot=S8, bcast=False):
+    def build(mem):
+        rng = np.random.default_rng(seed)
+        p = _abi.BmmParams()
+        p.x = qt(mem, _rand(rng, xt, (batch, k, m) if tx else (batch, m, k)), xt, 0.02, 3 if xt == S8 else 126)
+        p.y = qt(mem, _rand(rng, yt, ((1,) if bcast else (batch,)) + ((n, k) if ty else (k, n))), yt, 0.03, -2 if yt == S8 else 131)
+        p.out, out = qt_out(mem, (batch, m, n), ot, 0.02 * 0.03 * 74 * 74 * float(k) ** 0.5 / 30, 4 if ot == S8 else 120)
+        p.batch, p.m, p.k, p.n, p.transpose_x, p.transpose_y = batch, m, k, n, int(tx), int(ty)
+        p.batch_stride_x, p.batch_stride_y = m * k, 0 if bcast else k * n
+        return p, [out]
+    return SimpleCase("batch_matmul_q8", build)
+
+
+# tiles of 128 x 64 and 128 x 128 with remainders, fewer steps than stages, every layout, odd row lengths, every signedness
+BMM_CASES = {"%s%s_b%d_m%d_k%d_n%d" % ("T" if tx else "N", "T" if ty else "N", b, m, k, n):
+             (lambda i=i, b=b, m=m, k=k, n=n, tx=tx, ty=ty, t=t: bmm(40 + i, b, m, k, n, tx, ty, *t))
+             for i, (b, m, k, n, tx, ty, t) in enumerate((
+                 (1, 1, 1, 1, 0, 0, (S8, S8, S8)), (3, 129, 64, 64, 0, 1, (S8, S8, S8)), (2, 128, 65, 128, 0, 1, (U8, U8, U8)), (2, 130, 200, 65, 0, 0, (S8, U8, S8)),
+                 (2, 17, 512, 33, 0, 0, (U8, S8, S8)), (1, 64, 333, 129, 1, 0, (S8, S8, U8)), (2, 136, 128, 48, 1, 1, (S8, S8, S8)), (5, 96, 17, 17, 1, 1, (U8, U8, S8)),
+                 (2, 256, 256, 256, 1, 0, (S8, S8, S8)), (3, 77, 96, 77, 0, 1, (S8, S8, S8)), (3, 77, 77, 32, 0, 0, (S8, S8, S8)), (1, 128, 192, 20, 0, 0, (S8, S8, S8))))}
+BMM_CASES["broadcast"] = lambda: bmm(60, 4, 40, 72, 80, 0, 0, bcast=True)
+
+EXACT = {"bmm": BMM_CASES, "fc": FC_CASES, "f32": F32_CASES, "eltwise": ELTWISE_CASES, "resize": RESIZE_CASES, "arg": ARG_CASES, "mean": MEAN_CASES}
 ROUNDED = {"softmax": SOFTMAX_CASES}
 
 
