@@ -128,3 +128,26 @@ def test_pipelined_requests_match_blocking_enqueue():
     assert len({w.numpy().tobytes() for w in want}) > 1          # the requests really differ
     for w, g in zip(want, got):
         assert torch.equal(w, g)
+
+
+@pytest.mark.parametrize("elements", [1, 1000, 1 << 20, (1 << 20) + 1])
+def test_host_arrays_staged_and_direct(elements):
+    """Pageable and pinned host arrays on both sides of the staging limit, one output bound twice, changing inputs."""
+    import torch
+    from armnn_b200 import network
+    from armnn_b200.network import DataType, TensorInfo
+    net = network.INetwork()
+    a, act = net.AddInputLayer(0), net.AddActivationLayer(network.ActivationFunction.ReLu)
+    a.GetOutputSlot(0).Connect(act.GetInputSlot(0))
+    for layer in (a, act):
+        layer.GetOutputSlot(0).SetTensorInfo(TensorInfo((1, elements), DataType.QAsymmS8, 0.5, 3))
+    for i in range(2):
+        act.GetOutputSlot(0).Connect(net.AddOutputLayer(i).GetInputSlot(0))
+    rt, opt, ln = _load(net)
+    rng = np.random.default_rng(3)
+    for request in range(3):
+        x = rng.integers(-128, 128, size=(1, elements)).astype(np.int8)
+        y, pinned = np.zeros_like(x), torch.zeros((1, elements), dtype=torch.int8).pin_memory()
+        ln.EnqueueWorkload({0: x if request != 1 else torch.from_numpy(x).pin_memory()}, {0: y, 1: pinned})
+        want = np.maximum(x, 3)
+        assert np.array_equal(y, want) and np.array_equal(pinned.numpy(), want), request
