@@ -1,153 +1,502 @@
 // One QLstm step, reproducing RefQLstmWorkload::Execute operation by operation
 // (src/backends/reference/workloads/RefQLstmWorkload.cpp:46-541, LstmUtils.cpp:16-256 of the Arm NN tree).
 //
-// CpuRef keeps the gate pre-activations in int16 buffers and re-quantises them after EVERY
-// multiply-accumulate of the mat-vec products (LstmUtils.cpp:87-111), so a gate value is the end of a
-// K-long chain  acc <- Q16(deq(acc) + deq(w) * deq(x))  whose result depends on every intermediate rounding
-// and saturation.  An int32 dot product followed by one requantisation is a different function, so the
-// kernel evaluates the chains themselves: one chain per (gate, unit) of a batch row, all chains of a row
-// in one CTA, 2 chains per thread for instruction-level parallelism, and the GPU hides the chain latency
-// by running every (row, gate, unit) chain concurrently.  This is latency/issue-bound fp32 work: no
-// tensor cores.  The int16 accumulator is carried as an integer-valued float (the clamp keeps it in
-// [-32768, 32767], where float is exact), which removes two conversions per step without changing a bit.
+// CpuRef keeps the gate pre-activations in int16 buffers and re-quantises them after EVERY multiply-accumulate of the
+// mat-vec products (LstmUtils.cpp:87-111), so a gate value is the end of a K-long chain
+//     acc <- clamp16(round_half_away(fl(fl(fl(acc * sG) + fl(fl(w * sw) * x)) / sG)))
+// whose result depends on every intermediate rounding and saturation; an int32 dot product followed by one requantisation
+// is a different function.  But acc is an integer and acc * sG / sG is acc up to a few roundings, so the step adds
+// round(r), r = w x sw / sG, whatever acc is, unless r lies within
+//     E = 2^-24 (3 |acc| + 8 |r| + 8)
+// of a half or the sum reaches the clamp.  One fused multiply-add does that step:
+//     T' = RN(T + w xc),  xc = x sw / sG,  T = 1.5 * 2^23 + acc.
+// r depends on the product of two bytes only.  The host lists, per pair of gates, the input magnitudes for which SOME weight
+// byte comes that close to a half (with |acc| <= QL_LEVEL; with the scales of the reference's own test a third of the inputs
+// for two gates, one in a hundred for the others).  A block of eight steps without such an input is eight FMAs.  In any other
+// block d = w xc - (T' - T), exact, is formed as well, and its largest magnitude tells whether every rounding was the
+// reference's.  Blocks that cannot vouch for themselves (two per thread and row on average) are noted down with the
+// accumulators they began with, and their doubtful steps are evaluated with the reference's own arithmetic at the end of the
+// chain: as a step's increment does not depend on acc, a rounding that went the other way shifts everything after it by the
+// same integer.  A warp with an accumulator that might reach the clamp evaluates the block by the reference's arithmetic.
 //
-// One CTA handles one batch row through the whole step: mat-vecs -> (peephole) -> layer norm ->
-// activations -> cell update -> output gate -> hidden state -> projection -> outputs.  Layer-norm sums
-// are accumulated by a single thread per gate in index order because CpuRef's fp32 sums are sequential.
+// A cluster of CTAs works on R (1 or 2) batch rows: every CTA runs the chains of its share of the units (a thread has two
+// gates of one unit, a packed pair, and converts each weight once for all R rows; weights come through shared memory, a
+// tile ahead) and writes the results into the shared memory of the row's owner; CTA r of the cluster then takes row r
+// through (peephole) -> layer norm -> activations -> cell update -> output gate -> hidden state -> projection (chains of the
+// same kind) -> outputs.  Layer-norm sums are sequential in the reference: one thread per gate, its operands read ahead.
+//
+// Bound by the fp32 pipe in the chains and by the latency of the sequential sums.
+#include <mutex>
+#include <type_traits>
 #include "common.cuh"
 
 namespace b200k {
 
-constexpr int QL_THREADS = 1024;
+constexpr int QL_UNITS = 256;                    // units a CTA works on at a time: one thread per unit and pair of gates
+constexpr int QL_THREADS = 2 * QL_UNITS;
+constexpr int QL_SEG = 1024;                     // steps whose factors are staged at once, at most
+constexpr int QL_TILE = 64, QL_PITCH = QL_TILE + 16;     // weight bytes per row and tile; conflict-free 128-bit reads
+constexpr int QL_TILE_BYTES = 4 * QL_UNITS * QL_PITCH;
+constexpr int QL_NOTES = 8;                      // doubtful blocks a thread can note down per row
+constexpr float QL_LEVEL = 2048.0f;              // |acc| up to which the host's list of inputs holds
+constexpr float QL_NEAR_CLAMP = 32000.0f;        // |acc| from which on saturation is possible (zero points included)
+constexpr float QL_ULP = 6.0e-8f;                // a little more than 2^-24
+constexpr int QL_GATE_SLACK = 64;                // floats behind the gate buffers (the projection factors are padded)
+constexpr float QL_MAGIC = 12582912.0f;          // 1.5 * 2^23
 
-__device__ __forceinline__ float q16f(float v, float scale)          // Quantize<int16_t>, offset 0, as float
+// round_half_away(fl(v / scale)) without the division unit (inv = RN(1 / scale)): Markstein's correctly rounded quotient and
+// the 1.5 * 2^23 constant; exact halves, and whatever is not finite, go through the division.
+__device__ __forceinline__ float ql_round_div(float v, float scale, float inv)
 {
-    return fminf(fmaxf(roundf(__fdiv_rn(v, scale)), -32768.f), 32767.f);
+    const float p = __fmul_rn(v, inv);
+    const float q = __fmaf_rn(__fmaf_rn(-p, scale, v), inv, p);
+    float n = __fsub_rn(__fadd_rn(q, QL_MAGIC), QL_MAGIC);
+    if (!(fabsf(__fsub_rn(q, n)) < 0.5f)) n = roundf(__fdiv_rn(v, scale));
+    return n;
+}
+__device__ __forceinline__ float q16f(float v, float scale, float inv)          // Quantize<int16_t>, offset 0, as float
+{
+    return fminf(fmaxf(ql_round_div(v, scale, inv), -32768.f), 32767.f);
 }
 __device__ __forceinline__ float q16zf(float v, float scale, float zp)
 {
     return fminf(fmaxf(__fadd_rn(zp, roundf(__fdiv_rn(v, scale))), -32768.f), 32767.f);
 }
 
-// round_half_away(fl(v / scale)) without the division unit, for the long chains: with inv = RN(1 / scale)
-// (__frcp_rn), p = fl(v * inv) and q = fma(fma(-p, scale, v), inv, p) is the correctly rounded quotient (Markstein);
-// q is rounded with the 1.5 * 2^23 constant (halves to even), and only when q is an exact half or too large for the
-// constant does roundf decide.
-__device__ __forceinline__ float round_div_fast(float v, float scale, float inv)
-{
-    const float p = __fmul_rn(v, inv);
-    const float q = __fmaf_rn(__fmaf_rn(-p, scale, v), inv, p);
-    float n = __fsub_rn(__fadd_rn(q, 12582912.0f), 12582912.0f);
-    if (fabsf(__fsub_rn(q, n)) >= 0.5f) n = roundf(q);
-    return n;
-}
-__device__ __forceinline__ float q16f_fast(float v, float scale, float inv)
-{
-    return fminf(fmaxf(round_div_fast(v, scale, inv), -32768.f), 32767.f);
-}
-__device__ __forceinline__ float q16zf_fast(float v, float scale, float inv, float zp)
-{
-    return fminf(fmaxf(__fadd_rn(zp, round_div_fast(v, scale, inv)), -32768.f), 32767.f);
-}
+// Input magnitudes 0 .. 255 (|q - zero point|), one bit each, that can bring a product close to a half.
+struct QlDanger { uint32_t bits[8]; };
 
 struct QlArgs {
     b200k_qlstm_params p;
     int cifg, peephole, ln, proj;
+    int seg, both;                               // staged steps: a multiple of 16; both sources fit at once
+    int exact_only;                              // scales outside the range the error bound holds for: every step by the reference's arithmetic
+    int vec_i, vec_o, vec_p;                     // weight rows are whole aligned 16-byte pieces
+    int nbuf;                                    // weight tiles in shared memory: 1 or 2
+    int proj_staged;                             // the projection weights fit the tiles' space
+    unsigned tile_off;                           // where the weight tiles begin in shared memory
+    QlDanger danger[2][2], danger_p;             // [input, recurrent][pair of gates: (i, c), (f, o)]; projection
 };
 
-// acc <- chain over k of Q16(acc*sG + (w[k]*sw) * v[k]) for two independent chains (A and B), both evaluated by
-// packed two-wide fp32 instructions (the chains of a row keep the schedulers' issue slots busy, so halving the
-// instruction count is what counts).  v2 holds every value twice, as (x, x) pairs.  Products that the reference
-// rounds before adding are formed as fma2(a, b, 0): a packed multiply feeding a packed add would be contracted.
-// Quantize to int16: Markstein's correctly rounded quotient, the 1.5 * 2^23 rounding constant, and roundf for the
-// exact halves it rounds to even where the reference rounds away from zero (see round_div_fast).
-template <bool VEC>
-__device__ __forceinline__ void chain2(float& accA, float& accB, const int8_t* wA, const int8_t* wB, float swA, float swB,
-                                        const float2* v2, int K, float sGA, float sGB, bool hasB)
+__device__ __forceinline__ uint32_t ql_cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t ql_cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void ql_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void ql_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// a float into the shared memory of CTA `rank` of the cluster, at the address `mine` has in this CTA
+__device__ __forceinline__ void ql_store_remote(float* mine, uint32_t rank, float v)
 {
-    const float iGA = __frcp_rn(sGA), iGB = __frcp_rn(sGB);
-    const f32x2 sG2 = pack2(sGA, sGB), nsG2 = pack2(-sGA, -sGB), iG2 = pack2(iGA, iGB), sw2 = pack2(swA, swB);
-    const f32x2 zero2 = pack2(0.f, 0.f), magic2 = pack2(12582912.0f, 12582912.0f);
-    f32x2 acc2 = pack2(accA, accB);
-    auto step = [&](float wa, float wb, int k) {
-        const float2 xx = v2[k];
-        const f32x2 t2 = fma2(fma2(pack2(wa, wb), sw2, zero2), pack2(xx.x, xx.y), zero2);    // fl(fl(w * sw) * x)
-        const f32x2 a2 = add2(fma2(acc2, sG2, zero2), t2);                                    // fl(fl(acc * sG) + t)
-        const f32x2 p2 = mul2(a2, iG2);
-        const f32x2 q2 = fma2(fma2(p2, nsG2, a2), iG2, p2);                                   // RN(a / sG)
-        const f32x2 n2 = sub2(add2(q2, magic2), magic2);
-        float qa, qb, na, nb;
-        unpack2(q2, qa, qb); unpack2(n2, na, nb);
-        if (fabsf(__fsub_rn(qa, na)) >= 0.5f) na = roundf(qa);
-        if (fabsf(__fsub_rn(qb, nb)) >= 0.5f) nb = roundf(qb);
-        acc2 = pack2(fminf(fmaxf(na, -32768.f), 32767.f), fminf(fmaxf(nb, -32768.f), 32767.f));
-    };
-    if (VEC) {
-        for (int k0 = 0; k0 < K; k0 += 16) {
-            int8_t ra[16], rb[16];
-            *(uint4*)ra = *(const uint4*)(wA + k0);
-            if (hasB) *(uint4*)rb = *(const uint4*)(wB + k0);
-            else      *(uint4*)rb = make_uint4(0, 0, 0, 0);
-            #pragma unroll
-            for (int j = 0; j < 16; ++j) step((float)ra[j], (float)rb[j], k0 + j);
-        }
-    } else {
-        for (int k = 0; k < K; ++k) step((float)wA[k], hasB ? (float)wB[k] : 0.f, k);
-    }
-    unpack2(acc2, accA, accB);
+    const uint32_t local = (uint32_t)__cvta_generic_to_shared(mine);
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
+__device__ __forceinline__ void ql_copy16(void* dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void ql_copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void ql_copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// four weights of a row from k on, zeros beyond K
+__device__ __forceinline__ uint32_t ql_weights4(const int8_t* w, int k, int K)
+{
+    uint32_t v = 0;
+    #pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (k + i < K) v |= (uint32_t)(uint8_t)w[k + i] << (8 * i);
+    return v;
 }
 
-template <bool VEC_I, bool VEC_O>
-__global__ void __launch_bounds__(QL_THREADS) qlstm_step_kernel(const QlArgs a)
+// One step of a pair of chains with the reference's arithmetic.  acc2: integers; products that the reference rounds
+// before adding are fma2(a, b, 0) (a packed multiply feeding a packed add would be contracted); the quotient is
+// Markstein's correctly rounded one.
+struct QlExact {
+    f32x2 sG2, nsG2, iG2, sw2;
+    float lo, hi;                                // clamp
+    __device__ __forceinline__ void set(float sGa, float sGb, float swa, float swb, float l, float h)
+    {
+        sG2 = pack2(sGa, sGb); nsG2 = pack2(-sGa, -sGb); iG2 = pack2(__frcp_rn(sGa), __frcp_rn(sGb)); sw2 = pack2(swa, swb);
+        lo = l; hi = h;
+    }
+    __device__ __forceinline__ f32x2 quotient(f32x2 T, f32x2 w2, float x) const
+    {
+        const f32x2 zero2 = pack2(0.f, 0.f), magic2 = pack2(QL_MAGIC, QL_MAGIC);
+        const f32x2 t2 = fma2(fma2(w2, sw2, zero2), pack2(x, x), zero2);                      // fl(fl(w * sw) * x)
+        const f32x2 a2 = add2(fma2(sub2(T, magic2), sG2, zero2), t2);                         // fl(fl(acc * sG) + t)
+        const f32x2 p2 = mul2(a2, iG2);
+        return fma2(fma2(p2, nsG2, a2), iG2, p2);                                             // RN(a / sG)
+    }
+};
+
+// a byte of each of two words as a pair of floats, signed
+__device__ __forceinline__ f32x2 ql_weight_pair(uint32_t a, uint32_t b, int j, f32x2 off2)
+{
+    return sub2(pack2(__uint_as_float(__byte_perm(a, 0x4b000000u, 0x7440 + j)), __uint_as_float(__byte_perm(b, 0x4b000000u, 0x7440 + j))), off2);
+}
+
+// Eight steps by the reference's arithmetic, halves and clamp included.  x: the steps' dequantised values.
+__device__ __noinline__ f32x2 ql_slow8(f32x2 T, uint2 wa, uint2 wb, const float* x, const QlExact* e)
+{
+    const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC), woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
+    const uint32_t ma[2] = {wa.x ^ 0x80808080u, wa.y ^ 0x80808080u}, mb[2] = {wb.x ^ 0x80808080u, wb.y ^ 0x80808080u};
+    #pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const f32x2 q2 = e->quotient(T, ql_weight_pair(ma[j >> 2], mb[j >> 2], j & 3, woff2), x[j]);
+        float qa, qb, na, nb;
+        unpack2(q2, qa, qb);
+        unpack2(sub2(add2(q2, magic2), magic2), na, nb);
+        if (!(fabsf(__fsub_rn(qa, na)) < 0.5f)) na = roundf(qa);
+        if (!(fabsf(__fsub_rn(qb, nb)) < 0.5f)) nb = roundf(qb);
+        T = add2(pack2(fminf(fmaxf(na, e->lo), e->hi), fminf(fmaxf(nb, e->lo), e->hi)), magic2);
+    }
+    return T;
+}
+
+// Bounds of a block of eight steps: x = how far an accumulator can move in it (|w| <= 128, half a unit of rounding per step),
+// corrections that notes may bring included; y = the part of E that does not depend on the accumulators it begins with.
+__device__ __forceinline__ float2 ql_bounds(float sum_abs, float max_abs)
+{
+    const float s = __fmaf_rn(128.5f, sum_abs, 4.5f) + 8.0f * QL_NOTES;
+    return make_float2(s, QL_ULP * (3.0f * s + 8.0f * 128.0f * max_abs + 8.0f));
+}
+
+// A packed pair of chains and its doubtful blocks: first step of the block, the two accumulators before it (whose 16 bits
+// are the low halves of T's words).  Only the notes have an address, so that the rest stays in registers.
+struct QlChains {
+    f32x2 T;
+    int notes;
+    uint2* note;
+};
+
+// What noted blocks are corrected from: the staged arrays and the weight rows of the pair.
+struct QlSource {
+    const float2* xc;                            // factors of the pair, by position
+    const float* xf;                             // dequantised values
+    const float2* bounds;                        // by block
+    const QlExact* e;
+    const int8_t* wa; const int8_t* wb;          // weight rows: position 0 is step `first` of `K`
+    int first, K, aligned;                       // aligned: eight weights are one 8-byte word
+    __device__ __forceinline__ uint2 weights(const int8_t* w, int pos) const
+    {
+        if (aligned) return *(const uint2*)(w + first + pos);
+        return make_uint2(ql_weights4(w, first + pos, K), ql_weights4(w, first + pos + 4, K));
+    }
+};
+
+// Evaluates the doubtful steps of the noted blocks with the reference's arithmetic and corrects the accumulators.
+__device__ __noinline__ f32x2 ql_resolve(f32x2 end, int notes, const uint2* list, const QlSource src)
+{
+    const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC), woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
+    const QlExact e = *src.e;
+    f32x2 corr2 = pack2(0.f, 0.f);               // what the reference's accumulators are ahead by
+    #pragma unroll 1
+    for (int i = 0; i < notes; ++i) {
+        const uint2 note = list[i];
+        const int pos = (int)note.x;
+        const float a0 = (float)(short)(note.y & 0xffffu), a1 = (float)((int)note.y >> 16);
+        const uint2 wa = src.weights(src.wa, pos), wb = src.weights(src.wb, pos);
+        const float thr = 0.5f - __fmaf_rn(3.0f * QL_ULP, fmaxf(fabsf(a0), fabsf(a1)), src.bounds[pos >> 3].y);
+        const uint32_t ma[2] = {wa.x ^ 0x80808080u, wa.y ^ 0x80808080u}, mb[2] = {wb.x ^ 0x80808080u, wb.y ^ 0x80808080u};
+        f32x2 T[9], w2[8];
+        T[0] = pack2(a0 + QL_MAGIC, a1 + QL_MAGIC);
+        uint32_t doubtful = 0;
+        #pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            w2[j] = ql_weight_pair(ma[j >> 2], mb[j >> 2], j & 3, woff2);
+            const float2 c = src.xc[pos + j];
+            const f32x2 c2 = pack2(c.x, c.y);
+            T[j + 1] = fma2(w2[j], c2, T[j]);
+            float d0, d1;
+            unpack2(fma2(w2[j], c2, sub2(T[j], T[j + 1])), d0, d1);
+            if (!(fmaxf(fabsf(d0), fabsf(d1)) < thr)) doubtful |= 1u << j;
+        }
+        #pragma unroll 1
+        while (doubtful) {
+            const int k = __ffs((int)doubtful) - 1;
+            doubtful &= doubtful - 1;
+            f32x2 t = T[0], next = T[1], w = w2[0];
+            #pragma unroll
+            for (int j = 1; j < 8; ++j)
+                if (j == k) { t = T[j]; next = T[j + 1]; w = w2[j]; }
+            const f32x2 q2 = e.quotient(add2(t, corr2), w, src.xf[pos + k]);
+            float qa, qb, na, nb;
+            unpack2(q2, qa, qb);
+            unpack2(sub2(add2(q2, magic2), magic2), na, nb);
+            if (!(fabsf(__fsub_rn(qa, na)) < 0.5f)) na = roundf(qa);
+            if (!(fabsf(__fsub_rn(qb, nb)) < 0.5f)) nb = roundf(qb);
+            corr2 = sub2(pack2(na, nb), sub2(next, magic2));
+        }
+    }
+    return add2(end, corr2);
+}
+
+// Eight steps of a pair of chains from position `pos` on, whose weights are w2 (wa, wb as bytes).  listed: one of the inputs is on the
+// host's list.
+__device__ __forceinline__ void ql_steps8(QlChains& ch, const f32x2* w2, int pos, bool listed, const QlSource& src, bool exact_only)
+{
+    const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC);
+    const float2 bd = src.bounds[pos >> 3];
+    const f32x2 T0 = ch.T;
+    float f0, f1;
+    unpack2(sub2(T0, magic2), f0, f1);
+    const float amax = fmaxf(fabsf(f0), fabsf(f1));
+    bool checked = listed;
+    if (__any_sync(0xffffffffu, !(amax + bd.x <= QL_LEVEL) || ch.notes >= QL_NOTES)) {
+        checked = true;
+        const bool far = exact_only || __any_sync(0xffffffffu, !(amax + bd.x <= QL_NEAR_CLAMP));
+        if (far || __any_sync(0xffffffffu, ch.notes >= QL_NOTES)) {
+            ch.T = ql_resolve(ch.T, ch.notes, ch.note, src);
+            ch.notes = 0;
+            if (far) {
+                ch.T = ql_slow8(ch.T, src.weights(src.wa, pos), src.weights(src.wb, pos), src.xf + pos, src.e);
+                return;
+            }
+        }
+    }
+    f32x2 t = ch.T;
+    const f32x2 begin = t;
+    f32x2 c2[8];
+    #pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+        const float4 x = *(const float4*)(src.xc + pos + j);
+        c2[j] = pack2(x.x, x.y); c2[j + 1] = pack2(x.z, x.w);
+    }
+    if (!checked) {
+        #pragma unroll
+        for (int j = 0; j < 8; ++j) t = fma2(w2[j], c2[j], t);
+    } else {
+        float dmax = 0.f;
+        #pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const f32x2 next = fma2(w2[j], c2[j], t);
+            float d0, d1;
+            unpack2(fma2(w2[j], c2[j], sub2(t, next)), d0, d1);
+            dmax = fmaxf(fmaxf(dmax, fabsf(d0)), fabsf(d1));
+            t = next;
+        }
+        if (!(__fadd_rn(dmax, __fmaf_rn(3.0f * QL_ULP, amax, bd.y)) < 0.5f)) {
+            float t0, t1;
+            unpack2(begin, t0, t1);
+            ch.note[ch.notes++] = make_uint2((uint32_t)pos, __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x5410));
+        }
+    }
+    ch.T = t;
+}
+
+template <int R>
+__global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_constant__ QlArgs a)
 {
     pdl_enter();
     const b200k_qlstm_params& p = a.p;
     const int I = p.input_size, U = p.num_units, O = p.output_size;
-    const int b = blockIdx.x, tid = threadIdx.x;
-    extern __shared__ float sm[];
-    float2* xf = (float2*)sm;       // [I]   dequantised input row, every value twice (for the two-wide chains)
-    float2* hf = xf + I;            // [O]   dequantised previous output state, likewise
-    float* gate = (float*)(hf + O); // [4][U] int16 gate buffers as integer-valued floats (i, f, c, o)
-    float* cell = gate + 4 * U;     // [U]   new cell state (integer-valued)
-    float* hid = cell + U;          // [U]   dequantised hidden state
-    float* stat = hid + U;          // [4][2] mean, 1/stddev per gate
+    const int tid = threadIdx.x;
+    const int nct = (int)ql_cluster_size(), rank = (int)ql_cluster_rank();
+    const int b0 = (int)(blockIdx.x / (unsigned)nct) * R;    // first of the cluster's rows
+    if (nct > 1) ql_cluster_arrive();                        // (every CTA of the cluster runs before anyone writes to it)
 
-    for (int k = tid; k < I; k += QL_THREADS) {
-        const float v = dequantize_dev(p.input[(long long)b * I + k], p.input_scale, p.input_zp);
-        xf[k] = make_float2(v, v);
+    extern __shared__ float4 ql_smem[];
+    __shared__ QlDanger s_danger[2][2];
+    __shared__ QlExact s_exact[2][2];
+    float* gates = (float*)ql_smem;                          // [4][U] int16 gate buffers as integer-valued floats (o, i, f, c)
+    auto gate = [&](int g) { return gates + ((g + 1) & 3) * U; };
+    float* work = gates + ((4 * U + QL_GATE_SLACK + 3) & ~3);
+    // chains of the gates, by row and pair (i and c, f and o): factors of every step; by block of eight steps: its bounds, and
+    // whether one of its inputs is on the host's list
+    const int nblk = a.seg / 8;
+    float2* xc = (float2*)work;                              // [R][2][seg]
+    float2* bounds = xc + R * 2 * a.seg;                     // [R][2][nblk]
+    float* xf = (float*)(bounds + R * 2 * nblk);             // [R][seg] dequantised values
+    uint8_t* listed = (uint8_t*)(xf + R * a.seg);            // [R][2][nblk]
+    // afterwards, in the same place:
+    float* cell = work;                                      // [U] new cell state (integer-valued)
+    float* stat = cell + U;                                  // [4][2] mean, 1 / stddev per gate
+    float* hid = stat + 8;                                   // [U rounded up to 16] dequantised hidden state
+    // and, where the i, f and c gates were:
+    float2* hc = (float2*)(gates + ((U + 3) & ~3));          // [U rounded up to 16] projection factor of a unit, twice
+    float2* hbounds = hc + ((U + 15) & ~15);                 // [U rounded up to 16, / 8]
+    uint8_t* hlisted = (uint8_t*)(hbounds + ((U + 15) & ~15) / 8);   // the same
+    // weights: nbuf tiles of 4 x QL_UNITS rows (gate-major), then the whole projection matrix
+    uint8_t* tiles = (uint8_t*)ql_smem + a.tile_off;
+
+    const int8_t* wi[4] = {a.cifg ? p.w_i2f : p.w_i2i, p.w_i2f, p.w_i2c, p.w_i2o};       // (CIFG: a chain that nobody reads)
+    const int8_t* wr[4] = {a.cifg ? p.w_r2f : p.w_r2i, p.w_r2f, p.w_r2c, p.w_r2o};
+    const float si[4] = {a.cifg ? p.s_i2f : p.s_i2i, p.s_i2f, p.s_i2c, p.s_i2o};
+    const float sr[4] = {a.cifg ? p.s_r2f : p.s_r2i, p.s_r2f, p.s_r2c, p.s_r2o};
+    const float sint[4] = {a.cifg ? p.forget_intermediate_scale : p.input_intermediate_scale, p.forget_intermediate_scale,
+                           p.cell_intermediate_scale, p.output_intermediate_scale};
+    const f32x2 woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
+
+    for (int i = tid; i < (int)(sizeof(s_danger) / 4); i += QL_THREADS) ((uint32_t*)s_danger)[i] = ((const uint32_t*)a.danger)[i];
+    if (tid < 4) {
+        const int src = tid >> 1, pr = tid & 1;
+        s_exact[src][pr].set(pr ? sint[1] : sint[0], pr ? sint[3] : sint[2], src ? (pr ? sr[1] : sr[0]) : (pr ? si[1] : si[0]),
+                             src ? (pr ? sr[3] : sr[2]) : (pr ? si[3] : si[2]), -32768.f, 32767.f);
     }
-    for (int k = tid; k < O; k += QL_THREADS) {
-        const float v = dequantize_dev(p.output_state_in[(long long)b * O + k], p.output_state_scale, p.output_state_zp);
-        hf[k] = make_float2(v, v);
-    }
+
+    auto row_of = [&](int r) { return min(b0 + r, p.batch - 1); };          // a cluster's missing last row repeats its first
+    // n steps from k0 on of source `src` (0 input, 1 previous output), at position `at` of the staged arrays
+    auto stage = [&](int src, int k0, int n, int at) {
+        const int blocks = ((n + 15) & ~15) / 8;
+        float c[4];
+        #pragma unroll
+        for (int g = 0; g < 4; ++g) c[g] = __fdiv_rn(src == 0 ? si[g] : sr[g], sint[g]);
+        const int K = src == 0 ? I : O, zp = src == 0 ? p.input_zp : p.output_state_zp;
+        const float scale = src == 0 ? p.input_scale : p.output_state_scale;
+        const int8_t* base = src == 0 ? p.input : p.output_state_in;
+        __syncthreads();
+        for (int i = tid; i < R * blocks; i += QL_THREADS) {
+            const int r = i / blocks, blk = i - r * blocks;
+            const int8_t* x = base + (long long)row_of(r) * K + k0 + blk * 8;
+            float sum[2] = {0.f, 0.f}, mx[2] = {0.f, 0.f};
+            uint32_t on_list[2] = {0, 0};
+            #pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int q = blk * 8 + j < n ? (int)x[j] - zp : 0, mag = abs(q);
+                const float v = __fmul_rn(__int2float_rn(q), scale);
+                const int pos = at + blk * 8 + j;
+                xf[r * a.seg + pos] = v;
+                #pragma unroll
+                for (int pr = 0; pr < 2; ++pr) {
+                    const float2 f = make_float2(__fmul_rn(v, pr ? c[1] : c[0]), __fmul_rn(v, pr ? c[3] : c[2]));
+                    xc[(r * 2 + pr) * a.seg + pos] = f;
+                    const float m = fmaxf(fabsf(f.x), fabsf(f.y));
+                    sum[pr] += m; mx[pr] = fmaxf(mx[pr], m);
+                    on_list[pr] |= (s_danger[src][pr].bits[(mag >> 5) & 7] >> (mag & 31)) & 1u;
+                }
+            }
+            #pragma unroll
+            for (int pr = 0; pr < 2; ++pr) {
+                bounds[(r * 2 + pr) * nblk + at / 8 + blk] = ql_bounds(a.exact_only ? 1e30f : sum[pr], mx[pr]);
+                listed[(r * 2 + pr) * nblk + at / 8 + blk] = (uint8_t)on_list[pr];
+            }
+        }
+        __syncthreads();
+    };
+
+    // ---- the gates' chains: input weights first, then recurrent weights, continuing the same accumulators.  Usually both
+    // sources are staged side by side once; a long layer's are staged piece by piece.
+    const int Us = (U + nct - 1) / nct, u_lo = rank * Us, u_hi = min(U, u_lo + Us);
+    const int I16 = (I + 15) & ~15;
     __syncthreads();
+    if (a.both) { stage(0, 0, I, 0); stage(1, 0, O, I16); }
+    if (nct > 1) ql_cluster_wait();
+    const int pr = tid / QL_UNITS, ul = tid % QL_UNITS;      // this thread's gates: pr and pr + 2; its unit within the pass
+    for (int ub = u_lo; ub < u_hi; ub += QL_UNITS) {
+        const int units = min(QL_UNITS, u_hi - ub);
+        const bool busy = (ul & ~31) < units;                // (warp-uniform; lanes beyond the last unit repeat it)
+        QlChains ch[R];
+        uint2 notes[R][QL_NOTES];
+        #pragma unroll
+        for (int r = 0; r < R; ++r) { ch[r].T = pack2(QL_MAGIC, QL_MAGIC); ch[r].notes = 0; ch[r].note = notes[r]; }
+        // n steps from k0 on of source src, staged at `at`
+        auto run = [&](auto vec, int src, int k0, int n, int at) {
+            constexpr bool VEC = decltype(vec)::value;
+            const int K = src == 0 ? I : O;
+            auto fetch = [&](int t, int buf) {               // the tile of steps [t, t + QL_TILE)
+                #pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const int8_t* w = (src ? wr[g] : wi[g]) + (long long)ub * K + k0 + t;
+                    uint8_t* d = tiles + buf * QL_TILE_BYTES + g * QL_UNITS * QL_PITCH;
+                    if (VEC) {
+                        const int c = (tid & 3) * 16;
+                        #pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int row = h * (QL_THREADS / 4) + (tid >> 2);
+                            if (row < units && t + c < n) ql_copy16(d + row * QL_PITCH + c, w + (long long)row * K + c);
+                        }
+                    } else {
+                        const int c = (tid & 15) * 4;
+                        #pragma unroll 8
+                        for (int row = tid >> 4; row < units; row += QL_THREADS / 16)
+                            if (t + c < n) *(uint32_t*)(d + row * QL_PITCH + c) = ql_weights4(w + (long long)row * K, c, n - t);
+                    }
+                }
+                if (VEC) ql_copy_commit();
+            };
+            QlSource from[R];
+            #pragma unroll
+            for (int r = 0; r < R; ++r) {
+                from[r].xc = xc + (r * 2 + pr) * a.seg + at; from[r].xf = xf + r * a.seg + at;
+                from[r].bounds = bounds + (r * 2 + pr) * nblk + at / 8;
+                from[r].e = &s_exact[src][pr];
+                const long long row = (long long)(ub + min(ul, units - 1)) * K;
+                from[r].wa = (src ? (pr ? wr[1] : wr[0]) : (pr ? wi[1] : wi[0])) + row;
+                from[r].wb = (src ? (pr ? wr[3] : wr[2]) : (pr ? wi[3] : wi[2])) + row;
+                from[r].first = k0; from[r].K = K; from[r].aligned = VEC;
+            }
+            const uint8_t* ta = tiles + (pr * QL_UNITS + min(ul, units - 1)) * QL_PITCH;
+            fetch(0, 0);
+            int buf = 0;
+            for (int t = 0; t < n; t += QL_TILE) {
+                const bool ahead = a.nbuf == 2 && t + QL_TILE < n;
+                if (ahead) fetch(t + QL_TILE, buf ^ 1);
+                if (VEC) { if (ahead) ql_copy_wait<1>(); else ql_copy_wait<0>(); }
+                __syncthreads();
+                if (busy) {
+                    const uint8_t* tb = ta + buf * QL_TILE_BYTES;
+                    #pragma unroll 1
+                    for (int k = t; k < min(n, t + QL_TILE); k += 16) {
+                        const uint4 na = *(const uint4*)(tb + k - t), nb = *(const uint4*)(tb + 2 * QL_UNITS * QL_PITCH + k - t);
+                        const uint32_t ma[4] = {na.x ^ 0x80808080u, na.y ^ 0x80808080u, na.z ^ 0x80808080u, na.w ^ 0x80808080u};
+                        const uint32_t mb[4] = {nb.x ^ 0x80808080u, nb.y ^ 0x80808080u, nb.z ^ 0x80808080u, nb.w ^ 0x80808080u};
+                        #pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            f32x2 w2[8];
+                            #pragma unroll
+                            for (int j = 0; j < 8; ++j) w2[j] = ql_weight_pair(ma[h * 2 + (j >> 2)], mb[h * 2 + (j >> 2)], j & 3, woff2);
+                            #pragma unroll
+                            for (int r = 0; r < R; ++r)
+                                ql_steps8(ch[r], w2, k + h * 8, listed[(r * 2 + pr) * nblk + ((at + k) >> 3) + h] != 0, from[r], a.exact_only);
+                        }
+                    }
+                }
+                __syncthreads();                             // (everyone has left the tile before it is overwritten)
+                if (a.nbuf == 2) buf ^= 1;
+                else if (t + QL_TILE < n) fetch(t + QL_TILE, 0);
+            }
+            #pragma unroll
+            for (int r = 0; r < R; ++r) {
+                ch[r].T = ql_resolve(ch[r].T, ch[r].notes, ch[r].note, from[r]);
+                ch[r].notes = 0;
+            }
+        };
+        auto run_source = [&](int src, int k0, int n, int at) {
+            if (src == 0 ? a.vec_i : a.vec_o) run(std::integral_constant<bool, true>{}, src, k0, n, at);
+            else                              run(std::integral_constant<bool, false>{}, src, k0, n, at);
+        };
+        if (a.both) {
+            run_source(0, 0, I, 0);
+            run_source(1, 0, O, I16);
+        } else {
+            for (int src = 0; src < 2; ++src)
+                for (int s0 = 0; s0 < (src == 0 ? I : O); s0 += a.seg) {
+                    const int n = min(a.seg, (src == 0 ? I : O) - s0);
+                    stage(src, s0, n, 0);
+                    run_source(src, s0, n, 0);
+                }
+        }
+        if (ul < units) {
+            #pragma unroll
+            for (int r = 0; r < R; ++r) {
+                float f[2];
+                unpack2(sub2(ch[r].T, pack2(QL_MAGIC, QL_MAGIC)), f[0], f[1]);
+                #pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float* to = gate(pr + 2 * h) + ub + ul;
+                    if (nct > 1) ql_store_remote(to, (uint32_t)r, f[h]);
+                    else *to = f[h];
+                }
+            }
+        }
+    }
+    if (nct > 1) { ql_cluster_arrive(); ql_cluster_wait(); }
+    else __syncthreads();
+    // from here on CTA r works alone on row r
+    const int b = b0 + rank;
+    if (rank >= R || b >= p.batch) return;
 
-    const int8_t* wi[4] = {p.w_i2i, p.w_i2f, p.w_i2c, p.w_i2o};
-    const int8_t* wr[4] = {p.w_r2i, p.w_r2f, p.w_r2c, p.w_r2o};
-    const float si[4] = {p.s_i2i, p.s_i2f, p.s_i2c, p.s_i2o};
-    const float sr[4] = {p.s_r2i, p.s_r2f, p.s_r2c, p.s_r2o};
-    const float sint[4] = {p.input_intermediate_scale, p.forget_intermediate_scale, p.cell_intermediate_scale,
-                           p.output_intermediate_scale};
+    const float sc = p.cell_state_scale, isc = __frcp_rn(sc);
     const int g0 = a.cifg ? 1 : 0;
-    const int nchains = (4 - g0) * U;
-
-    // ---- mat-vec chains: input weights first, then recurrent weights, continuing the same accumulator
-    for (int c0 = tid; c0 < nchains; c0 += 2 * QL_THREADS) {
-        const int cA = c0, cB = c0 + QL_THREADS;
-        const bool hasB = cB < nchains;
-        const int gA = g0 + cA / U, uA = cA % U;
-        const int gB = hasB ? g0 + cB / U : gA, uB = hasB ? cB % U : uA;
-        float accA = 0.f, accB = 0.f;
-        chain2<VEC_I>(accA, accB, wi[gA] + (long long)uA * I, wi[gB] + (long long)uB * I, si[gA], si[gB], xf, I,
-                      sint[gA], sint[gB], hasB);
-        chain2<VEC_O>(accA, accB, wr[gA] + (long long)uA * O, wr[gB] + (long long)uB * O, sr[gA], sr[gB], hf, O,
-                      sint[gA], sint[gB], hasB);
-        gate[gA * U + uA] = accA;
-        if (hasB) gate[gB * U + uB] = accB;
-    }
-    __syncthreads();
-
-    const float sc = p.cell_state_scale;
     const int16_t* peep[4] = {p.w_c2i, p.w_c2f, nullptr, p.w_c2o};
     const float speep[4] = {p.s_c2i, p.s_c2f, 0.f, p.s_c2o};
     const int16_t* lnw[4] = {p.ln_i, p.ln_f, p.ln_c, p.ln_o};
@@ -155,16 +504,34 @@ __global__ void __launch_bounds__(QL_THREADS) qlstm_step_kernel(const QlArgs a)
     const int32_t* gbias[4] = {p.b_i, p.b_f, p.b_c, p.b_o};
     const float sgb[4] = {p.s_bi, p.s_bf, p.s_bc, p.s_bo};
 
+    // The projection weights, [O][U16 + 16] bytes, into the space of the weight tiles by threads [first, QL_THREADS): done
+    // by the warps that have nothing to do while the layer-norm sums run.
+    const int U16 = (U + 15) & ~15, ppitch = U16 + 16;
+    bool proj_pending = a.proj && a.proj_staged;
+    auto stage_projection = [&](int first) {
+        const int piece = a.vec_p ? 16 : 4, per_row = U16 / piece, step = QL_THREADS - first;
+        int j = (tid - first) / per_row, c = (tid - first) - j * per_row;
+        const int dj = step / per_row, dc = step - dj * per_row;
+        while (j < O) {
+            if (a.vec_p) ql_copy16(tiles + j * ppitch + c * 16, p.w_proj + (long long)j * U + c * 16);
+            else         *(uint32_t*)(tiles + j * ppitch + c * 4) = ql_weights4(p.w_proj + (long long)j * U, c * 4, U);
+            j += dj; c += dc;
+            if (c >= per_row) { c -= per_row; ++j; }
+        }
+        if (a.vec_p) ql_copy_commit();
+    };
+
     // Post-processing of gates [gfirst, glast]: peephole, layer norm, activation.  `cellsrc` is the cell
     // state the peephole reads (old state for i and f, new state for o), as integer-valued floats.
     auto gate_post = [&](int gfirst, int glast, const int16_t* cell_in_global, const float* cell_smem) {
         if (a.peephole) {
-            for (int t = tid; t < (glast - gfirst + 1) * U; t += QL_THREADS) {
-                const int g = gfirst + t / U, u = t % U;
+            for (int g = gfirst; g <= glast; ++g) {
                 if (!peep[g]) continue;
-                const float cv = cell_smem ? cell_smem[u] : (float)cell_in_global[(long long)b * U + u];
-                const float pr = __fmul_rn(__fmul_rn((float)peep[g][u], speep[g]), __fmul_rn(cv, sc));
-                gate[g * U + u] = q16f(__fadd_rn(__fmul_rn(gate[g * U + u], sint[g]), pr), sint[g]);
+                for (int u = tid; u < U; u += QL_THREADS) {
+                    const float cv = cell_smem ? cell_smem[u] : (float)cell_in_global[(long long)b * U + u];
+                    const float pv = __fmul_rn(__fmul_rn((float)peep[g][u], speep[g]), __fmul_rn(cv, sc));
+                    gate(g)[u] = q16f(__fadd_rn(__fmul_rn(gate(g)[u], sint[g]), pv), sint[g], __frcp_rn(sint[g]));
+                }
             }
             __syncthreads();
         }
@@ -173,12 +540,29 @@ __global__ void __launch_bounds__(QL_THREADS) qlstm_step_kernel(const QlArgs a)
             const int w = tid >> 5;
             if ((tid & 31) == 0 && w <= glast - gfirst) {
                 const int g = gfirst + w;
+                const float* v = gate(g);
+                const float s = sint[g];
                 float sum = 0.f, sum_sq = 0.f;
-                for (int i = 0; i < U; ++i) {
-                    const float v = __fmul_rn(gate[g * U + i], sint[g]);
-                    sum = __fadd_rn(sum, v);
-                    sum_sq = __fadd_rn(sum_sq, __fmul_rn(v, v));
+                auto add = [&](float q) {
+                    const float x = __fmul_rn(q, s);
+                    sum = __fadd_rn(sum, x);
+                    sum_sq = __fadd_rn(sum_sq, __fmul_rn(x, x));
+                };
+                int i = 0;
+                if ((U & 3) == 0 && U >= 8) {                // 128-bit reads, eight values ahead
+                    const float4* q = (const float4*)v;
+                    float4 c0 = q[0], c1 = q[1];
+                    #pragma unroll 1
+                    for (; i + 8 <= U; i += 8) {
+                        const int next = min((i >> 2) + 2, (U >> 2) - 2);
+                        const float4 n0 = q[next], n1 = q[next + 1];
+                        add(c0.x); add(c0.y); add(c0.z); add(c0.w);
+                        add(c1.x); add(c1.y); add(c1.z); add(c1.w);
+                        c0 = n0; c1 = n1;
+                    }
                 }
+                #pragma unroll 4
+                for (; i < U; ++i) add(v[i]);
                 const float fu = (float)U;
                 const float mean = __fdiv_rn(sum, fu);
                 const float variance = __fsub_rn(__fdiv_rn(sum_sq, fu), __fmul_rn(mean, mean));
@@ -186,70 +570,73 @@ __global__ void __launch_bounds__(QL_THREADS) qlstm_step_kernel(const QlArgs a)
                 stat[g * 2] = mean;
                 stat[g * 2 + 1] = __fdiv_rn(1.0f, sd);
             }
+            if (w >= 4 && proj_pending) stage_projection(128);
+            proj_pending = false;
             __syncthreads();
         }
-        for (int t = tid; t < (glast - gfirst + 1) * U; t += QL_THREADS) {
-            const int g = gfirst + t / U, u = t % U;
-            float q = gate[g * U + u];
-            float s = sint[g];
-            if (a.ln) {
-                const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f);
-                q = q16f(__fmul_rn(__fsub_rn(__fmul_rn(q, s), stat[g * 2]), stat[g * 2 + 1]), sln);       // normalise
-                q = q16f(__fmul_rn(__fmul_rn((float)lnw[g][u], slnw[g]), __fmul_rn(q, sln)), sln);           // * weight
-                q = q16f(__fadd_rn(__fmul_rn(q, sln), __fmul_rn(__int2float_rn(gbias[g][u]), sgb[g])), 1.f / 4096);  // + bias
-                s = 1.f / 4096;
+        for (int g = gfirst; g <= glast; ++g) {
+            const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f), isln = __frcp_rn(sln);
+            for (int u = tid; u < U; u += QL_THREADS) {
+                float q = gate(g)[u];
+                float s = sint[g];
+                if (a.ln) {
+                    q = q16f(__fmul_rn(__fsub_rn(__fmul_rn(q, s), stat[g * 2]), stat[g * 2 + 1]), sln, isln);      // normalise
+                    q = q16f(__fmul_rn(__fmul_rn((float)lnw[g][u], slnw[g]), __fmul_rn(q, sln)), sln, isln);       // * weight
+                    q = q16f(__fadd_rn(__fmul_rn(q, sln), __fmul_rn(__int2float_rn(gbias[g][u]), sgb[g])), 1.f / 4096, 4096.f);  // + bias
+                    s = 1.f / 4096;
+                }
+                const float v = __fmul_rn(q, s);
+                const float r = g == 2 ? tanhf(v) : __fdiv_rn(1.f, __fadd_rn(1.f, expf(-v)));
+                gate(g)[u] = q16f(r, sc, isc);
             }
-            const float v = __fmul_rn(q, s);
-            const float r = g == 2 ? tanhf(v) : __fdiv_rn(1.f, __fadd_rn(1.f, expf(-v)));
-            gate[g * U + u] = q16f(r, sc);
         }
         __syncthreads();
     };
 
-    gate_post(g0, 2, p.cell_state_in, nullptr);
+    // (without peephole the output gate does not see the new cell state: all gates at once)
+    gate_post(g0, a.peephole ? 2 : 3, p.cell_state_in, nullptr);
 
     // ---- cell state: c = Q(f * c_in); c = Q(c + g * i)  (or g * Q(1 - f) with CIFG); clip
     for (int u = tid; u < U; u += QL_THREADS) {
         const float cin = __fmul_rn((float)p.cell_state_in[(long long)b * U + u], sc);
-        const float f = gate[1 * U + u];
-        float c = q16f(__fmul_rn(__fmul_rn(f, sc), cin), sc);
-        const float ig = a.cifg ? q16f(__fsub_rn(1.0f, __fmul_rn(f, sc)), sc) : gate[0 * U + u];
-        c = q16f(__fadd_rn(__fmul_rn(c, sc), __fmul_rn(__fmul_rn(gate[2 * U + u], sc), __fmul_rn(ig, sc))), sc);
+        const float f = gate(1)[u];
+        float c = q16f(__fmul_rn(__fmul_rn(f, sc), cin), sc, isc);
+        const float ig = a.cifg ? q16f(__fsub_rn(1.0f, __fmul_rn(f, sc)), sc, isc) : gate(0)[u];
+        c = q16f(__fadd_rn(__fmul_rn(c, sc), __fmul_rn(__fmul_rn(gate(2)[u], sc), __fmul_rn(ig, sc))), sc, isc);
         if (p.cell_clip > 0.0f) {
             const float fv = __fmul_rn(c, sc);
             float r = (p.cell_clip < fv) ? p.cell_clip : fv;
             r = (-p.cell_clip > r) ? -p.cell_clip : r;
-            c = q16f(r, sc);
+            c = q16f(r, sc, isc);
         }
         cell[u] = c;
         p.cell_state_out[(long long)b * U + u] = (int16_t)c;
     }
     __syncthreads();
 
-    gate_post(3, 3, nullptr, cell);
+    if (a.peephole) gate_post(3, 3, nullptr, cell);
 
-    // ---- hidden = Q8(o * Q16(tanh(c)))
-    const float hzp = (float)p.hidden_state_zp;
-    for (int u = tid; u < U; u += QL_THREADS) {
-        const float t = q16f(tanhf(__fmul_rn(cell[u], sc)), sc);
-        const float hv = __fmul_rn(__fmul_rn(gate[3 * U + u], sc), __fmul_rn(t, sc));
+    // ---- hidden = Q8(o * Q16(tanh(c))), its projection factors and magnitudes
+    const float hzp = (float)p.hidden_state_zp, cp = a.proj ? __fdiv_rn(p.s_proj, p.output_scale) : 0.f;
+    for (int u = tid; u < U16; u += QL_THREADS) {
+        if (u >= U) { hc[u] = make_float2(0.f, 0.f); hid[u] = 0.f; continue; }
+        const float t = q16f(tanhf(__fmul_rn(cell[u], sc)), sc, isc);
+        const float hv = __fmul_rn(__fmul_rn(gate(3)[u], sc), __fmul_rn(t, sc));
         const float hq = fminf(fmaxf(__fadd_rn(hzp, roundf(__fdiv_rn(hv, p.hidden_state_scale))), -128.f), 127.f);
-        hid[u] = __fmul_rn(__fsub_rn(hq, hzp), p.hidden_state_scale);      // dequantised hidden state
+        const float h = __fmul_rn(__fsub_rn(hq, hzp), p.hidden_state_scale);      // dequantised hidden state
+        hid[u] = h;
+        cell[u] = fabsf(__fsub_rn(hq, hzp));                                      // (the cell state is done with: its magnitude)
+        const float f = __fmul_rn(h, cp);
+        hc[u] = make_float2(f, f);
     }
     __syncthreads();
 
     // ---- projection (int16 accumulator at the OUTPUT's scale and offset) and outputs
-    const float so = p.output_scale, zo = (float)p.output_zp, iso = __frcp_rn(p.output_scale);
-    for (int j = tid; j < O; j += QL_THREADS) {
+    if (proj_pending) stage_projection(0);
+    const float so = p.output_scale, zo = (float)p.output_zp;
+    auto finish = [&](int j, float acc) {                    // acc: int16 accumulator of output j (projection), or unused
         float out8;
         if (a.proj) {
-            float acc = 0.f;                                   // int16 buffer starts as raw zeros
-            if (p.b_proj) acc = q16zf(__fmul_rn(__int2float_rn(p.b_proj[j]), p.s_bproj), so, zo);
-            const int8_t* w = p.w_proj + (long long)j * U;
-            for (int k = 0; k < U; ++k) {
-                const float d = __fmul_rn(__fsub_rn(acc, zo), so);
-                acc = q16zf_fast(__fadd_rn(d, __fmul_rn(__fmul_rn((float)w[k], p.s_proj), hid[k])), so, iso, zo);
-            }
             out8 = fminf(fmaxf(__fadd_rn(zo, roundf(__fdiv_rn(__fmul_rn(__fsub_rn(acc, zo), so), so))), -128.f), 127.f);
             if (p.projection_clip > 0.0f) {
                 const float fv = __fmul_rn(__fsub_rn(out8, zo), so);
@@ -264,7 +651,104 @@ __global__ void __launch_bounds__(QL_THREADS) qlstm_step_kernel(const QlArgs a)
         const float ov = __fmul_rn(__fsub_rn(out8, zo), so);
         const float hs = fminf(fmaxf(__fadd_rn((float)p.output_state_zp, roundf(__fdiv_rn(ov, p.output_state_scale))), -128.f), 127.f);
         p.output_state_out[(long long)b * O + j] = (int8_t)hs;
+    };
+    if (!a.proj) {
+        for (int j = tid; j < O; j += QL_THREADS) finish(j, 0.f);
+        return;
     }
+    const int hblk = U16 / 8;
+    for (int blk = tid; blk < hblk; blk += QL_THREADS) {
+        float sum = 0.f, mx = 0.f;
+        uint32_t on_list = 0;
+        for (int j = 0; j < 8; ++j) {
+            const int u = blk * 8 + j, mag = u < U ? (int)cell[u] : 0;
+            const float m = fabsf(hc[u].x);
+            sum += m; mx = fmaxf(mx, m);
+            on_list |= (a.danger_p.bits[(mag >> 5) & 7] >> (mag & 31)) & 1u;
+        }
+        hbounds[blk] = ql_bounds(a.exact_only ? 1e30f : sum, mx);
+        hlisted[blk] = (uint8_t)on_list;
+    }
+    if (tid == 0) s_exact[0][0].set(so, so, p.s_proj, p.s_proj, -32768.f - zo, 32767.f - zo);
+    if (a.proj_staged && a.vec_p) ql_copy_wait<0>();
+    __syncthreads();
+    // two outputs, half of them apart, per thread; the chains run on acc - zo, an integer like the gates' accumulators
+    const int O2 = (O + 1) / 2;
+    for (int j0 = tid; (j0 & ~31) < O2; j0 += QL_THREADS) {
+        const int j = min(j0, O2 - 1), j1 = min(j + O2, O - 1);      // (idle lanes repeat the last pair)
+        const int8_t* w[2] = {p.w_proj + (long long)j * U, p.w_proj + (long long)j1 * U};
+        float first[2] = {0.f, 0.f};                         // the int16 buffer starts as raw zeros
+        if (p.b_proj) {
+            first[0] = q16zf(__fmul_rn(__int2float_rn(p.b_proj[j]), p.s_bproj), so, zo);
+            first[1] = q16zf(__fmul_rn(__int2float_rn(p.b_proj[j1]), p.s_bproj), so, zo);
+        }
+        QlChains ch;
+        uint2 notes[QL_NOTES];
+        ch.T = pack2(QL_MAGIC + (first[0] - zo), QL_MAGIC + (first[1] - zo));
+        ch.notes = 0; ch.note = notes;
+        QlSource from;
+        from.xc = hc; from.xf = hid; from.bounds = hbounds; from.e = &s_exact[0][0];
+        from.wa = a.proj_staged ? (const int8_t*)tiles + j * ppitch : w[0];
+        from.wb = a.proj_staged ? (const int8_t*)tiles + j1 * ppitch : w[1];
+        from.first = 0; from.K = U; from.aligned = a.proj_staged;
+        uint2 na = from.weights(from.wa, 0), nb = from.weights(from.wb, 0);
+        #pragma unroll 1
+        for (int k = 0; k < U16; k += 8) {
+            const uint32_t ma[2] = {na.x ^ 0x80808080u, na.y ^ 0x80808080u}, mb[2] = {nb.x ^ 0x80808080u, nb.y ^ 0x80808080u};
+            if (k + 8 < U16) { na = from.weights(from.wa, k + 8); nb = from.weights(from.wb, k + 8); }
+            f32x2 w2[8];
+            #pragma unroll
+            for (int i = 0; i < 8; ++i) w2[i] = ql_weight_pair(ma[i >> 2], mb[i >> 2], i & 3, woff2);
+            ql_steps8(ch, w2, k, hlisted[k >> 3] != 0, from, a.exact_only);
+        }
+        ch.T = ql_resolve(ch.T, ch.notes, ch.note, from);
+        float f0, f1;
+        unpack2(sub2(ch.T, pack2(QL_MAGIC, QL_MAGIC)), f0, f1);
+        if (j0 < O2) {
+            finish(j, f0 + zo);
+            if (j + O2 < O) finish(j + O2, f1 + zo);
+        }
+    }
+}
+
+// ---- host: which input magnitudes need the reference's arithmetic ----------------------------------------------------------
+
+// For one gate: r = |w| mag c over all weight magnitudes.  A function of the layer's scales alone, worked out once per set
+// of scales and kept in a small table (the oldest entry makes room).
+static QlDanger ql_danger_of(float sx, float sw, float sG)
+{
+    struct Entry { float sx, sw, sG; bool used; QlDanger d; };
+    static Entry table[64];
+    static int next = 0;
+    static std::mutex guard;
+    {
+        std::lock_guard<std::mutex> lock(guard);
+        for (const Entry& e : table)
+            if (e.used && e.sx == sx && e.sw == sw && e.sG == sG) return e.d;
+    }
+    const double c = (double)sx * (double)sw / (double)sG, unit = 1.0 / 16777216.0;
+    QlDanger d;
+    memset(&d, 0, sizeof(d));
+    for (int mag = 1; mag < 256; ++mag) {
+        double least = 1e300;                        // (distance from a half, less what does not depend on the accumulator) / unit
+        for (int w = 0; w <= 128; ++w) {
+            const double r = (double)(w * mag) * c;
+            const double near = fabs(r - (double)(long long)r - 0.5) / unit - 8.0 * r - 8.0;
+            least = near < least ? near : least;
+        }
+        if (least <= 3.0 * QL_LEVEL) d.bits[mag >> 5] |= 1u << (mag & 31);
+    }
+    std::lock_guard<std::mutex> lock(guard);
+    Entry& e = table[next];
+    next = (next + 1) & 63;
+    e.sx = sx; e.sw = sw; e.sG = sG; e.d = d; e.used = true;
+    return d;
+}
+static QlDanger ql_either(const QlDanger& a, const QlDanger& b)
+{
+    QlDanger d;
+    for (int i = 0; i < 8; ++i) d.bits[i] = a.bits[i] | b.bits[i];
+    return d;
 }
 
 }  // namespace b200k
@@ -292,20 +776,73 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
                   B200K_E_INVALID, "qlstm_step: layer norm needs all layer-norm weights and gate biases");
     B200K_REQUIRE(a.proj || p->num_units == p->output_size, B200K_E_INVALID,
                   "qlstm_step: without projection the output size must equal the number of units");
-    const size_t smem = sizeof(float) * (2 * ((size_t)p->input_size + p->output_size) + 6 * (size_t)p->num_units + 8);
-    B200K_REQUIRE(smem <= 200 * 1024, B200K_E_TOOBIG, "qlstm_step: layer too large for the shared-memory resident kernel");
-    const bool vi = (p->input_size % 16) == 0 &&
-                    ((((uintptr_t)p->w_i2i | (uintptr_t)p->w_i2f | (uintptr_t)p->w_i2c | (uintptr_t)p->w_i2o) & 15) == 0);
-    const bool vo = (p->output_size % 16) == 0 &&
-                    ((((uintptr_t)p->w_r2i | (uintptr_t)p->w_r2f | (uintptr_t)p->w_r2c | (uintptr_t)p->w_r2o) & 15) == 0);
+    const float scales[] = {p->input_scale, p->output_state_scale, p->input_intermediate_scale, p->forget_intermediate_scale,
+                            p->cell_intermediate_scale, p->output_intermediate_scale, p->s_i2f, p->s_i2c, p->s_i2o, p->s_r2f, p->s_r2c, p->s_r2o,
+                            a.cifg ? 1.f : p->s_i2i, a.cifg ? 1.f : p->s_r2i, p->output_scale, a.proj ? p->s_proj : 1.f, p->hidden_state_scale};
+    auto byte = [](int z) { return z >= -128 && z <= 127; };
+    a.exact_only = !byte(p->input_zp) || !byte(p->output_state_zp) || !byte(p->output_zp) || !byte(p->hidden_state_zp);
+    for (float s : scales) a.exact_only |= !(s >= 1e-8f && s <= 1e8f);
+    memset(a.danger, 0, sizeof(a.danger));
+    memset(&a.danger_p, 0, sizeof(a.danger_p));
+    if (!a.exact_only) {
+        const float si[4] = {a.cifg ? p->s_i2f : p->s_i2i, p->s_i2f, p->s_i2c, p->s_i2o}, sr[4] = {a.cifg ? p->s_r2f : p->s_r2i, p->s_r2f, p->s_r2c, p->s_r2o};
+        const float sint[4] = {a.cifg ? p->forget_intermediate_scale : p->input_intermediate_scale, p->forget_intermediate_scale,
+                               p->cell_intermediate_scale, p->output_intermediate_scale};
+        for (int pr = 0; pr < 2; ++pr) {
+            a.danger[0][pr] = ql_either(ql_danger_of(p->input_scale, si[pr], sint[pr]), ql_danger_of(p->input_scale, si[pr + 2], sint[pr + 2]));
+            a.danger[1][pr] = ql_either(ql_danger_of(p->output_state_scale, sr[pr], sint[pr]), ql_danger_of(p->output_state_scale, sr[pr + 2], sint[pr + 2]));
+        }
+        if (a.proj) a.danger_p = ql_danger_of(p->hidden_state_scale, p->s_proj, p->output_scale);
+    }
+    auto aligned = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
+    a.vec_i = p->input_size % 16 == 0 && aligned(p->w_i2i) && aligned(p->w_i2f) && aligned(p->w_i2c) && aligned(p->w_i2o);
+    a.vec_o = p->output_size % 16 == 0 && aligned(p->w_r2i) && aligned(p->w_r2f) && aligned(p->w_r2c) && aligned(p->w_r2o);
+    a.vec_p = p->num_units % 16 == 0 && aligned(p->w_proj);
     cudaStream_t s = (cudaStream_t)stream;
+    int dev = 0, sms = 0;
+    B200K_CUDA(cudaGetDevice(&dev));
+    B200K_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // Two rows per pair of CTAs (each weight converted once for both) as soon as that fills most SMs; below, the units of one
+    // row are spread over up to eight CTAs, so that a small batch still uses the machine.
+    int rows = 1, cs = 1;
+    if (p->batch >= 2 && p->batch * 5ll >= sms * 3ll) { rows = 2; cs = 2; }
+    else while (cs < 8 && p->batch * cs * 2 <= sms + sms / 4 && p->num_units >= 32 * cs) cs *= 2;
+    // Shared memory: the gates; the staged factors, or what comes after the chains; the weight tiles, or the projection
+    // matrix.  Very large layers make do with fewer staged steps and one tile.
+    auto up16 = [](int v) { return (v + 15) & ~15; };
+    const size_t limit = 226 * 1024, U = (size_t)p->num_units;
+    const size_t gates = 4 * ((4 * U + QL_GATE_SLACK + 3) & ~(size_t)3), after = 8 * U + 32 + 64;      // (64: padding)
+    const int wanted = up16(p->input_size) + up16(p->output_size);
+    a.seg = wanted < QL_SEG ? wanted : QL_SEG;
+    a.nbuf = 2;
+    size_t smem;
+    for (;;) {
+        const size_t staged = (size_t)rows * a.seg * (2 * 8 + 4) + (size_t)rows * 2 * (a.seg / 8) * (8 + 1);
+        a.tile_off = (unsigned)((gates + staged + 15) & ~(size_t)15);
+        smem = a.tile_off + (size_t)a.nbuf * QL_TILE_BYTES;
+        if (smem < gates + after) smem = gates + after;
+        if (smem <= limit) break;
+        if (a.nbuf == 2) a.nbuf = 1;
+        else if (a.seg > 128) a.seg = a.seg / 2 > 128 ? up16(a.seg / 2) : 128;
+        else if (rows == 2) rows = cs = 1;
+        else break;
+    }
+    B200K_REQUIRE(smem <= limit, B200K_E_TOOBIG, "qlstm_step: layer too large for the shared-memory resident kernel");
+    a.both = a.seg >= wanted;
+    // The projection matrix takes the tiles' place if the steps before it, whose data begin where the staged factors were,
+    // end before the tiles do (moved back if they need to be).
+    const size_t behind = (gates + after + 15) & ~(size_t)15;
+    if (a.proj && behind > a.tile_off && behind + (size_t)a.nbuf * QL_TILE_BYTES <= limit) {
+        a.tile_off = (unsigned)behind;
+        smem = a.tile_off + (size_t)a.nbuf * QL_TILE_BYTES;
+    }
+    const size_t whole = a.tile_off + (size_t)p->output_size * (up16(p->num_units) + 16);
+    a.proj_staged = a.proj && a.tile_off >= behind && whole <= limit;
+    if (a.proj_staged && whole > smem) smem = whole;
     auto launch = [&](auto kern) -> int {
-        if (smem > 48 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_pdl(kern, dim3((unsigned)p->batch), dim3(QL_THREADS), smem, s, a);
+        if (smem > 40 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        launch_pdl_cluster(kern, dim3((unsigned)((p->batch + rows - 1) / rows * cs)), dim3(QL_THREADS), smem, s, (unsigned)cs, a);
         return check_launch("qlstm_step_kernel");
     };
-    if (vi && vo)  return launch(qlstm_step_kernel<true, true>);
-    if (!vi && vo) return launch(qlstm_step_kernel<false, true>);
-    if (vi && !vo) return launch(qlstm_step_kernel<true, false>);
-    return launch(qlstm_step_kernel<false, false>);
+    return rows == 2 ? launch(qlstm_step_kernel<2>) : launch(qlstm_step_kernel<1>);
 }

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from cases import F32, S8, U8, SimpleCase, _abi, _rand, qt, qt_out, run_case
-from q8util import activation_clamp, diff_stats, random_fc_case
+from q8util import activation_clamp, diff_stats, random_qlstm_case, random_fc_case
 
 pytestmark = pytest.mark.gpu
 
@@ -192,8 +192,35 @@ BMM_CASES = {"%s%s_b%d_m%d_k%d_n%d" % ("T" if tx else "N", "T" if ty else "N", b
                  (2, 256, 256, 256, 1, 0, (S8, S8, S8)), (3, 77, 96, 77, 0, 1, (S8, S8, S8)), (3, 77, 77, 32, 0, 0, (S8, S8, S8)), (1, 128, 192, 20, 0, 0, (S8, S8, S8))))}
 BMM_CASES["broadcast"] = lambda: bmm(60, 4, 40, 72, 80, 0, 0, bcast=True)
 
+def qlstm(seed, batch, i, u, o, gate_scale=None, weight_scale=None, **kw):
+    """gate_scale 2^-7 with 2^-7 weights and inputs: products that fall on exact halves; larger weight scales: chains that
+    saturate"""
+    case = random_qlstm_case(seed, batch, i, u, o, **kw)
+    for g in "ifco":
+        if weight_scale is not None:
+            for k in ("s_i2" + g, "s_r2" + g):
+                if k in case.s:
+                    case.s[k] = weight_scale
+    if gate_scale is not None:
+        for g in ("input", "forget", "cell", "output"):
+            case.s[g + "_intermediate_scale"] = gate_scale
+    return case
+
+
+QLSTM_CASES = {
+    # clusters of one, two (one and two rows), four and eight CTAs; more units than threads; more steps than are staged
+    "batch1_u512": lambda: qlstm(1, 1, 40, 512, 64), "batch20_u130": lambda: qlstm(2, 20, 33, 130, 24), "batch60": lambda: qlstm(3, 60, 16, 64, 32),
+    "batch89_two_rows_odd": lambda: qlstm(4, 89, 24, 48, 16), "batch150_two_rows": lambda: qlstm(5, 150, 16, 32, 16),
+    "units_600_staged_in_two": lambda: qlstm(6, 2, 1100, 600, 32), "tiny": lambda: qlstm(7, 3, 1, 1, 1),
+    "exact_halves": lambda: qlstm(8, 4, 64, 48, 32, gate_scale=2.0 ** -7, weight_scale=2.0 ** -7),
+    "halves_everywhere": lambda: qlstm(9, 2, 64, 48, 32, gate_scale=2.0 ** -13, weight_scale=2.0 ** -7),
+    "saturating": lambda: qlstm(10, 4, 64, 48, 32, weight_scale=1.5), "large_accumulators": lambda: qlstm(11, 90, 256, 96, 64, weight_scale=0.05),
+    "no_projection_odd": lambda: qlstm(12, 5, 19, 37, 37, projection=False), "cifg_two_rows": lambda: qlstm(13, 90, 16, 40, 24, cifg=True, peephole=True),
+    "one_tile_of_a_large_layer": lambda: qlstm(14, 1, 24, 6000, 16), "projection_not_staged": lambda: qlstm(15, 1, 16, 700, 320),
+}
+
 EXACT = {"bmm": BMM_CASES, "fc": FC_CASES, "f32": F32_CASES, "eltwise": ELTWISE_CASES, "resize": RESIZE_CASES, "arg": ARG_CASES, "mean": MEAN_CASES}
-ROUNDED = {"softmax": SOFTMAX_CASES}
+ROUNDED = {"softmax": SOFTMAX_CASES, "qlstm": QLSTM_CASES}
 
 
 @pytest.mark.parametrize("group,name", [(g, n) for g, c in EXACT.items() for n in c])
@@ -209,4 +236,5 @@ def test_within_one_unit(built, group, name):
     want, got = run_case(ROUNDED[group][name](), "oracle"), run_case(ROUNDED[group][name](), "gpu")
     for w, g in zip(want, got):
         st = diff_stats(w, g)
-        assert st["max_abs"] <= 1 and st["mismatch_frac"] <= 0.01, (group, name, st)
+        # (the int16 cell state goes through two of them)
+        assert st["max_abs"] <= (2 if w.dtype == np.int16 else 1) and st["mismatch_frac"] <= 0.01, (group, name, st)
