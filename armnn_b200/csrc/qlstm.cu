@@ -12,9 +12,9 @@
 //     T' = RN(T + w xc),  xc = x sw / sG,  T = 1.5 * 2^23 + acc.
 // r depends on the product of two bytes only.  The host lists, per pair of gates, the input magnitudes for which SOME weight
 // byte comes that close to a half (with |acc| <= QL_LEVEL; with the scales of the reference's own test a third of the inputs
-// for two gates, one in a hundred for the others).  A block of eight steps without such an input is eight FMAs.  In any other
+// for two gates, one in a hundred for the others).  A block of 16 steps without such an input is 16 FMAs.  In any other
 // block d = w xc - (T' - T), exact, is formed as well, and its largest magnitude tells whether every rounding was the
-// reference's.  Blocks that cannot vouch for themselves (two per thread and row on average) are noted down with the
+// reference's.  Half blocks that cannot vouch for themselves (two per thread and row on average) are noted down with the
 // accumulators they began with, and their doubtful steps are evaluated with the reference's own arithmetic at the end of the
 // chain: as a step's increment does not depend on acc, a rounding that went the other way shifts everything after it by the
 // same integer.  A warp with an accumulator that might reach the clamp evaluates the block by the reference's arithmetic.
@@ -37,7 +37,8 @@ constexpr int QL_THREADS = 2 * QL_UNITS;
 constexpr int QL_SEG = 1024;                     // steps whose factors are staged at once, at most
 constexpr int QL_TILE = 64, QL_PITCH = QL_TILE + 16;     // weight bytes per row and tile; conflict-free 128-bit reads
 constexpr int QL_TILE_BYTES = 4 * QL_UNITS * QL_PITCH;
-constexpr int QL_NOTES = 8;                      // doubtful blocks a thread can note down per row
+constexpr int QL_NOTES = 8;                      // doubtful half blocks a thread can note down per row
+constexpr int QL_BLOCK = 16;                     // steps of a block
 constexpr float QL_LEVEL = 2048.0f;              // |acc| up to which the host's list of inputs holds
 constexpr float QL_NEAR_CLAMP = 32000.0f;        // |acc| from which on saturation is possible (zero points included)
 constexpr float QL_ULP = 6.0e-8f;                // a little more than 2^-24
@@ -75,7 +76,7 @@ struct QlArgs {
     int nbuf;                                    // weight tiles in shared memory: 1 or 2
     int proj_staged;                             // the projection weights fit the tiles' space
     unsigned tile_off;                           // where the weight tiles begin in shared memory
-    QlDanger danger[2][2], danger_p;             // [input, recurrent][pair of gates: (i, c), (f, o)]; projection
+    QlDanger danger[3][2];                       // [input, recurrent, projection][pair of gates: (i, c), (f, o)]
 };
 
 __device__ __forceinline__ uint32_t ql_cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
@@ -134,33 +135,59 @@ __device__ __forceinline__ f32x2 ql_weight_pair(uint32_t a, uint32_t b, int j, f
     return sub2(pack2(__uint_as_float(__byte_perm(a, 0x4b000000u, 0x7440 + j)), __uint_as_float(__byte_perm(b, 0x4b000000u, 0x7440 + j))), off2);
 }
 
-// Eight steps by the reference's arithmetic, halves and clamp included.  x: the steps' dequantised values.
-__device__ __noinline__ f32x2 ql_slow8(f32x2 T, uint2 wa, uint2 wb, const float* x, const QlExact* e)
+// A block of steps by the reference's arithmetic, halves and clamp included.  x: the steps' dequantised values.
+__device__ __noinline__ f32x2 ql_slow_block(f32x2 T, uint4 wa, uint4 wb, const float* x, const QlExact* e)
 {
     const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC), woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
-    const uint32_t ma[2] = {wa.x ^ 0x80808080u, wa.y ^ 0x80808080u}, mb[2] = {wb.x ^ 0x80808080u, wb.y ^ 0x80808080u};
-    #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const f32x2 q2 = e->quotient(T, ql_weight_pair(ma[j >> 2], mb[j >> 2], j & 3, woff2), x[j]);
-        float qa, qb, na, nb;
-        unpack2(q2, qa, qb);
-        unpack2(sub2(add2(q2, magic2), magic2), na, nb);
-        if (!(fabsf(__fsub_rn(qa, na)) < 0.5f)) na = roundf(qa);
-        if (!(fabsf(__fsub_rn(qb, nb)) < 0.5f)) nb = roundf(qb);
-        T = add2(pack2(fminf(fmaxf(na, e->lo), e->hi), fminf(fmaxf(nb, e->lo), e->hi)), magic2);
+    const QlExact ex = *e;
+    uint32_t ma[4] = {wa.x ^ 0x80808080u, wa.y ^ 0x80808080u, wa.z ^ 0x80808080u, wa.w ^ 0x80808080u};
+    uint32_t mb[4] = {wb.x ^ 0x80808080u, wb.y ^ 0x80808080u, wb.z ^ 0x80808080u, wb.w ^ 0x80808080u};
+    #pragma unroll 1
+    for (int j = 0; j < QL_BLOCK; j += 4) {
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const f32x2 q2 = ex.quotient(T, ql_weight_pair(ma[0], mb[0], i, woff2), x[j + i]);
+            float qa, qb, na, nb;
+            unpack2(q2, qa, qb);
+            unpack2(sub2(add2(q2, magic2), magic2), na, nb);
+            if (!(fabsf(__fsub_rn(qa, na)) < 0.5f)) na = roundf(qa);
+            if (!(fabsf(__fsub_rn(qb, nb)) < 0.5f)) nb = roundf(qb);
+            T = add2(pack2(fminf(fmaxf(na, ex.lo), ex.hi), fminf(fmaxf(nb, ex.lo), ex.hi)), magic2);
+        }
+        ma[0] = ma[1]; ma[1] = ma[2]; ma[2] = ma[3];
+        mb[0] = mb[1]; mb[1] = mb[2]; mb[2] = mb[3];
     }
     return T;
 }
 
-// Bounds of a block of eight steps: x = how far an accumulator can move in it (|w| <= 128, half a unit of rounding per step),
+// Bounds of a block: x = how far an accumulator can move in it (|w| <= 128, half a unit of rounding per step),
 // corrections that notes may bring included; y = the part of E that does not depend on the accumulators it begins with.
 __device__ __forceinline__ float2 ql_bounds(float sum_abs, float max_abs)
 {
-    const float s = __fmaf_rn(128.5f, sum_abs, 4.5f) + 8.0f * QL_NOTES;
+    const float s = __fmaf_rn(128.5f, sum_abs, 0.5f * QL_BLOCK + 0.5f) + 8.0f * QL_NOTES;
     return make_float2(s, QL_ULP * (3.0f * s + 8.0f * 128.0f * max_abs + 8.0f));
 }
 
-// A packed pair of chains and its doubtful blocks: first step of the block, the two accumulators before it (whose 16 bits
+// The bounds of a block whose largest factors (of the two chains) the lanes of half a warp have, a step each; listed: one of the
+// inputs is on the host's list.  Called by whole warps.
+struct QlBlockInfo { float2 bounds; uint8_t listed; };
+__device__ __forceinline__ QlBlockInfo ql_block_info(float factor, const QlDanger& danger, int mag, int exact_only)
+{
+    float sum = factor, mx = factor;
+    const uint32_t on_list = (danger.bits[(mag >> 5) & 7] >> (mag & 31)) & 1u;
+    #pragma unroll
+    for (int d = 1; d < QL_BLOCK; d *= 2) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+    }
+    const uint32_t votes = __ballot_sync(0xffffffffu, on_list != 0);
+    QlBlockInfo info;
+    info.bounds = ql_bounds(exact_only ? 1e30f : sum, mx);
+    info.listed = (votes >> (threadIdx.x & 16) & 0xffffu) != 0;
+    return info;
+}
+
+// A packed pair of chains and its doubtful half blocks: first step, the two accumulators before it (whose 16 bits
 // are the low halves of T's words).  Only the notes have an address, so that the rest stays in registers.
 struct QlChains {
     f32x2 T;
@@ -173,29 +200,40 @@ struct QlSource {
     const float2* xc;                            // factors of the pair, by position
     const float* xf;                             // dequantised values
     const float2* bounds;                        // by block
+    const uint8_t* listed;                       // by block: one of the inputs is on the host's list
     const QlExact* e;
     const int8_t* wa; const int8_t* wb;          // weight rows: position 0 is step `first` of `K`
-    int first, K, aligned;                       // aligned: eight weights are one 8-byte word
-    __device__ __forceinline__ uint2 weights(const int8_t* w, int pos) const
+    int first, K, aligned;                       // aligned: weights come in whole aligned words
+    __device__ __forceinline__ uint2 weights8(const int8_t* w, int pos) const
     {
         if (aligned) return *(const uint2*)(w + first + pos);
         return make_uint2(ql_weights4(w, first + pos, K), ql_weights4(w, first + pos + 4, K));
     }
+    __device__ __forceinline__ uint4 weights16(const int8_t* w, int pos) const
+    {
+        if (aligned) return *(const uint4*)(w + first + pos);
+        return make_uint4(ql_weights4(w, first + pos, K), ql_weights4(w, first + pos + 4, K), ql_weights4(w, first + pos + 8, K), ql_weights4(w, first + pos + 12, K));
+    }
 };
 
-// Evaluates the doubtful steps of the noted blocks with the reference's arithmetic and corrects the accumulators.
+// Evaluates the doubtful steps of the noted half blocks with the reference's arithmetic and corrects the accumulators.
 __device__ __noinline__ f32x2 ql_resolve(f32x2 end, int notes, const uint2* list, const QlSource src)
 {
     const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC), woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
     const QlExact e = *src.e;
     f32x2 corr2 = pack2(0.f, 0.f);               // what the reference's accumulators are ahead by
+    uint2 note = list[0], next_wa = make_uint2(0, 0), next_wb = next_wa;
+    if (notes > 0) { next_wa = src.weights8(src.wa, (int)note.x); next_wb = src.weights8(src.wb, (int)note.x); }
     #pragma unroll 1
     for (int i = 0; i < notes; ++i) {
-        const uint2 note = list[i];
         const int pos = (int)note.x;
         const float a0 = (float)(short)(note.y & 0xffffu), a1 = (float)((int)note.y >> 16);
-        const uint2 wa = src.weights(src.wa, pos), wb = src.weights(src.wb, pos);
-        const float thr = 0.5f - __fmaf_rn(3.0f * QL_ULP, fmaxf(fabsf(a0), fabsf(a1)), src.bounds[pos >> 3].y);
+        const uint2 wa = next_wa, wb = next_wb;
+        if (i + 1 < notes) {                     // (the weights of the next one are on their way meanwhile)
+            note = list[i + 1];
+            next_wa = src.weights8(src.wa, (int)note.x); next_wb = src.weights8(src.wb, (int)note.x);
+        }
+        const float thr = 0.5f - __fmaf_rn(3.0f * QL_ULP, fmaxf(fabsf(a0), fabsf(a1)), src.bounds[pos / QL_BLOCK].y);
         const uint32_t ma[2] = {wa.x ^ 0x80808080u, wa.y ^ 0x80808080u}, mb[2] = {wb.x ^ 0x80808080u, wb.y ^ 0x80808080u};
         f32x2 T[9], w2[8];
         T[0] = pack2(a0 + QL_MAGIC, a1 + QL_MAGIC);
@@ -230,57 +268,102 @@ __device__ __noinline__ f32x2 ql_resolve(f32x2 end, int notes, const uint2* list
     return add2(end, corr2);
 }
 
-// Eight steps of a pair of chains from position `pos` on, whose weights are w2 (wa, wb as bytes).  listed: one of the inputs is on the
-// host's list.
-__device__ __forceinline__ void ql_steps8(QlChains& ch, const f32x2* w2, int pos, bool listed, const QlSource& src, bool exact_only)
+// A block of steps, from position `pos` on, of the pairs of chains of R rows; ma, mb: the weight bytes with their sign flipped.
+template <int R>
+__device__ __forceinline__ void ql_block(QlChains (&ch)[R], const uint32_t (&ma)[4], const uint32_t (&mb)[4], int pos, const QlSource (&src)[R])
 {
-    const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC);
-    const float2 bd = src.bounds[pos >> 3];
-    const f32x2 T0 = ch.T;
-    float f0, f1;
-    unpack2(sub2(T0, magic2), f0, f1);
-    const float amax = fmaxf(fabsf(f0), fabsf(f1));
-    bool checked = listed;
-    if (__any_sync(0xffffffffu, !(amax + bd.x <= QL_LEVEL) || ch.notes >= QL_NOTES)) {
+    const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC), woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
+    float2 bd[R];
+    float amax[R];
+    bool checked = false, beyond = false, done[R];
+    #pragma unroll
+    for (int r = 0; r < R; ++r) {
+        bd[r] = src[r].bounds[pos / QL_BLOCK];
+        checked |= src[r].listed[pos / QL_BLOCK] != 0;
+        float f0, f1;
+        unpack2(sub2(ch[r].T, magic2), f0, f1);
+        amax[r] = fmaxf(fabsf(f0), fabsf(f1));
+        beyond |= !(amax[r] + bd[r].x <= QL_LEVEL) || ch[r].notes > QL_NOTES - 2;
+        done[r] = false;
+    }
+    if (__any_sync(0xffffffffu, beyond)) {
         checked = true;
-        const bool far = exact_only || __any_sync(0xffffffffu, !(amax + bd.x <= QL_NEAR_CLAMP));
-        if (far || __any_sync(0xffffffffu, ch.notes >= QL_NOTES)) {
-            ch.T = ql_resolve(ch.T, ch.notes, ch.note, src);
-            ch.notes = 0;
-            if (far) {
-                ch.T = ql_slow8(ch.T, src.weights(src.wa, pos), src.weights(src.wb, pos), src.xf + pos, src.e);
-                return;
+        #pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool far = __any_sync(0xffffffffu, !(amax[r] + bd[r].x <= QL_NEAR_CLAMP));
+            if (far || __any_sync(0xffffffffu, ch[r].notes > QL_NOTES - 2)) {
+                ch[r].T = ql_resolve(ch[r].T, ch[r].notes, ch[r].note, src[r]);
+                ch[r].notes = 0;
+                if (far) {
+                    ch[r].T = ql_slow_block(ch[r].T, src[r].weights16(src[r].wa, pos), src[r].weights16(src[r].wb, pos), src[r].xf + pos, src[r].e);
+                    done[r] = true;
+                }
             }
         }
     }
-    f32x2 t = ch.T;
-    const f32x2 begin = t;
-    f32x2 c2[8];
+    f32x2 t[R];
     #pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-        const float4 x = *(const float4*)(src.xc + pos + j);
-        c2[j] = pack2(x.x, x.y); c2[j + 1] = pack2(x.z, x.w);
-    }
+    for (int r = 0; r < R; ++r) t[r] = ch[r].T;
+    auto factors = [&](int r, int j, f32x2& c0, f32x2& c1) {
+        const float4 x = *(const float4*)(src[r].xc + pos + j);
+        c0 = pack2(x.x, x.y); c1 = pack2(x.z, x.w);
+    };
     if (!checked) {
         #pragma unroll
-        for (int j = 0; j < 8; ++j) t = fma2(w2[j], c2[j], t);
-    } else {
-        float dmax = 0.f;
-        #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const f32x2 next = fma2(w2[j], c2[j], t);
-            float d0, d1;
-            unpack2(fma2(w2[j], c2[j], sub2(t, next)), d0, d1);
-            dmax = fmaxf(fmaxf(dmax, fabsf(d0)), fabsf(d1));
-            t = next;
+        for (int j = 0; j < QL_BLOCK; j += 2) {
+            const f32x2 w0 = ql_weight_pair(ma[j >> 2], mb[j >> 2], j & 3, woff2), w1 = ql_weight_pair(ma[j >> 2], mb[j >> 2], (j + 1) & 3, woff2);
+            #pragma unroll
+            for (int r = 0; r < R; ++r) {
+                f32x2 c0, c1;
+                factors(r, j, c0, c1);
+                t[r] = fma2(w1, c1, fma2(w0, c0, t[r]));
+            }
         }
-        if (!(__fadd_rn(dmax, __fmaf_rn(3.0f * QL_ULP, amax, bd.y)) < 0.5f)) {
-            float t0, t1;
-            unpack2(begin, t0, t1);
-            ch.note[ch.notes++] = make_uint2((uint32_t)pos, __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x5410));
+        #pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (!done[r]) ch[r].T = t[r];
+        return;
+    }
+    float dmax[R][2];
+    f32x2 half[R];
+    #pragma unroll
+    for (int r = 0; r < R; ++r) dmax[r][0] = dmax[r][1] = 0.f;
+    #pragma unroll
+    for (int j = 0; j < QL_BLOCK; j += 2) {
+        const f32x2 w0 = ql_weight_pair(ma[j >> 2], mb[j >> 2], j & 3, woff2), w1 = ql_weight_pair(ma[j >> 2], mb[j >> 2], (j + 1) & 3, woff2);
+        #pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (j == QL_BLOCK / 2) half[r] = t[r];
+            f32x2 c0, c1;
+            factors(r, j, c0, c1);
+            const f32x2 t0 = t[r], t1 = fma2(w0, c0, t0), t2 = fma2(w1, c1, t1);
+            float d0, d1, d2, d3;
+            unpack2(fma2(w0, c0, sub2(t0, t1)), d0, d1);
+            unpack2(fma2(w1, c1, sub2(t1, t2)), d2, d3);
+            float& m = dmax[r][j >= QL_BLOCK / 2];
+            m = fmaxf(fmaxf(m, fabsf(d0)), fabsf(d1));
+            m = fmaxf(fmaxf(m, fabsf(d2)), fabsf(d3));
+            t[r] = t2;
         }
     }
-    ch.T = t;
+    #pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (done[r]) continue;
+        const float e = __fmaf_rn(3.0f * QL_ULP, amax[r], bd[r].y);
+        const bool n0 = !(__fadd_rn(dmax[r][0], e) < 0.5f), n1 = !(__fadd_rn(dmax[r][1], e) < 0.5f);
+        if (n0 || n1) {
+            float t0, t1;
+            if (n0) {
+                unpack2(ch[r].T, t0, t1);
+                ch[r].note[ch[r].notes++] = make_uint2((uint32_t)pos, __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x5410));
+            }
+            if (n1) {
+                unpack2(half[r], t0, t1);
+                ch[r].note[ch[r].notes++] = make_uint2((uint32_t)pos + QL_BLOCK / 2, __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x5410));
+            }
+        }
+        ch[r].T = t[r];
+    }
 }
 
 template <int R>
@@ -295,14 +378,14 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     if (nct > 1) ql_cluster_arrive();                        // (every CTA of the cluster runs before anyone writes to it)
 
     extern __shared__ float4 ql_smem[];
-    __shared__ QlDanger s_danger[2][2];
+    __shared__ QlDanger s_danger[3][2];
     __shared__ QlExact s_exact[2][2];
     float* gates = (float*)ql_smem;                          // [4][U] int16 gate buffers as integer-valued floats (o, i, f, c)
     auto gate = [&](int g) { return gates + ((g + 1) & 3) * U; };
     float* work = gates + ((4 * U + QL_GATE_SLACK + 3) & ~3);
-    // chains of the gates, by row and pair (i and c, f and o): factors of every step; by block of eight steps: its bounds, and
+    // chains of the gates, by row and pair (i and c, f and o): factors of every step; by block of steps: its bounds, and
     // whether one of its inputs is on the host's list
-    const int nblk = a.seg / 8;
+    const int nblk = a.seg / QL_BLOCK;
     float2* xc = (float2*)work;                              // [R][2][seg]
     float2* bounds = xc + R * 2 * a.seg;                     // [R][2][nblk]
     float* xf = (float*)(bounds + R * 2 * nblk);             // [R][seg] dequantised values
@@ -313,8 +396,8 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     float* hid = stat + 8;                                   // [U rounded up to 16] dequantised hidden state
     // and, where the i, f and c gates were:
     float2* hc = (float2*)(gates + ((U + 3) & ~3));          // [U rounded up to 16] projection factor of a unit, twice
-    float2* hbounds = hc + ((U + 15) & ~15);                 // [U rounded up to 16, / 8]
-    uint8_t* hlisted = (uint8_t*)(hbounds + ((U + 15) & ~15) / 8);   // the same
+    float2* hbounds = hc + ((U + 15) & ~15);                 // [U rounded up to 16, / 16]
+    uint8_t* hlisted = (uint8_t*)(hbounds + ((U + 15) & ~15) / QL_BLOCK);    // the same
     // weights: nbuf tiles of 4 x QL_UNITS rows (gate-major), then the whole projection matrix
     uint8_t* tiles = (uint8_t*)ql_smem + a.tile_off;
 
@@ -324,7 +407,6 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     const float sr[4] = {a.cifg ? p.s_r2f : p.s_r2i, p.s_r2f, p.s_r2c, p.s_r2o};
     const float sint[4] = {a.cifg ? p.forget_intermediate_scale : p.input_intermediate_scale, p.forget_intermediate_scale,
                            p.cell_intermediate_scale, p.output_intermediate_scale};
-    const f32x2 woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
 
     for (int i = tid; i < (int)(sizeof(s_danger) / 4); i += QL_THREADS) ((uint32_t*)s_danger)[i] = ((const uint32_t*)a.danger)[i];
     if (tid < 4) {
@@ -336,7 +418,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     auto row_of = [&](int r) { return min(b0 + r, p.batch - 1); };          // a cluster's missing last row repeats its first
     // n steps from k0 on of source `src` (0 input, 1 previous output), at position `at` of the staged arrays
     auto stage = [&](int src, int k0, int n, int at) {
-        const int blocks = ((n + 15) & ~15) / 8;
+        const int n16 = (n + 15) & ~15;
         float c[4];
         #pragma unroll
         for (int g = 0; g < 4; ++g) c[g] = __fdiv_rn(src == 0 ? si[g] : sr[g], sint[g]);
@@ -344,30 +426,22 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
         const float scale = src == 0 ? p.input_scale : p.output_state_scale;
         const int8_t* base = src == 0 ? p.input : p.output_state_in;
         __syncthreads();
-        for (int i = tid; i < R * blocks; i += QL_THREADS) {
-            const int r = i / blocks, blk = i - r * blocks;
-            const int8_t* x = base + (long long)row_of(r) * K + k0 + blk * 8;
-            float sum[2] = {0.f, 0.f}, mx[2] = {0.f, 0.f};
-            uint32_t on_list[2] = {0, 0};
-            #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int q = blk * 8 + j < n ? (int)x[j] - zp : 0, mag = abs(q);
-                const float v = __fmul_rn(__int2float_rn(q), scale);
-                const int pos = at + blk * 8 + j;
-                xf[r * a.seg + pos] = v;
-                #pragma unroll
-                for (int pr = 0; pr < 2; ++pr) {
-                    const float2 f = make_float2(__fmul_rn(v, pr ? c[1] : c[0]), __fmul_rn(v, pr ? c[3] : c[2]));
-                    xc[(r * 2 + pr) * a.seg + pos] = f;
-                    const float m = fmaxf(fabsf(f.x), fabsf(f.y));
-                    sum[pr] += m; mx[pr] = fmaxf(mx[pr], m);
-                    on_list[pr] |= (s_danger[src][pr].bits[(mag >> 5) & 7] >> (mag & 31)) & 1u;
-                }
-            }
+        // a step per thread; 16 neighbouring lanes have a block (whole warps take part in its reduction)
+        for (int i = tid; (i & ~31) < R * n16; i += QL_THREADS) {
+            const bool in = i < R * n16;
+            const int r = in ? i / n16 : 0, k = in ? i - r * n16 : 0;
+            const int q = in && k < n ? (int)base[(long long)row_of(r) * K + k0 + k] - zp : 0, mag = abs(q);
+            const float v = __fmul_rn(__int2float_rn(q), scale);
+            if (in) xf[r * a.seg + at + k] = v;
             #pragma unroll
             for (int pr = 0; pr < 2; ++pr) {
-                bounds[(r * 2 + pr) * nblk + at / 8 + blk] = ql_bounds(a.exact_only ? 1e30f : sum[pr], mx[pr]);
-                listed[(r * 2 + pr) * nblk + at / 8 + blk] = (uint8_t)on_list[pr];
+                const float2 f = make_float2(__fmul_rn(v, pr ? c[1] : c[0]), __fmul_rn(v, pr ? c[3] : c[2]));
+                if (in) xc[(r * 2 + pr) * a.seg + at + k] = f;
+                const QlBlockInfo info = ql_block_info(fmaxf(fabsf(f.x), fabsf(f.y)), s_danger[src][pr], mag, a.exact_only);
+                if (in && (tid & 15) == 0) {
+                    bounds[(r * 2 + pr) * nblk + (at + k) / QL_BLOCK] = info.bounds;
+                    listed[(r * 2 + pr) * nblk + (at + k) / QL_BLOCK] = info.listed;
+                }
             }
         }
         __syncthreads();
@@ -388,16 +462,19 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
         uint2 notes[R][QL_NOTES];
         #pragma unroll
         for (int r = 0; r < R; ++r) { ch[r].T = pack2(QL_MAGIC, QL_MAGIC); ch[r].notes = 0; ch[r].note = notes[r]; }
-        // n steps from k0 on of source src, staged at `at`
-        auto run = [&](auto vec, int src, int k0, int n, int at) {
-            constexpr bool VEC = decltype(vec)::value;
-            const int K = src == 0 ? I : O;
+        // by source, and by the pieces of it that are staged at once
+        #pragma unroll 1
+        for (int piece = 0, src = 0; src < 2; ) {
+            const int K = src == 0 ? I : O, step = a.both ? K : a.seg;
+            const int k0 = piece * step, n = min(step, K - k0), at = a.both && src ? I16 : 0;
+            const bool vec = src == 0 ? a.vec_i : a.vec_o;
+            if (!a.both) stage(src, k0, n, 0);
             auto fetch = [&](int t, int buf) {               // the tile of steps [t, t + QL_TILE)
                 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
                     const int8_t* w = (src ? wr[g] : wi[g]) + (long long)ub * K + k0 + t;
                     uint8_t* d = tiles + buf * QL_TILE_BYTES + g * QL_UNITS * QL_PITCH;
-                    if (VEC) {
+                    if (vec) {
                         const int c = (tid & 3) * 16;
                         #pragma unroll
                         for (int h = 0; h < 2; ++h) {
@@ -406,48 +483,42 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
                         }
                     } else {
                         const int c = (tid & 15) * 4;
-                        #pragma unroll 8
+                        #pragma unroll 4
                         for (int row = tid >> 4; row < units; row += QL_THREADS / 16)
                             if (t + c < n) *(uint32_t*)(d + row * QL_PITCH + c) = ql_weights4(w + (long long)row * K, c, n - t);
                     }
                 }
-                if (VEC) ql_copy_commit();
+                ql_copy_commit();
             };
             QlSource from[R];
             #pragma unroll
             for (int r = 0; r < R; ++r) {
                 from[r].xc = xc + (r * 2 + pr) * a.seg + at; from[r].xf = xf + r * a.seg + at;
-                from[r].bounds = bounds + (r * 2 + pr) * nblk + at / 8;
+                from[r].bounds = bounds + (r * 2 + pr) * nblk + at / QL_BLOCK;
+                from[r].listed = listed + (r * 2 + pr) * nblk + at / QL_BLOCK;
                 from[r].e = &s_exact[src][pr];
                 const long long row = (long long)(ub + min(ul, units - 1)) * K;
                 from[r].wa = (src ? (pr ? wr[1] : wr[0]) : (pr ? wi[1] : wi[0])) + row;
                 from[r].wb = (src ? (pr ? wr[3] : wr[2]) : (pr ? wi[3] : wi[2])) + row;
-                from[r].first = k0; from[r].K = K; from[r].aligned = VEC;
+                from[r].first = k0; from[r].K = K; from[r].aligned = vec;
             }
             const uint8_t* ta = tiles + (pr * QL_UNITS + min(ul, units - 1)) * QL_PITCH;
             fetch(0, 0);
             int buf = 0;
+            #pragma unroll 1
             for (int t = 0; t < n; t += QL_TILE) {
                 const bool ahead = a.nbuf == 2 && t + QL_TILE < n;
-                if (ahead) fetch(t + QL_TILE, buf ^ 1);
-                if (VEC) { if (ahead) ql_copy_wait<1>(); else ql_copy_wait<0>(); }
+                if (ahead) { fetch(t + QL_TILE, buf ^ 1); ql_copy_wait<1>(); }
+                else ql_copy_wait<0>();
                 __syncthreads();
                 if (busy) {
                     const uint8_t* tb = ta + buf * QL_TILE_BYTES;
                     #pragma unroll 1
-                    for (int k = t; k < min(n, t + QL_TILE); k += 16) {
+                    for (int k = t; k < min(n, t + QL_TILE); k += QL_BLOCK) {
                         const uint4 na = *(const uint4*)(tb + k - t), nb = *(const uint4*)(tb + 2 * QL_UNITS * QL_PITCH + k - t);
                         const uint32_t ma[4] = {na.x ^ 0x80808080u, na.y ^ 0x80808080u, na.z ^ 0x80808080u, na.w ^ 0x80808080u};
                         const uint32_t mb[4] = {nb.x ^ 0x80808080u, nb.y ^ 0x80808080u, nb.z ^ 0x80808080u, nb.w ^ 0x80808080u};
-                        #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            f32x2 w2[8];
-                            #pragma unroll
-                            for (int j = 0; j < 8; ++j) w2[j] = ql_weight_pair(ma[h * 2 + (j >> 2)], mb[h * 2 + (j >> 2)], j & 3, woff2);
-                            #pragma unroll
-                            for (int r = 0; r < R; ++r)
-                                ql_steps8(ch[r], w2, k + h * 8, listed[(r * 2 + pr) * nblk + ((at + k) >> 3) + h] != 0, from[r], a.exact_only);
-                        }
+                        ql_block<R>(ch, ma, mb, k, from);
                     }
                 }
                 __syncthreads();                             // (everyone has left the tile before it is overwritten)
@@ -459,21 +530,8 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
                 ch[r].T = ql_resolve(ch[r].T, ch[r].notes, ch[r].note, from[r]);
                 ch[r].notes = 0;
             }
-        };
-        auto run_source = [&](int src, int k0, int n, int at) {
-            if (src == 0 ? a.vec_i : a.vec_o) run(std::integral_constant<bool, true>{}, src, k0, n, at);
-            else                              run(std::integral_constant<bool, false>{}, src, k0, n, at);
-        };
-        if (a.both) {
-            run_source(0, 0, I, 0);
-            run_source(1, 0, O, I16);
-        } else {
-            for (int src = 0; src < 2; ++src)
-                for (int s0 = 0; s0 < (src == 0 ? I : O); s0 += a.seg) {
-                    const int n = min(a.seg, (src == 0 ? I : O) - s0);
-                    stage(src, s0, n, 0);
-                    run_source(src, s0, n, 0);
-                }
+            ++piece;
+            if (piece * step >= K) { piece = 0; ++src; }
         }
         if (ul < units) {
             #pragma unroll
@@ -524,6 +582,14 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     // Post-processing of gates [gfirst, glast]: peephole, layer norm, activation.  `cellsrc` is the cell
     // state the peephole reads (old state for i and f, new state for o), as integer-valued floats.
     auto gate_post = [&](int gfirst, int glast, const int16_t* cell_in_global, const float* cell_smem) {
+        // layer-norm weights and biases of this thread's first unit, on their way during the sums
+        int16_t lw[4];
+        int32_t gb[4];
+        #pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const bool need = a.ln && g >= gfirst && g <= glast && tid < U;
+            lw[g] = need ? lnw[g][tid] : (int16_t)0; gb[g] = need ? gbias[g][tid] : 0;
+        }
         if (a.peephole) {
             for (int g = gfirst; g <= glast; ++g) {
                 if (!peep[g]) continue;
@@ -574,15 +640,18 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
             proj_pending = false;
             __syncthreads();
         }
-        for (int g = gfirst; g <= glast; ++g) {
-            const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f), isln = __frcp_rn(sln);
-            for (int u = tid; u < U; u += QL_THREADS) {
+        for (int u = tid; u < U; u += QL_THREADS) {
+            #pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                if (g < gfirst || g > glast) continue;
                 float q = gate(g)[u];
                 float s = sint[g];
                 if (a.ln) {
+                    if (u != tid) { lw[g] = lnw[g][u]; gb[g] = gbias[g][u]; }
+                    const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f), isln = __frcp_rn(sln);
                     q = q16f(__fmul_rn(__fsub_rn(__fmul_rn(q, s), stat[g * 2]), stat[g * 2 + 1]), sln, isln);      // normalise
-                    q = q16f(__fmul_rn(__fmul_rn((float)lnw[g][u], slnw[g]), __fmul_rn(q, sln)), sln, isln);       // * weight
-                    q = q16f(__fadd_rn(__fmul_rn(q, sln), __fmul_rn(__int2float_rn(gbias[g][u]), sgb[g])), 1.f / 4096, 4096.f);  // + bias
+                    q = q16f(__fmul_rn(__fmul_rn((float)lw[g], slnw[g]), __fmul_rn(q, sln)), sln, isln);           // * weight
+                    q = q16f(__fadd_rn(__fmul_rn(q, sln), __fmul_rn(__int2float_rn(gb[g]), sgb[g])), 1.f / 4096, 4096.f);        // + bias
                     s = 1.f / 4096;
                 }
                 const float v = __fmul_rn(q, s);
@@ -618,18 +687,25 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
 
     // ---- hidden = Q8(o * Q16(tanh(c))), its projection factors and magnitudes
     const float hzp = (float)p.hidden_state_zp, cp = a.proj ? __fdiv_rn(p.s_proj, p.output_scale) : 0.f;
-    for (int u = tid; u < U16; u += QL_THREADS) {
-        if (u >= U) { hc[u] = make_float2(0.f, 0.f); hid[u] = 0.f; continue; }
-        const float t = q16f(tanhf(__fmul_rn(cell[u], sc)), sc, isc);
-        const float hv = __fmul_rn(__fmul_rn(gate(3)[u], sc), __fmul_rn(t, sc));
-        const float hq = fminf(fmaxf(__fadd_rn(hzp, roundf(__fdiv_rn(hv, p.hidden_state_scale))), -128.f), 127.f);
-        const float h = __fmul_rn(__fsub_rn(hq, hzp), p.hidden_state_scale);      // dequantised hidden state
-        hid[u] = h;
-        cell[u] = fabsf(__fsub_rn(hq, hzp));                                      // (the cell state is done with: its magnitude)
+    for (int u = tid; (u & ~31) < U16; u += QL_THREADS) {
+        float h = 0.f;
+        int mag = 0;
+        if (u < U) {
+            const float t = q16f(tanhf(__fmul_rn(cell[u], sc)), sc, isc);
+            const float hv = __fmul_rn(__fmul_rn(gate(3)[u], sc), __fmul_rn(t, sc));
+            const float hq = fminf(fmaxf(__fadd_rn(hzp, roundf(__fdiv_rn(hv, p.hidden_state_scale))), -128.f), 127.f);
+            const float d = __fsub_rn(hq, hzp);
+            h = __fmul_rn(d, p.hidden_state_scale);          // dequantised hidden state
+            mag = (int)fabsf(d);
+        }
         const float f = __fmul_rn(h, cp);
-        hc[u] = make_float2(f, f);
+        const QlBlockInfo info = ql_block_info(fabsf(f), s_danger[2][0], mag, a.exact_only);
+        if (u < U16) {
+            hid[u] = h;
+            hc[u] = make_float2(f, f);
+            if ((u & 15) == 0) { hbounds[u / QL_BLOCK] = info.bounds; hlisted[u / QL_BLOCK] = info.listed; }
+        }
     }
-    __syncthreads();
 
     // ---- projection (int16 accumulator at the OUTPUT's scale and offset) and outputs
     if (proj_pending) stage_projection(0);
@@ -653,21 +729,9 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
         p.output_state_out[(long long)b * O + j] = (int8_t)hs;
     };
     if (!a.proj) {
+        __syncthreads();
         for (int j = tid; j < O; j += QL_THREADS) finish(j, 0.f);
         return;
-    }
-    const int hblk = U16 / 8;
-    for (int blk = tid; blk < hblk; blk += QL_THREADS) {
-        float sum = 0.f, mx = 0.f;
-        uint32_t on_list = 0;
-        for (int j = 0; j < 8; ++j) {
-            const int u = blk * 8 + j, mag = u < U ? (int)cell[u] : 0;
-            const float m = fabsf(hc[u].x);
-            sum += m; mx = fmaxf(mx, m);
-            on_list |= (a.danger_p.bits[(mag >> 5) & 7] >> (mag & 31)) & 1u;
-        }
-        hbounds[blk] = ql_bounds(a.exact_only ? 1e30f : sum, mx);
-        hlisted[blk] = (uint8_t)on_list;
     }
     if (tid == 0) s_exact[0][0].set(so, so, p.s_proj, p.s_proj, -32768.f - zo, 32767.f - zo);
     if (a.proj_staged && a.vec_p) ql_copy_wait<0>();
@@ -682,28 +746,25 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
             first[0] = q16zf(__fmul_rn(__int2float_rn(p.b_proj[j]), p.s_bproj), so, zo);
             first[1] = q16zf(__fmul_rn(__int2float_rn(p.b_proj[j1]), p.s_bproj), so, zo);
         }
-        QlChains ch;
+        QlChains ch[1];
         uint2 notes[QL_NOTES];
-        ch.T = pack2(QL_MAGIC + (first[0] - zo), QL_MAGIC + (first[1] - zo));
-        ch.notes = 0; ch.note = notes;
-        QlSource from;
-        from.xc = hc; from.xf = hid; from.bounds = hbounds; from.e = &s_exact[0][0];
-        from.wa = a.proj_staged ? (const int8_t*)tiles + j * ppitch : w[0];
-        from.wb = a.proj_staged ? (const int8_t*)tiles + j1 * ppitch : w[1];
-        from.first = 0; from.K = U; from.aligned = a.proj_staged;
-        uint2 na = from.weights(from.wa, 0), nb = from.weights(from.wb, 0);
+        ch[0].T = pack2(QL_MAGIC + (first[0] - zo), QL_MAGIC + (first[1] - zo));
+        ch[0].notes = 0; ch[0].note = notes;
+        QlSource from[1];
+        from[0].xc = hc; from[0].xf = hid; from[0].bounds = hbounds; from[0].listed = hlisted; from[0].e = &s_exact[0][0];
+        from[0].wa = a.proj_staged ? (const int8_t*)tiles + j * ppitch : w[0];
+        from[0].wb = a.proj_staged ? (const int8_t*)tiles + j1 * ppitch : w[1];
+        from[0].first = 0; from[0].K = U; from[0].aligned = a.proj_staged;
+        uint4 na = from[0].weights16(from[0].wa, 0), nb = from[0].weights16(from[0].wb, 0);
         #pragma unroll 1
-        for (int k = 0; k < U16; k += 8) {
-            const uint32_t ma[2] = {na.x ^ 0x80808080u, na.y ^ 0x80808080u}, mb[2] = {nb.x ^ 0x80808080u, nb.y ^ 0x80808080u};
-            if (k + 8 < U16) { na = from.weights(from.wa, k + 8); nb = from.weights(from.wb, k + 8); }
-            f32x2 w2[8];
-            #pragma unroll
-            for (int i = 0; i < 8; ++i) w2[i] = ql_weight_pair(ma[i >> 2], mb[i >> 2], i & 3, woff2);
-            ql_steps8(ch, w2, k, hlisted[k >> 3] != 0, from, a.exact_only);
+        for (int k = 0; k < U16; k += QL_BLOCK) {
+            const uint32_t ma[4] = {na.x ^ 0x80808080u, na.y ^ 0x80808080u, na.z ^ 0x80808080u, na.w ^ 0x80808080u};
+            const uint32_t mb[4] = {nb.x ^ 0x80808080u, nb.y ^ 0x80808080u, nb.z ^ 0x80808080u, nb.w ^ 0x80808080u};
+            if (k + QL_BLOCK < U16) { na = from[0].weights16(from[0].wa, k + QL_BLOCK); nb = from[0].weights16(from[0].wb, k + QL_BLOCK); }
+            ql_block<1>(ch, ma, mb, k, from);
         }
-        ch.T = ql_resolve(ch.T, ch.notes, ch.note, from);
         float f0, f1;
-        unpack2(sub2(ch.T, pack2(QL_MAGIC, QL_MAGIC)), f0, f1);
+        unpack2(sub2(ql_resolve(ch[0].T, ch[0].notes, ch[0].note, from[0]), pack2(QL_MAGIC, QL_MAGIC)), f0, f1);
         if (j0 < O2) {
             finish(j, f0 + zo);
             if (j + O2 < O) finish(j + O2, f1 + zo);
@@ -783,7 +844,6 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
     a.exact_only = !byte(p->input_zp) || !byte(p->output_state_zp) || !byte(p->output_zp) || !byte(p->hidden_state_zp);
     for (float s : scales) a.exact_only |= !(s >= 1e-8f && s <= 1e8f);
     memset(a.danger, 0, sizeof(a.danger));
-    memset(&a.danger_p, 0, sizeof(a.danger_p));
     if (!a.exact_only) {
         const float si[4] = {a.cifg ? p->s_i2f : p->s_i2i, p->s_i2f, p->s_i2c, p->s_i2o}, sr[4] = {a.cifg ? p->s_r2f : p->s_r2i, p->s_r2f, p->s_r2c, p->s_r2o};
         const float sint[4] = {a.cifg ? p->forget_intermediate_scale : p->input_intermediate_scale, p->forget_intermediate_scale,
@@ -792,7 +852,7 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
             a.danger[0][pr] = ql_either(ql_danger_of(p->input_scale, si[pr], sint[pr]), ql_danger_of(p->input_scale, si[pr + 2], sint[pr + 2]));
             a.danger[1][pr] = ql_either(ql_danger_of(p->output_state_scale, sr[pr], sint[pr]), ql_danger_of(p->output_state_scale, sr[pr + 2], sint[pr + 2]));
         }
-        if (a.proj) a.danger_p = ql_danger_of(p->hidden_state_scale, p->s_proj, p->output_scale);
+        if (a.proj) a.danger[2][0] = ql_danger_of(p->hidden_state_scale, p->s_proj, p->output_scale);
     }
     auto aligned = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     a.vec_i = p->input_size % 16 == 0 && aligned(p->w_i2i) && aligned(p->w_i2f) && aligned(p->w_i2c) && aligned(p->w_i2o);
@@ -817,7 +877,7 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
     a.nbuf = 2;
     size_t smem;
     for (;;) {
-        const size_t staged = (size_t)rows * a.seg * (2 * 8 + 4) + (size_t)rows * 2 * (a.seg / 8) * (8 + 1);
+        const size_t staged = (size_t)rows * a.seg * (2 * 8 + 4) + (size_t)rows * 2 * (a.seg / QL_BLOCK) * (8 + 1);
         a.tile_off = (unsigned)((gates + staged + 15) & ~(size_t)15);
         smem = a.tile_off + (size_t)a.nbuf * QL_TILE_BYTES;
         if (smem < gates + after) smem = gates + after;
