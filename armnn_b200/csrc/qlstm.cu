@@ -187,15 +187,20 @@ __device__ __forceinline__ QlBlockInfo ql_block_info(float factor, const QlDange
     return info;
 }
 
-// A packed pair of chains and its doubtful half blocks: first step, the two accumulators before it (whose 16 bits
-// are the low halves of T's words).  Only the notes have an address, so that the rest stays in registers.
+// A doubtful half block: the two accumulators before it (whose 16 bits are the low halves of T's words), its weight bytes as
+// ql_block has them (fetching them again at the end of the chain cost more than the evaluation), and its first step.
+struct QlNote {
+    uint4 w;
+    uint32_t acc, pos;
+};
+// A packed pair of chains and its doubtful half blocks.  Only the notes have an address, so that the rest stays in registers.
 struct QlChains {
     f32x2 T;
     int notes;
-    uint2* note;
+    QlNote* note;
 };
 
-// What noted blocks are corrected from: the staged arrays and the weight rows of the pair.
+// What noted half blocks are corrected from, and the weight rows of the pair.
 struct QlSource {
     const float2* xc;                            // factors of the pair, by position
     const float* xf;                             // dequantised values
@@ -204,11 +209,6 @@ struct QlSource {
     const QlExact* e;
     const int8_t* wa; const int8_t* wb;          // weight rows: position 0 is step `first` of `K`
     int first, K, aligned;                       // aligned: weights come in whole aligned words
-    __device__ __forceinline__ uint2 weights8(const int8_t* w, int pos) const
-    {
-        if (aligned) return *(const uint2*)(w + first + pos);
-        return make_uint2(ql_weights4(w, first + pos, K), ql_weights4(w, first + pos + 4, K));
-    }
     __device__ __forceinline__ uint4 weights16(const int8_t* w, int pos) const
     {
         if (aligned) return *(const uint4*)(w + first + pos);
@@ -217,31 +217,27 @@ struct QlSource {
 };
 
 // Evaluates the doubtful steps of the noted half blocks with the reference's arithmetic and corrects the accumulators.
-__device__ __noinline__ f32x2 ql_resolve(f32x2 end, int notes, const uint2* list, const QlSource src)
+__device__ __noinline__ f32x2 ql_resolve(f32x2 end, int notes, const QlNote* list, const float2* xc, const float* xf, const float2* bounds, const QlExact* exact)
 {
     const f32x2 magic2 = pack2(QL_MAGIC, QL_MAGIC), woff2 = pack2(8388608.0f + 128.0f, 8388608.0f + 128.0f);
-    const QlExact e = *src.e;
+    const QlExact e = *exact;
     f32x2 corr2 = pack2(0.f, 0.f);               // what the reference's accumulators are ahead by
-    uint2 note = list[0], next_wa = make_uint2(0, 0), next_wb = next_wa;
-    if (notes > 0) { next_wa = src.weights8(src.wa, (int)note.x); next_wb = src.weights8(src.wb, (int)note.x); }
+    QlNote next = list[0];
     #pragma unroll 1
     for (int i = 0; i < notes; ++i) {
-        const int pos = (int)note.x;
-        const float a0 = (float)(short)(note.y & 0xffffu), a1 = (float)((int)note.y >> 16);
-        const uint2 wa = next_wa, wb = next_wb;
-        if (i + 1 < notes) {                     // (the weights of the next one are on their way meanwhile)
-            note = list[i + 1];
-            next_wa = src.weights8(src.wa, (int)note.x); next_wb = src.weights8(src.wb, (int)note.x);
-        }
-        const float thr = 0.5f - __fmaf_rn(3.0f * QL_ULP, fmaxf(fabsf(a0), fabsf(a1)), src.bounds[pos / QL_BLOCK].y);
-        const uint32_t ma[2] = {wa.x ^ 0x80808080u, wa.y ^ 0x80808080u}, mb[2] = {wb.x ^ 0x80808080u, wb.y ^ 0x80808080u};
+        const QlNote note = next;
+        if (i + 1 < notes) next = list[i + 1];
+        const int pos = (int)note.pos;
+        const float a0 = (float)(short)(note.acc & 0xffffu), a1 = (float)((int)note.acc >> 16);
+        const float thr = 0.5f - __fmaf_rn(3.0f * QL_ULP, fmaxf(fabsf(a0), fabsf(a1)), bounds[pos / QL_BLOCK].y);
+        const uint32_t ma[2] = {note.w.x, note.w.y}, mb[2] = {note.w.z, note.w.w};
         f32x2 T[9], w2[8];
         T[0] = pack2(a0 + QL_MAGIC, a1 + QL_MAGIC);
         uint32_t doubtful = 0;
         #pragma unroll
         for (int j = 0; j < 8; ++j) {
             w2[j] = ql_weight_pair(ma[j >> 2], mb[j >> 2], j & 3, woff2);
-            const float2 c = src.xc[pos + j];
+            const float2 c = xc[pos + j];
             const f32x2 c2 = pack2(c.x, c.y);
             T[j + 1] = fma2(w2[j], c2, T[j]);
             float d0, d1;
@@ -256,7 +252,7 @@ __device__ __noinline__ f32x2 ql_resolve(f32x2 end, int notes, const uint2* list
             #pragma unroll
             for (int j = 1; j < 8; ++j)
                 if (j == k) { t = T[j]; next = T[j + 1]; w = w2[j]; }
-            const f32x2 q2 = e.quotient(add2(t, corr2), w, src.xf[pos + k]);
+            const f32x2 q2 = e.quotient(add2(t, corr2), w, xf[pos + k]);
             float qa, qb, na, nb;
             unpack2(q2, qa, qb);
             unpack2(sub2(add2(q2, magic2), magic2), na, nb);
@@ -292,7 +288,7 @@ __device__ __forceinline__ void ql_block(QlChains (&ch)[R], const uint32_t (&ma)
         for (int r = 0; r < R; ++r) {
             const bool far = __any_sync(0xffffffffu, !(amax[r] + bd[r].x <= QL_NEAR_CLAMP));
             if (far || __any_sync(0xffffffffu, ch[r].notes > QL_NOTES - 2)) {
-                ch[r].T = ql_resolve(ch[r].T, ch[r].notes, ch[r].note, src[r]);
+                ch[r].T = ql_resolve(ch[r].T, ch[r].notes, ch[r].note, src[r].xc, src[r].xf, src[r].bounds, src[r].e);
                 ch[r].notes = 0;
                 if (far) {
                     ch[r].T = ql_slow_block(ch[r].T, src[r].weights16(src[r].wa, pos), src[r].weights16(src[r].wb, pos), src[r].xf + pos, src[r].e);
@@ -352,15 +348,16 @@ __device__ __forceinline__ void ql_block(QlChains (&ch)[R], const uint32_t (&ma)
         const float e = __fmaf_rn(3.0f * QL_ULP, amax[r], bd[r].y);
         const bool n0 = !(__fadd_rn(dmax[r][0], e) < 0.5f), n1 = !(__fadd_rn(dmax[r][1], e) < 0.5f);
         if (n0 || n1) {
-            float t0, t1;
-            if (n0) {
-                unpack2(ch[r].T, t0, t1);
-                ch[r].note[ch[r].notes++] = make_uint2((uint32_t)pos, __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x5410));
-            }
-            if (n1) {
-                unpack2(half[r], t0, t1);
-                ch[r].note[ch[r].notes++] = make_uint2((uint32_t)pos + QL_BLOCK / 2, __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x5410));
-            }
+            auto note = [&](f32x2 begin, int h) {
+                float t0, t1;
+                unpack2(begin, t0, t1);
+                QlNote& to = ch[r].note[ch[r].notes++];
+                to.w = make_uint4(ma[2 * h], ma[2 * h + 1], mb[2 * h], mb[2 * h + 1]);
+                to.acc = __byte_perm(__float_as_uint(t0), __float_as_uint(t1), 0x5410);
+                to.pos = (uint32_t)(pos + h * (QL_BLOCK / 2));
+            };
+            if (n0) note(ch[r].T, 0);
+            if (n1) note(half[r], 1);
         }
         ch[r].T = t[r];
     }
@@ -459,7 +456,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
         const int units = min(QL_UNITS, u_hi - ub);
         const bool busy = (ul & ~31) < units;                // (warp-uniform; lanes beyond the last unit repeat it)
         QlChains ch[R];
-        uint2 notes[R][QL_NOTES];
+        QlNote notes[R][QL_NOTES];
         #pragma unroll
         for (int r = 0; r < R; ++r) { ch[r].T = pack2(QL_MAGIC, QL_MAGIC); ch[r].notes = 0; ch[r].note = notes[r]; }
         // by source, and by the pieces of it that are staged at once
@@ -527,7 +524,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
             }
             #pragma unroll
             for (int r = 0; r < R; ++r) {
-                ch[r].T = ql_resolve(ch[r].T, ch[r].notes, ch[r].note, from[r]);
+                ch[r].T = ql_resolve(ch[r].T, ch[r].notes, ch[r].note, from[r].xc, from[r].xf, from[r].bounds, from[r].e);
                 ch[r].notes = 0;
             }
             ++piece;
@@ -747,7 +744,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
             first[1] = q16zf(__fmul_rn(__int2float_rn(p.b_proj[j1]), p.s_bproj), so, zo);
         }
         QlChains ch[1];
-        uint2 notes[QL_NOTES];
+        QlNote notes[QL_NOTES];
         ch[0].T = pack2(QL_MAGIC + (first[0] - zo), QL_MAGIC + (first[1] - zo));
         ch[0].notes = 0; ch[0].note = notes;
         QlSource from[1];
@@ -764,7 +761,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
             ql_block<1>(ch, ma, mb, k, from);
         }
         float f0, f1;
-        unpack2(sub2(ql_resolve(ch[0].T, ch[0].notes, ch[0].note, from[0]), pack2(QL_MAGIC, QL_MAGIC)), f0, f1);
+        unpack2(sub2(ql_resolve(ch[0].T, ch[0].notes, ch[0].note, from[0].xc, from[0].xf, from[0].bounds, from[0].e), pack2(QL_MAGIC, QL_MAGIC)), f0, f1);
         if (j0 < O2) {
             finish(j, f0 + zo);
             if (j + O2 < O) finish(j + O2, f1 + zo);
