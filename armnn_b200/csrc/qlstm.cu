@@ -25,7 +25,10 @@
 // through (peephole) -> layer norm -> activations -> cell update -> output gate -> hidden state -> projection (chains of the
 // same kind) -> outputs.  Layer-norm sums are sequential in the reference: one thread per gate, its operands read ahead.
 //
-// Bound by the fp32 pipe in the chains and by the latency of the sequential sums.
+// Bound by the fp32 and integer pipes in the chains (about 60 % of the time at 512 units) and by the latency of the sequential
+// sums and of the projection's chains.  Three layers (40 or 256 -> 512 units -> 256) at batch 128: 475 us with one CTA per row and
+// the reference's arithmetic in every step, 310 us with blocks of eight steps, 283 us with 16 and both rows interleaved, 251 us
+// since notes keep their weights.
 #include <mutex>
 #include <type_traits>
 #include "common.cuh"
