@@ -314,7 +314,9 @@ bool bmm_mma_eligible(const b200k_bmm_params* p)
     if (!p->x.data || !p->y.data || !p->out.data) return false;
     if (!is_q8(p->x.dtype) || !is_q8(p->y.dtype) || !is_q8(p->out.dtype)) return false;
     if (p->batch < 1 || p->batch > 65535 || p->m < 1 || p->k < 1 || p->n < 1) return false;
-    if ((p->m + BM_T - 1) / BM_T > 65535 || !ordinary_quant(p->out)) return false;
+    if ((p->m + BM_T - 1) / BM_T > 65535) return false;
+    // (the accumulator is below 2^31 in magnitude)
+    if (!quotient_holds(2147483648.0 * fabs((double)p->x.scale * (double)p->y.scale), p->out)) return false;
     // (the int32 accumulator of the reference and of the generic kernel has the same range)
     return true;
 }

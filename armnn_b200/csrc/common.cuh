@@ -73,10 +73,15 @@ inline float rn_reciprocal(float b)
     return best;
 }
 
-// Whether the division-free quotients (and, for the zero point, the 2^23 byte-to-float trick) are exact for a tensor's
-// quantisation parameters; anything else takes the kernels with the IEEE division.
+// Whether a tensor's quantisation parameters are in the range that the division-free quotients (and, for the zero point, the
+// 2^23 byte-to-float trick) are exact for; anything else takes the kernels with the IEEE division.  The range is not closed
+// under division: quotient_holds says whether values of up to vmax have quotients by the scale that stay finite on the way
+// (an infinite product v * (1 / scale) would become NaN in the correction step, where the division saturates).
 inline bool ordinary_scale(float s) { return s >= 1e-20f && s <= 1e20f; }
 inline bool ordinary_quant(const b200k_qtensor& t) { return ordinary_scale(t.scale) && t.zero_point > -(1 << 20) && t.zero_point < (1 << 20); }
+inline bool quotient_holds(double vmax, const b200k_qtensor& t) { return ordinary_quant(t) && vmax < 1e38 && vmax < 1e30 * (double)t.scale; }
+// largest |dequantised value| of an 8-bit tensor
+inline double value_bound(const b200k_qtensor& t) { return (256.0 + fabs((double)t.zero_point)) * fabs((double)t.scale); }
 
 // The contraction epilogue v = fl(fl(acc * m) + b); q = clamp(zy + round_half_away(fl(v / sy)), lo, hi) without the
 // division unit: with y = RN(1 / sy) from the host, p = fl(v * y) and q = fma(fma(-p, sy, v), y, p) is the correctly

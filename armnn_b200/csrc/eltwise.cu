@@ -229,9 +229,10 @@ extern "C" int b200k_eltwise_q8(const b200k_eltwise_params* p, void* stream)
     }
     cudaStream_t s = (cudaStream_t)stream;
     const uintptr_t al = (uintptr_t)p->a.data | (uintptr_t)p->b.data | (uintptr_t)p->out.data;
+    const double va = value_bound(p->a), vb = value_bound(p->b), vmax = p->op == ELT_MUL ? va * vb : va + vb;
     const bool fast_op = p->op == ELT_ADD || p->op == ELT_SUB || p->op == ELT_MUL || p->op == ELT_MAX || p->op == ELT_MIN;
     if (same && fast_op && is_q8(p->a.dtype) && is_q8(p->b.dtype) && is_q8(p->out.dtype) && (al & 15) == 0 &&
-        ordinary_quant(p->a) && ordinary_quant(p->b) && ordinary_quant(p->out)) {
+        ordinary_quant(p->a) && ordinary_quant(p->b) && quotient_holds(vmax, p->out)) {
         EltVecArgs v;
         v.a = (const uint8_t*)p->a.data; v.b = (const uint8_t*)p->b.data; v.out = (uint8_t*)p->out.data;
         v.flip_a = p->a.dtype == B200K_S8 ? 0x80808080u : 0u; v.flip_b = p->b.dtype == B200K_S8 ? 0x80808080u : 0u;

@@ -200,7 +200,7 @@ extern "C" int b200k_resize_q(const b200k_resize_params* p, void* stream)
     const long long images = p->nchw ? (long long)p->n * p->c : p->n;
     const long long width = (long long)p->out_w * (p->nchw ? 1 : p->c), in_width = (long long)p->in_w * (p->nchw ? 1 : p->c);
     const unsigned row_blocks = div_up(p->out_h, RZ_ROWS);
-    if (is_q8(p->x.dtype) && is_q8(p->y.dtype) && ordinary_quant(p->x) && ordinary_quant(p->y) && images <= 65535 && row_blocks <= 65535 &&
+    if (is_q8(p->x.dtype) && is_q8(p->y.dtype) && ordinary_quant(p->x) && quotient_holds(2.0 * value_bound(p->x), p->y) && images <= 65535 && row_blocks <= 65535 &&
         width < (1ll << 30) && in_width < (1ll << 30)) {
         ResizeArgs r = a;
         if (p->nchw) { r.N = (int)images; r.C = 1; r.nchw = 0; }
