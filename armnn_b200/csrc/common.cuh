@@ -58,10 +58,15 @@ __device__ __forceinline__ int quantize_dev(float v, float scale, int zp, float 
     return __float2int_rz(q);
 }
 
+// The scales that the division-free quotients below are exact for: reciprocals and remainders stay normal numbers.
+inline bool ordinary_scale(float s) { return s >= 1e-20f && s <= 1e20f; }
+
 // RN(1 / b): the double quotient rounded to float is within one ulp; the exact residuals 1 - b * y (products of two
-// 24-bit significands are exact in double) pick the nearest of the three candidates.
+// 24-bit significands are exact in double) pick the nearest of the three candidates.  NaN for any other scale: every quotient
+// formed with it is NaN, which the tensor-core epilogue's tests send to the IEEE division.
 inline float rn_reciprocal(float b)
 {
+    if (!ordinary_scale(b)) return NAN;
     const float y = (float)(1.0 / (double)b);
     const float cand[3] = {nextafterf(y, 0.f), y, nextafterf(y, INFINITY)};
     float best = y;
@@ -77,7 +82,6 @@ inline float rn_reciprocal(float b)
 // 2^23 byte-to-float trick) are exact for; anything else takes the kernels with the IEEE division.  The range is not closed
 // under division: quotient_holds says whether values of up to vmax have quotients by the scale that stay finite on the way
 // (an infinite product v * (1 / scale) would become NaN in the correction step, where the division saturates).
-inline bool ordinary_scale(float s) { return s >= 1e-20f && s <= 1e20f; }
 inline bool ordinary_quant(const b200k_qtensor& t) { return ordinary_scale(t.scale) && t.zero_point > -(1 << 20) && t.zero_point < (1 << 20); }
 inline bool quotient_holds(double vmax, const b200k_qtensor& t) { return ordinary_quant(t) && vmax < 1e38 && vmax < 1e30 * (double)t.scale; }
 // largest |dequantised value| of an 8-bit tensor
@@ -86,11 +90,15 @@ inline double value_bound(const b200k_qtensor& t) { return (256.0 + fabs((double
 // The contraction epilogue v = fl(fl(acc * m) + b); q = clamp(zy + round_half_away(fl(v / sy)), lo, hi) without the
 // division unit: with y = RN(1 / sy) from the host, p = fl(v * y) and q = fma(fma(-p, sy, v), y, p) is the correctly
 // rounded quotient (Markstein); it is rounded with the 1.5 * 2^23 constant (halves to even) and only exact halves, or
-// values too large for the constant, go through roundf.  lo / hi: type range intersected with the activation clamp.
+// values too large for the constant, go through roundf.  lo / hi: type range intersected with the activation clamp.  For
+// ordinary parameters of the output (ordinary_quant): v is limited to quotients of +-2^24, which saturate, as a product that
+// overflowed would leave NaN.
 __device__ __forceinline__ int requant_fast(int acc, float m, float b, bool has_bias, float sy, float inv_sy, float zy, float lo, float hi)
 {
+    const float most = __fmul_rn(sy, 16777216.0f);
     float v = __fmul_rn(__int2float_rn(acc), m);
     if (has_bias) v = __fadd_rn(v, b);
+    v = fminf(fmaxf(v, -most), most);
     const float p = __fmul_rn(v, inv_sy);
     const float q = __fmaf_rn(__fmaf_rn(-p, sy, v), inv_sy, p);
     float n = __fsub_rn(__fadd_rn(q, 12582912.0f), 12582912.0f);
@@ -305,7 +313,13 @@ __device__ __forceinline__ void requant_fast2(int acc0, int acc1, f32x2 m2, f32x
                                               float& r0, float& r1)
 {
     const f32x2 zero2 = pack2(0.f, 0.f), magic2 = pack2(12582912.0f, 12582912.0f);
-    const f32x2 v2 = add2(fma2(pack2(__int2float_rn(acc0), __int2float_rn(acc1)), m2, zero2), b2);   // fl(fl(acc * m) + b)
+    f32x2 v2 = add2(fma2(pack2(__int2float_rn(acc0), __int2float_rn(acc1)), m2, zero2), b2);         // fl(fl(acc * m) + b)
+    {
+        float v0, v1, nsy, unused;
+        unpack2(v2, v0, v1); unpack2(sy2n, nsy, unused);
+        const float most = __fmul_rn(nsy, -16777216.0f);
+        v2 = pack2(fminf(fmaxf(v0, -most), most), fminf(fmaxf(v1, -most), most));
+    }
     const f32x2 p2 = mul2(v2, inv2);
     const f32x2 q2 = fma2(fma2(p2, sy2n, v2), inv2, p2);
     const f32x2 n2 = sub2(add2(q2, magic2), magic2);
@@ -399,6 +413,22 @@ __device__ __forceinline__ float epi_make_bq(float b, int cc, float m, float sy,
     const float rem = __fadd_rn(__fmaf_rn(-q0, sy, hi), lo);
     const float q = __fmaf_rn(rem, inv_sy, q0);
     return __fadd_rn(q, zoff);
+}
+
+__device__ __forceinline__ float max4_nan(float a, float b, float c, float d)      // NaN if any of them is
+{
+    float m;
+    asm("{ .reg .f32 t; max.NaN.f32 t, %1, %2, %3; max.NaN.f32 %0, t, %4; }" : "=f"(m) : "f"(a), "f"(b), "f"(c), "f"(d));
+    return m;
+}
+
+// max(m, |v|) of the magnitudes that a rounding bound is made of.  NaN and infinity, which fmaxf would drop and the hot path
+// cannot work with, become 0 in v and a huge bound, which sends every value to the reference's arithmetic.
+constexpr float BOUND_HUGE = 3.0e38f;
+__host__ __device__ __forceinline__ float bound_max(float m, float& v)
+{
+    if (!(fabsf(v) <= BOUND_HUGE)) { v = 0.f; return BOUND_HUGE; }
+    return fmaxf(m, fabsf(v));
 }
 
 // Programmatic dependent launch.  A grid launched with launch_pdl may be scheduled while its predecessor in the stream

@@ -541,7 +541,7 @@ __device__ __noinline__ uint32_t epi_fix_group(int a0, int a1, int a2, int a3, u
     const float2 t01 = __fadd2_rn(q01, ec.magic2), t23 = __fadd2_rn(q23, ec.magic2);
     const float2 n01 = __fadd2_rn(t01, ec.nmagic2), n23 = __fadd2_rn(t23, ec.nmagic2);
     const float2 d01 = __ffma2_rn(n01, ec.neg2, q01), d23 = __ffma2_rn(n23, ec.neg2, q23);
-    const float dmax = fmaxf(fmaxf(fabsf(d01.x), fabsf(d01.y)), fmaxf(fabsf(d23.x), fabsf(d23.y)));
+    const float dmax = max4_nan(fabsf(d01.x), fabsf(d01.y), fabsf(d23.x), fabsf(d23.y));
     const float2 z01 = __fadd2_rn(t01, zoff2), z23 = __fadd2_rn(t23, zoff2);
     const float z[4] = {z01.x, z01.y, z23.x, z23.y};
     uint32_t bits[4];
@@ -557,7 +557,7 @@ __device__ __noinline__ uint32_t epi_fix_group(int a0, int a1, int a2, int a3, u
     }
     uint32_t out = __byte_perm(__byte_perm(bits[0], bits[1], 0x0040), __byte_perm(bits[2], bits[3], 0x0040), 0x5410);
     if (!(dmax < 0.5f) || x->always) {
-        // (no usable table, an exact half, or a value too large for the constant)
+        // (no usable table, an exact half, or a value too large for the constant or, as NaN, for the quotient)
         out = 0;
         #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -960,7 +960,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const int ch = min(n0 + j, a.OC - 1);           // columns beyond OC are padding: any finite constants do
                     const float m = __fmul_rn(a.rq.sx, a.w_scales ? a.w_scales[ch] : a.w_scale);
                     s_m[j] = m;
-                    s_mq[j] = __fdiv_rn(m, a.rq.sy);
+                    float mq = __fdiv_rn(m, a.rq.sy);
+                    if (bound_max(0.f, mq) == BOUND_HUGE) bq_max = BOUND_HUGE;
+                    s_mq[j] = mq;
                     s_bterm[j] = a.bias ? __fmul_rn(__int2float_rn(a.bias[ch]), a.b_scales ? a.b_scales[ch] : a.b_scale) : 0.f;
                 }
                 for (int i = etid; i < a.ncls * BN; i += 32 * TC_EPI_WARPS) {
@@ -980,14 +982,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     // (recomputed rather than read back: another thread wrote s_m[j] and s_bterm[j])
                     const float m = __fmul_rn(a.rq.sx, a.w_scales ? a.w_scales[ch] : a.w_scale);
                     const float b = a.bias ? __fmul_rn(__int2float_rn(a.bias[ch]), a.b_scales ? a.b_scales[ch] : a.b_scale) : 0.f;
-                    const float bq = epi_make_bq(b, v, m, a.rq.sy, a.inv_sy, zoff);
+                    float bq = epi_make_bq(b, v, m, a.rq.sy, a.inv_sy, zoff), by = __fmul_rn(b, a.inv_sy);
+                    bq_max = bound_max(bq_max, bq);
+                    bsy_max = bound_max(bsy_max, by);
                     s_bq[i] = bq;
-                    bq_max = fmaxf(bq_max, fabsf(bq));
-                    bsy_max = fmaxf(bsy_max, fabsf(__fmul_rn(b, a.inv_sy)));
                 }
-                // (NaN or infinity anywhere turns into a huge bound: no hot path for this n-tile)
-                const uint32_t w0 = __reduce_max_sync(0xffffffffu, __float_as_uint(bq_max <= 3.0e38f ? bq_max : 3.0e38f));
-                const uint32_t w1 = __reduce_max_sync(0xffffffffu, __float_as_uint(bsy_max <= 3.0e38f ? bsy_max : 3.0e38f));
+                // (NaN or infinity anywhere has turned into a huge bound: no hot path for this n-tile)
+                const uint32_t w0 = __reduce_max_sync(0xffffffffu, __float_as_uint(bq_max));
+                const uint32_t w1 = __reduce_max_sync(0xffffffffu, __float_as_uint(bsy_max));
                 if (lane == 0) { atomicMax(&emax[0], w0); atomicMax(&emax[1], w1); }
                 epi_barrier();
                 {
@@ -1862,14 +1864,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
                 const float b = a.bias ? __fmul_rn(__int2float_rn(a.bias[j]), a.b_scales ? a.b_scales[j] : a.b_scale) : 0.f;
                 const int cc = a.zx * a.wsum[j];
                 s_m[j] = m; s_bterm[j] = b; s_cc[j] = cc;
-                s_mq[j] = __fdiv_rn(m, a.rq.sy);
-                const float bq = epi_make_bq(b, cc, m, a.rq.sy, a.inv_sy, zy1);
+                float mq = __fdiv_rn(m, a.rq.sy), bq = epi_make_bq(b, cc, m, a.rq.sy, a.inv_sy, zy1), by = __fmul_rn(b, a.inv_sy);
+                if (bound_max(0.f, mq) == BOUND_HUGE) bq_max = BOUND_HUGE;
+                bq_max = bound_max(bq_max, bq);
+                bsy_max = bound_max(bsy_max, by);
+                s_mq[j] = mq;
                 s_bq[j] = bq;
-                bq_max = fmaxf(bq_max, fabsf(bq));
-                bsy_max = fmaxf(bsy_max, fabsf(__fmul_rn(b, a.inv_sy)));
             }
-            const uint32_t w0 = __reduce_max_sync(0xffffffffu, __float_as_uint(bq_max <= 3.0e38f ? bq_max : 3.0e38f));
-            const uint32_t w1 = __reduce_max_sync(0xffffffffu, __float_as_uint(bsy_max <= 3.0e38f ? bsy_max : 3.0e38f));
+            const uint32_t w0 = __reduce_max_sync(0xffffffffu, __float_as_uint(bq_max));
+            const uint32_t w1 = __reduce_max_sync(0xffffffffu, __float_as_uint(bsy_max));
             if (lane == 0) { atomicMax(&s_emax[0], w0); atomicMax(&s_emax[1], w1); }
         }
         epi_barrier();
@@ -2200,14 +2203,15 @@ static bool host_tables_for(const b200k_conv2d_params* p, const TcArgs& a, TcTab
         const float m = sx * (p->w.scales ? hp->ws[ch] : p->w.scale);
         const float b = p->bias.data ? (float)hp->bias_v[ch] * (p->bias.scales ? hp->bs[ch] : p->bias.scale) : 0.f;
         const int cc = a.need_corr ? a.zx * hp->wsum[ch] - p->kh * p->kw * a.kvalid_c * a.zx * a.zw : 0;
-        tabs->mq[ch] = m / sy;
-        const float bq = host_make_bq(b, cc, m, sy, inv_sy, zoff);
+        float mq = m / sy, bq = host_make_bq(b, cc, m, sy, inv_sy, zoff), by = b * inv_sy;
+        bq_max = bound_max(bq_max, bq);
+        bsy_max = bound_max(bsy_max, by);
+        if (bound_max(0.f, mq) == BOUND_HUGE) bq_max = BOUND_HUGE;
+        tabs->mq[ch] = mq;
         tabs->bq[ch] = bq;
-        bq_max = fmaxf(bq_max, fabsf(bq));
-        bsy_max = fmaxf(bsy_max, fabsf(b * inv_sy));
     }
     for (int ch = p->oc; ch < TC_PTAB_MAX; ++ch) { tabs->mq[ch] = 0.f; tabs->bq[ch] = 0.f; }
-    if (!(bq_max <= 3.0e38f) || !(bsy_max <= 3.0e38f)) return false;
+    if (bq_max == BOUND_HUGE || bsy_max == BOUND_HUGE) return false;
     const float rz = 257.0f;
     const float rmax = fmaxf(fabsf(a.rq.tlo - 1.0f - zy1), fabsf(a.rq.thi + 1.0f - zy1));
     const float big = a.acc_big ? 1.0f : 0.0f;

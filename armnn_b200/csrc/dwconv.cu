@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(256, 2) dw3x3_rows_kernel(const __grid_constan
         }
         mq01 = pack2(mq[0], mq[1]); mq23 = pack2(mq[2], mq[3]);
         bq01 = pack2(bq[0], bq[1]); bq23 = pack2(bq[2], bq[3]);
-        // (a 3 x 3 accumulator is below 2^24: its conversion to fp32 is exact.  NaN or infinity anywhere: no hot path.)
+        // (A 3 x 3 accumulator is below 2^24: its conversion to fp32 is exact.  Where bq is NaN, bsy is infinite: no hot path.  An
+        // infinite mq or q" leaves a NaN in d.)
         const float e = 1.1f * 5.9604645e-8f * (a3.e_const + 1.0001f * bsy + 3.0f * bqm);
         thr = !(e < 0.0625f) ? 0.0f : 0.5f - e;
     }
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(256, 2) dw3x3_rows_kernel(const __grid_constan
             const f32x2 d01 = sub2(q01, n01), d23 = sub2(q23, n23);                                      // q" - n (exact)
             float d0, d1, d2, d3, z0, z1, z2, z3;
             unpack2(d01, d0, d1); unpack2(d23, d2, d3);
-            dw[s] = fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(d2), fabsf(d3)));
+            dw[s] = max4_nan(fabsf(d0), fabsf(d1), fabsf(d2), fabsf(d3));                                // (overflow: inf - inf)
             unpack2(n01, z0, z1); unpack2(n23, z2, z3);
             if (!FULL) { z0 = fminf(z0, span); z1 = fminf(z1, span); z2 = fminf(z2, span); z3 = fminf(z3, span); }
             int i0, i1, i2, i3;
@@ -408,12 +409,12 @@ __global__ void __launch_bounds__(256, 2) dw3x3_rows_kernel(const __grid_constan
             asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(i1), "r"(i0), "r"(hi16));
             outw[s] = (w + lo4) ^ flip4;
         }
-        if (fmaxf(fmaxf(dw[0], dw[1]), fmaxf(dw[2], dw[3])) >= thr || dump) {
+        if (!(max4_nan(dw[0], dw[1], dw[2], dw[3]) < thr) || dump) {
             // (rare) some value is too close to a rounding boundary for the hot path to vouch for: the reference chain
             // for its word of four channels; and the accumulator dump of the tests
             #pragma unroll
             for (int s = 0; s < DWR_S; ++s) {
-                if (dw[s] >= thr) {
+                if (!(dw[s] < thr)) {
                     const f32x2 nsy2 = pack2(-a.rq.sy, -a.rq.sy), inv2 = pack2(a3.inv_sy, a3.inv_sy), zy2 = pack2((float)a.rq.zy, (float)a.rq.zy);
                     const f32x2 m01 = pack2(s_mb[0][threadIdx.x], s_mb[1][threadIdx.x]), m23 = pack2(s_mb[2][threadIdx.x], s_mb[3][threadIdx.x]);
                     const f32x2 b01 = pack2(s_mb[4][threadIdx.x], s_mb[5][threadIdx.x]), b23 = pack2(s_mb[6][threadIdx.x], s_mb[7][threadIdx.x]);
@@ -546,7 +547,7 @@ extern "C" int b200k_dwconv2d_q8(const b200k_conv2d_params* p, void* stream)
     const uintptr_t al = (uintptr_t)a.x | (uintptr_t)a.w | (uintptr_t)a.y;
     cudaStream_t s = (cudaStream_t)stream;
     if (a.dm == 1 && a.KH == 3 && a.KW == 3 && a.dh == 1 && a.dw == 1 && a.sh == a.sw && (a.sh == 1 || a.sh == 2) &&
-        (a.C % 4) == 0 && (al & 3) == 0) {
+        (a.C % 4) == 0 && (al & 3) == 0 && ordinary_quant(p->y)) {
         const int zw_eff = a.zw - (a.w_u8 ? 128 : 0);
         if (zw_eff >= -127 && zw_eff <= 127 && ((long long)p->n * p->h + 4) * (p->wd + 4) * p->c < (1ll << 31) &&
             (long long)p->n * p->oh * p->ow * p->oc < (1ll << 31)) {

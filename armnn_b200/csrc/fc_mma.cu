@@ -165,7 +165,7 @@ bool fc_mma_eligible(const b200k_fc_params* p)
     if (!is_q8(p->x.dtype) || !is_q8(p->w.dtype) || !is_q8(p->y.dtype)) return false;
     if (p->bias.data && p->bias.dtype != B200K_S32) return false;
     if (p->w.scales && p->w.zero_point != 0) return false;
-    if (!ordinary_scale(p->y.scale)) return false;
+    if (!ordinary_quant(p->y)) return false;
     return (p->m + FM_T - 1) / FM_T <= 65535;
 }
 

@@ -287,7 +287,7 @@ bool fc_stream_eligible(const b200k_fc_params* p)
     if (!is_q8(p->x.dtype) || !is_q8(p->w.dtype) || !is_q8(p->y.dtype)) return false;
     if (p->bias.data && p->bias.dtype != B200K_S32) return false;
     if (((((uintptr_t)p->x.data) | ((uintptr_t)p->w.data)) & 15) != 0) return false;
-    if (p->w.scales && p->w.zero_point != 0) return false;
+    if ((p->w.scales && p->w.zero_point != 0) || !ordinary_quant(p->y)) return false;
     // the input rows and at least two one-row stages must fit
     const size_t pitch = (size_t)p->k + 64;
     return (size_t)(p->m + 2) * pitch + 16 * 1024 <= 227 * 1024 && (long long)p->k * 255 * 255 < (1ll << 31);

@@ -195,7 +195,7 @@ static bool fc_rows_eligible(const b200k_fc_params* p)
     if (!is_q8(p->x.dtype) || !is_q8(p->w.dtype) || !is_q8(p->y.dtype)) return false;
     if (p->bias.data && p->bias.dtype != B200K_S32) return false;
     if (p->k % 16 != 0 || ((((uintptr_t)p->x.data) | ((uintptr_t)p->w.data)) & 15) != 0) return false;
-    if (p->w.scales && p->w.zero_point != 0) return false;
+    if ((p->w.scales && p->w.zero_point != 0) || !ordinary_quant(p->y)) return false;
     return true;
 }
 

@@ -4,17 +4,20 @@ Sparse operands with values of 0 and +-1 put zero and overflowing quotients side
 import numpy as np
 import pytest
 
-from cases import S8, SimpleCase, _abi, qt, qt_out, run_case
+from cases import S8, U8, SimpleCase, _abi, qt, qt_out, run_case
+from q8util import ConvCase, FcCase
 
 pytestmark = pytest.mark.gpu
 
 # input scale, weight (second operand) scale, output scale
 ELT_SCALES = {"overflow": (1e20, 1e20, 1e-20), "half_way": (1e16, 1e3, 1e-16), "ordinary": (0.02, 0.03, 0.05), "tiny": (1e-20, 1e-20, 1e-20),
               "near_the_bound": (3e9, 3e9, 1e-20), "output_huge": (1e19, 1e18, 1e20)}
+MAC_SCALES = {"overflow": (1e20, 1.0, 1e-20), "some_overflow": (1e18, 1e18, 1.0), "tiny": (1e-15, 1e-15, 2e-30), "subnormal": (1e-20, 1e-19, 3e-39),
+              "output_huge": (1e16, 1e19, 1e35), "output_beyond_normal_reciprocals": (1e18, 2e19, 2e38), "ordinary": (0.02, 0.03, 0.002), "by_channel": (1e15, [1e15, 3e-35, 2e-35], 1e-20)}
 
 
-def _sparse(rng, shape):
-    return (rng.integers(0, 3, size=shape) == 0).astype(np.int8) * np.where(rng.integers(0, 2, size=shape) == 0, -1, 1).astype(np.int8)
+def _sparse(rng, shape, lo=-1):
+    return (rng.integers(0, 3, size=shape) == 0).astype(np.int8) * np.where(rng.integers(0, 2, size=shape) == 0, lo, 1).astype(np.int8)
 
 
 def _bytes(rng, shape):
@@ -59,6 +62,35 @@ def _bmm(scales, ty):
     return SimpleCase("batch_matmul_q8", build)
 
 
+def _conv(scales, c, oc, k, n=2, h=9, stride=1, depthwise=False, weights_u8=False, relu=False, add=False):
+    rng = np.random.default_rng(c * 100 + k)
+    x = _sparse(rng, (n, h, h, c))
+    w = _sparse(rng, (1, k, k, oc) if depthwise else (oc, k, k, c), lo=1 if weights_u8 else -1)
+    pad = (k // 2,) * 4
+    case = ConvCase(x, w.astype(np.uint8) if weights_u8 else w, None, (scales[0], 0), (scales[1], 0), (scales[2], 3), stride=(stride, stride), pad=pad,
+                    act=(1, 0., 0.) if relu else (0, 0., 0.), depthwise=depthwise, w_dtype=U8 if weights_u8 else S8)
+    if isinstance(scales[1], list):                          # by channel: next to each other a scale that overflows and one that does not
+        case.w_scales, case.w_q = np.resize(np.asarray(scales[1], np.float32), oc), (1.0, 0)
+    if add:
+        other = rng.integers(-128, 128, size=(n, case.oh, case.ow, oc)).astype(np.int8)
+        case.add = (other, (scales[2] * 0.8, -3), (scales[2], 1))
+    return case
+
+
+def _fc(scales, m, k, n):
+    rng = np.random.default_rng(m + n)
+    return FcCase(_sparse(rng, (m, k)), _sparse(rng, (n, k)), None, (scales[0], 0), (scales[1], 0), (scales[2], 3))
+
+
+MACS = {
+    "conv_tc": lambda s: _conv(s, 64, 64, 1), "conv_tc_3x3_relu": lambda s: _conv(s, 64, 64, 3, relu=True), "conv_tc_add": lambda s: _conv(s, 64, 128, 1, add=True),
+    "conv_grouped": lambda s: _conv(s, 16, 32, 1, n=8, h=8), "conv_stem": lambda s: _conv(s, 3, 64, 7, h=32, stride=2), "conv_dp4a": lambda s: _conv(s, 5, 7, 3),
+    "dw_rows": lambda s: _conv(s, 32, 32, 3, depthwise=True), "dw_rows_relu": lambda s: _conv(s, 32, 32, 3, stride=2, depthwise=True, relu=True),
+    "dw3x3": lambda s: _conv(s, 32, 32, 3, depthwise=True, weights_u8=True),
+    "fc_stream": lambda s: _fc(s, 4, 64, 48), "fc_rows": lambda s: _fc(s, 2, 48, 33), "fc_mma": lambda s: _fc(s, 40, 51, 33),
+}
+
+
 @pytest.mark.parametrize("scales", ELT_SCALES)
 @pytest.mark.parametrize("name,case", [("op%d" % op, lambda s, op=op: _eltwise(op, s)) for op in (0, 2, 3, 4, 5)] +
                          [("bilinear", lambda s: _resize(0, s)), ("nearest", lambda s: _resize(1, s)), ("bmm", lambda s: _bmm(s, False)), ("bmm_t", lambda s: _bmm(s, True))])
@@ -66,4 +98,12 @@ def test_values(built, name, case, scales):
     if name.startswith("bmm") and scales == "overflow":
         scales = "near_the_bound"                            # (the product of the scales is not a float)
     want, got = run_case(case(ELT_SCALES[scales]), "oracle"), run_case(case(ELT_SCALES[scales]), "gpu")
+    assert np.array_equal(want[0], got[0]), (name, scales, int((want[0] != got[0]).sum()), want[0].size)
+
+
+@pytest.mark.parametrize("name,scales", [(n, s) for n in MACS for s in MAC_SCALES if s != "by_channel" or n[:3] in ("con", "dw_")])
+def test_contractions(built, name, scales):
+    case = MACS[name](MAC_SCALES[scales])
+    want, got = case.run_oracle(), case.run_gpu()
+    assert np.array_equal(want[1], got[1])
     assert np.array_equal(want[0], got[0]), (name, scales, int((want[0] != got[0]).sum()), want[0].size)
