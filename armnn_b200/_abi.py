@@ -166,6 +166,10 @@ class ResizeParams(C.Structure):
 _P, _F, _I = C.c_void_p, C.c_float, C.c_int32
 
 
+class QLstmPlan(C.Structure):
+    _fields_ = [("scales", _F * 17), ("magnitudes", C.c_uint32 * 8 * 2 * 3)]
+
+
 class QLstmParams(C.Structure):
     _fields_ = [
         ("batch", _I), ("input_size", _I), ("num_units", _I), ("output_size", _I),
@@ -190,6 +194,7 @@ class QLstmParams(C.Structure):
         ("input_intermediate_scale", _F), ("forget_intermediate_scale", _F),
         ("cell_intermediate_scale", _F), ("output_intermediate_scale", _F),
         ("hidden_state_scale", _F), ("hidden_state_zp", _I),
+        ("plan", C.POINTER(QLstmPlan)),
     ]
 
 
@@ -246,7 +251,7 @@ KERNEL_ENTRY_POINTS = {
 EXPORTED_SYMBOLS = ["b200k_" + k for k in KERNEL_ENTRY_POINTS] + [
     "b200k_device_open", "b200k_device_count", "b200k_last_error", "b200k_version",
     "b200k_activation_clamp", "b200k_conv2d_pack_bytes", "b200k_conv2d_pack", "b200k_conv2d_scratch_bytes", "b200k_conv2d_q8_static", "b200k_sizeof_params", "b200k_poll_status",
-    "b200k_kernel_launches", "b200k_int8_mma_peak",
+    "b200k_kernel_launches", "b200k_int8_mma_peak", "b200k_qlstm_prepare",
 ]
 
 
@@ -270,6 +275,8 @@ def declare_product(lib):
     lib.b200k_conv2d_pack_bytes.restype = C.c_size_t
     lib.b200k_conv2d_pack.argtypes = [C.POINTER(Conv2dParams), C.c_void_p, C.c_void_p]
     lib.b200k_conv2d_pack.restype = C.c_int
+    lib.b200k_qlstm_prepare.argtypes = [C.POINTER(QLstmParams), C.POINTER(QLstmPlan)]
+    lib.b200k_qlstm_prepare.restype = C.c_int
     lib.b200k_poll_status.restype = C.c_int
     lib.b200k_int8_mma_peak.argtypes = [C.POINTER(C.c_double), C.c_void_p]
     lib.b200k_int8_mma_peak.restype = C.c_int

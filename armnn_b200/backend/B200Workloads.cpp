@@ -1050,12 +1050,18 @@ std::unique_ptr<IWorkload> MakeLstm(const QueueDescriptor& d, const WorkloadInfo
     });
 }
 
+struct QLstmState : SimpleState<b200k_qlstm_params>
+{
+    using SimpleState<b200k_qlstm_params>::SimpleState;
+    b200k_qlstm_plan plan;
+};
+
 // Device copies of the QLstm weights: the descriptor's ConstTensorHandles are released by the layer right after
 // CreateWorkload (src/armnn/LoadedNetwork.cpp:396), as RefQLstmWorkload's AssignScopedTensorHandle copies show.
 std::unique_ptr<IWorkload> MakeQLstm(const QueueDescriptor& d, const WorkloadInfo& info, const ContextPtr& ctx)
 {
     const auto& qd = *PolymorphicDowncast<const QLstmQueueDescriptor*>(&d);
-    auto st = std::make_shared<SimpleState<b200k_qlstm_params>>(ctx);
+    auto st = std::make_shared<QLstmState>(ctx);
     b200k_qlstm_params& p = st->p;
     std::memset(&p, 0, sizeof(p));
     const TensorInfo& x = info.m_InputTensorInfos[0];
@@ -1120,6 +1126,8 @@ std::unique_ptr<IWorkload> MakeQLstm(const QueueDescriptor& d, const WorkloadInf
     p.cell_intermediate_scale = prm.m_CellIntermediateScale;
     p.output_intermediate_scale = prm.m_OutputIntermediateScale;
     p.hidden_state_scale = prm.m_HiddenStateScale; p.hidden_state_zp = prm.m_HiddenStateZeroPoint;
+    B200CheckStatus(b200k_qlstm_prepare(&p, &st->plan));
+    p.plan = &st->plan;
     return Make<QLstmQueueDescriptor>(d, info, ctx, [st](const QLstmQueueDescriptor& data, cudaStream_t s)
     {
         b200k_qlstm_params& q = st->p;

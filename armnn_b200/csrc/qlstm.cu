@@ -774,47 +774,84 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
 
 // ---- host: which input magnitudes need the reference's arithmetic ----------------------------------------------------------
 
-// For one gate: r = |w| mag c over all weight magnitudes.  A function of the layer's scales alone, worked out once per set
-// of scales and kept in a small table (the oldest entry makes room).
-static QlDanger ql_danger_of(float sx, float sw, float sG)
+// For one gate: r = |w| mag c over all weight magnitudes.  r less its nearest integer through 1.5 * 2^52 (where that stops
+// being exact, from 2^51 on, the bound has long exceeded a half): 33 000 steps that vectorise, 45 us on a host core against
+// 130 with a conversion to an integer.
+static void ql_list_magnitudes(float sx, float sw, float sG, uint32_t* bits)
 {
-    struct Entry { float sx, sw, sG; bool used; QlDanger d; };
-    static Entry table[64];
-    static int next = 0;
+    const double c = (double)sx * (double)sw / (double)sG, unit = 1.0 / 16777216.0, magic = 6755399441055744.0;
+    for (int mag = 1; mag < 256; ++mag) {
+        int near = 0;
+        for (int w = 0; w <= 128; ++w) {
+            const double r = (double)(w * mag) * c, t = r - ((r + magic) - magic);
+            near |= 0.5 - fabs(t) <= (8.0 * r + 8.0 + 3.0 * QL_LEVEL) * unit;
+        }
+        if (near) bits[mag >> 5] |= 1u << (mag & 31);
+    }
+}
+
+// The scales of a layer that its plan depends on, gates i, f, c, o in turn (CIFG: the input gate's chains are repeats of the
+// forget gate's).
+static void ql_plan_scales(const b200k_qlstm_params* p, float* s)
+{
+    const bool cifg = p->w_i2i == nullptr;
+    const float all[17] = {p->input_scale, p->output_state_scale, p->hidden_state_scale, p->output_scale, p->w_proj ? p->s_proj : 1.f,
+                           cifg ? p->s_i2f : p->s_i2i, p->s_i2f, p->s_i2c, p->s_i2o, cifg ? p->s_r2f : p->s_r2i, p->s_r2f, p->s_r2c, p->s_r2o,
+                           cifg ? p->forget_intermediate_scale : p->input_intermediate_scale, p->forget_intermediate_scale,
+                           p->cell_intermediate_scale, p->output_intermediate_scale};
+    memcpy(s, all, sizeof(all));
+}
+// scales that the error bound holds for
+static bool ql_plan_ordinary(const b200k_qlstm_plan& plan)
+{
+    for (float s : plan.scales)
+        if (!(s >= 1e-8f && s <= 1e8f)) return false;
+    return true;
+}
+static void ql_make_plan(b200k_qlstm_plan& plan)             // from its scales
+{
+    memset(plan.magnitudes, 0, sizeof(plan.magnitudes));
+    if (!ql_plan_ordinary(plan)) return;
+    const float *s = plan.scales, *si = s + 5, *sr = s + 9, *sint = s + 13;
+    for (int g = 0; g < 4; ++g) {
+        ql_list_magnitudes(s[0], si[g], sint[g], plan.magnitudes[0][g & 1]);
+        ql_list_magnitudes(s[1], sr[g], sint[g], plan.magnitudes[1][g & 1]);
+    }
+    ql_list_magnitudes(s[2], s[4], s[3], plan.magnitudes[2][0]);
+}
+
+// Plans of the layers that are stepped without one of their own (a bounded table: the oldest makes room).
+static b200k_qlstm_plan ql_plan_for(const float* scales)
+{
+    static b200k_qlstm_plan table[256];
+    static int used = 0, next = 0;
     static std::mutex guard;
     {
         std::lock_guard<std::mutex> lock(guard);
-        for (const Entry& e : table)
-            if (e.used && e.sx == sx && e.sw == sw && e.sG == sG) return e.d;
+        for (int i = 0; i < used; ++i)
+            if (memcmp(table[i].scales, scales, sizeof(table[i].scales)) == 0) return table[i];
     }
-    const double c = (double)sx * (double)sw / (double)sG, unit = 1.0 / 16777216.0;
-    QlDanger d;
-    memset(&d, 0, sizeof(d));
-    for (int mag = 1; mag < 256; ++mag) {
-        double least = 1e300;                        // (distance from a half, less what does not depend on the accumulator) / unit
-        for (int w = 0; w <= 128; ++w) {
-            const double r = (double)(w * mag) * c;
-            const double near = fabs(r - (double)(long long)r - 0.5) / unit - 8.0 * r - 8.0;
-            least = near < least ? near : least;
-        }
-        if (least <= 3.0 * QL_LEVEL) d.bits[mag >> 5] |= 1u << (mag & 31);
-    }
+    b200k_qlstm_plan plan;
+    memcpy(plan.scales, scales, sizeof(plan.scales));
+    ql_make_plan(plan);
     std::lock_guard<std::mutex> lock(guard);
-    Entry& e = table[next];
-    next = (next + 1) & 63;
-    e.sx = sx; e.sw = sw; e.sG = sG; e.d = d; e.used = true;
-    return d;
-}
-static QlDanger ql_either(const QlDanger& a, const QlDanger& b)
-{
-    QlDanger d;
-    for (int i = 0; i < 8; ++i) d.bits[i] = a.bits[i] | b.bits[i];
-    return d;
+    table[next] = plan;
+    next = (next + 1) & 255;
+    if (used < 256) ++used;
+    return plan;
 }
 
 }  // namespace b200k
 
 using namespace b200k;
+
+extern "C" int b200k_qlstm_prepare(const b200k_qlstm_params* p, b200k_qlstm_plan* plan)
+{
+    B200K_REQUIRE(p && plan, B200K_E_INVALID, "qlstm_prepare: null params or plan");
+    ql_plan_scales(p, plan->scales);
+    ql_make_plan(*plan);
+    return B200K_OK;
+}
 
 extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
 {
@@ -837,23 +874,14 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
                   B200K_E_INVALID, "qlstm_step: layer norm needs all layer-norm weights and gate biases");
     B200K_REQUIRE(a.proj || p->num_units == p->output_size, B200K_E_INVALID,
                   "qlstm_step: without projection the output size must equal the number of units");
-    const float scales[] = {p->input_scale, p->output_state_scale, p->input_intermediate_scale, p->forget_intermediate_scale,
-                            p->cell_intermediate_scale, p->output_intermediate_scale, p->s_i2f, p->s_i2c, p->s_i2o, p->s_r2f, p->s_r2c, p->s_r2o,
-                            a.cifg ? 1.f : p->s_i2i, a.cifg ? 1.f : p->s_r2i, p->output_scale, a.proj ? p->s_proj : 1.f, p->hidden_state_scale};
+    float scales[17];
+    ql_plan_scales(p, scales);
+    const bool own = p->plan && memcmp(p->plan->scales, scales, sizeof(scales)) == 0;
+    const b200k_qlstm_plan plan = own ? *p->plan : ql_plan_for(scales);
     auto byte = [](int z) { return z >= -128 && z <= 127; };
-    a.exact_only = !byte(p->input_zp) || !byte(p->output_state_zp) || !byte(p->output_zp) || !byte(p->hidden_state_zp);
-    for (float s : scales) a.exact_only |= !(s >= 1e-8f && s <= 1e8f);
-    memset(a.danger, 0, sizeof(a.danger));
-    if (!a.exact_only) {
-        const float si[4] = {a.cifg ? p->s_i2f : p->s_i2i, p->s_i2f, p->s_i2c, p->s_i2o}, sr[4] = {a.cifg ? p->s_r2f : p->s_r2i, p->s_r2f, p->s_r2c, p->s_r2o};
-        const float sint[4] = {a.cifg ? p->forget_intermediate_scale : p->input_intermediate_scale, p->forget_intermediate_scale,
-                               p->cell_intermediate_scale, p->output_intermediate_scale};
-        for (int pr = 0; pr < 2; ++pr) {
-            a.danger[0][pr] = ql_either(ql_danger_of(p->input_scale, si[pr], sint[pr]), ql_danger_of(p->input_scale, si[pr + 2], sint[pr + 2]));
-            a.danger[1][pr] = ql_either(ql_danger_of(p->output_state_scale, sr[pr], sint[pr]), ql_danger_of(p->output_state_scale, sr[pr + 2], sint[pr + 2]));
-        }
-        if (a.proj) a.danger[2][0] = ql_danger_of(p->hidden_state_scale, p->s_proj, p->output_scale);
-    }
+    a.exact_only = !byte(p->input_zp) || !byte(p->output_state_zp) || !byte(p->output_zp) || !byte(p->hidden_state_zp) || !ql_plan_ordinary(plan);
+    static_assert(sizeof(a.danger) == sizeof(plan.magnitudes), "a plan holds what the kernel reads");
+    memcpy(a.danger, plan.magnitudes, sizeof(a.danger));
     auto aligned = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     a.vec_i = p->input_size % 16 == 0 && aligned(p->w_i2i) && aligned(p->w_i2f) && aligned(p->w_i2c) && aligned(p->w_i2o);
     a.vec_o = p->output_size % 16 == 0 && aligned(p->w_r2i) && aligned(p->w_r2f) && aligned(p->w_r2c) && aligned(p->w_r2o);

@@ -1625,6 +1625,9 @@ class GraphProgram:
         p.cell_intermediate_scale = d["CellIntermediateScale"]
         p.output_intermediate_scale = d["OutputIntermediateScale"]
         p.hidden_state_scale, p.hidden_state_zp = d["HiddenStateScale"], d["HiddenStateZeroPoint"]
+        plan = _abi.QLstmPlan()
+        lib.check(lib.load_library().b200k_qlstm_prepare(ctypes.byref(p), ctypes.byref(plan)))
+        p.plan = ctypes.pointer(plan)      # (the struct keeps the plan alive)
         return "qlstm_step", p
 
 

@@ -578,6 +578,15 @@ int b200k_cast_q(const b200k_convert_params* p, void* stream);
  * int16 gate buffers after every multiply-accumulate (LstmUtils.cpp:87-111).
  * Weight pointers are device pointers; a NULL pointer disables the corresponding option exactly as
  * the reference's m_CifgEnabled / m_PeepholeEnabled / m_ProjectionEnabled / m_LayerNormEnabled do. */
+
+/* What a step needs to know about a layer's scales beyond the scales themselves: the input magnitudes that can bring a product
+ * close to a rounding boundary.  A function of the scales alone (kept with them, so that a plan is never used for others), worked
+ * out by b200k_qlstm_prepare on the host in about half a millisecond: once per layer, when it is created.  Plain host memory. */
+typedef struct {
+    float    scales[17];
+    uint32_t magnitudes[3][2][8];    /* [input, recurrent, projection][gates i and c, gates f and o]: a bit per |q - zero point| */
+} b200k_qlstm_plan;
+
 typedef struct {
     int32_t batch, input_size, num_units, output_size;
     /* tensors */
@@ -602,9 +611,14 @@ typedef struct {
     float input_intermediate_scale, forget_intermediate_scale, cell_intermediate_scale,
           output_intermediate_scale;
     float hidden_state_scale; int32_t hidden_state_zp;
+    const b200k_qlstm_plan* plan;    /* host memory, read during the call; NULL or made for other scales: the library's own, of the
+                                      * last 256 layers stepped that way */
 } b200k_qlstm_params;
 
 int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream);
+
+/* Fills the plan of a layer (scales, descriptor values and which weights there are; p->plan is ignored).  No device is needed. */
+int b200k_qlstm_prepare(const b200k_qlstm_params* p, b200k_qlstm_plan* plan);
 
 /* One step of armnn::LstmImpl on Float32 tensors (src/backends/reference/workloads/Lstm.cpp:14-259 with LstmUtils.cpp;
  * the Lstm layer, and every time step of UnidirectionalSequenceLstm): gate pre-activations accumulated term by term in
