@@ -341,12 +341,12 @@ int launch_bmm_mma(const b200k_bmm_params* p, cudaStream_t stream)
     auto operand = [](bool kc, int rows) { return kc ? rows * BM_PITCH_K : BM_K * (rows + 8); };
     const size_t stages = (size_t)BM_STAGES * ((operand(!tx, BM_T) + operand(!ty, bn) + 15) & ~15), tile = (size_t)BM_T * (bn + 16);
     const size_t smem = stages > tile ? stages : tile;
-    auto go = [&](auto kern) -> int {
-        if (smem > 47 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_pdl(kern, grid, dim3(narrow ? 128 : 256), smem, stream, a);
+    auto go = [&](auto tag) -> int {
+        if (const int rc = allow_shared<decltype(tag)::kernel>(smem)) return rc;
+        launch_pdl(tag.kernel, grid, dim3(narrow ? 128 : 256), smem, stream, a);
         return check_launch("bmm_mma_kernel");
     };
-    #define B200K_BMM_WIDTH(TX, TY, XU, YU) (narrow ? go(bmm_mma_kernel<TX, TY, XU, YU, 2>) : go(bmm_mma_kernel<TX, TY, XU, YU, 4>))
+    #define B200K_BMM_WIDTH(TX, TY, XU, YU) (narrow ? go(KernelTag<bmm_mma_kernel<TX, TY, XU, YU, 2>>()) : go(KernelTag<bmm_mma_kernel<TX, TY, XU, YU, 4>>()))
     #define B200K_BMM_TYPES(TX, TY)                                                                                    \
         (xu ? (yu ? B200K_BMM_WIDTH(TX, TY, true, true) : B200K_BMM_WIDTH(TX, TY, true, false))                        \
             : (yu ? B200K_BMM_WIDTH(TX, TY, false, true) : B200K_BMM_WIDTH(TX, TY, false, false)))

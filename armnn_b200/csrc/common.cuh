@@ -5,6 +5,8 @@
 // intrinsics (no fused multiply-add, IEEE division), because the reference is built for baseline
 // x86-64 without FMA contraction (cmake/GlobalConfig.cmake:107,126 of the Arm NN tree).
 #pragma once
+#include <atomic>
+#include <mutex>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
@@ -34,6 +36,29 @@ inline int check_launch(const char* what)
     if (e != cudaSuccess) { set_error("launch of %s failed: %s", what, cudaGetErrorString(e)); return B200K_E_CUDA; }
     return B200K_OK;
 }
+
+// Opts a kernel into this much dynamic shared memory on the current device, where that is beyond what every launch may use.  The
+// driver is asked when a kernel first needs more than before, not on each launch.  The lock is for two threads whose launches
+// differ in size: the driver keeps the last size it was given, which must not be the smaller one.
+constexpr int MAX_DEVICES = 64;
+template <auto Kernel>
+inline int allow_shared(size_t bytes)
+{
+    static std::atomic<size_t> allowed[MAX_DEVICES];
+    static std::mutex guard;
+    if (bytes <= 40 * 1024) return B200K_OK;                 // (static shared memory comes on top)
+    int dev = 0;
+    B200K_CUDA(cudaGetDevice(&dev));
+    const bool known = dev >= 0 && dev < MAX_DEVICES;
+    if (known && bytes <= allowed[dev].load(std::memory_order_acquire)) return B200K_OK;
+    std::lock_guard<std::mutex> lock(guard);
+    if (known && bytes <= allowed[dev].load(std::memory_order_relaxed)) return B200K_OK;
+    B200K_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (known) allowed[dev].store(bytes, std::memory_order_release);
+    return B200K_OK;
+}
+// A kernel as an argument of a generic lambda that has to know it at compile time (for allow_shared).
+template <auto Kernel> struct KernelTag { static constexpr auto kernel = Kernel; };
 
 inline bool is_q8(int dtype) { return dtype == B200K_U8 || dtype == B200K_S8; }
 

@@ -299,8 +299,8 @@ static int launch_contract_f32(F32Args& a, int batch, bool conv, bool akc, bool 
     const long long big = ((a.M + 63) / 64) * ((a.N + 63) / 64) * batch;
     const int bm = big >= 148 ? 64 : 32, bn = bm;
     const size_t smem = ((size_t)a.CC * a.T * 2 * (bm + 4 + bn + 4) + 2 * (bm + 4)) * sizeof(float);   // and a slack row of each
-    auto go = [&](auto kern) -> int {
-        if (smem > 48 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto go = [&](auto tag) -> int {
+        if (const int rc = allow_shared<decltype(tag)::kernel>(smem)) return rc;
         // (more than 65535 batches or column tiles: several launches)
         F32Args q = a;
         for (int b0 = 0; b0 < batch; b0 += 65535)
@@ -308,7 +308,7 @@ static int launch_contract_f32(F32Args& a, int batch, bool conv, bool akc, bool 
                 q.x = a.x + b0 * a.bsa; q.w = a.w + b0 * a.bsb; q.y = a.y + b0 * a.bso;
                 q.n_off = (int)j0;
                 const long long cols = a.N - j0 < 65535ll * bn ? a.N - j0 : 65535ll * bn;
-                launch_pdl(kern, dim3(div_up(a.M, bm), div_up(cols, bn), (unsigned)(batch - b0 < 65535 ? batch - b0 : 65535)),
+                launch_pdl(tag.kernel, dim3(div_up(a.M, bm), div_up(cols, bn), (unsigned)(batch - b0 < 65535 ? batch - b0 : 65535)),
                            dim3(F32_THREADS), smem, s, q);
                 const int rc = check_launch("contract_f32_kernel");
                 if (rc) return rc;
@@ -317,15 +317,15 @@ static int launch_contract_f32(F32Args& a, int batch, bool conv, bool akc, bool 
     };
     #define B200K_F32_KERNELS(TM, TN)                                                                                  \
         do {                                                                                                           \
-            if (regs && conv && one) return go(contract_f32_kernel<TM, TN, true, true, true, true, true>);             \
-            if (regs && conv)        return go(contract_f32_kernel<TM, TN, true, true, true, false, true>);            \
-            if (regs)                return go(contract_f32_kernel<TM, TN, false, true, true, true, true>);            \
-            if (conv && one)         return go(contract_f32_kernel<TM, TN, true, true, true, true, false>);            \
-            if (conv)                return go(contract_f32_kernel<TM, TN, true, true, true, false, false>);           \
-            if (akc && bkc)          return go(contract_f32_kernel<TM, TN, false, true, true, true, false>);           \
-            if (akc)                 return go(contract_f32_kernel<TM, TN, false, true, false, true, false>);          \
-            if (bkc)                 return go(contract_f32_kernel<TM, TN, false, false, true, true, false>);          \
-            return go(contract_f32_kernel<TM, TN, false, false, false, true, false>);                                  \
+            if (regs && conv && one) return go(KernelTag<contract_f32_kernel<TM, TN, true, true, true, true, true>>()); \
+            if (regs && conv)        return go(KernelTag<contract_f32_kernel<TM, TN, true, true, true, false, true>>()); \
+            if (regs)                return go(KernelTag<contract_f32_kernel<TM, TN, false, true, true, true, true>>()); \
+            if (conv && one)         return go(KernelTag<contract_f32_kernel<TM, TN, true, true, true, true, false>>()); \
+            if (conv)                return go(KernelTag<contract_f32_kernel<TM, TN, true, true, true, false, false>>()); \
+            if (akc && bkc)          return go(KernelTag<contract_f32_kernel<TM, TN, false, true, true, true, false>>()); \
+            if (akc)                 return go(KernelTag<contract_f32_kernel<TM, TN, false, true, false, true, false>>()); \
+            if (bkc)                 return go(KernelTag<contract_f32_kernel<TM, TN, false, false, true, true, false>>()); \
+            return go(KernelTag<contract_f32_kernel<TM, TN, false, false, false, true, false>>());                     \
         } while (0)
     if (bm == 64) B200K_F32_KERNELS(4, 8);
     B200K_F32_KERNELS(4, 2);

@@ -1541,15 +1541,7 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     if (a2.bstat) a2.stage_tx = (uint32_t)(a.stage_tx - L::B_BYTES);
     const size_t smem = fixed + (size_t)stages * group * stride;
     auto kern = conv_tc_kernel<BN, SWZ, EG, PTAB>;
-    // per instantiation and device: the largest dynamic shared-memory size opted into so far (a racing second thread
-    // at worst repeats the call)
-    static std::atomic<size_t> configured[TC_MAX_DEVICES];
-    const int dev = current_device();
-    if (smem > configured[dev].load(std::memory_order_acquire)) {
-        B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        size_t seen = configured[dev].load(std::memory_order_relaxed);
-        while (seen < smem && !configured[dev].compare_exchange_weak(seen, smem, std::memory_order_release)) {}
-    }
+    if (const int rc = allow_shared<conv_tc_kernel<BN, SWZ, EG, PTAB>>(smem)) return rc;
     const long long tiles = (long long)a.ntn * a.ntm;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     // Programmatic dependent launch: the grid may start while its predecessor in the stream drains (its set-up touches

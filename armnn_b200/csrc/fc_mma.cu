@@ -10,7 +10,6 @@
 //
 // Zero points as in the other kernels: sum (x - zx)(w - zw) = sum x w - zw sum x - zx sum w + K zx zw, the row and column
 // sums from MMAs against ones.
-#include <atomic>
 #include "common.cuh"
 
 namespace b200k {
@@ -188,14 +187,13 @@ int launch_fc_mma(const b200k_fc_params* p, cudaStream_t stream)
     const size_t smem = operands > sums ? operands : sums;
     const bool vec = p->k % 16 == 0 && (((uintptr_t)p->x.data | (uintptr_t)p->w.data) & 15) == 0;
     const dim3 grid(div_up(p->n, FM_T), div_up(p->m, FM_T), 1);
-    auto go = [&](auto kern) -> int {
-        // (the opt-in is per device, and cheap)
-        if (smem > 47 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_pdl(kern, grid, dim3(FM_THREADS), smem, stream, a);
+    auto go = [&](auto tag) -> int {
+        if (const int rc = allow_shared<decltype(tag)::kernel>(smem)) return rc;
+        launch_pdl(tag.kernel, grid, dim3(FM_THREADS), smem, stream, a);
         return check_launch("fc_mma_kernel");
     };
     const bool xu = p->x.dtype == B200K_U8, wu = p->w.dtype == B200K_U8;
-    #define B200K_FC_MMA(XU, WU) (vec ? go(fc_mma_kernel<XU, WU, true>) : go(fc_mma_kernel<XU, WU, false>))
+    #define B200K_FC_MMA(XU, WU) (vec ? go(KernelTag<fc_mma_kernel<XU, WU, true>>()) : go(KernelTag<fc_mma_kernel<XU, WU, false>>()))
     if (xu) return wu ? B200K_FC_MMA(true, true) : B200K_FC_MMA(true, false);
     return wu ? B200K_FC_MMA(false, true) : B200K_FC_MMA(false, false);
     #undef B200K_FC_MMA

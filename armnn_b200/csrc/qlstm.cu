@@ -927,10 +927,10 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
     const size_t whole = a.tile_off + (size_t)p->output_size * (up16(p->num_units) + 16);
     a.proj_staged = a.proj && a.tile_off >= behind && whole <= limit;
     if (a.proj_staged && whole > smem) smem = whole;
-    auto launch = [&](auto kern) -> int {
-        if (smem > 40 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_pdl_cluster(kern, dim3((unsigned)((p->batch + rows - 1) / rows * cs)), dim3(QL_THREADS), smem, s, (unsigned)cs, a);
+    auto launch = [&](auto tag) -> int {
+        if (const int rc = allow_shared<decltype(tag)::kernel>(smem)) return rc;
+        launch_pdl_cluster(tag.kernel, dim3((unsigned)((p->batch + rows - 1) / rows * cs)), dim3(QL_THREADS), smem, s, (unsigned)cs, a);
         return check_launch("qlstm_step_kernel");
     };
-    return rows == 2 ? launch(qlstm_step_kernel<2>) : launch(qlstm_step_kernel<1>);
+    return rows == 2 ? launch(KernelTag<qlstm_step_kernel<2>>()) : launch(KernelTag<qlstm_step_kernel<1>>());
 }

@@ -336,32 +336,32 @@ static int launch_rows(const b200k_softmax_params* p, void* stream, int mode, co
         r.tlo = a.y.tlo; r.thi = a.y.thi;
         r.axis = p->axis_size; r.pitch = (p->axis_size + 27) / 32 * 32 + 4; r.rows = rows;
         const bool words = (p->axis_size & 3) == 0 && (((uintptr_t)p->x.data | (uintptr_t)p->y.data) & 3) == 0;
-        auto go = [&](auto kern, int warps) -> int {
+        auto go = [&](auto tag, int warps) -> int {
             const size_t bytes = ((size_t)warps * SMR_ROWS * r.pitch + CHAIN_SLACK) * sizeof(float);
-            if (bytes > 47 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-            launch_pdl(kern, dim3(div_up(rows, warps * SMR_ROWS)), dim3(32 * warps), bytes, s, r);
+            if (const int rc = allow_shared<decltype(tag)::kernel>(bytes)) return rc;
+            launch_pdl(tag.kernel, dim3(div_up(rows, warps * SMR_ROWS)), dim3(32 * warps), bytes, s, r);
             return check_launch("softmax_rows_kernel");
         };
         // 66 KiB of exponentials per block at most: three blocks per SM
         if (words) {
-            if (p->axis_size <= 128)  return go(softmax_rows_kernel<1, true, 8>, 8);
-            if (p->axis_size <= 512)  return go(softmax_rows_kernel<4, true, 8>, 8);
-            if (p->axis_size <= 1024) return go(softmax_rows_kernel<8, true, 4>, 4);
-            return go(softmax_rows_kernel<16, true, 2>, 2);
+            if (p->axis_size <= 128)  return go(KernelTag<softmax_rows_kernel<1, true, 8>>(), 8);
+            if (p->axis_size <= 512)  return go(KernelTag<softmax_rows_kernel<4, true, 8>>(), 8);
+            if (p->axis_size <= 1024) return go(KernelTag<softmax_rows_kernel<8, true, 4>>(), 4);
+            return go(KernelTag<softmax_rows_kernel<16, true, 2>>(), 2);
         }
-        if (p->axis_size <= 128)  return go(softmax_rows_kernel<1, false, 8>, 8);
-        if (p->axis_size <= 512)  return go(softmax_rows_kernel<4, false, 8>, 8);
-        if (p->axis_size <= 1024) return go(softmax_rows_kernel<8, false, 4>, 4);
-        return go(softmax_rows_kernel<16, false, 2>, 2);
+        if (p->axis_size <= 128)  return go(KernelTag<softmax_rows_kernel<1, false, 8>>(), 8);
+        if (p->axis_size <= 512)  return go(KernelTag<softmax_rows_kernel<4, false, 8>>(), 8);
+        if (p->axis_size <= 1024) return go(KernelTag<softmax_rows_kernel<8, false, 4>>(), 4);
+        return go(KernelTag<softmax_rows_kernel<16, false, 2>>(), 2);
     }
-    auto go = [&](auto kern) -> int {
-        if (smem > 47 * 1024) B200K_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_pdl(kern, dim3((unsigned)rows), dim3(SM_THREADS), smem, s, a);
+    auto go = [&](auto tag) -> int {
+        if (const int rc = allow_shared<decltype(tag)::kernel>(smem)) return rc;
+        launch_pdl(tag.kernel, dim3((unsigned)rows), dim3(SM_THREADS), smem, s, a);
         return check_launch("softmax_kernel");
     };
-    if (mode == ROW_SOFTMAX)     return go(softmax_kernel<ROW_SOFTMAX>);
-    if (mode == ROW_LOG_SOFTMAX) return go(softmax_kernel<ROW_LOG_SOFTMAX>);
-    return go(softmax_kernel<ROW_L2_NORM>);
+    if (mode == ROW_SOFTMAX)     return go(KernelTag<softmax_kernel<ROW_SOFTMAX>>());
+    if (mode == ROW_LOG_SOFTMAX) return go(KernelTag<softmax_kernel<ROW_LOG_SOFTMAX>>());
+    return go(KernelTag<softmax_kernel<ROW_L2_NORM>>());
 }
 
 extern "C" int b200k_softmax_q8(const b200k_softmax_params* p, void* stream)
