@@ -37,10 +37,25 @@ inline int check_launch(const char* what)
     return B200K_OK;
 }
 
+// What CUDA keeps per device (the number of SMs, a kernel's shared-memory limit) is remembered per device: a process may drive
+// several GPUs, one network and one host thread each.
+constexpr int MAX_DEVICES = 64;
+inline int sm_count()
+{
+    static std::atomic<int> counts[MAX_DEVICES];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) dev = 0;
+    n = counts[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        counts[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // Opts a kernel into this much dynamic shared memory on the current device, where that is beyond what every launch may use.  The
 // driver is asked when a kernel first needs more than before, not on each launch.  The lock is for two threads whose launches
 // differ in size: the driver keeps the last size it was given, which must not be the smaller one.
-constexpr int MAX_DEVICES = 64;
 template <auto Kernel>
 inline int allow_shared(size_t bytes)
 {

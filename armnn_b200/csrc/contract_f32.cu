@@ -295,9 +295,12 @@ static int launch_contract_f32(F32Args& a, int batch, bool conv, bool akc, bool 
     const bool regs = akc && bkc && a.T <= F32_QUADS && (a.C & 3) == 0 && (((uintptr_t)a.x | (uintptr_t)a.w) & 15) == 0 &&
                       (a.a_row & 3) == 0 && (a.b_col & 3) == 0 && (a.bsa & 3) == 0 && (a.bsb & 3) == 0 && a.b_tap < (1 << 20);
     if (regs && !one) a.CC = a.T <= F32_QUADS / 2 ? (F32_QUADS / a.T >= 4 ? 16 : 8) : 4;
-    // the 64 x 64 tile (4 x 8 outputs per thread) where it gives every SM a CTA, else 32 x 32
+    // The 64 x 64 tile (4 x 8 outputs per thread) where it gives every SM a CTA, else 32 x 32.  Measured on both sides (us, 64
+    // against 32): matrices of K = 512 with 64 tiles of the large kind 30.9 / 29.4, 135 tiles 31.1 / 47.9, 160 tiles 54.5 / 59.3,
+    // 512 tiles 103 / 160; 3 x 3 convolutions with 49 tiles 26.7 / 19.3, 98 - 100 tiles 27.0 / 25.7 and 60.9 / 45.0, 147 tiles
+    // 31.9 / 31.8, 196 tiles 38.1 / 40.2: convolutions change sides at one CTA per SM, matrices already at about half of that.
     const long long big = ((a.M + 63) / 64) * ((a.N + 63) / 64) * batch;
-    const int bm = big >= 148 ? 64 : 32, bn = bm;
+    const int bm = big >= sm_count() ? 64 : 32, bn = bm;
     const size_t smem = ((size_t)a.CC * a.T * 2 * (bm + 4 + bn + 4) + 2 * (bm + 4)) * sizeof(float);   // and a slack row of each
     auto go = [&](auto tag) -> int {
         if (const int rc = allow_shared<decltype(tag)::kernel>(smem)) return rc;

@@ -1340,29 +1340,6 @@ static bool load_driver_entry_points()
     return true;
 }
 
-// State that CUDA keeps per device (SM count, the opt-in shared-memory size of a kernel) is cached per device: a
-// process may drive several GPUs, one network and one host thread each.
-constexpr int TC_MAX_DEVICES = 64;
-
-static int current_device()
-{
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= TC_MAX_DEVICES) dev = 0;
-    return dev;
-}
-
-static int sm_count()
-{
-    static std::atomic<int> cached[TC_MAX_DEVICES];
-    const int dev = current_device();
-    int n = cached[dev].load(std::memory_order_relaxed);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        cached[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
-
 // Tile width.  The kernel is persistent with one CTA per SM, and on the network shapes a tile's cost is its epilogue
 // (proportional to its columns) plus a fixed part, so the estimate of a launch is waves x (columns + fixed), with
 // waves = ceil(tiles / SMs): narrow tiles fill the SMs when there are few rows, wide tiles win when there are many
@@ -2083,13 +2060,7 @@ static int launch_conv_stem(const b200k_conv2d_params* p, cudaStream_t stream)
         a.ep.hi = TC_MAGIC + hi1;
     }
     a.wait_limit = TC_WAIT_LIMIT_CYCLES;
-    static std::atomic<bool> configured[TC_MAX_DEVICES];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= TC_MAX_DEVICES) dev = 0;
-    if (!configured[dev].load(std::memory_order_acquire)) {
-        B200K_CUDA(cudaFuncSetAttribute(conv_stem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        configured[dev].store(true, std::memory_order_release);
-    }
+    if (const int rc = allow_shared<conv_stem_kernel>(227 * 1024)) return rc;
     const int sms = sm_count();
     const int grid = a.tiles < sms ? a.tiles : sms;
     launch_pdl(conv_stem_kernel, dim3((unsigned)grid), dim3(ST_THREADS), pl.smem, stream, a);
@@ -2387,7 +2358,10 @@ int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid
         const CUtensorMapSwizzle usw = uw == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
         // Epilogue groups: with one n-tile and no fused Add, 256 / bn (at most 4) tiles are in the epilogue at once, each
         // on its own accumulator buffer and a quarter (half) of the epilogue warps.  (Measured on ResNet-50's layers at
-        // batch 256: 1x1 and 3x3 convolutions with 64 or 128 output channels run 10 - 30 % faster this way.)
+        // batch 256: 1x1 and 3x3 convolutions with 64 or 128 output channels run 10 - 30 % faster this way.  With 64 columns and
+        // at most one tile per CTA, where only one group has work, a single group would be 8 - 17 % faster by itself - 56 x 56 x
+        // 64, 3 x 3: 5.6 us against 6.1 - and ResNet-50 at batch 3 and MobileNet-v2 at batch 1 measure the same either way; with
+        // 128 columns there is no difference.)
         a.eg = (a.ntn == 1 && !fa.res && !row_mode) ? (bn == 64 ? 4 : (bn == 128 ? 2 : 1)) : 1;
         // row-window mode (network stems): two groups (0.41 -> 0.32 ms for ResNet-50's stem at batch 256; four were slower
         // than one there)

@@ -236,7 +236,6 @@ __global__ void __launch_bounds__(256) dwconv3x3_kernel(const Dw3Args a3)
 // |q" - rint(q")| >= 0.5 - E is redone with the reference chain (requant_fast2; its per-channel constants wait in
 // shared memory, one private slot per thread).
 constexpr int DWR_S = 4;
-constexpr long long DWR_MIN_THREADS = 148 * 512;    // a heuristic only: two blocks of threads per SM of a B200
 
 struct DwRowsArgs {
     DwArgs d;
@@ -563,11 +562,11 @@ extern "C" int b200k_dwconv2d_q8(const b200k_conv2d_params* p, void* stream)
             r.lo4 = 0x01010101u * (uint32_t)(int)(r.lo - a.rq.tlo);
             r.flip4 = p->y.dtype == B200K_U8 ? 0u : 0x80808080u;
             r.strips = (a.OW + DWR_S - 1) / DWR_S;
-            // output rows per thread: as many as leave every SM a few blocks of threads (an input row is then read
+            // output rows per thread: as many as leave every SM two blocks of threads (an input row is then read
             // (rows + 2) / rows times at stride 1)
             const long long per_row_threads = (long long)p->n * r.strips * (a.C / 4);
             int rows = 8;
-            while (rows > 1 && per_row_threads * ((a.OH + rows - 1) / rows) < DWR_MIN_THREADS) rows >>= 1;
+            while (rows > 1 && per_row_threads * ((a.OH + rows - 1) / rows) < sm_count() * 512ll) rows >>= 1;
             r.rows = rows;
             r.rowblocks = (a.OH + rows - 1) / rows;
             r.d.total = per_row_threads * r.rowblocks;

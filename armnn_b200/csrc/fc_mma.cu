@@ -5,8 +5,12 @@
 // instead: the whole K extent (up to FM_KT at a time) of the 64 operand rows is copied to shared memory at once - one
 // round trip to memory instead of one per K step - every warp multiplies each eighth 32-byte slice, and the partial sums meet
 // in shared memory.  The weights do not depend on the kernel before this one, so their copies start before the wait for it.
-// Bound by that round trip and the reduction: 200 x 1280 x 1001 takes 6.5 us against 25.2 us with a warp per output column
-// and dp4a, whose 32 CTA rows read every activation byte through the L1 once per eight columns.
+// Up to a few hundred rows bound by that round trip and the reduction: 200 x 1280 x 1001 takes 6.4 us against 25.3 us with a
+// warp per output column and dp4a, whose 32 CTA rows read every activation byte through the L1 once per eight columns.  Many
+// rows are bound by the operands' traffic from L2 (each is read again for every 32 rows or columns of the other) and, above
+// 1700 bytes of K per pass, by one CTA per SM whose copies and MMAs take turns: 4096 x 1280 x 1001 74 us, 4096 x 4096 x 1001
+// 231 us (146 TOP/s), 4096 x 4099 x 4099 1351 us; the dp4a kernels take 446, 1102 and 6767 us.  No size from 5 to 4096
+// rows is slower than there.
 //
 // Zero points as in the other kernels: sum (x - zx)(w - zw) = sum x w - zw sum x - zx sum w + K zx zw, the row and column
 // sums from MMAs against ones.

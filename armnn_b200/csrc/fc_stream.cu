@@ -21,7 +21,6 @@
 //
 // Every wait on an mbarrier is bounded: a wait that gives up raises a status word (b200k_poll_status) and the CTA
 // drains and returns.
-#include <atomic>
 #include "common.cuh"
 
 namespace b200k {
@@ -295,15 +294,7 @@ bool fc_stream_eligible(const b200k_fc_params* p)
 
 int launch_fc_stream(const b200k_fc_params* p, cudaStream_t stream)
 {
-    static std::atomic<int> sm_count[64];
-    static std::atomic<bool> configured[64][4];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-    int sms = sm_count[dev].load(std::memory_order_acquire);
-    if (sms == 0) {
-        B200K_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        sm_count[dev].store(sms, std::memory_order_release);
-    }
+    const int sms = sm_count();
     FsArgs a;
     a.x = (const uint8_t*)p->x.data; a.w = (const uint8_t*)p->w.data; a.bias = (const int32_t*)p->bias.data;
     a.y = (uint8_t*)p->y.data; a.acc_out = p->acc_out;
@@ -345,18 +336,13 @@ int launch_fc_stream(const b200k_fc_params* p, cudaStream_t stream)
     const int units = (p->n + a.R - 1) / a.R;
     const dim3 grid((unsigned)(units < sms ? units : sms));
     const bool xu = p->x.dtype == B200K_U8, wu = p->w.dtype == B200K_U8;
-    #define B200K_FS_LAUNCH(XU, WU, IDX)                                                                              \
-        do {                                                                                                          \
-            if (!configured[dev][IDX].load(std::memory_order_acquire)) {                                              \
-                B200K_CUDA(cudaFuncSetAttribute(fc_stream_kernel<XU, WU>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); \
-                configured[dev][IDX].store(true, std::memory_order_release);                                          \
-            }                                                                                                         \
-            launch_pdl(fc_stream_kernel<XU, WU>, grid, dim3(FS_THREADS), smem, stream, a);                            \
-        } while (0)
-    if (xu) { if (wu) B200K_FS_LAUNCH(true, true, 0); else B200K_FS_LAUNCH(true, false, 1); }
-    else    { if (wu) B200K_FS_LAUNCH(false, true, 2); else B200K_FS_LAUNCH(false, false, 3); }
-    #undef B200K_FS_LAUNCH
-    return check_launch("fc_stream_kernel");
+    auto go = [&](auto tag) -> int {
+        if (const int rc = allow_shared<decltype(tag)::kernel>(227 * 1024)) return rc;
+        launch_pdl(tag.kernel, grid, dim3(FS_THREADS), smem, stream, a);
+        return check_launch("fc_stream_kernel");
+    };
+    if (xu) return wu ? go(KernelTag<fc_stream_kernel<true, true>>()) : go(KernelTag<fc_stream_kernel<true, false>>());
+    return wu ? go(KernelTag<fc_stream_kernel<false, true>>()) : go(KernelTag<fc_stream_kernel<false, false>>());
 }
 
 // 0, or the code of the wait that gave up (1 producer / ring slot, 2 consumer / weights); resets the word

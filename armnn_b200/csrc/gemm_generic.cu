@@ -90,6 +90,9 @@ extern "C" int b200k_batch_matmul_q8(const b200k_bmm_params* p, void* stream)
 
 // ---- FullyConnected with [N, K] weights and at most FC_ROWS rows whose K the weight-streaming kernel cannot take
 //
+// (K a multiple of 16 but not of 64, or too long for its ring.)  fc_mma.cu, which takes more rows and every other K, needs 1.1 to
+// 1.5 times as long there: 1 x 1296 x 1001 2.9 us against 3.8, 4 x 4112 x 1001 6.0 against 8.5, 2 x 4112 x 4095 8.6 against 11.5;
+// only a short K under many columns is even (48 or 528 x 4095: 0.95 to 1.08).
 // A block owns FC_COLS output columns (one per warp) and all rows of x, which it stages in shared memory once.
 // A warp streams its weight row through registers 16 bytes per lane at a time and multiplies it with every staged row
 // (dp4a); the per-lane partial sums of the FC_ROWS rows are then reduced across the warp so that lane r ends up with

@@ -160,15 +160,7 @@ extern "C" int b200k_lstm_step_f32(const b200k_lstm_params* p, void* stream)
     // shared memory before anything is written, and a cell value is read and written by the same thread.
     const size_t smem = ((size_t)p->input_size + p->output_size + 5 * (size_t)p->num_units) * sizeof(float);
     B200K_REQUIRE(smem <= 200 * 1024, B200K_E_TOOBIG, "lstm_step_f32: %zu bytes of shared memory per row exceed 200 KiB", smem);
-    static thread_local int opted_device = -1;
-    if (smem > 48 * 1024) {
-        int dev = 0;
-        B200K_CUDA(cudaGetDevice(&dev));
-        if (opted_device != dev) {
-            B200K_CUDA(cudaFuncSetAttribute(lstm_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            opted_device = dev;
-        }
-    }
+    if (const int rc = allow_shared<lstm_step_kernel>(smem)) return rc;
     launch_pdl(lstm_step_kernel, dim3((unsigned)p->batch), dim3(LSTM_THREADS), smem, (cudaStream_t)stream, *p);
     return check_launch("lstm_step_kernel");
 }

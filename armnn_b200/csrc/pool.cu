@@ -266,7 +266,7 @@ extern "C" int b200k_pool2d_q8(const b200k_pool2d_params* p, void* stream)
     int vec = pick_vec(p->x, p->y, p->c);
     // few outputs with large windows (global average pooling): narrower vectors give more threads to hide the latency
     // of the window's loads
-    if (vec == 16 && (long long)p->n * p->oh * p->ow * (p->c / 16) < 148 * 1024) vec = 4;
+    if (vec == 16 && (long long)p->n * p->oh * p->ow * (p->c / 16) < sm_count() * 1024ll) vec = 4;
     a.total = (long long)p->n * p->oh * p->ow * (p->c / vec);
     cudaStream_t s = (cudaStream_t)stream;
     if (vec == 16 && p->pool_type == 0 && p->x.dtype == p->y.dtype && p->x.scale == p->y.scale &&

@@ -887,9 +887,7 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
     a.vec_o = p->output_size % 16 == 0 && aligned(p->w_r2i) && aligned(p->w_r2f) && aligned(p->w_r2c) && aligned(p->w_r2o);
     a.vec_p = p->num_units % 16 == 0 && aligned(p->w_proj);
     cudaStream_t s = (cudaStream_t)stream;
-    int dev = 0, sms = 0;
-    B200K_CUDA(cudaGetDevice(&dev));
-    B200K_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int sms = sm_count();
     // Two rows per pair of CTAs (each weight converted once for both) as soon as that fills most SMs; below, the units of one
     // row are spread over up to eight CTAs, so that a small batch still uses the machine.
     int rows = 1, cs = 1;
