@@ -48,7 +48,9 @@ constexpr float QL_ULP = 6.0e-8f;                // a little more than 2^-24
 constexpr int QL_GATE_SLACK = 64;                // floats behind the gate buffers (the projection factors are padded)
 constexpr float QL_MAGIC = 12582912.0f;          // 1.5 * 2^23
 
-// round_half_away(fl(v / scale)) without the division unit (inv = RN(1 / scale)): Markstein's correctly rounded quotient and
+// RN(1 / scale) for the quotients below; NaN, which sends them to the division, for a scale that they do not hold for
+__device__ __forceinline__ float ql_inverse(float scale) { return scale >= 1e-20f && scale <= 1e20f ? __frcp_rn(scale) : __int_as_float(0x7fffffff); }
+// round_half_away(fl(v / scale)) without the division unit (inv = ql_inverse(scale)): Markstein's correctly rounded quotient and
 // the 1.5 * 2^23 constant; exact halves, and whatever is not finite, go through the division.
 __device__ __forceinline__ float ql_round_div(float v, float scale, float inv)
 {
@@ -119,14 +121,18 @@ struct QlExact {
     float lo, hi;                                // clamp
     __device__ __forceinline__ void set(float sGa, float sGb, float swa, float swb, float l, float h)
     {
-        sG2 = pack2(sGa, sGb); nsG2 = pack2(-sGa, -sGb); iG2 = pack2(__frcp_rn(sGa), __frcp_rn(sGb)); sw2 = pack2(swa, swb);
+        sG2 = pack2(sGa, sGb); nsG2 = pack2(-sGa, -sGb); iG2 = pack2(ql_inverse(sGa), ql_inverse(sGb)); sw2 = pack2(swa, swb);
         lo = l; hi = h;
     }
-    __device__ __forceinline__ f32x2 quotient(f32x2 T, f32x2 w2, float x) const
+    // fl(acc * sG) + t, to be divided by sG
+    __device__ __forceinline__ f32x2 dividend(f32x2 T, f32x2 w2, float x) const
     {
         const f32x2 zero2 = pack2(0.f, 0.f), magic2 = pack2(QL_MAGIC, QL_MAGIC);
         const f32x2 t2 = fma2(fma2(w2, sw2, zero2), pack2(x, x), zero2);                      // fl(fl(w * sw) * x)
-        const f32x2 a2 = add2(fma2(sub2(T, magic2), sG2, zero2), t2);                         // fl(fl(acc * sG) + t)
+        return add2(fma2(sub2(T, magic2), sG2, zero2), t2);
+    }
+    __device__ __forceinline__ f32x2 quotient(f32x2 a2) const
+    {
         const f32x2 p2 = mul2(a2, iG2);
         return fma2(fma2(p2, nsG2, a2), iG2, p2);                                             // RN(a / sG)
     }
@@ -149,12 +155,17 @@ __device__ __noinline__ f32x2 ql_slow_block(f32x2 T, uint4 wa, uint4 wb, const f
     for (int j = 0; j < QL_BLOCK; j += 4) {
         #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const f32x2 q2 = ex.quotient(T, ql_weight_pair(ma[0], mb[0], i, woff2), x[j + i]);
+            const f32x2 a2 = ex.dividend(T, ql_weight_pair(ma[0], mb[0], i, woff2), x[j + i]), q2 = ex.quotient(a2);
             float qa, qb, na, nb;
             unpack2(q2, qa, qb);
             unpack2(sub2(add2(q2, magic2), magic2), na, nb);
-            if (!(fabsf(__fsub_rn(qa, na)) < 0.5f)) na = roundf(qa);
-            if (!(fabsf(__fsub_rn(qb, nb)) < 0.5f)) nb = roundf(qb);
+            const bool ha = !(fabsf(__fsub_rn(qa, na)) < 0.5f), hb = !(fabsf(__fsub_rn(qb, nb)) < 0.5f);
+            if (ha || hb) {                                  // (halves, and quotients that overflow on the way)
+                float aa, ab, sa, sb;
+                unpack2(a2, aa, ab); unpack2(ex.sG2, sa, sb);
+                if (ha) na = roundf(__fdiv_rn(aa, sa));
+                if (hb) nb = roundf(__fdiv_rn(ab, sb));
+            }
             T = add2(pack2(fminf(fmaxf(na, ex.lo), ex.hi), fminf(fmaxf(nb, ex.lo), ex.hi)), magic2);
         }
         ma[0] = ma[1]; ma[1] = ma[2]; ma[2] = ma[3];
@@ -255,7 +266,7 @@ __device__ __noinline__ f32x2 ql_resolve(f32x2 end, int notes, const QlNote* lis
             #pragma unroll
             for (int j = 1; j < 8; ++j)
                 if (j == k) { t = T[j]; next = T[j + 1]; w = w2[j]; }
-            const f32x2 q2 = e.quotient(add2(t, corr2), w, xf[pos + k]);
+            const f32x2 q2 = e.quotient(e.dividend(add2(t, corr2), w, xf[pos + k]));
             float qa, qb, na, nb;
             unpack2(q2, qa, qb);
             unpack2(sub2(add2(q2, magic2), magic2), na, nb);
@@ -553,7 +564,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     const int b = b0 + rank;
     if (rank >= R || b >= p.batch) return;
 
-    const float sc = p.cell_state_scale, isc = __frcp_rn(sc);
+    const float sc = p.cell_state_scale, isc = ql_inverse(sc);
     const int g0 = a.cifg ? 1 : 0;
     const int16_t* peep[4] = {p.w_c2i, p.w_c2f, nullptr, p.w_c2o};
     const float speep[4] = {p.s_c2i, p.s_c2f, 0.f, p.s_c2o};
@@ -596,7 +607,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
                 for (int u = tid; u < U; u += QL_THREADS) {
                     const float cv = cell_smem ? cell_smem[u] : (float)cell_in_global[(long long)b * U + u];
                     const float pv = __fmul_rn(__fmul_rn((float)peep[g][u], speep[g]), __fmul_rn(cv, sc));
-                    gate(g)[u] = q16f(__fadd_rn(__fmul_rn(gate(g)[u], sint[g]), pv), sint[g], __frcp_rn(sint[g]));
+                    gate(g)[u] = q16f(__fadd_rn(__fmul_rn(gate(g)[u], sint[g]), pv), sint[g], ql_inverse(sint[g]));
                 }
             }
             __syncthreads();
@@ -648,7 +659,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
                 float s = sint[g];
                 if (a.ln) {
                     if (u != tid) { lw[g] = lnw[g][u]; gb[g] = gbias[g][u]; }
-                    const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f), isln = __frcp_rn(sln);
+                    const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f), isln = ql_inverse(sln);
                     q = q16f(__fmul_rn(__fsub_rn(__fmul_rn(q, s), stat[g * 2]), stat[g * 2 + 1]), sln, isln);      // normalise
                     q = q16f(__fmul_rn(__fmul_rn((float)lw[g], slnw[g]), __fmul_rn(q, sln)), sln, isln);           // * weight
                     q = q16f(__fadd_rn(__fmul_rn(q, sln), __fmul_rn(__int2float_rn(gb[g]), sgb[g])), 1.f / 4096, 4096.f);        // + bias

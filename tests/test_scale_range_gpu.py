@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from cases import S8, U8, SimpleCase, _abi, qt, qt_out, run_case
-from q8util import ConvCase, FcCase
+from q8util import ConvCase, FcCase, diff_stats, random_qlstm_case
 
 pytestmark = pytest.mark.gpu
 
@@ -107,3 +107,22 @@ def test_contractions(built, name, scales):
     want, got = case.run_oracle(), case.run_gpu()
     assert np.array_equal(want[1], got[1])
     assert np.array_equal(want[0], got[0]), (name, scales, int((want[0] != got[0]).sum()), want[0].size)
+
+
+@pytest.mark.parametrize("projection", [False, True])
+@pytest.mark.parametrize("batch", [2, 90])
+def test_qlstm_products_that_overflow(built, batch, projection):
+    """A product over the gate's scale is infinite: the step saturates, in the direction of its sign."""
+    case = random_qlstm_case(batch, batch, 16, 20, 12 if projection else 20, layer_norm=False, projection=projection)
+    case.x, case.h = _sparse(np.random.default_rng(1), case.x.shape), _sparse(np.random.default_rng(2), case.h.shape)
+    case.s["input_scale"] = case.s["output_state_scale"] = 1e17
+    for g in "ifco":
+        case.s["s_i2" + g] = case.s["s_r2" + g] = 1e17
+        for k in ("w_i2" + g, "w_r2" + g):
+            case.w[k] = _sparse(np.random.default_rng(ord(g)), case.w[k].shape)
+    for g in ("input", "forget", "cell", "output"):
+        case.s[g + "_intermediate_scale"] = 2.0 ** -18
+    want, got = case.run_oracle(), case.run_gpu()
+    for w, g in zip(want, got):
+        st = diff_stats(w, g)                  # (exp and tanh: see test_shape_edges_gpu.py)
+        assert st["max_abs"] <= (2 if w.dtype == np.int16 else 1) and st["mismatch_frac"] <= 0.01, st
