@@ -39,23 +39,6 @@ struct BmmTcArgs {
     int s8;                                          // output type
 };
 
-template <bool AU, bool BU>
-__device__ __forceinline__ void bm_mma(int* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    if (AU && BU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else if (AU && !BU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else if (!AU && BU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // w[j] = four consecutive rows' bytes at k + j  ->  o[i] = row i's bytes at k .. k + 3
 __device__ __forceinline__ void bm_transpose4(const uint32_t* w, uint32_t* o)
 {
@@ -217,7 +200,7 @@ __global__ void __launch_bounds__(64 * WN, WN == 4 ? 2 : 4) bmm_mma_kernel(const
             for (int mi = 0; mi < 4; ++mi)
                 #pragma unroll
                 for (int ni = 0; ni < 4; ++ni)
-                    bm_mma<XU, YU>(acc[mi][ni], fa[mi][0], fa[mi][1], fa[mi][2], fa[mi][3], fb[ni][0], fb[ni][1]);
+                    mma_8bit<XU, YU>(acc[mi][ni], fa[mi][0], fa[mi][1], fa[mi][2], fa[mi][3], fb[ni][0], fb[ni][1]);
             if (a.zy != 0) {
                 #pragma unroll
                 for (int mi = 0; mi < 4; ++mi)

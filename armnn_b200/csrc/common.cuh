@@ -158,6 +158,18 @@ __device__ __forceinline__ int dp4a_mixed(uint32_t x, uint32_t w, int acc)
     return d;
 }
 
+// c (16 x 8, int32) += a (16 x 32) b (32 x 8) on 8-bit operands, each signed or unsigned: the fragments of a warp
+template <bool AU, bool BU>
+__device__ __forceinline__ void mma_8bit(int* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    #define B200K_MMA_8BIT(AT, BT)                                                                                     \
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32." AT "." BT ".s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};" \
+                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1))
+    if (AU) { if (BU) B200K_MMA_8BIT("u8", "u8"); else B200K_MMA_8BIT("u8", "s8"); }
+    else    { if (BU) B200K_MMA_8BIT("s8", "u8"); else B200K_MMA_8BIT("s8", "s8"); }
+    #undef B200K_MMA_8BIT
+}
+
 // Sixteen bytes from any address, the first n of them (zeros for the rest; n may be <= 0 or > 16): from the aligned words that
 // hold them, of which only those with at least one wanted byte are read.
 __device__ __forceinline__ uint4 load16_any(const uint8_t* p, int n)

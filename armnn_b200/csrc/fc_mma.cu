@@ -9,8 +9,8 @@
 // warp per output column and dp4a, whose 32 CTA rows read every activation byte through the L1 once per eight columns.  Many
 // rows are bound by the operands' traffic from L2 (each is read again for every 32 rows or columns of the other) and, above
 // 1700 bytes of K per pass, by one CTA per SM whose copies and MMAs take turns: 4096 x 1280 x 1001 74 us, 4096 x 4096 x 1001
-// 231 us (146 TOP/s), 4096 x 4099 x 4099 1351 us; the dp4a kernels take 446, 1102 and 6767 us.  No size from 5 to 4096
-// rows is slower than there.
+// 231 us (146 TOP/s), 4096 x 4099 x 4099 1351 us; the dp4a kernels take 446, 1102 and 6767 us.  No size measured from
+// 5 to 4096 rows is slower than with them.
 //
 // Zero points as in the other kernels: sum (x - zx)(w - zw) = sum x w - zw sum x - zx sum w + K zx zw, the row and column
 // sums from MMAs against ones.
@@ -31,23 +31,6 @@ struct FcMmaArgs {
     Requant rq;
     float inv_sy, lo, hi;
 };
-
-template <bool AU, bool BU>
-__device__ __forceinline__ void fm_mma(int* c, const uint32_t* a, uint32_t b0, uint32_t b1)
-{
-    if (AU && BU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-    else if (AU && !BU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-    else if (!AU && BU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-    else
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 // bytes [k0, k0 + kt) of 32 rows of a [rows, K] matrix from row r0 on, zeros beyond it; VEC: whole aligned 16-byte pieces
 template <bool VEC>
@@ -100,6 +83,7 @@ __global__ void __launch_bounds__(FM_THREADS) fc_mma_kernel(const FcMmaArgs a)
         __syncthreads();
         const int kend = min(a.kt, a.K - k0);
         for (int k = warp * 32; k < kend; k += 32 * FM_WARPS) {
+            constexpr uint32_t ones = 0x01010101u;
             uint32_t fa[2][4], fb[4][2];
             #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -115,15 +99,14 @@ __global__ void __launch_bounds__(FM_THREADS) fc_mma_kernel(const FcMmaArgs a)
             #pragma unroll
             for (int i = 0; i < 2; ++i)
                 #pragma unroll
-                for (int j = 0; j < 4; ++j) fm_mma<XU, WU>(acc[i][j], fa[i], fb[j][0], fb[j][1]);
+                for (int j = 0; j < 4; ++j) mma_8bit<XU, WU>(acc[i][j], fa[i][0], fa[i][1], fa[i][2], fa[i][3], fb[j][0], fb[j][1]);
             if (a.zw != 0) {
                 #pragma unroll
-                for (int i = 0; i < 2; ++i) fm_mma<XU, WU>(rsum[i], fa[i], 0x01010101u, 0x01010101u);
+                for (int i = 0; i < 2; ++i) mma_8bit<XU, WU>(rsum[i], fa[i][0], fa[i][1], fa[i][2], fa[i][3], ones, ones);
             }
             if (a.zx != 0) {
-                const uint32_t ones[4] = {0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u};
                 #pragma unroll
-                for (int j = 0; j < 4; ++j) fm_mma<XU, WU>(csum[j], ones, fb[j][0], fb[j][1]);
+                for (int j = 0; j < 4; ++j) mma_8bit<XU, WU>(csum[j], ones, ones, ones, ones, fb[j][0], fb[j][1]);
             }
         }
     }

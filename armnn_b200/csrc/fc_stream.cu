@@ -73,23 +73,6 @@ __device__ __forceinline__ uint4 fs_lds128(uint32_t addr)
     return v;
 }
 
-template <bool XU, bool WU>
-__device__ __forceinline__ void fs_mma(int* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    if (XU && WU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else if (XU && !WU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else if (!XU && WU)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 __device__ __forceinline__ void fs_consumer_barrier()
 {
     asm volatile("bar.sync 1, %0;" ::"n"(32 * FS_WARPS) : "memory");
@@ -218,10 +201,10 @@ __global__ void __launch_bounds__(FS_THREADS, 2) fc_stream_kernel(const FsArgs a
                     const uint4 xa1 = (second && row_a) ? fs_lds128(xa_addr + b2 * 64) : make_uint4(0, 0, 0, 0);
                     const uint4 xb1 = (second && row_b) ? fs_lds128(xb_addr + b2 * 64) : make_uint4(0, 0, 0, 0);
                     const uint4 wv1 = (second && wrow) ? fs_lds128(w_addr + b2 * 64) : make_uint4(0, 0, 0, 0);
-                    fs_mma<XU, WU>(acc[0], xa0.x, xb0.x, xa0.y, xb0.y, wv0.x, wv0.y);
-                    fs_mma<XU, WU>(acc[1], xa0.z, xb0.z, xa0.w, xb0.w, wv0.z, wv0.w);
-                    fs_mma<XU, WU>(acc[2], xa1.x, xb1.x, xa1.y, xb1.y, wv1.x, wv1.y);
-                    fs_mma<XU, WU>(acc[3], xa1.z, xb1.z, xa1.w, xb1.w, wv1.z, wv1.w);
+                    mma_8bit<XU, WU>(acc[0], xa0.x, xb0.x, xa0.y, xb0.y, wv0.x, wv0.y);
+                    mma_8bit<XU, WU>(acc[1], xa0.z, xb0.z, xa0.w, xb0.w, wv0.z, wv0.w);
+                    mma_8bit<XU, WU>(acc[2], xa1.x, xb1.x, xa1.y, xb1.y, wv1.x, wv1.y);
+                    mma_8bit<XU, WU>(acc[3], xa1.z, xb1.z, xa1.w, xb1.w, wv1.z, wv1.w);
                     if (a.zx != 0) {
                         wl = dp4a_mixed<WU, true>(wv0.x, 0x01010101u, wl); wl = dp4a_mixed<WU, true>(wv0.y, 0x01010101u, wl);
                         wl = dp4a_mixed<WU, true>(wv0.z, 0x01010101u, wl); wl = dp4a_mixed<WU, true>(wv0.w, 0x01010101u, wl);
