@@ -17,7 +17,7 @@ no collective on the data path).  Prints ONE JSON line on rank 0:
   roofline   conv2d_q8 (the dominant kernel): int8 ops / CUDA-event time against the int8 tensor peak measured on
              this device by an MMA-only kernel, plus the step's time against its binding roof (per layer
              max(ops / tensor peak, bytes / HBM bandwidth), summed)
-  cpu_baseline  the reference's CpuRef timed on this box's host cores on a bounded sample (N = 1 only)
+  cpu_baseline  the reference's CpuRef (kind "reference"), or where it is not built its C restatement (kind "port"), on this box's host cores, a bounded sample (N = 1 only)
 """
 import argparse
 import ctypes
@@ -150,12 +150,18 @@ def cpuref_images_per_s(steps, warmup, cores=None):
     mean = sum(per_step) / len(per_step)
     return {"value": cores / mean, "unit": "images/s", "cores": cores, "kind": kind,
             "sample": "%d timed step(s) after %d warm-up of 1 image per core (batch-1 ResNet-50 224x224 graph, %d "
-                      "single-threaded CpuRef instances in parallel)" % (steps, warmup, cores), "ms_per_step": mean * 1e3}
+                      "single-threaded %s instances in parallel)" % (steps, warmup, cores, "CpuRef" if kind == "reference" else "C restatement"),
+            "ms_per_step": mean * 1e3}
 
 
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    from armnn_b200 import armnn_host
+    if not armnn_host.available():
+        # (the C restatement that stands in for CpuRef as the host baseline is not the reference)
+        print(json.dumps({"impl": "reference", "unavailable": "the Arm NN runtime with CpuRef (libarmnn.so and its binding) is not built here"}), flush=True)
         return
     base = cpuref_images_per_s(args.steps, max(args.warmup, 0))
     line = {"impl": "reference", "metric": "int8 ResNet-50 images/s", "value": base["value"], "unit": "images/s",
