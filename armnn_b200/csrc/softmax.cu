@@ -224,7 +224,8 @@ __global__ void __launch_bounds__(32 * WARPS) softmax_rows_kernel(const RowsArgs
                 float z[4], d[4];
                 unpack2(z01, z[0], z[1]); unpack2(z23, z[2], z[3]);
                 unpack2(sub2(q01, z01), d[0], d[1]); unpack2(sub2(q23, z23), d[2], d[3]);
-                if (!(fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fmaxf(fabsf(d[2]), fabsf(d[3]))) < 0.499f)) {
+                // (an exponential that overflowed, as with a negative beta, leaves NaN)
+                if (!(max4_nan(fabsf(d[0]), fabsf(d[1]), fabsf(d[2]), fabsf(d[3])) < 0.499f)) {
                     z[0] = exact(v.x, s); z[1] = exact(v.y, s); z[2] = exact(v.z, s); z[3] = exact(v.w, s);
                 }
                 ((uint32_t*)y)[i] = sat_pack4(z, s8);

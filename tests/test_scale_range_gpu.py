@@ -6,6 +6,7 @@ import pytest
 
 from cases import S8, U8, SimpleCase, _abi, qt, qt_out, run_case
 from q8util import ConvCase, FcCase, diff_stats, random_qlstm_case
+from test_shape_edges_gpu import softmax
 
 pytestmark = pytest.mark.gpu
 
@@ -107,6 +108,15 @@ def test_contractions(built, name, scales):
     want, got = case.run_oracle(), case.run_gpu()
     assert np.array_equal(want[1], got[1])
     assert np.array_equal(want[0], got[0]), (name, scales, int((want[0] != got[0]).sum()), want[0].size)
+
+
+@pytest.mark.parametrize("rows,axis", [(2100, 64), (2100, 63), (3, 64)])
+def test_softmax_exponentials_that_overflow(built, rows, axis):
+    """beta < 0: the reference's exponentials and their sum are infinite, and infinity over infinity is not a number."""
+    case = softmax(rows, rows, axis, S8, beta=-40.0)
+    want, got = run_case(case, "oracle"), run_case(case, "gpu")
+    assert set(np.unique(want[0])) == {-128}
+    assert np.array_equal(want[0], got[0]), int((want[0] != got[0]).sum())
 
 
 @pytest.mark.parametrize("projection", [False, True])
