@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) pool2d_kernel(const PoolArgs a)
     store_vec_f<VEC>(a.y, oi, r);
 }
 
-// Max pooling whose input and output share type, scale and offset: dequantisation is monotone (scale > 0) and
+// Max pooling whose input and output share type, scale and offset: dequantisation is monotone and, for an ordinary scale,
 // Quantize(Dequantize(q)) == q, so the result is the maximum of the quantised bytes themselves — SIMD byte maxima, no
 // floating point.  A window with no valid tap yields Quantize(lowest float) = the type minimum, a padding-only window
 // Quantize(0) = the zero point, as in the general kernel.
@@ -269,8 +269,10 @@ extern "C" int b200k_pool2d_q8(const b200k_pool2d_params* p, void* stream)
     if (vec == 16 && (long long)p->n * p->oh * p->ow * (p->c / 16) < sm_count() * 1024ll) vec = 4;
     a.total = (long long)p->n * p->oh * p->ow * (p->c / vec);
     cudaStream_t s = (cudaStream_t)stream;
+    int lo, hi;
+    type_range(p->x.dtype, lo, hi);
     if (vec == 16 && p->pool_type == 0 && p->x.dtype == p->y.dtype && p->x.scale == p->y.scale &&
-        p->x.zero_point == p->y.zero_point && p->x.scale > 0.f) {
+        p->x.zero_point == p->y.zero_point && ordinary_scale(p->x.scale) && p->x.zero_point >= lo && p->x.zero_point <= hi) {
         launch_pdl(maxpool_same_quant_kernel, dim3((unsigned)(div_up(a.total, 256))), dim3(256), 0, s, a);
         return check_launch("maxpool_same_quant_kernel");
     }

@@ -119,6 +119,25 @@ def test_softmax_exponentials_that_overflow(built, rows, axis):
     assert np.array_equal(want[0], got[0]), int((want[0] != got[0]).sum())
 
 
+@pytest.mark.parametrize("scale,zp", [(0.05, 7), (3e37, 0), (0.05, 300), (1e-39, -4)])
+def test_max_pooling_without_requantisation(built, scale, zp):
+    """Values that overflow when dequantised, and a zero point outside the type's range in windows that lie in the padding."""
+    def build(mem):
+        rng = np.random.default_rng(5)
+        p = _abi.Pool2dParams()
+        n, h, oh, c = 8, 284, 144, 16
+        p.x = qt(mem, rng.integers(0, 256, size=(n, h, h, c)).astype(np.uint8), U8, scale, zp)
+        p.y, y = qt_out(mem, (n, oh, oh, c), U8, scale, zp)
+        p.n, p.h, p.wd, p.c, p.oh, p.ow = n, h, h, c, oh, oh
+        p.pool_h = p.pool_w = p.stride_h = p.stride_w = 2
+        p.pad_top = p.pad_bottom = p.pad_left = p.pad_right = 2
+        p.pool_type, p.padding_method = 0, 1
+        return p, [y]
+    case = SimpleCase("pool2d_q8", build)
+    want, got = run_case(case, "oracle"), run_case(case, "gpu")
+    assert np.array_equal(want[0], got[0]), int((want[0] != got[0]).sum())
+
+
 @pytest.mark.parametrize("projection", [False, True])
 @pytest.mark.parametrize("batch", [2, 90])
 def test_qlstm_products_that_overflow(built, batch, projection):
