@@ -27,7 +27,7 @@
 //
 // Bound by the fp32 and integer pipes in the chains (about 60 % of the time at 512 units) and by the latency of the sequential
 // sums and of the projection's chains.  Three layers (40 or 256 -> 512 units -> 256) at batch 128: 475 us with one CTA per row and
-// the reference's arithmetic in every step, 310 us with blocks of eight steps, 283 us with 16 and both rows interleaved, 251 us
+// the reference's arithmetic in every step, 310 us with blocks of eight steps, 283 us with 16 and both rows interleaved, 255 us
 // since notes keep their weights.
 #include <mutex>
 #include <type_traits>
@@ -48,10 +48,9 @@ constexpr float QL_ULP = 6.0e-8f;                // a little more than 2^-24
 constexpr int QL_GATE_SLACK = 64;                // floats behind the gate buffers (the projection factors are padded)
 constexpr float QL_MAGIC = 12582912.0f;          // 1.5 * 2^23
 
-// RN(1 / scale) for the quotients below; NaN, which sends them to the division, for a scale that they do not hold for
-__device__ __forceinline__ float ql_inverse(float scale) { return scale >= 1e-20f && scale <= 1e20f ? __frcp_rn(scale) : __int_as_float(0x7fffffff); }
-// round_half_away(fl(v / scale)) without the division unit (inv = ql_inverse(scale)): Markstein's correctly rounded quotient and
-// the 1.5 * 2^23 constant; exact halves, and whatever is not finite, go through the division.
+// round_half_away(fl(v / scale)) without the division unit (inv = rn_reciprocal(scale), NaN where the quotient does not hold):
+// Markstein's correctly rounded quotient and the 1.5 * 2^23 constant; exact halves, and whatever is not finite, go through the
+// division.
 __device__ __forceinline__ float ql_round_div(float v, float scale, float inv)
 {
     const float p = __fmul_rn(v, inv);
@@ -81,6 +80,7 @@ struct QlArgs {
     int nbuf;                                    // weight tiles in shared memory: 1 or 2
     int proj_staged;                             // the projection weights fit the tiles' space
     unsigned tile_off;                           // where the weight tiles begin in shared memory
+    float inv_gate[4], inv_ln[4], inv_cell, inv_out;     // reciprocals of the scales that are divided by, gates i, f, c, o
     QlDanger danger[3][2];                       // [input, recurrent, projection][pair of gates: (i, c), (f, o)]
 };
 
@@ -119,9 +119,9 @@ __device__ __forceinline__ uint32_t ql_weights4(const int8_t* w, int k, int K)
 struct QlExact {
     f32x2 sG2, nsG2, iG2, sw2;
     float lo, hi;                                // clamp
-    __device__ __forceinline__ void set(float sGa, float sGb, float swa, float swb, float l, float h)
+    __device__ __forceinline__ void set(float sGa, float sGb, float iGa, float iGb, float swa, float swb, float l, float h)
     {
-        sG2 = pack2(sGa, sGb); nsG2 = pack2(-sGa, -sGb); iG2 = pack2(ql_inverse(sGa), ql_inverse(sGb)); sw2 = pack2(swa, swb);
+        sG2 = pack2(sGa, sGb); nsG2 = pack2(-sGa, -sGb); iG2 = pack2(iGa, iGb); sw2 = pack2(swa, swb);
         lo = l; hi = h;
     }
     // fl(acc * sG) + t, to be divided by sG
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     for (int i = tid; i < (int)(sizeof(s_danger) / 4); i += QL_THREADS) ((uint32_t*)s_danger)[i] = ((const uint32_t*)a.danger)[i];
     if (tid < 4) {
         const int src = tid >> 1, pr = tid & 1;
-        s_exact[src][pr].set(pr ? sint[1] : sint[0], pr ? sint[3] : sint[2], src ? (pr ? sr[1] : sr[0]) : (pr ? si[1] : si[0]),
+        s_exact[src][pr].set(pr ? sint[1] : sint[0], pr ? sint[3] : sint[2], a.inv_gate[pr], a.inv_gate[pr + 2], src ? (pr ? sr[1] : sr[0]) : (pr ? si[1] : si[0]),
                              src ? (pr ? sr[3] : sr[2]) : (pr ? si[3] : si[2]), -32768.f, 32767.f);
     }
 
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
     const int b = b0 + rank;
     if (rank >= R || b >= p.batch) return;
 
-    const float sc = p.cell_state_scale, isc = ql_inverse(sc);
+    const float sc = p.cell_state_scale, isc = a.inv_cell;
     const int g0 = a.cifg ? 1 : 0;
     const int16_t* peep[4] = {p.w_c2i, p.w_c2f, nullptr, p.w_c2o};
     const float speep[4] = {p.s_c2i, p.s_c2f, 0.f, p.s_c2o};
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
                 for (int u = tid; u < U; u += QL_THREADS) {
                     const float cv = cell_smem ? cell_smem[u] : (float)cell_in_global[(long long)b * U + u];
                     const float pv = __fmul_rn(__fmul_rn((float)peep[g][u], speep[g]), __fmul_rn(cv, sc));
-                    gate(g)[u] = q16f(__fadd_rn(__fmul_rn(gate(g)[u], sint[g]), pv), sint[g], ql_inverse(sint[g]));
+                    gate(g)[u] = q16f(__fadd_rn(__fmul_rn(gate(g)[u], sint[g]), pv), sint[g], a.inv_gate[g]);
                 }
             }
             __syncthreads();
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
                 float s = sint[g];
                 if (a.ln) {
                     if (u != tid) { lw[g] = lnw[g][u]; gb[g] = gbias[g][u]; }
-                    const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f), isln = ql_inverse(sln);
+                    const float sln = __fmul_rn(__fmul_rn(p.input_scale, slnw[g]), 1024.f), isln = a.inv_ln[g];
                     q = q16f(__fmul_rn(__fsub_rn(__fmul_rn(q, s), stat[g * 2]), stat[g * 2 + 1]), sln, isln);      // normalise
                     q = q16f(__fmul_rn(__fmul_rn((float)lw[g], slnw[g]), __fmul_rn(q, sln)), sln, isln);           // * weight
                     q = q16f(__fadd_rn(__fmul_rn(q, sln), __fmul_rn(__int2float_rn(gb[g]), sgb[g])), 1.f / 4096, 4096.f);        // + bias
@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qlstm_step_kernel(const __grid_
         for (int j = tid; j < O; j += QL_THREADS) finish(j, 0.f);
         return;
     }
-    if (tid == 0) s_exact[0][0].set(so, so, p.s_proj, p.s_proj, -32768.f - zo, 32767.f - zo);
+    if (tid == 0) s_exact[0][0].set(so, so, a.inv_out, a.inv_out, p.s_proj, p.s_proj, -32768.f - zo, 32767.f - zo);
     if (a.proj_staged && a.vec_p) ql_copy_wait<0>();
     __syncthreads();
     // two outputs, half of them apart, per thread; the chains run on acc - zo, an integer like the gates' accumulators
@@ -831,7 +831,8 @@ static void ql_make_plan(b200k_qlstm_plan& plan)             // from its scales
     ql_list_magnitudes(s[2], s[4], s[3], plan.magnitudes[2][0]);
 }
 
-// Plans of the layers that are stepped without one of their own (a bounded table: the oldest makes room).
+// The plans made last (a bounded table: the oldest makes room): a network that is loaded again, or several times, does not make
+// them again, and layers that are stepped without a plan of their own have theirs here.
 static b200k_qlstm_plan ql_plan_for(const float* scales)
 {
     static b200k_qlstm_plan table[256];
@@ -859,8 +860,9 @@ using namespace b200k;
 extern "C" int b200k_qlstm_prepare(const b200k_qlstm_params* p, b200k_qlstm_plan* plan)
 {
     B200K_REQUIRE(p && plan, B200K_E_INVALID, "qlstm_prepare: null params or plan");
-    ql_plan_scales(p, plan->scales);
-    ql_make_plan(*plan);
+    float scales[17];
+    ql_plan_scales(p, scales);
+    *plan = ql_plan_for(scales);
     return B200K_OK;
 }
 
@@ -893,6 +895,13 @@ extern "C" int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream)
     a.exact_only = !byte(p->input_zp) || !byte(p->output_state_zp) || !byte(p->output_zp) || !byte(p->hidden_state_zp) || !ql_plan_ordinary(plan);
     static_assert(sizeof(a.danger) == sizeof(plan.magnitudes), "a plan holds what the kernel reads");
     memcpy(a.danger, plan.magnitudes, sizeof(a.danger));
+    const float ln[4] = {p->s_lni, p->s_lnf, p->s_lnc, p->s_lno};
+    for (int g = 0; g < 4; ++g) {
+        a.inv_gate[g] = rn_reciprocal(scales[13 + g]);
+        a.inv_ln[g] = rn_reciprocal(p->input_scale * ln[g] * 1024.f);
+    }
+    a.inv_cell = rn_reciprocal(p->cell_state_scale);
+    a.inv_out = rn_reciprocal(p->output_scale);
     auto aligned = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     a.vec_i = p->input_size % 16 == 0 && aligned(p->w_i2i) && aligned(p->w_i2f) && aligned(p->w_i2c) && aligned(p->w_i2o);
     a.vec_o = p->output_size % 16 == 0 && aligned(p->w_r2i) && aligned(p->w_r2f) && aligned(p->w_r2c) && aligned(p->w_r2o);

@@ -611,8 +611,8 @@ typedef struct {
     float input_intermediate_scale, forget_intermediate_scale, cell_intermediate_scale,
           output_intermediate_scale;
     float hidden_state_scale; int32_t hidden_state_zp;
-    const b200k_qlstm_plan* plan;    /* host memory, read during the call; NULL or made for other scales: the library's own, of the
-                                      * last 256 layers stepped that way */
+    const b200k_qlstm_plan* plan;    /* host memory, read during the call; NULL or made for other scales: the library's own copy, kept
+                                      * for the last 256 layers */
 } b200k_qlstm_params;
 
 int b200k_qlstm_step(const b200k_qlstm_params* p, void* stream);
