@@ -33,7 +33,7 @@
 // (per-tensor asymmetric weights) is accumulated by the tensor core itself from constant B tiles holding -zw.
 //
 // Requantisation is the same function as in the CUDA-core kernel and the CPU oracle (IEEE fp32, unfused), evaluated
-// without the division unit and bit-identically (see epi_chunk_fast and epi_fix_group).
+// without the division unit and bit-identically (see epi_chunk_fast and epi_fix_values).
 //
 // Every wait on an mbarrier is bounded; when a bound is hit the kernel raises a status word (read with
 // b200k_poll_status), drains and returns, so a logic error cannot hang the device.
@@ -96,7 +96,7 @@ __device__ __forceinline__ void tc_trace(int i)
 struct EpiConsts {
     float2 inv2, nsy2, magic2, zero2, neg2;      // RN(1 / sy), -sy, MAGIC, 0, -1
     float2 nmagic2;                              // -MAGIC
-    float2 zoff_lut2, zoff_sat2, zoff_clamp2;    // what is added to t = MAGIC + n (see epi_fix_group), per way of ending
+    float2 zoff_lut2, zoff_sat2, zoff_clamp2;    // what is added to t = MAGIC + n (see epi_fix_values), per way of ending
     float lo, hi;                                // EPI_CLAMP: clamp bounds in the biased domain (MAGIC + ...)
 };
 
@@ -128,7 +128,7 @@ struct TcArgs {
     // fused ElementwiseBinary Add (res != null): y = Q2(deq(Q(conv)) + deq(res)), clamp in rq2
     const uint8_t* res; float res_scale; int res_zp; int res_u8;
     Requant rq2;
-    float inv_sy;                               // RN(1 / rq.sy), correctly rounded (see epi_fix_group)
+    float inv_sy;                               // RN(1 / rq.sy), correctly rounded (see epi_fix_values)
     EpiConsts ep;                               // the hot path's constants
     const uint8_t* add_lut;                     // fused-add table built by b200k_conv2d_pack (+ its tag), or null
     uint32_t lut_tag[TC_LUT_TAG_WORDS];         // the tag a table made for exactly this launch carries
@@ -302,6 +302,12 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* r)
                  : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t* r)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]) :: "memory");
+}
 // The same load split in two, so that several can be in flight: the registers must not be touched between issue and
 // wait, which the wait enforces by claiming to modify them.
 __device__ __forceinline__ void tc_ld16_issue(uint32_t taddr, uint32_t* r)
@@ -431,7 +437,7 @@ __device__ __forceinline__ void lds_f2x2(uint32_t addr, float2& a, float2& b)   
 // do).  t = q" + MAGIC rounds q" to an integer n; whenever |q" - n| < 0.5 - E the reference's q lies on the same side of
 // every rounding boundary, so n is the reference's result and the halves-away-from-zero rule cannot matter.  A group of
 // four values in which some lane sees |q" - n| >= 0.5 - E (about one group in twenty) is re-evaluated with the
-// reference arithmetic itself (epi_fix_group).  Values whose q" is huge lose the integer grid of the magic constant:
+// reference arithmetic itself (epi_fix_values).  Values whose q" is huge lose the integer grid of the magic constant:
 // either they are flagged like the others or they saturate, as the reference's do.
 // Where mq and bq come from.  TabFast: tables in shared memory, read with 128-bit loads that every lane of the warp
 // repeats (all lanes work on the same columns; bq: this lane's class row): four wavefronts of the shared-memory pipe per
@@ -459,8 +465,14 @@ constexpr int TC_PTAB_MAX = 2048;               // output channels whose tables 
 struct TcTabs { float mq[TC_PTAB_MAX]; float bq[TC_PTAB_MAX]; };
 struct TcNoTabs { int unused; };
 
+__device__ __forceinline__ void epi_to_float(const uint32_t* r, float2* acc)       // 16 accumulators
+{
+    #pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = make_float2(__int2float_rn((int)r[2 * i]), __int2float_rn((int)r[2 * i + 1]));
+}
+
 template <int KIND, class Tab>
-__device__ __forceinline__ uint4 epi_chunk_fast(const uint32_t* r, const uint4 rv, const Tab& ad, const EpiConsts& ec, const uint32_t lut,
+__device__ __forceinline__ uint4 epi_chunk_fast(const float2* acc, const uint4 rv, const Tab& ad, const EpiConsts& ec, const uint32_t lut,
                                                 float* dmg)
 {
     const uint32_t resw[4] = {rv.x, rv.y, rv.z, rv.w};
@@ -469,9 +481,7 @@ __device__ __forceinline__ uint4 epi_chunk_fast(const uint32_t* r, const uint4 r
     for (int g = 0; g < 4; ++g) {
         float2 m01, m23, b01, b23;
         ad.load(g, m01, m23, b01, b23);
-        const float2 a01 = make_float2(__int2float_rn((int)r[g * 4 + 0]), __int2float_rn((int)r[g * 4 + 1]));
-        const float2 a23 = make_float2(__int2float_rn((int)r[g * 4 + 2]), __int2float_rn((int)r[g * 4 + 3]));
-        const float2 q01 = __ffma2_rn(a01, m01, b01), q23 = __ffma2_rn(a23, m23, b23);
+        const float2 q01 = __ffma2_rn(acc[g * 2], m01, b01), q23 = __ffma2_rn(acc[g * 2 + 1], m23, b23);
         const float2 t01 = __fadd2_rn(q01, ec.magic2), t23 = __fadd2_rn(q23, ec.magic2);
         const float2 n01 = __fadd2_rn(t01, ec.nmagic2), n23 = __fadd2_rn(t23, ec.nmagic2);       // rint(q") (exact)
         const float2 d01 = __ffma2_rn(n01, ec.neg2, q01), d23 = __ffma2_rn(n23, ec.neg2, q23);   // q" - n (exact)
@@ -523,8 +533,8 @@ __device__ __forceinline__ uint4 epi_chunk_fast(const uint32_t* r, const uint4 r
 // arithmetic (exact_value).  Kept out of line: it runs for a few per cent of the groups and would otherwise be inlined
 // sixteen times into every tile loop.
 template <int KIND>
-__device__ __noinline__ uint32_t epi_fix_group(int a0, int a1, int a2, int a3, uint32_t a_m, uint32_t a_b, uint32_t a_cc, uint32_t resw,
-                                               const EpiConsts* ecp, uint32_t lut, const EpiExact* x)
+__device__ __forceinline__ uint32_t epi_fix_values(int a0, int a1, int a2, int a3, uint32_t a_m, uint32_t a_b, uint32_t a_cc, uint32_t resw,
+                                                   const EpiConsts* ecp, uint32_t lut, const EpiExact* x)
 {
     const EpiConsts& ec = *ecp;
     const float2 zoff2 = KIND == EPI_LUT ? ec.zoff_lut2 : (KIND == EPI_CLAMP ? ec.zoff_clamp2 : ec.zoff_sat2);
@@ -567,28 +577,37 @@ __device__ __noinline__ uint32_t epi_fix_group(int a0, int a1, int a2, int a3, u
     }
     return out;
 }
-
-// The cold pass of one chunk (rare, or the accumulator dump of the tests): from the 16 accumulators still in
-// registers, (fix) evaluate them with the reference arithmetic (other operand's bytes at res_slot, result to out_slot)
-// and / or (acc_row) write the raw accumulators of a valid row out for the bit-exactness tests.
-__device__ __forceinline__ void epi_cold(const uint32_t* r, uint32_t res_slot, uint32_t out_slot, uint32_t a_m, uint32_t a_b,
-                                         uint32_t a_cc, const EpiExact& x, bool fix, int32_t* acc_row)
+// one group from registers
+template <int KIND>
+__device__ __noinline__ uint32_t epi_fix_group(int a0, int a1, int a2, int a3, uint32_t a_m, uint32_t a_b, uint32_t a_cc,
+                                               const EpiConsts* ecp, const EpiExact* x)
 {
-    if (acc_row) {
-        #pragma unroll
-        for (int j = 0; j < 16; ++j) acc_row[j] = (int)r[j] - lds_s32(a_cc + j * 4);
+    return epi_fix_values<KIND>(a0, a1, a2, a3, a_m, a_b, a_cc, 0u, ecp, 0u, x);
+}
+// The flagged groups (a bit each, the same for the whole warp) of a chunk of 16 columns whose accumulators are still at taddr
+// in tensor memory; the other operand's bytes at res_addr, the results to out_addr.  Reading the accumulators again, instead
+// of keeping them in registers and passing them, leaves one call in the tile loop where four were.
+template <int KIND>
+__device__ __noinline__ void epi_fix_chunk(uint32_t groups, uint32_t taddr, uint32_t a_m, uint32_t a_b, uint32_t a_cc, uint32_t res_addr,
+                                           uint32_t out_addr, const EpiConsts* ecp, uint32_t lut, const EpiExact* x)
+{
+    #pragma unroll 1
+    for (; groups; groups &= groups - 1u) {
+        const uint32_t g = (uint32_t)__ffs((int)groups) - 1u;
+        uint32_t r[4];
+        tc_ld4(taddr + g * 4u, r);
+        const uint32_t resw = KIND == EPI_LUT || x->always ? (uint32_t)lds_s32(res_addr + g * 4u) : 0u;
+        const uint32_t out = epi_fix_values<KIND>((int)r[0], (int)r[1], (int)r[2], (int)r[3], a_m + g * 16u, a_b + g * 16u, a_cc + g * 16u, resw,
+                                                  ecp, lut, x);
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(out_addr + g * 4u), "r"(out) : "memory");
     }
-    if (!fix) return;
-    const uint4 rv = x.fused ? lds128(res_slot) : make_uint4(0, 0, 0, 0);
-    const uint32_t resw[4] = {rv.x, rv.y, rv.z, rv.w};
-    uint32_t out[4] = {0, 0, 0, 0};
+}
+
+// The raw accumulators of one chunk of a valid row, for the bit-exactness tests.
+__device__ __forceinline__ void epi_dump(const uint32_t* r, uint32_t a_cc, int32_t* acc_row)
+{
     #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const int q = exact_value((int)r[j] - lds_s32(a_cc + j * 4), lds_f32(a_m + j * 4), lds_f32(a_b + j * 4),
-                                  (resw[j >> 2] >> (8 * (j & 3))) & 0xffu, x);
-        out[j >> 2] |= ((uint32_t)q & 0xffu) << (8 * (j & 3));
-    }
-    sts128(out_slot, make_uint4(out[0], out[1], out[2], out[3]));
+    for (int j = 0; j < 16; ++j) acc_row[j] = (int)r[j] - lds_s32(a_cc + j * 4);
 }
 
 template <int BN, int SWZ>
@@ -669,7 +688,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     float* s_mq = (float*)(s_cc + a.ncls * BN);             // [BN] hot-path multiplier m / sy
     float* s_bq = s_mq + BN;                                // [classes][BN] hot-path addend (see epi_chunk_fast)
     uint32_t* s_emax = (uint32_t*)(s_bq + a.ncls * BN);     // [2][2] max |bq|, max |b / sy| of a staging (bit patterns), double-buffered
-    EpiExact* s_ex = (EpiExact*)(s_emax + 4);               // the reference arithmetic's constants (epi_fix_group)
+    EpiExact* s_ex = (EpiExact*)(s_emax + 4);               // the reference arithmetic's constants (epi_fix_values)
     uint8_t* s_lut = (uint8_t*)(((uintptr_t)(s_emax + 4 + 16) + 255) & ~(uintptr_t)255);   // fused-add table, 256-byte aligned
     // per K-slice: {channel offset, im2col offsets (x | y << 16), weight column, packed-row offset}: the producers read
     // their coordinates from here instead of carrying tap counters through every slice
@@ -918,9 +937,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (ew == 0) TC_TRACE(5);
         const bool always_fix = fused && !lut_ok;            // no table: every chunk takes the reference arithmetic
         const bool dump_acc = a.acc_out != nullptr;
-        // the reference arithmetic's constants: only the cold pass uses them, which rebuilds them from the launch
-        // arguments instead of keeping them in registers through the hot loop
-        auto make_exact = [&]() {
+        // the reference arithmetic's constants (published by the first staging's barriers)
+        if (etid == 0) {
             EpiExact ex;
             ex.sy1 = a.rq.sy; ex.zy1 = (float)a.rq.zy;
             ex.lo1 = fmaxf(a.rq.tlo, (float)a.rq.clo); ex.hi1 = fminf(a.rq.thi, (float)a.rq.chi);
@@ -928,10 +946,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             ex.sy2 = a.rq2.sy; ex.zy2 = (float)a.rq2.zy;
             ex.lo2 = fmaxf(a.rq2.tlo, (float)a.rq2.clo); ex.hi2 = fminf(a.rq2.thi, (float)a.rq2.chi);
             ex.always = always_fix;
-            return ex;
-        };
+            *s_ex = ex;
+        }
         static_assert(sizeof(EpiExact) <= 64, "EpiExact outgrew its shared-memory slot");
-        if (etid == 0) *s_ex = make_exact();                  // (published by the first staging's barriers)
         const float lo1 = fmaxf(a.rq.tlo, (float)a.rq.clo), hi1 = fminf(a.rq.thi, (float)a.rq.chi), zy1 = (float)a.rq.zy;
         // how the hot path ends (warp-uniform, fixed for the launch)
         const int kind = use_lut ? EPI_LUT
@@ -1016,10 +1033,46 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // find itself without a tile
         if (eg > 1) stage_constants(0);
         if (ew == 0) TC_TRACE(6);
-        // The tile loop exists once per way the hot path ends (KIND, fixed for the launch), chosen by one switch below, so
-        // that the per-chunk code is straight-line.
-        auto run_tiles = [&](auto kind_tag) {
+        // The chunks of one unit.  This loop exists once per way the hot path ends (KIND), chosen per unit; everything around it
+        // exists once.  An SM comes to a launch without its instructions, and the first tile's way through the code takes
+        // two to three times a later tile's (5 - 11 us against 2 - 3.5 in ResNet-50 at batch 256, 2.5 against 1 at batch 3): with
+        // a copy of the whole tile loop per KIND and a fix-up call per group, the same layers ran 2 - 5 % slower.  Left as
+        // a loop over chunks, the code is smaller still and every later tile slower: 3230 us against 3010.
+        // The first load has been issued; the next one is as soon as the values before it have left their registers.
+        auto unit_chunks = [&](auto kind_tag, uint32_t* r, uint32_t tcol, int col0, uint32_t res_row, uint32_t st_row, uint32_t a_m, uint32_t a_b,
+                               uint32_t a_cc, uint32_t a_mq, uint32_t a_bq, int n0) {
             constexpr int KIND = decltype(kind_tag)::value;
+            #pragma unroll
+            for (int j = 0; j < NCH; ++j, tcol += 16, col0 += 16) {
+                float2 acc[8];
+                tc_ld16_wait(r);
+                epi_to_float(r, acc);
+                if (j + 1 < NCH) tc_ld16_issue(tcol + 16, r);
+                const uint32_t res_addr = res_row + ((((uint32_t)(part * NCH + j)) ^ sw_x) << 4);
+                const uint4 rv = KIND == EPI_LUT ? lds128(res_addr) : make_uint4(0, 0, 0, 0);
+                float dmg[4];
+                uint4 outv;
+                if constexpr (PTAB) {
+                    const TabFastP ad = {tabs.mq + n0 + col0, tabs.bq + n0 + col0};
+                    outv = epi_chunk_fast<KIND>(acc, rv, ad, a.ep, lut_addr, dmg);
+                } else {
+                    const TabFast ad = {a_mq + col0 * 4, a_bq + col0 * 4};
+                    outv = epi_chunk_fast<KIND>(acc, rv, ad, a.ep, lut_addr, dmg);
+                }
+                const uint32_t out_addr = st_row + (((uint32_t)j ^ st_sw) << 4);
+                sts128(out_addr, outv);
+                // groups the hot path cannot vouch for (|q" - n| within E of a half, a huge value, or no usable
+                // table at all: thr = 0) take the reference arithmetic, from the accumulators still in tensor memory
+                if (__any_sync(0xffffffffu, fmaxf(fmaxf(dmg[0], dmg[1]), fmaxf(dmg[2], dmg[3])) >= thr)) {
+                    uint32_t groups = 0;
+                    #pragma unroll
+                    for (int g = 0; g < 4; ++g) groups |= __any_sync(0xffffffffu, dmg[g] >= thr) ? 1u << g : 0u;
+                    if (j + 1 < NCH) tc_ld16_wait(r);        // (no load in flight across the call)
+                    epi_fix_chunk<KIND>(groups, tcol, a_m + col0 * 4, a_b + col0 * 4, a_cc + col0 * 4, res_addr, out_addr, &a.ep, lut_addr, s_ex);
+                }
+            }
+        };
+        {
             int it = 0;
             int ub = 0; uint32_t uph = 0;                    // operand-buffer position (kept without divisions)
             uint32_t st_base = st_base0;
@@ -1030,7 +1083,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const int n0 = ntn == 1 ? 0 : (t - tm * ntn) * BN;
                 const long long m0 = (long long)tm * a.tile_rows;
                 const int buf = it & ((1 << NACC_LOG2) - 1);
-                if (n0 != cur_n0) stage_constants(n0);
+                if (eg == 1 && n0 != cur_n0) stage_constants(n0);
                 if (ew == 0 && it < 8) TC_TRACE(56 + it);
                 if (!dead && !mbar_wait(&acc_full[buf], ((uint32_t)it >> NACC_LOG2) & 1u, a.wait_limit)) { atomicExch(&g_tc_status, 3); dead = true; }
                 if (ew == 0 && t == blockIdx.x) TC_TRACE(7);
@@ -1065,12 +1118,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int us = 0; us < nact; ++us) {
                     const int colw = us * UW + part * (int)W;      // first column of this warp in this unit
                     const uint32_t res_row = smem_u32(s_io + (size_t)(NSTG_UNITS + ub) * IO_BYTES + row * UW);    // (fused: eg == 1)
-                    // The warp's NCH chunks of 16 columns go through two register sets that take turns: the loads of
-                    // the first two are issued before the unit's waits; a set is reloaded (chunk + 2) as soon as its
-                    // chunk has been computed.  (tcgen05.wait::ld waits for every load the thread has issued.)
-                    uint32_t r[2][16];
-                    tc_ld16_issue(tacc + (uint32_t)colw, r[0]);
-                    if (NCH > 1) tc_ld16_issue(tacc + (uint32_t)(colw + 16), r[1]);
+                    uint32_t r[16];
+                    tc_ld16_issue(tacc + (uint32_t)colw, r);
                     if (fused && !dead && !mbar_wait(&io_full[ub], uph, a.wait_limit)) { atomicExch(&g_tc_status, 5); dead = true; }
                     // the store that last used this staging buffer has read it out
                     if (lane == 0) {
@@ -1079,52 +1128,21 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     __syncwarp();
                     const uint32_t st_row = st_base + (uint32_t)lane * W;
-                    #pragma unroll
-                    for (int j = 0; j < NCH; ++j) {
-                        if ((j & 1) == 0) {
-                            tc_ld16_wait(r[0]);
-                            if (j + 1 < NCH) tc_ld16_wait(r[1]);
-                        }
-                        const int col0 = colw + j * 16;
-                        const uint4 rv = KIND == EPI_LUT ? lds128(res_row + ((((uint32_t)(part * NCH + j)) ^ sw_x) << 4)) : make_uint4(0, 0, 0, 0);
-                        float dmg[4];
-                        uint4 outv;
-                        if constexpr (PTAB) {
-                            const TabFastP ad = {tabs.mq + n0 + col0, tabs.bq + n0 + col0};
-                            outv = epi_chunk_fast<KIND>(r[j & 1], rv, ad, a.ep, lut_addr, dmg);
-                        } else {
-                            const TabFast ad = {a_mq + col0 * 4, a_bq + col0 * 4};
-                            outv = epi_chunk_fast<KIND>(r[j & 1], rv, ad, a.ep, lut_addr, dmg);
-                        }
-                        // groups the hot path cannot vouch for (|q" - n| within E of a half, a huge value, or no usable
-                        // table at all: thr = 0) take the reference arithmetic, from the accumulators still in registers
-                        if (__any_sync(0xffffffffu, fmaxf(fmaxf(dmg[0], dmg[1]), fmaxf(dmg[2], dmg[3])) >= thr)) {
-                            const uint32_t* rr = r[j & 1];
-                            const uint32_t resw[4] = {rv.x, rv.y, rv.z, rv.w};
-                            uint32_t w[4] = {outv.x, outv.y, outv.z, outv.w};
-                            #pragma unroll
-                            for (int g = 0; g < 4; ++g) {
-                                if (__any_sync(0xffffffffu, dmg[g] >= thr))
-                                    w[g] = epi_fix_group<KIND>((int)rr[g * 4], (int)rr[g * 4 + 1], (int)rr[g * 4 + 2], (int)rr[g * 4 + 3],
-                                                               a_m + (col0 + g * 4) * 4, a_b + (col0 + g * 4) * 4, a_cc + (col0 + g * 4) * 4, resw[g],
-                                                               &a.ep, lut_addr, s_ex);
-                            }
-                            outv = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
-                        sts128(st_row + (((uint32_t)j ^ st_sw) << 4), outv);
-                        if (j + 2 < NCH) tc_ld16_issue(tacc + (uint32_t)(colw + (j + 2) * 16), r[j & 1]);
+                    auto chunks = [&](auto kind_tag) { unit_chunks(kind_tag, r, tacc + (uint32_t)colw, colw, res_row, st_row, a_m, a_b, a_cc, a_mq, a_bq, n0); };
+                    switch (kind) {
+                        case EPI_LUT:    chunks(std::integral_constant<int, EPI_LUT>{}); break;
+                        case EPI_SAT_U8: chunks(std::integral_constant<int, EPI_SAT_U8>{}); break;
+                        case EPI_SAT_S8: chunks(std::integral_constant<int, EPI_SAT_S8>{}); break;
+                        default:         chunks(std::integral_constant<int, EPI_CLAMP>{}); break;
                     }
                     // the accumulator dump of the tests: from a second read of the accumulators
                     if (dump_acc) {
-                        const EpiExact ex = make_exact();
                         #pragma unroll 1
                         for (int j = 0; j < NCH; ++j) {
                             const int col0 = colw + j * 16;
                             uint32_t rr[16];
                             tc_ld16(tacc + (uint32_t)col0, rr);
-                            epi_cold(rr, res_row + ((((uint32_t)(part * NCH + j)) ^ sw_x) << 4), st_row + (((uint32_t)j ^ st_sw) << 4),
-                                     a_m + col0 * 4, a_b + col0 * 4, a_cc + col0 * 4, ex, false,
-                                     (mvalid && n0 + col0 < a.OC) ? a.acc_out + m * a.OC + n0 + col0 : nullptr);
+                            if (mvalid && n0 + col0 < a.OC) epi_dump(rr, a_cc + col0 * 4, a.acc_out + m * a.OC + n0 + col0);
                         }
                     }
                     if (fused) {
@@ -1164,12 +1182,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (ew == 0 && it < 8) TC_TRACE(40 + it);
                 if (ew == 0) TC_TRACE(9);
             }
-        };
-        switch (kind) {
-            case EPI_LUT:    run_tiles(std::integral_constant<int, EPI_LUT>{}); break;
-            case EPI_SAT_U8: run_tiles(std::integral_constant<int, EPI_SAT_U8>{}); break;
-            case EPI_SAT_S8: run_tiles(std::integral_constant<int, EPI_SAT_S8>{}); break;
-            default:         run_tiles(std::integral_constant<int, EPI_CLAMP>{}); break;
         }
         // shared memory may go once the last store has read it; its global writes complete with the kernel
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -1894,15 +1906,17 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
                 uint8_t* orow = a.y + ((long long)t * a.OW + px) * a.OC;
                 const TabFast ad = {a_mq + c * 64, a_bq + c * 64};
                 float dmg[4];
-                uint4 outv = epi_chunk_fast<KIND>(rc, make_uint4(0, 0, 0, 0), ad, a.ep, 0u, dmg);
+                float2 acc[8];
+                epi_to_float(rc, acc);
+                uint4 outv = epi_chunk_fast<KIND>(acc, make_uint4(0, 0, 0, 0), ad, a.ep, 0u, dmg);
                 if (__any_sync(0xffffffffu, fmaxf(fmaxf(dmg[0], dmg[1]), fmaxf(dmg[2], dmg[3])) >= thr)) {
                     uint32_t w[4] = {outv.x, outv.y, outv.z, outv.w};
                     #pragma unroll
                     for (int g = 0; g < 4; ++g) {
                         if (__any_sync(0xffffffffu, dmg[g] >= thr))
                             w[g] = epi_fix_group<KIND>((int)rc[g * 4], (int)rc[g * 4 + 1], (int)rc[g * 4 + 2], (int)rc[g * 4 + 3],
-                                                       a_m + (c * 16 + g * 4) * 4, a_b + (c * 16 + g * 4) * 4, a_cc + (c * 16 + g * 4) * 4, 0u,
-                                                       &a.ep, 0u, s_ex);
+                                                       a_m + (c * 16 + g * 4) * 4, a_b + (c * 16 + g * 4) * 4, a_cc + (c * 16 + g * 4) * 4,
+                                                       &a.ep, s_ex);
                     }
                     outv = make_uint4(w[0], w[1], w[2], w[3]);
                 }
