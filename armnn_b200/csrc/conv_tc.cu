@@ -91,6 +91,13 @@ __device__ __forceinline__ void tc_trace(int i)
 #define TC_TRACE(i) do { } while (0)
 #endif
 
+// The fused Add as arithmetic (see add_formula_bytes).  Pairs are the same value twice.
+struct AddFormula {
+    float2 roff2, k2, c02, range2, base2;        // -(2^23 + zero point) of the other operand's byte; its factor; addend; hi - lo; MAGIC + lo
+    float k1;                                    // factor of the convolution's output
+    uint32_t flip;                               // 0x80808080 where the other operand is int8
+};
+
 // Constants of the hot path, filled in by the host: they sit in the kernel's parameter space, so the packed
 // instructions read them as constant-bank operands and they take no registers.  Each is the same value twice.
 struct EpiConsts {
@@ -98,6 +105,7 @@ struct EpiConsts {
     float2 nmagic2;                              // -MAGIC
     float2 zoff_lut2, zoff_sat2, zoff_clamp2;    // what is added to t = MAGIC + n (see epi_fix_values), per way of ending
     float lo, hi;                                // EPI_CLAMP: clamp bounds in the biased domain (MAGIC + ...)
+    AddFormula add;                              // EPI_ADD
 };
 
 struct TcArgs {
@@ -414,7 +422,36 @@ __device__ __forceinline__ uint32_t lds_u8(uint32_t addr)
 
 // What the last step of the hot path is: look the fused Add up in its table, convert with the output type's own
 // saturation (the clamp is exactly the type's range), or clamp to a narrower activation range.
-enum { EPI_LUT = 0, EPI_SAT_U8 = 1, EPI_SAT_S8 = 2, EPI_CLAMP = 3 };
+enum { EPI_LUT = 0, EPI_SAT_U8 = 1, EPI_SAT_S8 = 2, EPI_CLAMP = 3, EPI_ADD = 4 };
+
+// The fused Add of four values without its table.  n: the convolution's output less the type minimum, an integer that may lie
+// outside 0 .. 255; res: the other operand's bytes.  Both operands are 8-bit, so the reference's
+//     clamp(z3 + round_half_away(fl(fl(fl((q1 - z1) s1) + fl((r - z2) s2)) / s3)), lo, hi)
+// is a function of 65536 pairs, and a linear form in n and r rounds to the same integers unless a pair lies within about 2e-5
+// of a half.  b200k_conv2d_pack tries 32 forms that differ in the last bits of their constants on all 65536 pairs, with these very
+// instructions, and a launch uses one that gave every entry of the table (see tc_pack_host_tables); where none did (exact halves,
+// as with scales in powers of two), the table stays.  Saturating multiplications clamp both stages for nothing: c is the
+// clamped n / 255, s the clamped position of the sum between lo and hi.
+// The table is 65 KiB that every CTA of every launch fetches, and a look-up costs 3.5 wavefronts of the shared-memory pipe: together
+// with kernels compiled per way of ending, ResNet-50 takes 2720 us at batch 256 (2969) and 350 at batch 3 (373).
+__device__ __forceinline__ uint32_t add_formula_bytes(const float* n, uint32_t res, const AddFormula& f)
+{
+    res ^= f.flip;
+    const float2 r01 = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(res, 0x4b000000u, 0x7440)), __uint_as_float(__byte_perm(res, 0x4b000000u, 0x7441))), f.roff2);
+    const float2 r23 = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(res, 0x4b000000u, 0x7442)), __uint_as_float(__byte_perm(res, 0x4b000000u, 0x7443))), f.roff2);
+    const float2 u01 = __ffma2_rn(r01, f.k2, f.c02), u23 = __ffma2_rn(r23, f.k2, f.c02);
+    const float u[4] = {u01.x, u01.y, u23.x, u23.y};
+    float sum[4];
+    #pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        float c;
+        asm("mul.rn.sat.f32 %0, %1, 0f3B808081;" : "=f"(c) : "f"(n[e]));                        // 1 / 255; 255 gives 1
+        asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(sum[e]) : "f"(c), "f"(f.k1), "f"(u[e]));
+    }
+    const float2 t01 = __ffma2_rn(make_float2(sum[0], sum[1]), f.range2, f.base2), t23 = __ffma2_rn(make_float2(sum[2], sum[3]), f.range2, f.base2);
+    return __byte_perm(__byte_perm(__float_as_uint(t01.x), __float_as_uint(t01.y), 0x0040),
+                       __byte_perm(__float_as_uint(t23.x), __float_as_uint(t23.y), 0x0040), 0x5410);
+}
 
 __device__ __forceinline__ void lds_f2x2(uint32_t addr, float2& a, float2& b)   // four consecutive floats as two pairs
 {
@@ -494,6 +531,8 @@ __device__ __forceinline__ uint4 epi_chunk_fast(const float2* acc, const uint4 r
             #pragma unroll
             for (int e = 0; e < 4; ++e) bits[e] = __float_as_uint(fminf(fmaxf(tt[e], ec.lo), ec.hi));
             packed[g] = __byte_perm(__byte_perm(bits[0], bits[1], 0x0040), __byte_perm(bits[2], bits[3], 0x0040), 0x5410);
+        } else if (KIND == EPI_ADD) {
+            packed[g] = add_formula_bytes(z, resw[g], ec.add);
         } else if (KIND == EPI_LUT) {
             uint32_t bits[4];
             #pragma unroll
@@ -537,7 +576,7 @@ __device__ __forceinline__ uint32_t epi_fix_values(int a0, int a1, int a2, int a
                                                    const EpiConsts* ecp, uint32_t lut, const EpiExact* x)
 {
     const EpiConsts& ec = *ecp;
-    const float2 zoff2 = KIND == EPI_LUT ? ec.zoff_lut2 : (KIND == EPI_CLAMP ? ec.zoff_clamp2 : ec.zoff_sat2);
+    const float2 zoff2 = KIND == EPI_LUT || KIND == EPI_ADD ? ec.zoff_lut2 : (KIND == EPI_CLAMP ? ec.zoff_clamp2 : ec.zoff_sat2);
     float2 m01, m23, b01, b23;
     lds_f2x2(a_m, m01, m23);
     lds_f2x2(a_b, b01, b23);
@@ -565,7 +604,8 @@ __device__ __forceinline__ uint32_t epi_fix_values(int a0, int a1, int a2, int a
             if (KIND == EPI_LUT) bits[e] = lds_u8(bits[e] * (uint32_t)TC_LUT_PITCH + __byte_perm(resw, lut, 0x7650 + e));
         }
     }
-    uint32_t out = __byte_perm(__byte_perm(bits[0], bits[1], 0x0040), __byte_perm(bits[2], bits[3], 0x0040), 0x5410);
+    uint32_t out = KIND == EPI_ADD ? add_formula_bytes(z, resw, ec.add)
+                                   : __byte_perm(__byte_perm(bits[0], bits[1], 0x0040), __byte_perm(bits[2], bits[3], 0x0040), 0x5410);
     if (!(dmax < 0.5f) || x->always) {
         // (no usable table, an exact half, or a value too large for the constant or, as NaN, for the quotient)
         out = 0;
@@ -596,7 +636,7 @@ __device__ __noinline__ void epi_fix_chunk(uint32_t groups, uint32_t taddr, uint
         const uint32_t g = (uint32_t)__ffs((int)groups) - 1u;
         uint32_t r[4];
         tc_ld4(taddr + g * 4u, r);
-        const uint32_t resw = KIND == EPI_LUT || x->always ? (uint32_t)lds_s32(res_addr + g * 4u) : 0u;
+        const uint32_t resw = KIND == EPI_LUT || KIND == EPI_ADD || x->always ? (uint32_t)lds_s32(res_addr + g * 4u) : 0u;
         const uint32_t out = epi_fix_values<KIND>((int)r[0], (int)r[1], (int)r[2], (int)r[3], a_m + g * 16u, a_b + g * 16u, a_cc + g * 16u, resw,
                                                   ecp, lut, x);
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(out_addr + g * 4u), "r"(out) : "memory");
@@ -648,12 +688,17 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 // rows beyond the tensor; before the buffer is written again that lane has waited for the store to have read it.  No
 // epilogue warp waits for another one.  With a fused Add the producer TMA-loads the other operand's unit into one of
 // two shared buffers; every epilogue warp releases it after reading its part.
-template <int BN, int SWZ, int EG, bool PTAB>
+//
+// What a launch ends in is compiled in (MODE), so that none carries the others' code and registers: no fused Add; a fused Add by
+// its table or by its formula, each with the per-channel constants in shared memory or in the parameter space.
+enum { TC_PLAIN = 0, TC_LUT = 1, TC_LUT_PTAB = 2, TC_ADD = 3, TC_ADD_PTAB = 4 };
+template <int BN, int SWZ, int EG, int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmR,
-               const __grid_constant__ TcArgs a, const __grid_constant__ std::conditional_t<PTAB, TcTabs, TcNoTabs> tabs)
+               const __grid_constant__ TcArgs a, const __grid_constant__ std::conditional_t<MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB, TcTabs, TcNoTabs> tabs)
 {
+    constexpr bool PTAB = MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB, fused = MODE != TC_PLAIN, formula = MODE == TC_ADD || MODE == TC_ADD_PTAB;
     using L = TcSmem<BN, SWZ>;
     constexpr int MAX_STAGES = L::MAX_STAGES;
     constexpr int UW = L::UW, UNITS = L::UNITS, IO_BYTES = L::IO_BYTES;
@@ -769,7 +814,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int s = 0; s < a.nslices; ++s)
                     tma_load_2d(s_wst + (size_t)s * L::B_BYTES, &tmB, w_full, (int)s_tab[s].z, 0);
             }
-            if (a.add_lut && prod == 0 && elect_one()) {
+            if (fused && !formula && a.add_lut && prod == 0 && elect_one()) {
                 // the fused-add table: one bulk copy (the epilogue checks its tag before using it)
                 mbar_expect_tx(lut_full, (uint32_t)TC_LUT_BYTES);
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -837,7 +882,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     if (++st == STAGES) { st = 0; ph ^= 1u; }
                 }
                 if (prod == 0 && (t - (int)blockIdx.x) / (int)gridDim.x < 8) TC_TRACE(16 + (t - (int)blockIdx.x) / (int)gridDim.x);
-                if (a.res && alive && !skip_loads && prod == 0) {
+                if (fused && alive && !skip_loads && prod == 0) {
                     // the fused Add's other operand, one unit at a time, into the buffer the epilogue will overwrite
                     if (!have) locate();
                     for (int us = 0; us < UNITS; ++us) {
@@ -932,11 +977,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int row = quad * 32 + lane;
         const uint32_t sw_x = UW == 128 ? (uint32_t)(row & 7) : (uint32_t)((row >> 1) & 3);   // TMA swizzle of this row
         const int pw = a.KW + 1;
-        const bool fused = a.res != nullptr;
         // The fused-add table arrives by a bulk copy the producer has issued.  A table is used only if it was built
         // for exactly this launch's quantisation parameters.
         bool lut_ok = false;
-        if (a.add_lut) {
+        if (fused && !formula && a.add_lut) {
             if (etid == 0) {
                 uint32_t ok = 1;
                 const uint32_t* tag = (const uint32_t*)(a.add_lut + TC_LUT_BYTES);
@@ -950,7 +994,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         const bool use_lut = fused && lut_ok;
         if (ew == 0) TC_TRACE(5);
-        const bool always_fix = fused && !lut_ok;            // no table: every chunk takes the reference arithmetic
+        const bool always_fix = fused && !formula && !lut_ok;            // no table: every chunk takes the reference arithmetic
         const bool dump_acc = a.acc_out != nullptr;
         // the reference arithmetic's constants (published by the first staging's barriers)
         if (etid == 0) {
@@ -966,7 +1010,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         static_assert(sizeof(EpiExact) <= 64, "EpiExact outgrew its shared-memory slot");
         const float lo1 = fmaxf(a.rq.tlo, (float)a.rq.clo), hi1 = fminf(a.rq.thi, (float)a.rq.chi), zy1 = (float)a.rq.zy;
         // how the hot path ends (warp-uniform, fixed for the launch)
-        const int kind = use_lut ? EPI_LUT
+        const int kind = formula ? EPI_ADD : fused ? EPI_LUT
                        : (lo1 == a.rq.tlo && hi1 == a.rq.thi) ? (a.rq.tlo == 0.f ? EPI_SAT_U8 : EPI_SAT_S8) : EPI_CLAMP;
         const uint32_t lut_addr = smem_u32(s_lut);
         int cur_n0 = -1;
@@ -979,7 +1023,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint32_t st_sw = W == 64 ? (uint32_t)((lane >> 1) & 3) : (W == 32 ? (uint32_t)((lane >> 2) & 1) : 0u);
         bool dead = false;
         // what the hot path adds to the requantised value: the output zero point; with the table also minus the type minimum
-        const float zoff = use_lut ? zy1 - a.rq.tlo : zy1;
+        const float zoff = use_lut || formula ? zy1 - a.rq.tlo : zy1;
         float thr = 0.0f;                                    // 0.5 - E of the staged n-tile (see epi_chunk_fast); 0: no hot path
         int stagings = 0;
         auto stage_constants = [&](int n0) {
@@ -1064,10 +1108,10 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 epi_to_float(r, acc);
                 if (j + 1 < NCH) tc_ld16_issue(tcol + 16, r);
                 const uint32_t res_addr = res_row + ((((uint32_t)(part * NCH + j)) ^ sw_x) << 4);
-                const uint4 rv = KIND == EPI_LUT ? lds128(res_addr) : make_uint4(0, 0, 0, 0);
+                const uint4 rv = KIND == EPI_LUT || KIND == EPI_ADD ? lds128(res_addr) : make_uint4(0, 0, 0, 0);
                 float dmg[4];
                 uint4 outv;
-                if constexpr (PTAB) {
+                if constexpr (MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB) {
                     const TabFastP ad = {tabs.mq + n0 + col0, tabs.bq + n0 + col0};
                     outv = epi_chunk_fast<KIND>(acc, rv, ad, a.ep, lut_addr, dmg);
                 } else {
@@ -1144,12 +1188,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     __syncwarp();
                     const uint32_t st_row = st_base + (uint32_t)lane * W;
                     auto chunks = [&](auto kind_tag) { unit_chunks(kind_tag, r, tacc + (uint32_t)colw, colw, res_row, st_row, a_m, a_b, a_cc, a_mq, a_bq, n0); };
-                    switch (kind) {
-                        case EPI_LUT:    chunks(std::integral_constant<int, EPI_LUT>{}); break;
-                        case EPI_SAT_U8: chunks(std::integral_constant<int, EPI_SAT_U8>{}); break;
-                        case EPI_SAT_S8: chunks(std::integral_constant<int, EPI_SAT_S8>{}); break;
-                        default:         chunks(std::integral_constant<int, EPI_CLAMP>{}); break;
-                    }
+                    if constexpr (formula)    chunks(std::integral_constant<int, EPI_ADD>{});
+                    else if constexpr (fused) chunks(std::integral_constant<int, EPI_LUT>{});      // (without a table its results are all replaced)
+                    else if (kind == EPI_SAT_U8) chunks(std::integral_constant<int, EPI_SAT_U8>{});
+                    else if (kind == EPI_SAT_S8) chunks(std::integral_constant<int, EPI_SAT_S8>{});
+                    else chunks(std::integral_constant<int, EPI_CLAMP>{});
                     // the accumulator dump of the tests: from a second read of the accumulators
                     if (dump_acc) {
                         #pragma unroll 1
@@ -1311,7 +1354,42 @@ __global__ void __launch_bounds__(256) row_input_pack_kernel(const RowInputArgs 
 
 // ---- fused-add table ---------------------------------------------------------------------------------------------
 
-struct AddLutArgs { uint8_t* lut; int y_u8, res_u8; float sy; int zy; float sr; int zr; Requant out; uint32_t tag[TC_LUT_TAG_WORDS]; };
+// The 32 forms of the fused Add that are tried: addend and factor off by parts of their last bits.
+struct AddForms {
+    AddFormula common;
+    float k1[4], c0[8];
+    __host__ __device__ AddFormula form(int i) const
+    {
+        AddFormula f = common;
+        f.k1 = k1[i >> 3];
+        f.c02 = make_float2(c0[i & 7], c0[i & 7]);
+        return f;
+    }
+};
+static AddForms make_add_forms(const b200k_conv2d_params* p)
+{
+    const Requant out = make_requant(0.f, p->add_out, p->clamp_lo, p->clamp_hi);
+    const double lo = out.clo, range = out.chi - out.clo, s3 = p->add_out.scale;
+    const double tlo = p->y.dtype == B200K_U8 ? 0.0 : -128.0;
+    const double k1 = 255.0 * p->y.scale / s3 / range, k2 = p->add_operand.scale / s3 / range;
+    const double c0 = (p->add_out.zero_point - lo + (tlo - p->y.zero_point) * (double)p->y.scale / s3) / range;
+    auto two = [](float v) { return make_float2(v, v); };
+    AddForms a;
+    memset(&a, 0, sizeof(a));
+    const bool s8 = p->add_operand.dtype == B200K_S8;
+    a.common.flip = s8 ? 0x80808080u : 0u;
+    a.common.roff2 = two(-(8388608.0f + (float)(p->add_operand.zero_point + (s8 ? 128 : 0))));
+    a.common.k2 = two((float)k2);
+    a.common.range2 = two((float)range);
+    a.common.base2 = two(TC_MAGIC + (float)lo);
+    const float k = (float)k1;
+    const float ks[4] = {k, nextafterf(k, INFINITY), nextafterf(k, -INFINITY), nextafterf(nextafterf(k, INFINITY), INFINITY)};
+    for (int i = 0; i < 4; ++i) a.k1[i] = ks[i];
+    for (int i = 0; i < 8; ++i) a.c0[i] = (float)(c0 + (i & 1 ? -1 : 1) * ((i + 1) / 2) * 2.9802322e-8);      // steps of 2^-25
+    return a;
+}
+
+struct AddLutArgs { uint8_t* lut; int y_u8, res_u8; float sy; int zy; float sr; int zr; Requant out; uint32_t tag[TC_LUT_TAG_WORDS]; AddForms forms; };
 
 // lut[(conv value - type minimum) * pitch + other operand's byte] = output byte of RefElementwiseBinaryWorkload(Add)
 // followed by the fused activation, evaluated once per pair of 8-bit values with the reference fp32 arithmetic.  The
@@ -1325,7 +1403,15 @@ __global__ void add_lut_kernel(const AddLutArgs a)
     const float fa = __fmul_rn(__int2float_rn(q1 - a.zy), a.sy);
     const float fb = __fmul_rn(__int2float_rn(q2 - a.zr), a.sr);
     const int q = quantize_dev(__fadd_rn(fa, fb), a.out.sy, a.out.zy, a.out.tlo, a.out.thi);
-    a.lut[b1 * TC_LUT_PITCH + b2] = (uint8_t)min(max(q, a.out.clo), a.out.chi);
+    const uint8_t entry = (uint8_t)min(max(q, a.out.clo), a.out.chi);
+    a.lut[b1 * TC_LUT_PITCH + b2] = entry;
+    // behind the tag, a bit for each form that does not give every entry (zeros before this launch)
+    const float n[4] = {(float)b1, (float)b1, (float)b1, (float)b1};
+    uint32_t wrong = 0;
+    for (int f = 0; f < 32; ++f)
+        if ((add_formula_bytes(n, (uint32_t)b2, a.forms.form(f)) & 0xffu) != entry) wrong |= 1u << f;
+    wrong = __reduce_or_sync(0xffffffffu, wrong);
+    if (wrong && (threadIdx.x & 31) == 0) atomicOr((uint32_t*)(a.lut + TC_LUT_BYTES) + TC_LUT_TAG_WORDS, wrong);
     if (i < TC_LUT_TAG_WORDS) ((uint32_t*)(a.lut + TC_LUT_BYTES))[i] = a.tag[i];
 }
 
@@ -1500,12 +1586,15 @@ bool conv_tc_eligible(const b200k_conv2d_params* p)
 }
 
 
-template <int BN, int SWZ, int EG, bool PTAB = false>
+template <int BN, int SWZ, int EG, int MODE = TC_PLAIN>
 static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR,
-                     const TcArgs& a, cudaStream_t stream, const TcTabs* tabs = nullptr)
+                     const TcArgs& a, cudaStream_t stream, const TcTabs* tabs = nullptr, bool formula = false)
 {
-    if constexpr (EG == 1 && !PTAB) {
-        if (tabs) return launch_tc<BN, SWZ, EG, true>(tmA, tmB, tmY, tmR, a, stream, tabs);
+    if constexpr (EG == 1 && MODE == TC_PLAIN) {
+        if (a.res) {
+            if (formula) return tabs ? launch_tc<BN, SWZ, EG, TC_ADD_PTAB>(tmA, tmB, tmY, tmR, a, stream, tabs) : launch_tc<BN, SWZ, EG, TC_ADD>(tmA, tmB, tmY, tmR, a, stream);
+            return tabs ? launch_tc<BN, SWZ, EG, TC_LUT_PTAB>(tmA, tmB, tmY, tmR, a, stream, tabs) : launch_tc<BN, SWZ, EG, TC_LUT>(tmA, tmB, tmY, tmR, a, stream);
+        }
     }
     using L = TcSmem<BN, SWZ>;
     const size_t budget = 227 * 1024;                                   // opt-in shared memory per CTA on sm_100
@@ -1544,8 +1633,8 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     a2.nprod = stages >= TC_PRODUCERS ? TC_PRODUCERS : (stages >= 2 ? 2 : 1);
     if (a2.bstat) a2.stage_tx = (uint32_t)(a.stage_tx - L::B_BYTES);
     const size_t smem = fixed + (size_t)stages * group * stride;
-    auto kern = conv_tc_kernel<BN, SWZ, EG, PTAB>;
-    if (const int rc = allow_shared<conv_tc_kernel<BN, SWZ, EG, PTAB>>(smem)) return rc;
+    auto kern = conv_tc_kernel<BN, SWZ, EG, MODE>;
+    if (const int rc = allow_shared<conv_tc_kernel<BN, SWZ, EG, MODE>>(smem)) return rc;
     const long long tiles = (long long)a.ntn * a.ntm;
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     // Programmatic dependent launch: the grid may start while its predecessor in the stream drains (its set-up touches
@@ -1561,7 +1650,7 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if constexpr (PTAB) {
+    if constexpr (MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB) {
         B200K_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmY, tmR, a2, *tabs));
     } else {
         const TcNoTabs none = {0};
@@ -2109,6 +2198,7 @@ struct HostPack {
     int oc, kh, kw, c;
     std::vector<float> ws, bs;
     std::vector<int32_t> bias_v, wsum;
+    uint32_t tag[TC_LUT_TAG_WORDS + 1];                      // what the fused-add table was built for, and the forms that do not give it
     // the tables of the last launch and what they were computed from (a layer is launched with the same quantisation
     // parameters every time: the ~2 k table entries are then formed once, not per launch)
     std::mutex mu;
@@ -2139,6 +2229,7 @@ int tc_pack_host_tables(const b200k_conv2d_params* p, void* packed, cudaStream_t
     if (p->w.scales) { hp->ws.resize(n); B200K_CUDA(cudaMemcpyAsync(hp->ws.data(), p->w.scales, n * 4, cudaMemcpyDeviceToHost, stream)); }
     if (p->bias.data) { hp->bias_v.resize(n); B200K_CUDA(cudaMemcpyAsync(hp->bias_v.data(), p->bias.data, n * 4, cudaMemcpyDeviceToHost, stream)); }
     if (p->bias.data && p->bias.scales) { hp->bs.resize(n); B200K_CUDA(cudaMemcpyAsync(hp->bs.data(), p->bias.scales, n * 4, cudaMemcpyDeviceToHost, stream)); }
+    B200K_CUDA(cudaMemcpyAsync(hp->tag, (const uint8_t*)packed + add_lut_offset(p->oc, p->kh, p->kw, p->c) + TC_LUT_BYTES, sizeof(hp->tag), cudaMemcpyDeviceToHost, stream));
     B200K_CUDA(cudaStreamSynchronize(stream));
     std::lock_guard<std::mutex> lock(g_hp_mutex);
     g_hp[packed] = hp;
@@ -2167,8 +2258,9 @@ static float host_make_bq(float b, int cc, float m, float sy, float inv_sy, floa
     return q + zoff;
 }
 
-// Fills the parameter-space tables of a fused-Add launch from the host copies; false: not available for this launch.
-static bool host_tables_for(const b200k_conv2d_params* p, const TcArgs& a, TcTabs* tabs, float* thr_out)
+// Fills the parameter-space tables of a fused-Add launch from the host copies, and the form of the Add that gives its table's
+// every entry (-1: none); false: not available for this launch.
+static bool host_tables_for(const b200k_conv2d_params* p, const TcArgs& a, TcTabs* tabs, float* thr_out, int* form)
 {
     if (!p->packed || a.ncls != 1 || a.im2col == 2 || p->oc > TC_PTAB_MAX) return false;
     std::shared_ptr<HostPack> hp;
@@ -2182,6 +2274,8 @@ static bool host_tables_for(const b200k_conv2d_params* p, const TcArgs& a, TcTab
         hp->oc != p->oc || hp->kh != p->kh || hp->kw != p->kw || hp->c != p->c) return false;
     const float sx = a.rq.sx, sy = a.rq.sy, inv_sy = a.inv_sy, zy1 = (float)a.rq.zy;
     const float zoff = zy1 - a.rq.tlo;                       // the table's index: minus the type minimum
+    *form = -1;
+    if (memcmp(hp->tag, a.lut_tag, sizeof(a.lut_tag)) == 0 && ~hp->tag[TC_LUT_TAG_WORDS] != 0u) *form = __builtin_ctz(~hp->tag[TC_LUT_TAG_WORDS]);
     const float key[8] = {sx, sy, inv_sy, zy1, a.rq.tlo, a.rq.thi, p->w.scale, p->bias.scale};
     const int ikey[6] = {a.zx, a.zw, a.kvalid_c, a.need_corr, a.acc_big, p->bias.data ? 1 : 0};
     std::lock_guard<std::mutex> lock(hp->mu);
@@ -2418,17 +2512,31 @@ int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid
     TcTabs tabs_storage;
     const TcTabs* host_tabs = nullptr;
     a.thr_host = 0.f;
-    if (fa.res && a.eg == 1 && kvalid_c == 0 && host_tables_for(p, a, &tabs_storage, &a.thr_host)) host_tabs = &tabs_storage;
-    if (swz == 128) {
-        if (bn == 256) return launch_tc<256, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs);
-        if (bn == 128) return grouped ? launch_tc<128, 128, 2>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<128, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs);
-        if (a.eg == 2) return launch_tc<64, 128, 2>(tmA, tmB, tmY, tmR, a, stream);
-        return grouped ? launch_tc<64, 128, 4>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<64, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs);
+    int form = -1;
+    bool formula = false;
+    if (fa.res && a.eg == 1 && kvalid_c == 0 && host_tables_for(p, a, &tabs_storage, &a.thr_host, &form)) {
+        host_tabs = &tabs_storage;
+        if (form >= 0) {
+            formula = true;
+            a.add_lut = nullptr;
+            a.ep.add = make_add_forms(p).form(form);
+            // Without table look-ups the shared-memory pipe has room for the constants; 16 KiB of parameters, which an SM reads
+            // for the first time in every launch, only pay over several tiles.  ResNet-50 at batch 3 (one tile per CTA): 359 us
+            // with the constants in the parameter space, 350 in shared memory; MobileNet-v2 at batch 64 (one to three) 824 and
+            // 821; ResNet-50 at batch 256 (5 to 42, and several n-tiles) 2720 and 2751.
+            if ((long long)a.ntn * a.ntm <= 2ll * sm_count()) host_tabs = nullptr;
+        }
     }
-    if (bn == 256) return launch_tc<256, 64, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs);
-    if (bn == 128) return grouped ? launch_tc<128, 64, 2>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<128, 64, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs);
+    if (swz == 128) {
+        if (bn == 256) return launch_tc<256, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
+        if (bn == 128) return grouped ? launch_tc<128, 128, 2>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<128, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
+        if (a.eg == 2) return launch_tc<64, 128, 2>(tmA, tmB, tmY, tmR, a, stream);
+        return grouped ? launch_tc<64, 128, 4>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<64, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
+    }
+    if (bn == 256) return launch_tc<256, 64, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
+    if (bn == 128) return grouped ? launch_tc<128, 64, 2>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<128, 64, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
     if (a.eg == 2) return launch_tc<64, 64, 2>(tmA, tmB, tmY, tmR, a, stream);
-    return grouped ? launch_tc<64, 64, 4>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<64, 64, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs);
+    return grouped ? launch_tc<64, 64, 4>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<64, 64, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
 }
 
 
@@ -2473,6 +2581,8 @@ int tc_pack(const b200k_conv2d_params* p, void* packed, cudaStream_t stream)
         la.sy = p->y.scale; la.zy = p->y.zero_point; la.sr = p->add_operand.scale; la.zr = p->add_operand.zero_point;
         la.out = make_requant(0.f, p->add_out, p->clamp_lo, p->clamp_hi);
         make_lut_tag(p, la.tag);
+        la.forms = make_add_forms(p);
+        B200K_CUDA(cudaMemsetAsync(lut + TC_LUT_BYTES, 0, 64, (cudaStream_t)stream));
         add_lut_kernel<<<256, 256, 0, (cudaStream_t)stream>>>(la);
         rc = check_launch("add_lut_kernel");
         if (rc) return rc;

@@ -1,0 +1,36 @@
+"""A convolution with a fused Add: the Add as arithmetic where that gives its table's every entry, by the table elsewhere."""
+import numpy as np
+import pytest
+
+from cases import S8, U8, run_case
+from q8util import random_conv_case
+
+pytestmark = pytest.mark.gpu
+
+# (type, convolution's output, other operand, Add's output, fused ReLU).  Scales in powers of two put sums on exact halves, which
+# no linear form rounds away from zero on both sides; 1e-3 for the output saturates most sums; 40.0 leaves a few output values.
+QUANT = {
+    "s8": (S8, (0.02, 3), (0.031, -7), (0.043, 5), 0), "s8_relu": (S8, (0.02, 3), (0.031, -7), (0.043, -20), 1),
+    "u8": (U8, (0.017, 121), (0.029, 140), (0.033, 118), 0), "u8_relu": (U8, (0.017, 0), (0.029, 255), (0.033, 9), 1),
+    "halves": (S8, (2.0 ** -6, 0), (2.0 ** -6, 1), (2.0 ** -5, 0), 0), "saturating": (S8, (0.02, 0), (0.03, 0), (1e-3, 0), 0),
+    "coarse": (U8, (0.02, 100), (0.03, 90), (40.0, 7), 0), "other_dominates": (S8, (1e-4, 0), (0.5, 0), (0.51, 0), 0),
+    "one_value_left": (S8, (0.02, 3), (0.031, -7), (0.043, 127), 1),
+}
+# one tile per CTA with constants in shared memory; the first number of row tiles beyond two per SM (148); narrow and ragged n-tiles
+SHAPES = {"small": (1, 9, 15, 64, 128), "many_tiles": (1, 2, 148 * 128 + 1, 32, 256), "ragged": (2, 31, 33, 48, 176), "narrow": (3, 16, 16, 128, 64)}
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("quant", QUANT)
+def test_exact(built, quant, shape):
+    dtype, y_q, other_q, out_q, relu = QUANT[quant]
+    n, h, w, c, oc = SHAPES[shape]
+    u8 = dict(x_dtype=U8, w_dtype=U8, y_dtype=U8, x_q=(0.02, 128)) if dtype == U8 else {}
+
+    def case():
+        k = random_conv_case(31, n, h, w, c, oc, 1, 1, act=(1, 0, 0) if relu else (0, 0, 0), fused_add=True, **u8)
+        k.y_q, k.add = y_q, (k.add[0], other_q, out_q)
+        return k
+    want, got = run_case(case(), "oracle"), run_case(case(), "gpu")
+    for a, b in zip(want, got):
+        assert a.shape == b.shape and np.array_equal(a, b), (quant, shape, int((a != b).sum()))
