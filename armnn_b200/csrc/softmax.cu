@@ -116,22 +116,29 @@ __global__ void __launch_bounds__(SM_THREADS) softmax_kernel(const SoftmaxArgs a
 // exponentials to shared memory; one warp of the block then runs all the block's chains, a row per lane (a pitch of 4 mod
 // 32 words makes eight lanes' 128-bit reads one conflict-free wavefront), while the SM's other blocks compute; finally
 // every warp divides and re-quantises its rows.
-// The division and the re-quantisation are one multiplication by 1 / (sum * output scale): its result is within 4e-7
-// relative of the reference's twice-rounded quotient, so whenever it is not within 1e-3 of a rounding boundary it rounds
-// to the same integer; the rest (a group of four in a hundred) take the reference's divisions.
-// Bound by instruction issue, about 20 per element, eight of them expf; a chain of 512 takes about 2300 cycles, which is
-// why a block's rows share one (with eight rows per warp and a chain per warp the chains alone took a quarter of the
-// issue slots).  32768 rows of 512: 101.9 us with one CTA and one summing thread per row,
-// 25.7 us now.
+// The division and the re-quantisation are one multiplication by 1 / (sum * output scale) and a test that its error cannot matter
+// (rows_sure); a value that fails it, one in 3500, takes the reference's divisions with its group of four, and so does its warp.
+// Bound by instruction issue, about 16 per element, eight of them expf; a chain of 512 takes about 2300 cycles, while the SM's
+// other blocks compute: with four warps a block six of them, and whatever phase one is in, others are in the other two.
+// 32768 rows of 512: 101.9 us with one CTA and one summing thread per row; 28.7 with a margin of 1e-3 in the test (a group in a
+// hundred, but one warp in three) and eight warps per block, 25.5 now (both alone, with cold caches).
 constexpr int SMR_ROWS = 4, SMR_MAX_AXIS = 2048;             // rows per warp
 
 struct RowsArgs {
     const uint8_t* x; uint8_t* y;
     uint32_t flip;                               // 0x80 for int8 input: bytes are compared and converted as byte + 128
-    float off_x, sx, beta, sy, zy, tlo, thi;
+    float off_x, sx, beta, sy, zy, tlo, thi, sure;
     int axis, pitch;
     long long rows;
 };
+// How far e / (s sy) + zy, evaluated as fma(e, 1 / (s sy), zy), may lie from an integer for the reference's value, two rounded
+// divisions and a rounding, to be that integer.  With u = 2^-24 the product differs from the quotient by 2 u, the reference's
+// by another 2 u, relative to a quotient of at most 257 + |zy| where the result does not saturate; the sum is rounded once more.
+static float rows_sure(int zp)
+{
+    const double error = 1.1 * 5.9604645e-8 * (4.01 * (257.0 + fabs((double)zp)) + 257.0);
+    return error < 0.25 ? (float)(0.5 - error) : -1.0f;      // (-1: nothing is sure)
+}
 
 // WPL: 4-byte words per lane and row (axis <= 128 WPL).  WORDS: rows are whole 4-byte words; otherwise every lane handles
 // single bytes, 32 apart.
@@ -225,7 +232,7 @@ __global__ void __launch_bounds__(32 * WARPS) softmax_rows_kernel(const RowsArgs
                 unpack2(z01, z[0], z[1]); unpack2(z23, z[2], z[3]);
                 unpack2(sub2(q01, z01), d[0], d[1]); unpack2(sub2(q23, z23), d[2], d[3]);
                 // (an exponential that overflowed, as with a negative beta, leaves NaN)
-                if (!(max4_nan(fabsf(d[0]), fabsf(d[1]), fabsf(d[2]), fabsf(d[3])) < 0.499f)) {
+                if (!(max4_nan(fabsf(d[0]), fabsf(d[1]), fabsf(d[2]), fabsf(d[3])) < a.sure)) {
                     z[0] = exact(v.x, s); z[1] = exact(v.y, s); z[2] = exact(v.z, s); z[3] = exact(v.w, s);
                 }
                 ((uint32_t*)y)[i] = sat_pack4(z, s8);
@@ -233,7 +240,7 @@ __global__ void __launch_bounds__(32 * WARPS) softmax_rows_kernel(const RowsArgs
         } else {
             for (int i = lane; i < a.axis; i += 32) {
                 const float q = __fmaf_rn(e[i], inv, a.zy), z = __fsub_rn(__fadd_rn(q, 12582912.0f), 12582912.0f);
-                const bool fine = fabsf(__fsub_rn(q, z)) < 0.499f;
+                const bool fine = fabsf(__fsub_rn(q, z)) < a.sure;
                 y[i] = (uint8_t)(int)(fine ? fminf(fmaxf(z, a.tlo), a.thi) : exact(e[i], s));
             }
         }
@@ -335,6 +342,7 @@ static int launch_rows(const b200k_softmax_params* p, void* stream, int mode, co
         r.off_x = 8388608.0f + (float)(p->x.zero_point + (int)r.flip);
         r.sx = p->x.scale; r.beta = p->beta; r.sy = p->y.scale; r.zy = (float)p->y.zero_point;
         r.tlo = a.y.tlo; r.thi = a.y.thi;
+        r.sure = rows_sure(p->y.zero_point);
         r.axis = p->axis_size; r.pitch = (p->axis_size + 27) / 32 * 32 + 4; r.rows = rows;
         const bool words = (p->axis_size & 3) == 0 && (((uintptr_t)p->x.data | (uintptr_t)p->y.data) & 3) == 0;
         auto go = [&](auto tag, int warps) -> int {
@@ -346,7 +354,8 @@ static int launch_rows(const b200k_softmax_params* p, void* stream, int mode, co
         // 66 KiB of exponentials per block at most: three blocks per SM
         if (words) {
             if (p->axis_size <= 128)  return go(KernelTag<softmax_rows_kernel<1, true, 8>>(), 8);
-            if (p->axis_size <= 512)  return go(KernelTag<softmax_rows_kernel<4, true, 8>>(), 8);
+            // (rows of 512: 96.9 us for an attention layer with two warps per block, 96.5 with four, 99.1 with eight, 100.5 with one)
+            if (p->axis_size <= 512)  return go(KernelTag<softmax_rows_kernel<4, true, 4>>(), 4);
             if (p->axis_size <= 1024) return go(KernelTag<softmax_rows_kernel<8, true, 4>>(), 4);
             return go(KernelTag<softmax_rows_kernel<16, true, 2>>(), 2);
         }
