@@ -387,7 +387,7 @@ __device__ __forceinline__ void requant_fast2(int acc0, int acc1, f32x2 m2, f32x
 
 
 // zero point + round_half_away(fl(v / sy)) of four values (integer-valued floats, not clamped): Markstein's correctly
-// rounded quotient with inv = RN(1 / sy), the 1.5 * 2^23 constant, roundf for exact halves (see requant_fast; values too
+// rounded quotient with inv = RN(1 / sy), the 1.5 * 2^23 constant, exact halves put right (see requant_fast; values too
 // large for the constant are far outside every 8-bit range).  One test for the four.
 struct Quant4 {
     float sy, inv_sy, zy;
@@ -404,9 +404,14 @@ struct Quant4 {
             float q[4], n[4];
             unpack2(q01, q[0], q[1]); unpack2(q23, q[2], q[3]);
             unpack2(n01, n[0], n[1]); unpack2(n23, n[2], n[3]);
+            // An exact half that the constant rounded towards zero goes the other way.  (Interpolation and sums of tensors whose
+            // scales are in simple ratios are full of halves: a Resize, an Add and an ArgMax of 11 MB took 32.6 us with the
+            // calls of roundf that were here, and take 29.3.)
             #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (fabsf(d[k]) >= 0.5f) n[k] = roundf(q[k]);
+            for (int k = 0; k < 4; ++k) {
+                const float h = copysignf(0.5f, q[k]);
+                if (d[k] == h) n[k] = __fadd_rn(q[k], h);
+            }
             n01 = pack2(n[0], n[1]); n23 = pack2(n[2], n[3]);
         }
         unpack2(add2(n01, zy2), z[0], z[1]);

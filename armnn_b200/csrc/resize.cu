@@ -95,7 +95,7 @@ __device__ __forceinline__ AxisSample axis_sample(int o, float scale, bool half,
 // weights are worked out once, and the two horizontally interpolated input rows are kept while the output rows stay
 // between them, so an enlarged row costs the vertical interpolation and the requantisation only.  Instruction-bound:
 // 8 x 64 x 64 x 21 -> 256 x 256 took 117 us with one element per thread (64-bit index divisions, coordinates and four
-// samples for every element), 13.8 us now.
+// samples for every element), 13.8 with a division and a coordinate per byte in the set-up and roundf for exact halves, about 11 now.
 constexpr int RZ_ROWS = 16, RZ_THREADS = 128;
 
 template <bool BILINEAR>
@@ -114,12 +114,24 @@ __global__ void __launch_bounds__(RZ_THREADS) resize_rows_kernel(const ResizeArg
     uint8_t* y = (uint8_t*)a.y.data + ((long long)n * a.OH + oy0) * width + j0;
     int off0[4], off1[4];
     float xw[4];
-    #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int j = min(j0 + k, width - 1), ox = j / a.C, c = j - ox * a.C;
-        const AxisSample s = axis_sample(ox, a.scale_x, half, a.method, align, a.IW);
-        off0[k] = s.i0 * a.C + c; off1[k] = s.i1 * a.C + c;
-        xw[k] = s.w;
+    if (a.C >= 4) {                                          // four bytes of at most two neighbouring pixels
+        const int ox = j0 / a.C, c0 = j0 - ox * a.C;
+        const AxisSample s0 = axis_sample(ox, a.scale_x, half, a.method, align, a.IW), s1 = axis_sample(min(ox + 1, a.OW - 1), a.scale_x, half, a.method, align, a.IW);
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool second = c0 + k >= a.C;
+            const int c = second ? c0 + k - a.C : c0 + k;    // (bytes beyond the row: any of the row's samples)
+            off0[k] = (second ? s1.i0 : s0.i0) * a.C + c; off1[k] = (second ? s1.i1 : s0.i1) * a.C + c;
+            xw[k] = second ? s1.w : s0.w;
+        }
+    } else {
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int j = min(j0 + k, width - 1), ox = j / a.C, c = j - ox * a.C;
+            const AxisSample s = axis_sample(ox, a.scale_x, half, a.method, align, a.IW);
+            off0[k] = s.i0 * a.C + c; off1[k] = s.i1 * a.C + c;
+            xw[k] = s.w;
+        }
     }
     // a byte as a float: 2^23 + byte (int8: + 128), minus 2^23 and the zero point (see bytes_minus_zp)
     const bool su = a.x.dtype == B200K_U8;
