@@ -263,6 +263,46 @@ __device__ __forceinline__ void tma_load_im2col_s(uint32_t dst, const CUtensorMa
                  " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
                  ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h) : "memory");
 }
+// CTA pairs (cta_group::2): loads into this CTA's shared memory that signal a barrier of either CTA, MMAs over both CTAs' operands
+// and accumulators, commits that arrive at the same barrier of both.
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank)          // the address in CTA `rank` of what saddr is here
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y)
+{
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void pair_load_im2col(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c, int w, int h, int n, uint16_t off_w, uint16_t off_h)
+{
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes.cta_group::2"
+                 " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+                 ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h) : "memory");
+}
+__device__ __forceinline__ void pair_commit(uint32_t bar)
+{
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void pair_mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx_s(uint32_t bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -692,7 +732,12 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 // What a launch ends in is compiled in (MODE), so that none carries the others' code and registers: no fused Add; a fused Add by
 // its table or by its formula, each with the per-channel constants in shared memory or in the parameter space.
 enum { TC_PLAIN = 0, TC_LUT = 1, TC_LUT_PTAB = 2, TC_ADD = 3, TC_ADD_PTAB = 4 };
-template <int BN, int SWZ, int EG, int MODE>
+//
+// PAIR: two CTAs of a cluster work on two neighbouring M-tiles and one n-tile as one 256 x BN MMA: each loads its own 128 rows of A
+// and half of the weight tile, the first CTA's issuer multiplies for both, each reads its own accumulators.  A wide tile's
+// weights come from L2 once per pair, and what a CTA loads per K-slice goes from 128 + 256 rows to 128 + 128: with
+// K of a thousand and more the loads, not the MMAs, bound the wide tiles.
+template <int BN, int SWZ, int EG, int MODE, bool PAIR = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmR,
@@ -700,6 +745,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 {
     constexpr bool PTAB = MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB, fused = MODE != TC_PLAIN, formula = MODE == TC_ADD || MODE == TC_ADD_PTAB;
     using L = TcSmem<BN, SWZ>;
+    static_assert(!PAIR || (EG == 1 && SWZ == 128), "CTA pairs: one tile per CTA in the epilogue");
+    constexpr int B_BYTES = PAIR ? L::B_BYTES / 2 : L::B_BYTES;          // what this CTA loads of a slice's weight tile
+    const uint32_t rank = PAIR ? cluster_rank() : 0u;
     constexpr int MAX_STAGES = L::MAX_STAGES;
     constexpr int UW = L::UW, UNITS = L::UNITS, IO_BYTES = L::IO_BYTES;
     constexpr int NACC_LOG2 = EG == 1 ? 1 : (EG == 2 ? 2 : 3);          // 2, 4 or 8 accumulator buffers in TMEM
@@ -714,7 +762,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint8_t* s_zw = smem;
     uint8_t* s_wst = smem + (size_t)a.nzw * L::B_BYTES;
     // weight-stationary launches: all K-slices of the (only) weight tile first, then a ring of activation tiles only
-    const int stage_stride = a.bstat ? L::A_BYTES : L::STAGE_BYTES;
+    const int stage_stride = a.bstat ? L::A_BYTES : L::A_BYTES + B_BYTES;
     uint8_t* ring = s_wst + (a.bstat ? (size_t)a.nslices * L::B_BYTES : 0);
     uint8_t* s_io = ring + (size_t)STAGES * a.group * stage_stride;
     float* s_m = (float*)(s_io + (size_t)(a.nstg * EG + NIO) * IO_BYTES);   // first the warps' staging buffers (nstg * eg units' worth), then NIO operand units
@@ -743,7 +791,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");     // the next kernel of the stream may begin its set-up
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp: provably uniform
     const int ntn = a.ntn;                                  // n-tiles; the last one may reach beyond OC (zero weights, clipped stores)
-    const int ntiles = ntn * a.ntm;
+    const int ntiles = ntn * (PAIR ? (a.ntm + 1) / 2 : a.ntm);          // (of pairs: the last one's second tile may lie beyond M)
+    const int tile0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, tstep = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 
     {
         // the barriers lie in one array (full, empty, acc_full, acc_empty, io_full, io_empty, w_full, lut_full): one
@@ -753,13 +802,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (i < NBAR) {
             const bool acc_e = i >= 2 * MAX_STAGES + L::MAX_ACC && i < 2 * MAX_STAGES + 2 * L::MAX_ACC;
             const bool io_e = i >= 2 * MAX_STAGES + 2 * L::MAX_ACC + L::MAX_IO && i < 2 * MAX_STAGES + 2 * L::MAX_ACC + 2 * L::MAX_IO;
-            mbar_init(&full[i], acc_e ? TC_EPI_WARPS / EG : (io_e ? TC_EPI_WARPS : 1));
+            mbar_init(&full[i], acc_e ? (PAIR ? 2 : 1) * TC_EPI_WARPS / EG : (io_e ? TC_EPI_WARPS : 1));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(BN << NACC_LOG2) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(BN << NACC_LOG2) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(BN << NACC_LOG2) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     if (a.nzw) {
         // BN identical logical rows (in row-window mode: zero on the bytes of a slice that are no real taps), each stored
@@ -782,6 +836,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();                     // both CTAs' barriers are there before either signals the other's
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     if (threadIdx.x == 0) TC_TRACE(1);
@@ -802,6 +857,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int ub = 0; uint32_t uph = 0;                    // unit-buffer position (kept without divisions)
             bool alive = true;
             const uint32_t ring_addr = smem_u32(ring), full_addr = smem_u32(full), empty_addr = smem_u32(empty);
+            const uint32_t signal_addr = PAIR ? cluster_map(full_addr, 0u) : full_addr;      // (pairs: the first CTA's barriers count both CTAs' loads)
             const uint32_t tab_addr = smem_u32(s_tab);
             const int mode = a.im2col;
             const bool bstat = a.bstat != 0, skip_loads = a.skip_loads != 0;
@@ -828,21 +884,24 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (elect_one()) {
                     const uint32_t fb = full_addr + g * 8;
                     uint32_t sa = ring_addr + (uint32_t)g * group_stride + L::A_BYTES;
-                    mbar_expect_tx_s(fb, group_tx);
-                    for (int gs = 0; gs < group; ++gs, sa += (uint32_t)stage_stride)
-                        tma_load_2d_s(sa, &tmB, fb, (int)lds128(tab_addr + 16u * (uint32_t)(g * group + gs)).z, ((int)blockIdx.x % ntn) * BN);
+                    if (!PAIR || rank == 0) mbar_expect_tx_s(fb, group_tx);
+                    for (int gs = 0; gs < group; ++gs, sa += (uint32_t)stage_stride) {
+                        const int col = (int)lds128(tab_addr + 16u * (uint32_t)(g * group + gs)).z, n0 = (tile0 % ntn) * BN;
+                        if constexpr (PAIR) pair_load_2d(sa, &tmB, signal_addr + g * 8, col, n0 + (int)rank * (BN / 2));
+                        else                tma_load_2d_s(sa, &tmB, fb, col, n0);
+                    }
                 }
             }
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
-                if (prod == 0 && t == blockIdx.x) TC_TRACE(2);
+            for (int t = tile0; t < ntiles && alive; t += tstep) {
+                if (prod == 0 && t == tile0) TC_TRACE(2);
                 // tile coordinates: only worked out by a producer that loads something of this tile
                 int n0 = 0, tm = 0, w0 = 0, h0 = 0, nimg = 0;
                 long long m0 = 0;
                 bool have = false;
                 auto locate = [&]() {
                     n0 = (t % ntn) * BN;
-                    tm = t / ntn;
+                    tm = PAIR ? t / ntn * 2 + (int)rank : t / ntn;
                     m0 = (long long)tm * a.tile_rows;
                     if (a.im2col == 2) {
                         nimg = tm / a.OH;
@@ -866,10 +925,17 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         // (self-test: no loads are issued, so the stage never fills and every waiter runs into its limit)
                         if (alive && !skip_loads && elect_one()) {
                             const bool weights = !bstat && ahead <= 0;
-                            if (ahead <= 0) mbar_expect_tx_s(fb, group_tx);
+                            if (ahead <= 0 && (!PAIR || rank == 0)) mbar_expect_tx_s(fb, group_tx);
                             uint32_t sa = ring_addr + (uint32_t)st * group_stride;
                             for (int gs = 0; gs < group; ++gs, sa += (uint32_t)stage_stride) {
                                 const uint4 e = lds128(te + 16u * (uint32_t)gs);
+                                if constexpr (PAIR) {
+                                    const uint32_t sb = signal_addr + st * 8;
+                                    if (mode == 1) pair_load_im2col(sa, &tmA, sb, (int)e.x, w0, h0, nimg, (uint16_t)(e.y & 0xffffu), (uint16_t)(e.y >> 16));
+                                    else           pair_load_2d(sa, &tmA, sb, (int)e.x, (int)m0);
+                                    if (weights) pair_load_2d(sa + L::A_BYTES, &tmB, sb, (int)e.z, n0 + (int)rank * (BN / 2));
+                                    continue;
+                                }
                                 if (mode == 2)      tma_load_4d_s(sa, &tmA, fb, 0, 0, h0 + (int)e.w, nimg);      // slice = filter row
                                 else if (mode == 1) tma_load_im2col_s(sa, &tmA, fb, (int)e.x, w0, h0, nimg, (uint16_t)(e.y & 0xffffu), (uint16_t)(e.y >> 16));
                                 else                tma_load_2d_s(sa, &tmA, fb, (int)e.x, (int)m0);
@@ -881,7 +947,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     ahead = max(ahead - 1, 0);
                     if (++st == STAGES) { st = 0; ph ^= 1u; }
                 }
-                if (prod == 0 && (t - (int)blockIdx.x) / (int)gridDim.x < 8) TC_TRACE(16 + (t - (int)blockIdx.x) / (int)gridDim.x);
+                if (prod == 0 && (t - tile0) / tstep < 8) TC_TRACE(16 + (t - tile0) / tstep);
                 if (fused && alive && !skip_loads && prod == 0) {
                     // the fused Add's other operand, one unit at a time, into the buffer the epilogue will overwrite
                     if (!have) locate();
@@ -898,12 +964,12 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        // ===================== MMA issuer =====================
-        {
+        // ===================== MMA issuer (of a pair: the first CTA's) =====================
+        if (!PAIR || rank == 0) {
             // instruction descriptor: D = S32 (bits 4-5 = 2); A / B format at bits 7 / 10 (1 = signed 8-bit,
             // 0 = unsigned 8-bit); both operands K-major (bits 15, 16 = 0); N >> 3 at bit 17; M >> 4 at bit 24
             const uint32_t id = (2u << 4) | ((uint32_t)a.a_signed << 7) | ((uint32_t)a.b_signed << 10) |
-                                ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+                                ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((PAIR ? 2 : 1) * TC_BM >> 4) << 24);
             // the zero-point MMAs: same A, B = a constant int8 tile
             const uint32_t id_zw = (2u << 4) | ((uint32_t)a.a_signed << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
             const int group = a.group, gpt = a.nslices / a.group;          // slices per stage, stages per tile
@@ -925,7 +991,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (bstat && !__all_sync(0xffffffffu, mbar_wait(w_full, 0, wait_limit))) { atomicExch(&g_tc_status, 7); alive = false; }
             TC_TRACE(3);
             tc_fence_after();
-            for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x, ++it) {
+            for (int t = tile0; t < ntiles && alive; t += tstep, ++it) {
                 const int buf = it & ((1 << NACC_LOG2) - 1);
                 // the epilogue must have drained this accumulator buffer (one round of the buffers ago)
                 if (!__all_sync(0xffffffffu, mbar_wait_idle(smem_u32(&acc_empty[buf]), (((uint32_t)it >> NACC_LOG2) & 1u) ^ 1u, wait_limit))) { atomicExch(&g_tc_status, 4); break; }
@@ -940,6 +1006,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         uint64_t da = da0 + dgroup * (uint64_t)st;
                         uint64_t db = bstat ? dbs : db0 + dgroup * (uint64_t)st;
                         for (int gs = 0; gs < group; ++gs, da += dstage, db += dbstep) {
+                            if constexpr (PAIR) {
+                                #pragma unroll
+                                for (int k = 0; k < SWZ / 32; ++k) pair_mma_i8(tacc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), id, (uint32_t)(g | gs | k));
+                                continue;
+                            }
                             tc_mma_i8(tacc, da, db, id, (uint32_t)(g | gs));        // the tile's first MMA overwrites
                             #pragma unroll
                             for (int k = 1; k < SWZ / 32; ++k) tc_mma_i8_acc(tacc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), id);
@@ -949,11 +1020,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 for (int k = 0; k < SWZ / 32; ++k) tc_mma_i8_acc(tacc, da + (uint64_t)(k * 2), dz + (uint64_t)(k * 2), id_zw);
                             }
                         }
-                        tc_commit_s(eb);           // stage reusable once these MMAs have read it
+                        if constexpr (PAIR) pair_commit(eb);
+                        else tc_commit_s(eb);      // stage reusable once these MMAs have read it
                     }
                     if (++st == STAGES) { st = 0; ph ^= 1u; }
                 }
-                if (alive && elect_one()) tc_commit(&acc_full[buf]);  // accumulator of this tile complete
+                if (alive && elect_one()) {                          // accumulator of this tile complete
+                    if constexpr (PAIR) pair_commit(smem_u32(&acc_full[buf]));
+                    else tc_commit(&acc_full[buf]);
+                }
                 if (it == 0) TC_TRACE(4);
                 if (it < 8) TC_TRACE(24 + it);
             }
@@ -1135,17 +1210,18 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int it = 0;
             int ub = 0; uint32_t uph = 0;                    // operand-buffer position (kept without divisions)
             uint32_t st_base = st_base0;
-            for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+            for (int t = tile0; t < ntiles; t += tstep, ++it) {
                 if ((it & (eg - 1)) != grp) continue;
                 // (a single n-tile is the common case of the epilogue-bound layers: no divisions then)
-                const int tm = ntn == 1 ? t : t / ntn;
-                const int n0 = ntn == 1 ? 0 : (t - tm * ntn) * BN;
+                const int tq = ntn == 1 ? t : t / ntn;
+                const int n0 = ntn == 1 ? 0 : (t - tq * ntn) * BN;
+                const int tm = PAIR ? tq * 2 + (int)rank : tq;
                 const long long m0 = (long long)tm * a.tile_rows;
                 const int buf = it & ((1 << NACC_LOG2) - 1);
                 if (eg == 1 && n0 != cur_n0) stage_constants(n0);
                 if (ew == 0 && it < 8) TC_TRACE(56 + it);
                 if (!dead && !mbar_wait(&acc_full[buf], ((uint32_t)it >> NACC_LOG2) & 1u, a.wait_limit)) { atomicExch(&g_tc_status, 3); dead = true; }
-                if (ew == 0 && t == blockIdx.x) TC_TRACE(7);
+                if (ew == 0 && t == tile0) TC_TRACE(7);
                 if (ew == 0 && it < 8) TC_TRACE(32 + it);
                 tc_fence_after();
                 const long long m = m0 + row;
@@ -1235,8 +1311,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (ew == 0 && it < 8) TC_TRACE(48 + it);
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[buf]);
-                if (ew == 0 && t == blockIdx.x) TC_TRACE(8);
+                if (lane == 0) {
+                    if constexpr (PAIR) mbar_arrive_cluster(cluster_map(smem_u32(&acc_empty[buf]), 0u));
+                    else mbar_arrive(&acc_empty[buf]);
+                }
+                if (ew == 0 && t == tile0) TC_TRACE(8);
                 if (ew == 0 && it < 8) TC_TRACE(40 + it);
                 if (ew == 0) TC_TRACE(9);
             }
@@ -1248,9 +1327,11 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();                     // neither CTA's shared memory goes while the other may use it
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(BN << NACC_LOG2) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(BN << NACC_LOG2) : "memory");
+        else                asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(BN << NACC_LOG2) : "memory");
         TC_TRACE(11);
     }
 }
@@ -1586,17 +1667,44 @@ bool conv_tc_eligible(const b200k_conv2d_params* p)
 }
 
 
-template <int BN, int SWZ, int EG, int MODE = TC_PLAIN>
+// How many CTA pairs the device can run at once (0: none).
+static int tc_pairs()
+{
+    constexpr auto kern = conv_tc_kernel<256, 128, 1, TC_PLAIN, true>;
+    static std::atomic<int> counts[MAX_DEVICES];             // count + 1
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 0;
+    int n = counts[dev].load(std::memory_order_relaxed);
+    if (n > 0) return n - 1;
+    const size_t smem = 227 * 1024;
+    if (allow_shared<kern>(smem) != B200K_OK) return 0;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(sm_count() & ~1), 1, 1);
+    cfg.blockDim = dim3(TC_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    counts[dev].store(n + 1, std::memory_order_relaxed);
+    return n;
+}
+
+template <int BN, int SWZ, int EG, int MODE = TC_PLAIN, bool PAIR = false>
 static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR,
                      const TcArgs& a, cudaStream_t stream, const TcTabs* tabs = nullptr, bool formula = false)
 {
-    if constexpr (EG == 1 && MODE == TC_PLAIN) {
+    if constexpr (EG == 1 && MODE == TC_PLAIN && !PAIR) {
         if (a.res) {
             if (formula) return tabs ? launch_tc<BN, SWZ, EG, TC_ADD_PTAB>(tmA, tmB, tmY, tmR, a, stream, tabs) : launch_tc<BN, SWZ, EG, TC_ADD>(tmA, tmB, tmY, tmR, a, stream);
             return tabs ? launch_tc<BN, SWZ, EG, TC_LUT_PTAB>(tmA, tmB, tmY, tmR, a, stream, tabs) : launch_tc<BN, SWZ, EG, TC_LUT>(tmA, tmB, tmY, tmR, a, stream);
         }
     }
     using L = TcSmem<BN, SWZ>;
+    constexpr size_t slice = PAIR ? L::A_BYTES + L::B_BYTES / 2 : L::STAGE_BYTES;
     const size_t budget = 227 * 1024;                                   // opt-in shared memory per CTA on sm_100
     TcArgs a2 = a;
     size_t rest = 1024 + L::CONST_BYTES + ((size_t)a.ncls * 2 + 1) * BN * 4 + 16 + 64 + (size_t)(EG + a.nio) * L::IO_BYTES + (a.add_lut ? TC_LUT_BYTES : 0) + 256 +
@@ -1605,14 +1713,14 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     // a second staging buffer per epilogue warp, then a third buffer for the fused Add's other operand (its loads then
     // run a whole unit ahead of the epilogue), each when the ring keeps at least three stages
     a2.nstg = 1;
-    if (rest + (size_t)EG * L::IO_BYTES + 3 * L::STAGE_BYTES <= budget) { a2.nstg = 2; rest += (size_t)EG * L::IO_BYTES; }
-    if (a.nio == 2 && rest + L::IO_BYTES + 3 * L::STAGE_BYTES <= budget) { a2.nio = 3; rest += L::IO_BYTES; }
-    B200K_REQUIRE(rest + 2 * L::STAGE_BYTES <= budget, B200K_E_TOOBIG, "conv2d_q8: shared memory exhausted (%zu bytes of tables)", rest);
+    if (rest + (size_t)EG * L::IO_BYTES + 3 * slice <= budget) { a2.nstg = 2; rest += (size_t)EG * L::IO_BYTES; }
+    if (a.nio == 2 && rest + L::IO_BYTES + 3 * slice <= budget) { a2.nio = 3; rest += L::IO_BYTES; }
+    B200K_REQUIRE(rest + 2 * slice <= budget, B200K_E_TOOBIG, "conv2d_q8: shared memory exhausted (%zu bytes of tables)", rest);
     // One n-tile and a weight tile of at most 64 KiB over all of K: keep it in shared memory for the whole launch, so
     // that the ring (and the L2 bandwidth behind it) carries activations only.
     const size_t wbytes = (size_t)a.nslices * L::B_BYTES;
-    a2.bstat = (a.ntn == 1 && wbytes <= 64 * 1024 && rest + wbytes + 4 * L::A_BYTES <= budget) ? 1 : 0;
-    const size_t stride = a2.bstat ? L::A_BYTES : L::STAGE_BYTES;
+    a2.bstat = (!PAIR && a.ntn == 1 && wbytes <= 64 * 1024 && rest + wbytes + 4 * L::A_BYTES <= budget) ? 1 : 0;
+    const size_t stride = a2.bstat ? L::A_BYTES : slice;
     const size_t fixed = rest + (a2.bstat ? wbytes : 0);
     // Ring: `stages` stages of `group` K-slices each.  Waiting for a stage, arming and releasing its barriers cost the
     // producer and the MMA issuer about as much as issuing two MMAs, so narrow tiles (short MMAs) want several slices per
@@ -1632,11 +1740,13 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     // slices back) must lie within the same ring pass as the slot it waits for, i.e. nprod <= stages.
     a2.nprod = stages >= TC_PRODUCERS ? TC_PRODUCERS : (stages >= 2 ? 2 : 1);
     if (a2.bstat) a2.stage_tx = (uint32_t)(a.stage_tx - L::B_BYTES);
+    if (PAIR) a2.stage_tx = (uint32_t)(2 * slice);            // (counted by the first CTA's barrier, for both)
     const size_t smem = fixed + (size_t)stages * group * stride;
-    auto kern = conv_tc_kernel<BN, SWZ, EG, MODE>;
-    if (const int rc = allow_shared<conv_tc_kernel<BN, SWZ, EG, MODE>>(smem)) return rc;
+    auto kern = conv_tc_kernel<BN, SWZ, EG, MODE, PAIR>;
+    if (const int rc = allow_shared<conv_tc_kernel<BN, SWZ, EG, MODE, PAIR>>(smem)) return rc;
     const long long tiles = (long long)a.ntn * a.ntm;
-    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+    const long long pairs = (long long)a.ntn * ((a.ntm + 1) / 2);
+    const int grid = PAIR ? 2 * (int)(pairs < tc_pairs() ? pairs : tc_pairs()) : (int)(tiles < sm_count() ? tiles : sm_count());
     // Programmatic dependent launch: the grid may start while its predecessor in the stream drains (its set-up touches
     // nothing the predecessor writes); the producer threads wait for the predecessor before their first activation load.
     cudaLaunchConfig_t cfg;
@@ -1645,11 +1755,13 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     cfg.blockDim = dim3(TC_THREADS, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = PAIR ? 2 : 1;
     if constexpr (MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB) {
         B200K_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmY, tmR, a2, *tabs));
     } else {
@@ -2404,7 +2516,12 @@ int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid
     a.skip_loads = p->selftest_us > 0 ? 1 : 0;
     a.wait_limit = p->selftest_us > 0 ? (long long)p->selftest_us * 2000ll : TC_WAIT_LIMIT_CYCLES;
 
-    const int bn = pick_bn(p->oc, a.ntm);
+    // CTA pairs on 256 x 256 tiles: from K = 2048 on (16 slices), where the loads bound a wide tile, and with a tile for every
+    // pair.  FullyConnected 4096 x 4096 x 4096 takes 55.2 us without and 48.5 with them, 512 -> 512 channels, 3 x 3, 64 x 14 x 14
+    // 36.5 and 33.7; all of ResNet-50 at batch 256 2685 from 16 slices on, 2686 from 9, 2702 from 4 (K = 1024 gains nothing).
+    const bool pair = swz == 128 && !row_mode && a.nzw == 0 && !fa.res && p->selftest_us == 0 && p->oc >= 256 && (size_t)a.ncls * 256 * 4 <= 32 * 1024 &&
+                      a.nslices >= 16 && ((p->oc + 255) / 256) * (((long long)a.ntm + 1) / 2) >= tc_pairs() && tc_pairs() > 0;
+    const int bn = pair ? 256 : pick_bn(p->oc, a.ntm);
     a.ntn = (p->oc + bn - 1) / bn;
     CUtensorMap tmA, tmB;
     const CUtensorMapSwizzle swizzle = swz == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
@@ -2414,7 +2531,7 @@ int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid
         const void* wptr = row_mode ? (const void*)((const uint8_t*)p->packed + rowp.wpack_offset) : p->w.data;
         cuuint64_t dims[2] = {K, (cuuint64_t)p->oc};
         cuuint64_t strides[1] = {K};
-        cuuint32_t box[2] = {(cuuint32_t)swz, (cuuint32_t)bn};
+        cuuint32_t box[2] = {(cuuint32_t)swz, (cuuint32_t)(pair ? bn / 2 : bn)};
         cuuint32_t estr[2] = {1, 1};
         CUresult r = g_encode_tiled(&tmB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)wptr, dims, strides, box, estr,
                                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -2528,6 +2645,7 @@ int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid
         }
     }
     if (swz == 128) {
+        if (pair) return launch_tc<256, 128, 1, TC_PLAIN, true>(tmA, tmB, tmY, tmR, a, stream);
         if (bn == 256) return launch_tc<256, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
         if (bn == 128) return grouped ? launch_tc<128, 128, 2>(tmA, tmB, tmY, tmR, a, stream) : launch_tc<128, 128, 1>(tmA, tmB, tmY, tmR, a, stream, host_tabs, formula);
         if (a.eg == 2) return launch_tc<64, 128, 2>(tmA, tmB, tmY, tmR, a, stream);
