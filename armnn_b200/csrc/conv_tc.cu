@@ -1793,9 +1793,16 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
 constexpr int ST_SLOTS = 32;                    // packed-row ring (a power of two)
 constexpr int ST_LOOKAHEAD = 4;                 // tiles the expanders may run ahead of the MMAs
 constexpr int ST_DONE = 8;                      // ring of per-tile "MMAs complete" barriers (a power of two)
-constexpr int ST_EXPANDERS = 4;
+// Eight warps expand rows: with four a tile waited for its two new rows.  ResNet-50's stem at batch 256 takes 269 us with four
+// expanders and one issuer, 213 with eight and two, 230 or more with only one of the two.
+constexpr int ST_EXPANDERS = 8;
 constexpr int ST_RAW = 16;                      // ring of raw input rows (bulk copies in flight ahead of the expanders)
-constexpr int ST_THREADS = 32 * (2 + ST_EXPANDERS + TC_EPI_WARPS);     // MMA issuer, row loader, expanders, epilogue
+constexpr int ST_ACC = 4;                       // accumulator buffers at most
+// Waiting for a tile's rows and issuing its MMAs takes a warp 1.3 us, of which the MMAs themselves are a fraction: two warps issue,
+// every other tile each.
+constexpr int ST_ISSUERS = 2;
+// issuer, row loader, expanders, epilogue, the other issuer
+constexpr int ST_THREADS = 32 * (1 + ST_EXPANDERS + TC_EPI_WARPS + ST_ISSUERS);
 
 struct StemArgs {
     const uint8_t* x; uint8_t* y; int32_t* acc_out;
@@ -1803,7 +1810,7 @@ struct StemArgs {
     const int32_t* bias; const float* w_scales; const float* b_scales;
     float w_scale, b_scale;
     int N, H, W, C, OH, OW, OC, KH, KW, sh, sw, pt, pl;
-    int cpad, WB, slot_bytes, raw_bytes, Hp, Wp, tiles, tmem_cols;
+    int cpad, WB, slot_bytes, raw_bytes, Hp, Wp, tiles, tmem_cols, acc_log2;
     int split;                                  // 4-byte pixels, even / odd output pixels as the two 64-row halves of a tile
     int zx, a_signed, b_signed, acc_big;
     Requant rq;
@@ -1837,9 +1844,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
     EpiExact* s_ex = (EpiExact*)(s_emax + 4);
     uint64_t* row_full = (uint64_t*)(s_emax + 4 + 16);                 // [ST_SLOTS]
     uint64_t* mma_done = row_full + ST_SLOTS;                          // [ST_DONE]
-    uint64_t* acc_full = mma_done + ST_DONE;                           // [2]
-    uint64_t* acc_empty = acc_full + 2;                                // [2]
-    uint64_t* w_full = acc_empty + 2;
+    uint64_t* acc_full = mma_done + ST_DONE;                           // [ST_ACC]
+    uint64_t* acc_empty = acc_full + ST_ACC;                           // [ST_ACC]
+    uint64_t* w_full = acc_empty + ST_ACC;
     uint64_t* raw_full = w_full + 1;                                   // [ST_RAW] a raw row has landed
     uint64_t* raw_empty = raw_full + ST_RAW;                           // [ST_RAW] its expander has read it
     uint32_t* tmem_slot = (uint32_t*)(raw_empty + ST_RAW);
@@ -1854,9 +1861,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
     const long long v0 = (long long)(t_begin / a.OH) * a.Hp + (long long)(t_begin % a.OH) * a.sh;     // first virtual row
     const long long wait_limit = a.wait_limit;
 
-    if (threadIdx.x < ST_SLOTS + ST_DONE + 5 + 2 * ST_RAW) {
+    const int acc_log2 = a.acc_log2, acc_mask = (1 << acc_log2) - 1;
+    if (threadIdx.x < ST_SLOTS + ST_DONE + 2 * ST_ACC + 1 + 2 * ST_RAW) {
         const int i = threadIdx.x;
-        mbar_init(&row_full[i], (i >= ST_SLOTS + ST_DONE + 2 && i < ST_SLOTS + ST_DONE + 4) ? TC_EPI_WARPS : 1);
+        mbar_init(&row_full[i], (i >= ST_SLOTS + ST_DONE + ST_ACC && i < ST_SLOTS + ST_DONE + 2 * ST_ACC) ? TC_EPI_WARPS : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (threadIdx.x < 4) s_emax[threadIdx.x] = 0u;
@@ -1869,9 +1877,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
-        // ===================== weights, then the MMAs =====================
-        if (elect_one()) {
+    const int issuer = warp == 0 ? 0 : warp - (1 + ST_EXPANDERS + TC_EPI_WARPS);       // (0 and from 1 on; the others are not above 0)
+    if (warp == 0 || issuer > 0) {
+        // ===================== weights, then the MMAs of every ST_ISSUERS-th tile =====================
+        if (warp == 0 && elect_one()) {
             const uint32_t wbytes = (uint32_t)(a.KH * a.OC * a.WB);
             mbar_expect_tx(w_full, wbytes);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -1893,14 +1902,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
         const int base_n = n, base_oy = oy;                 // (v0 = base_n * Hp + base_oy * sh)
         int waited = 0;                                      // packed rows [0, waited) have been seen complete
         for (int i = 0; i < ntiles && alive; ++i) {
+            if (i % ST_ISSUERS != issuer) { if (++oy == a.OH) { oy = 0; ++n; } continue; }
             const int lo = (n - base_n) * a.Hp + (oy - base_oy) * a.sh;                              // first packed row, relative
-            const int buf = i & 1;
+            const int buf = i & acc_mask;
             for (int rv = lo > waited ? lo : waited; rv < lo + a.KH && alive; ++rv) {
                 if (!__all_sync(0xffffffffu, mbar_wait(&row_full[rv & (ST_SLOTS - 1)], (uint32_t)(rv / ST_SLOTS) & 1u, wait_limit))) { atomicExch(&g_tc_status, 2); alive = false; }
             }
             waited = lo + a.KH;
             if (i < 8) TC_TRACE(16 + i);
-            if (alive && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (((uint32_t)i >> 1) & 1u) ^ 1u, wait_limit))) { atomicExch(&g_tc_status, 4); alive = false; }
+            if (alive && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (((uint32_t)i >> acc_log2) & 1u) ^ 1u, wait_limit))) { atomicExch(&g_tc_status, 4); alive = false; }
             if (!alive) break;
             tc_fence_after();
             if (elect_one()) {
@@ -2097,10 +2107,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
             // chunk k of tile i (this warp's k-th: column chunk part + 4 k); the first chunk of a tile waits for its accumulator
             auto issue = [&](int i, int k, uint32_t* dst) {
                 if (k == 0) {
-                    if (!dead && !mbar_wait(&acc_full[i & 1], ((uint32_t)i >> 1) & 1u, wait_limit)) { atomicExch(&g_tc_status, 3); dead = true; }
+                    if (!dead && !mbar_wait(&acc_full[i & acc_mask], ((uint32_t)i >> acc_log2) & 1u, wait_limit)) { atomicExch(&g_tc_status, 3); dead = true; }
                     tc_fence_after();
                 }
-                tc_ld16_issue(tmem_base + (uint32_t)((i & 1) * a.OC) + ((uint32_t)(quad * 32) << 16) + (uint32_t)((part + 4 * k) * 16), dst);
+                tc_ld16_issue(tmem_base + (uint32_t)((i & acc_mask) * a.OC) + ((uint32_t)(quad * 32) << 16) + (uint32_t)((part + 4 * k) * 16), dst);
             };
             int i = 0, k = 0;                                 // the chunk whose load is in flight / being worked on
             if (cpw > 0 && ntiles > 0) issue(0, 0, r0);
@@ -2115,7 +2125,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
                     // the warp's last chunk of tile i is in registers
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[i & 1]);
+                    if (lane == 0) mbar_arrive(&acc_empty[i & acc_mask]);
                     nk = 0; ni = i + 1;
                 }
                 if (ni < ntiles) issue(ni, nk, rn);
@@ -2154,9 +2164,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
             // warps without a chunk (fewer than four chunks per tile) still release every accumulator buffer
             if (cpw == 0) {
                 for (int j = 0; j < ntiles; ++j) {
-                    if (!dead && !mbar_wait(&acc_full[j & 1], ((uint32_t)j >> 1) & 1u, wait_limit)) { atomicExch(&g_tc_status, 3); dead = true; }
+                    if (!dead && !mbar_wait(&acc_full[j & acc_mask], ((uint32_t)j >> acc_log2) & 1u, wait_limit)) { atomicExch(&g_tc_status, 3); dead = true; }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[j & 1]);
+                    if (lane == 0) mbar_arrive(&acc_empty[j & acc_mask]);
                 }
             }
         };
@@ -2175,7 +2185,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
     }
 }
 
-struct StemPlan { bool ok; int cpad, WB, slot_bytes, raw_bytes, Wp, Hp, split; size_t wbytes, smem; int tmem_cols; };
+struct StemPlan { bool ok; int cpad, WB, slot_bytes, raw_bytes, Wp, Hp, split; size_t wbytes, smem; int tmem_cols, acc_log2; };
 
 static StemPlan stem_plan(const b200k_conv2d_params* p)
 {
@@ -2202,11 +2212,12 @@ static StemPlan stem_plan(const b200k_conv2d_params* p)
     r.wbytes = (size_t)p->kh * p->oc * r.WB;
     if (r.wbytes > 64 * 1024) return r;
     r.tmem_cols = 32;
-    while (r.tmem_cols < 2 * p->oc) r.tmem_cols <<= 1;
+    r.acc_log2 = p->oc * 4 <= 512 ? 2 : 1;
+    while (r.tmem_cols < p->oc << r.acc_log2) r.tmem_cols <<= 1;
     // raw rows arrive by bulk copies: whole rows of a multiple of 16 bytes
     if (((long long)p->wd * p->c) % 16 != 0) return r;
     r.raw_bytes = (p->wd * p->c + 8 + 127) & ~127;         // (+8: the expanders read whole words around a pixel)
-    r.smem = 1024 + (size_t)ST_SLOTS * r.slot_bytes + r.wbytes + (size_t)p->oc * 20 + 16 + 64 + (ST_SLOTS + ST_DONE + 5 + 2 * ST_RAW) * 8 + 16 +
+    r.smem = 1024 + (size_t)ST_SLOTS * r.slot_bytes + r.wbytes + (size_t)p->oc * 20 + 16 + 64 + (ST_SLOTS + ST_DONE + 2 * ST_ACC + 1 + 2 * ST_RAW) * 8 + 16 +
              128 + (size_t)ST_RAW * r.raw_bytes;
     r.ok = r.smem <= 227 * 1024;
     return r;
@@ -2267,7 +2278,7 @@ static int launch_conv_stem(const b200k_conv2d_params* p, cudaStream_t stream)
     a.KH = p->kh; a.KW = p->kw; a.sh = p->stride_h; a.sw = p->stride_w; a.pt = p->pad_top; a.pl = p->pad_left;
     a.cpad = pl.cpad; a.WB = pl.WB; a.slot_bytes = pl.slot_bytes; a.raw_bytes = pl.raw_bytes; a.Hp = pl.Hp; a.Wp = pl.Wp;
     a.split = pl.split;
-    a.tiles = p->n * p->oh; a.tmem_cols = pl.tmem_cols;
+    a.tiles = p->n * p->oh; a.tmem_cols = pl.tmem_cols; a.acc_log2 = pl.acc_log2;
     a.zx = p->x.zero_point;
     a.a_signed = p->x.dtype == B200K_S8; a.b_signed = p->w.dtype == B200K_S8;
     {
