@@ -1745,8 +1745,15 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
     auto kern = conv_tc_kernel<BN, SWZ, EG, MODE, PAIR>;
     if (const int rc = allow_shared<conv_tc_kernel<BN, SWZ, EG, MODE, PAIR>>(smem)) return rc;
     const long long tiles = (long long)a.ntn * a.ntm;
-    const long long pairs = (long long)a.ntn * ((a.ntm + 1) / 2);
-    const int grid = PAIR ? 2 * (int)(pairs < tc_pairs() ? pairs : tc_pairs()) : (int)(tiles < sm_count() ? tiles : sm_count());
+    const long long work = PAIR ? (long long)a.ntn * ((a.ntm + 1) / 2) : tiles;
+    const int units = PAIR ? tc_pairs() : sm_count();
+    int walkers = (int)(work < units ? work : units);
+    // With several n-tiles a CTA that steps by a multiple of their number stays with one of them, and prepares its per-channel
+    // constants once instead of once a tile: so many walkers where that costs none of them another tile (ResNet-50 at batch 256
+    // 2612 -> 2590 us, MobileNet-v2 at batch 64 816 -> 807).
+    const int whole = walkers - walkers % a.ntn;
+    if (whole > 0 && (work + whole - 1) / whole == (work + walkers - 1) / walkers) walkers = whole;
+    const int grid = PAIR ? 2 * walkers : walkers;
     // Programmatic dependent launch: the grid may start while its predecessor in the stream drains (its set-up touches
     // nothing the predecessor writes); the producer threads wait for the predecessor before their first activation load.
     cudaLaunchConfig_t cfg;
