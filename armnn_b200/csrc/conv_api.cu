@@ -171,8 +171,9 @@ static GroupPlan group_plan(int oc, int kh, int kw, int c)
         // zero-padded copy of the (small) input.  24 -> 144 channels at 56 x 56 (56 % of a tile, 75 % of three with g = 4):
         // MobileNet-v2 at batch 64 takes 807 us with the copy, 791 with g = 4, 793 with 8, 804 with 16.
         for (g = 2; g <= 4; g *= 2)
-            if ((g * c) % 16 == 0 && g * oc * 10 >= (g * oc + 255) / 256 * 256 * 7) break;
-        if (g > 4) return r;
+            if ((g * c) % 16 == 0 && (long long)g * oc * 10 >= (g * oc + 255ll) / 256 * 256 * 7) break;
+        // (small matrices only: the multiplications grow with g, and the tables of b200k_conv2d_q8_static have to hold them)
+        if (g > 4 || (long long)g * c * g * oc > 256 * 1024) return r;
     } else {
         while (g <= 16 && ((g * c) % 16 != 0 || (g * oc) % 16 != 0 || g * c < 32 || g * oc < 64)) g *= 2;
     }
