@@ -1793,7 +1793,7 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
 //   * the weights are re-packed at load time as [ky][OC / 8][WB / 16][8][16] (the same canonical layout) with zero in
 //     the padded channel lanes, and stay in shared memory for the whole launch;
 //   * a CTA walks a contiguous range of output rows (a tile is one output row), so every input row is expanded once per
-//     CTA and serves KH / stride_h tiles; accumulators are double-buffered in tensor memory and sixteen epilogue warps
+//     CTA and serves KH / stride_h tiles; up to four accumulators wait in tensor memory and sixteen epilogue warps
 //     requantise them with the same code as the main kernel and store their bytes directly.
 // Padding taps hold the zero point, so sum (x - zx) w = sum x w - zx sum_all w: one correction per channel, no border
 // classes.  Symmetric weights only (zero point 0).  Every wait is bounded as in the main kernel.
