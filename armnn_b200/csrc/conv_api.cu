@@ -13,7 +13,7 @@
 namespace b200k {
 
 int launch_conv_dp4a(const b200k_conv2d_params* p, cudaStream_t stream);
-int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid_c);   // B200K_E_UNSUPPORTED if not eligible
+int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid_c, bool packed_weights);   // B200K_E_UNSUPPORTED if not eligible
 bool conv_tc_eligible(const b200k_conv2d_params* p);
 size_t tc_pack_bytes(int oc, int kh, int kw, int c);
 size_t tc_scratch_bytes(const b200k_conv2d_params* p);
@@ -129,7 +129,7 @@ static int launch_padded(const b200k_conv2d_params* p, const PadPlan& pl, const 
         int rc = check_launch("repitch_rows_kernel");
         if (rc) return rc;
     }
-    int rc = launch_conv_tc(&q, stream, p->c);
+    int rc = launch_conv_tc(&q, stream, p->c, true);
     if (rc) return rc;
     if (p->oc % 16 != 0) {
         launch_pdl(repitch_rows_kernel, dim3((unsigned)div_up(pixels_out * (p->oc / 8), 256)), dim3(256), 0, stream,
@@ -258,8 +258,8 @@ int conv2d_dispatch(const b200k_conv2d_params* p, cudaStream_t stream)
     if (p->algo != 1) {
         b200k_conv2d_params q;
         // (group_plan only has a plan where groups of pixels beat what the kernel would do with the tensors as they are)
-        if (grouped_path_eligible(p, q)) return launch_conv_tc(&q, stream, 0);
-        if (conv_tc_eligible(p)) return launch_conv_tc(p, stream, 0);
+        if (grouped_path_eligible(p, q)) return launch_conv_tc(&q, stream, 0, true);
+        if (conv_tc_eligible(p)) return launch_conv_tc(p, stream, 0, false);
         PadPlan pl;
         if (wants_padding(p->oc, p->c) && padded_path_eligible(p, pl, q)) return launch_padded(p, pl, q, stream);
         B200K_REQUIRE(p->algo != 2, B200K_E_UNSUPPORTED, "conv2d_q8: shape/alignment not eligible for the tcgen05 kernel");

@@ -130,6 +130,7 @@ struct TcArgs {
     int cchunks;                                // C / BK
     int nslices;                                // KH*KW*cchunks
     int need_corr;                              // zx != 0
+    int weights_early;                          // the first tile's weights may be read before the kernels ahead of this one have finished
     int need_rect;                              // need_corr and some tap can fall outside the image
     int a_signed, b_signed;                     // operand element types: 1 = int8, 0 = uint8
     Requant rq;                                 // the convolution's own output quantisation
@@ -877,9 +878,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                              ::"r"(smem_u32(s_lut)), "l"(a.add_lut), "r"((uint32_t)TC_LUT_BYTES), "r"(smem_u32(lut_full)) : "memory");
             }
             // So the first tile's weights, as far as the ring holds them, are on their way before the activations exist
-            // (ResNet-50 at batch 256: 3044 us without this, 3015 with; at batch 3 383 and 381; MobileNet-v2 at batch 64 885 and 879).
-            // Weights that were never packed might be the previous kernel's output, and wait.
-            int ahead = bstat || skip_loads || !a.prefix ? 0 : min(STAGES, gpt);        // stages of the first tile whose weights are loaded here
+            // (ResNet-50 at batch 256: 3044 us without this, 3015 with; at batch 3 383 and 381).  Weights that the caller may
+            // rewrite without packing them again wait (see weights_early).
+            int ahead = bstat || skip_loads || !a.weights_early ? 0 : min(STAGES, gpt);        // stages of the first tile whose weights are loaded here
             for (int g = prod < a.nprod ? prod : ahead; g < ahead; g += a.nprod) {
                 if (elect_one()) {
                     const uint32_t fb = full_addr + g * 8;
@@ -2442,7 +2443,8 @@ static bool host_tables_for(const b200k_conv2d_params* p, const TcArgs& a, TcTab
     return true;
 }
 
-int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid_c)
+// kvalid_c: real channels of a channel-padded problem, else 0.  packed_weights: p->w lies in the packed tables, as a copy.
+int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid_c, bool packed_weights)
 {
     // few-channel stems: straight from the NHWC input when the geometry allows it (no re-packed copy of the input)
     if (p->c <= 16 && kvalid_c == 0 && stem_direct_eligible(p)) return launch_conv_stem(p, stream);
@@ -2477,6 +2479,10 @@ int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid
     a.ntm = row_mode ? p->n * p->oh : (int)((a.M + TC_BM - 1) / TC_BM);
     a.kstride = row_mode ? swz : p->c;
     a.need_corr = a.zx != 0;
+    // Weights are read ahead of the stream's order only where a new set of them needs new tables in any case, and packing is an
+    // ordinary launch that everything before it has finished for: a copy inside the tables, or sums of the weights that this
+    // launch uses.  Otherwise the kernel before this one may be writing them.
+    a.weights_early = p->packed && (a.need_corr || row_mode || packed_weights) ? 1 : 0;
     // can any tap of any output pixel leave the image?
     const int last_y = (p->oh - 1) * p->stride_h - p->pad_top + (p->kh - 1) * p->dil_h;
     const int last_x = (p->ow - 1) * p->stride_w - p->pad_left + (p->kw - 1) * p->dil_w;

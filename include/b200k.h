@@ -124,7 +124,11 @@ int b200k_conv2d_q8(const b200k_conv2d_params* p, void* stream);
  * CpuRef re-decodes the weights on every inference (ConvImpl.cpp:111-115); this replaces that.
  * `packed` must hold b200k_conv2d_pack_bytes() bytes of device memory; only w, oc, kh, kw, c of the
  * parameter struct are read.  Without a packed table, convolutions whose input zero point is not 0
- * run on the CUDA-core kernel. */
+ * run on the CUDA-core kernel.
+ * Weights, bias and scales are constants of a layer, which b200k_conv2d_q8 and b200k_fully_connected_q8 may read
+ * before the kernels ahead of them in the stream have finished (programmatic dependent launch).  To change them, write
+ * them and call b200k_conv2d_pack again on the same stream: its kernels are ordinary launches, which wait for what is
+ * ahead of them and which the next layer waits for. */
 size_t b200k_conv2d_pack_bytes(int32_t oc, int32_t kh, int32_t kw, int32_t c);
 int b200k_conv2d_pack(const b200k_conv2d_params* p, void* packed, void* stream);
 /* Bytes of per-call scratch b200k_conv2d_q8 wants for this geometry (0 for most shapes).  For c <= 16 the packed
