@@ -1800,7 +1800,7 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
 // classes.  Symmetric weights only (zero point 0).  Every wait is bounded as in the main kernel.
 constexpr int ST_SLOTS = 32;                    // packed-row ring (a power of two)
 constexpr int ST_LOOKAHEAD = 4;                 // tiles the expanders may run ahead of the MMAs
-constexpr int ST_DONE = 8;                      // ring of per-tile "MMAs complete" barriers (a power of two)
+constexpr int ST_DONE = 16;                     // ring of per-tile "MMAs complete" barriers (a power of two)
 // Eight warps expand rows: with four a tile waited for its two new rows.  ResNet-50's stem at batch 256 takes 269 us with four
 // expanders and one issuer, 213 with eight and two, 230 or more with only one of the two.
 constexpr int ST_EXPANDERS = 8;
@@ -1809,6 +1809,11 @@ constexpr int ST_ACC = 4;                       // accumulator buffers at most
 // Waiting for a tile's rows and issuing its MMAs takes a warp 1.3 us, of which the MMAs themselves are a fraction: two warps issue,
 // every other tile each.
 constexpr int ST_ISSUERS = 2;
+// An expander that is late tells the phases of mma_done apart by their parity, so the MMAs must not get ST_DONE tiles past the one it
+// waits for, however late it is.  Ahead of tile i it waits for tile i - ST_LOOKAHEAD.  Every tile needs a row that no tile before it
+// needs, so some tile t <= i + ST_EXPANDERS - 1 needs one that this expander still owes; the others wait for t ahead of
+// tile t + ST_LOOKAHEAD, and the MMAs end at the tile before that.
+static_assert(ST_DONE > (ST_EXPANDERS - 1) + (ST_LOOKAHEAD - 1) + ST_LOOKAHEAD, "a phase of mma_done could be taken for the one before last");
 // issuer, row loader, expanders, epilogue, the other issuer
 constexpr int ST_THREADS = 32 * (1 + ST_EXPANDERS + TC_EPI_WARPS + ST_ISSUERS);
 
