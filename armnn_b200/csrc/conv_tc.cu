@@ -1207,6 +1207,15 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
             }
         };
+        // A fused Add whose table is missing or made for other parameters: the reference arithmetic for every value, and no look-up
+        // (a launch without packed tables has no table in its shared memory either).
+        auto exact_chunks = [&](uint32_t* r, uint32_t tcol, int col0, uint32_t res_row, uint32_t st_row, uint32_t a_m, uint32_t a_b, uint32_t a_cc) {
+            tc_ld16_wait(r);                                 // (no load in flight across the call)
+            #pragma unroll 1
+            for (int j = 0; j < NCH; ++j, tcol += 16, col0 += 16)
+                epi_fix_chunk<EPI_SAT_U8>(0xfu, tcol, a_m + col0 * 4, a_b + col0 * 4, a_cc + col0 * 4, res_row + ((((uint32_t)(part * NCH + j)) ^ sw_x) << 4),
+                                          st_row + (((uint32_t)j ^ st_sw) << 4), &a.ep, 0u, s_ex);
+        };
         {
             int it = 0;
             int ub = 0; uint32_t uph = 0;                    // operand-buffer position (kept without divisions)
@@ -1266,7 +1275,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const uint32_t st_row = st_base + (uint32_t)lane * W;
                     auto chunks = [&](auto kind_tag) { unit_chunks(kind_tag, r, tacc + (uint32_t)colw, colw, res_row, st_row, a_m, a_b, a_cc, a_mq, a_bq, n0); };
                     if constexpr (formula)    chunks(std::integral_constant<int, EPI_ADD>{});
-                    else if constexpr (fused) chunks(std::integral_constant<int, EPI_LUT>{});      // (without a table its results are all replaced)
+                    else if constexpr (fused) { if (use_lut) chunks(std::integral_constant<int, EPI_LUT>{}); else exact_chunks(r, tacc + (uint32_t)colw, colw, res_row, st_row, a_m, a_b, a_cc); }
                     else if (kind == EPI_SAT_U8) chunks(std::integral_constant<int, EPI_SAT_U8>{});
                     else if (kind == EPI_SAT_S8) chunks(std::integral_constant<int, EPI_SAT_S8>{});
                     else chunks(std::integral_constant<int, EPI_CLAMP>{});

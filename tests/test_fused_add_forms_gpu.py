@@ -2,8 +2,9 @@
 import numpy as np
 import pytest
 
+from armnn_b200 import lib
 from cases import S8, U8, run_case
-from q8util import random_conv_case
+from q8util import Cuda, gpu_pack, random_conv_case
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +35,30 @@ def test_exact(built, quant, shape):
     want, got = run_case(case(), "oracle"), run_case(case(), "gpu")
     for a, b in zip(want, got):
         assert a.shape == b.shape and np.array_equal(a, b), (quant, shape, int((a != b).sum()))
+
+
+# Without packed tables (which input zero point 0 does not need), and with a table that was made for another output scale: every
+# value takes the reference arithmetic, and shared memory holds no table to look anything up in.
+@pytest.mark.parametrize("table", ["none", "made_for_another_scale"])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("quant", ["s8_relu", "u8"])
+def test_no_usable_table(built, quant, shape, table):
+    dtype, y_q, other_q, out_q, relu = QUANT[quant]
+    n, h, w, c, oc = SHAPES[shape]
+    u8 = dict(x_dtype=U8, y_dtype=U8) if dtype == U8 else {}
+    case = random_conv_case(33, n, h, w, c, oc, 1, 1, act=(1, 0, 0) if relu else (0, 0, 0), fused_add=True, x_q=(0.02, 0), **u8)
+    case.y_q, case.add = y_q, (case.add[0], other_q, out_q)
+    want, got = case.run_oracle()[0], _without_table(case, table)
+    assert np.array_equal(want, got), (quant, shape, int((want != got).sum()))
+
+
+def _without_table(case, table):
+    if table == "none":
+        return case.run_gpu(want_acc=False, algo=2, pack=False)[0]
+    mem = Cuda()
+    p, y, _ = case.params(mem, False, 2)
+    scale, p.add_out.scale = p.add_out.scale, p.add_out.scale * 1.5
+    p.packed = gpu_pack(mem, p)
+    p.add_out.scale = scale
+    lib.call("conv2d_q8", p)
+    return mem.fetch(y)
