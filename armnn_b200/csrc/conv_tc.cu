@@ -1832,7 +1832,7 @@ struct StemArgs {
     const int32_t* bias; const float* w_scales; const float* b_scales;
     float w_scale, b_scale;
     int N, H, W, C, OH, OW, OC, KH, KW, sh, sw, pt, pl;
-    int cpad, WB, slot_bytes, raw_bytes, Hp, Wp, tiles, tmem_cols, acc_log2;
+    int cpad, WB, slot_bytes, raw_bytes, step, Hp, Wp, tiles, tmem_cols, acc_log2;
     int split;                                  // 4-byte pixels, even / odd output pixels as the two 64-row halves of a tile
     int zx, a_signed, b_signed, acc_big;
     Requant rq;
@@ -1880,7 +1880,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
     // this CTA's contiguous range of tiles (output rows)
     const int t_begin = (int)((long long)a.tiles * blockIdx.x / gridDim.x), t_end = (int)((long long)a.tiles * (blockIdx.x + 1) / gridDim.x);
     const int ntiles = t_end - t_begin;
-    const long long v0 = (long long)(t_begin / a.OH) * a.Hp + (long long)(t_begin % a.OH) * a.sh;     // first virtual row
+    const long long v0 = (long long)(t_begin / a.OH) * a.Hp + (long long)(t_begin % a.OH) * a.step;   // first virtual row
     const long long wait_limit = a.wait_limit;
 
     const int acc_log2 = a.acc_log2, acc_mask = (1 << acc_log2) - 1;
@@ -1921,11 +1921,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
         const uint64_t da_slot = (uint64_t)(a.slot_bytes >> 4), db_ky = (uint64_t)((a.OC * a.WB) >> 4);
         const int kks = a.WB / 32;
         int n = t_begin / a.OH, oy = t_begin - n * a.OH;
-        const int base_n = n, base_oy = oy;                 // (v0 = base_n * Hp + base_oy * sh)
+        const int base_n = n, base_oy = oy;                 // (v0 = base_n * Hp + base_oy * step)
         int waited = 0;                                      // packed rows [0, waited) have been seen complete
         for (int i = 0; i < ntiles && alive; ++i) {
             if (i % ST_ISSUERS != issuer) { if (++oy == a.OH) { oy = 0; ++n; } continue; }
-            const int lo = (n - base_n) * a.Hp + (oy - base_oy) * a.sh;                              // first packed row, relative
+            const int lo = (n - base_n) * a.Hp + (oy - base_oy) * a.step;                            // first packed row, relative
             const int buf = i & acc_mask;
             for (int rv = lo > waited ? lo : waited; rv < lo + a.KH && alive; ++rv) {
                 if (!__all_sync(0xffffffffu, mbar_wait(&row_full[rv & (ST_SLOTS - 1)], (uint32_t)(rv / ST_SLOTS) & 1u, wait_limit))) { atomicExch(&g_tc_status, 2); alive = false; }
@@ -1961,7 +1961,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
             for (int i = 0; i < ntiles && alive; ++i) {
                 const int t = t_begin + i;
                 const int n = t / a.OH, oy = t % a.OH;
-                const long long lo = (long long)n * a.Hp + (long long)oy * a.sh - v0;
+                const long long lo = (long long)n * a.Hp + (long long)oy * a.step - v0;
                 for (long long rv = lo > next ? lo : next; rv < lo + a.KH && alive; ++rv) {
                     const int iy = (int)(rv - lo) + oy * a.sh - a.pt;
                     if (iy < 0 || iy >= a.H) continue;                       // a padding row: nothing to load
@@ -1987,7 +1987,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
         for (int i = 0; i < ntiles && alive; ++i) {
             const int t = t_begin + i;
             const int n = t / a.OH, oy = t % a.OH;
-            const long long lo = (long long)n * a.Hp + (long long)oy * a.sh - v0;
+            const long long lo = (long long)n * a.Hp + (long long)oy * a.step - v0;
             if (e == 0 && i == 1) TC_TRACE(12);
             if (i >= ST_LOOKAHEAD) {
                 const int j = i - ST_LOOKAHEAD;
@@ -2207,7 +2207,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
     }
 }
 
-struct StemPlan { bool ok; int cpad, WB, slot_bytes, raw_bytes, Wp, Hp, split; size_t wbytes, smem; int tmem_cols, acc_log2; };
+struct StemPlan { bool ok; int cpad, WB, slot_bytes, raw_bytes, Wp, step, Hp, split; size_t wbytes, smem; int tmem_cols, acc_log2; };
 
 static StemPlan stem_plan(const b200k_conv2d_params* p)
 {
@@ -2230,7 +2230,11 @@ static StemPlan stem_plan(const b200k_conv2d_params* p)
     r.slot_bytes = ((TC_BM - 1) * 16 + r.WB + 127) & ~127;
     r.Wp = (p->ow - 1) * p->stride_w + p->kw;
     if ((long long)r.Wp * r.cpad > r.slot_bytes) return r;
-    r.Hp = (p->oh - 1) * p->stride_h + p->kh;
+    // Packed rows are the rows that some tile reads, one after another: with a stride above the filter's height the rows between
+    // two tiles are no packed rows, or the waits for a ring slot (by the parity of packed row / ST_SLOTS) would count rows that
+    // nobody writes.
+    r.step = p->kh < p->stride_h ? p->kh : p->stride_h;
+    r.Hp = (p->oh - 1) * r.step + p->kh;
     r.wbytes = (size_t)p->kh * p->oc * r.WB;
     if (r.wbytes > 64 * 1024) return r;
     r.tmem_cols = 32;
@@ -2298,7 +2302,7 @@ static int launch_conv_stem(const b200k_conv2d_params* p, cudaStream_t stream)
     a.w_scale = p->w.scale; a.b_scale = p->bias.scale;
     a.N = p->n; a.H = p->h; a.W = p->wd; a.C = p->c; a.OH = p->oh; a.OW = p->ow; a.OC = p->oc;
     a.KH = p->kh; a.KW = p->kw; a.sh = p->stride_h; a.sw = p->stride_w; a.pt = p->pad_top; a.pl = p->pad_left;
-    a.cpad = pl.cpad; a.WB = pl.WB; a.slot_bytes = pl.slot_bytes; a.raw_bytes = pl.raw_bytes; a.Hp = pl.Hp; a.Wp = pl.Wp;
+    a.cpad = pl.cpad; a.WB = pl.WB; a.slot_bytes = pl.slot_bytes; a.raw_bytes = pl.raw_bytes; a.step = pl.step; a.Hp = pl.Hp; a.Wp = pl.Wp;
     a.split = pl.split;
     a.tiles = p->n * p->oh; a.tmem_cols = pl.tmem_cols; a.acc_log2 = pl.acc_log2;
     a.zx = p->x.zero_point;

@@ -15,6 +15,9 @@ CASES = {
     "5x5_c1": lambda: random_conv_case(3, 64, 64, 64, 1, 32, 5, 5, pad=(2, 2, 2, 2)), "7x7_no_padding": lambda: random_conv_case(4, 60, 70, 80, 3, 16, 7, 7),
     "3x3_stride_2": lambda: random_conv_case(5, 128, 96, 96, 3, 32, 3, 3, stride=(2, 2), pad=(0, 1, 0, 1), act=(1, 0, 0)), "7x7_stride_2_oc256": lambda: random_conv_case(6, 32, 64, 64, 3, 256, 7, 7, stride=(2, 2), pad=(3, 2, 3, 2)),
     "11x11_stride_4_rows": lambda: random_conv_case(7, 40, 200, 64, 3, 64, 11, 3, stride=(4, 2), pad=(2, 2, 1, 0)), "3x3_stride_3_rows": lambda: random_conv_case(8, 64, 96, 64, 4, 48, 3, 3, stride=(3, 1), pad=(0, 0, 1, 1)),
+    # strides above the filter's height: rows between two tiles that none reads
+    "1x1_stride_2_rows": lambda: random_conv_case(9, 400, 15, 32, 3, 16, 1, 1, stride=(2, 1)), "2x2_stride_3_rows": lambda: random_conv_case(10, 400, 23, 32, 3, 16, 2, 2, stride=(3, 2), **U8X),
+    "3x3_stride_4_rows": lambda: random_conv_case(11, 400, 31, 48, 1, 32, 3, 3, stride=(4, 1), act=(1, 0, 0)), "1x3_stride_4_rows": lambda: random_conv_case(12, 600, 18, 32, 2, 48, 1, 3, stride=(4, 1), pad=(1, 0, 1, 1)),
 }
 
 

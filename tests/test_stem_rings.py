@@ -13,8 +13,9 @@ K = {name: int(value) for name, value in re.findall(r"^constexpr int (ST_\w+) = 
 class Rings:
     """The waits and signals of a CTA that walks `tiles` output rows from the `first` on.  Barriers are counters of completed phases."""
 
-    def __init__(self, kh, step, oh, first, tiles, accumulators):
+    def __init__(self, kh, stride, oh, first, tiles, accumulators):
         self.count, self.mma, self.written, self.fault = {}, [False] * tiles, {}, None
+        step = min(kh, stride)                                      # (packed rows are the rows that some tile reads)
         hp = (oh - 1) * step + kh
         rows = [t // oh * hp + t % oh * step for t in range(first, first + tiles)]
         self.lo, self.kh = [r - rows[0] for r in rows], kh
@@ -86,15 +87,15 @@ class Rings:
         return stopped is None or self.waiting[stopped] is not None
 
 
-def check(kh, step, oh, first, tiles=44, accumulators=4):
+def check(kh, stride, oh, first, tiles=44, accumulators=4):
     """None, or what goes wrong."""
-    free = Rings(kh, step, oh, first, tiles, accumulators)
+    free = Rings(kh, stride, oh, first, tiles, accumulators)
     free.run()
     if any(w is not None for w in free.waiting):
         return "no end: %s" % free.waiting
     for w in range(len(free.warps)):
         for n in range(10 ** 6):
-            r = Rings(kh, step, oh, first, tiles, accumulators)
+            r = Rings(kh, stride, oh, first, tiles, accumulators)
             if not r.run(w, n):
                 break
             barrier, phase = r.waiting[w]
@@ -107,7 +108,7 @@ def check(kh, step, oh, first, tiles=44, accumulators=4):
 
 # filter rows, stride, output rows per image, first output row
 @pytest.mark.parametrize("kh,stride,oh,first", [(1, 1, 50, 0), (2, 1, 7, 3), (3, 1, 50, 0), (3, 1, 5, 2), (5, 1, 50, 0), (7, 1, 9, 8), (3, 2, 50, 0), (7, 2, 50, 0),
-                                                (7, 2, 3, 1), (11, 4, 50, 0), (11, 4, 3, 2), (11, 1, 4, 0), (4, 4, 6, 0), (3, 3, 50, 0)])
+                                                (7, 2, 3, 1), (11, 4, 50, 0), (11, 4, 3, 2), (11, 1, 4, 0), (4, 4, 6, 0), (3, 3, 50, 0), (1, 2, 8, 0), (1, 4, 5, 3), (2, 3, 8, 1), (3, 4, 7, 0)])
 @pytest.mark.parametrize("accumulators", [2, 4])
 def test_no_wait_is_overtaken(kh, stride, oh, first, accumulators):
     assert check(kh, stride, oh, first, accumulators=accumulators) is None
