@@ -1808,7 +1808,7 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
 // Padding taps hold the zero point, so sum (x - zx) w = sum x w - zx sum_all w: one correction per channel, no border
 // classes.  Symmetric weights only (zero point 0).  Every wait is bounded as in the main kernel.
 constexpr int ST_SLOTS = 32;                    // packed-row ring (a power of two)
-constexpr int ST_LOOKAHEAD = 4;                 // tiles the expanders may run ahead of the MMAs
+constexpr int ST_LOOKAHEAD = 4;                 // tiles the expanders may run ahead of the MMAs, at most (see stem_plan)
 constexpr int ST_DONE = 16;                     // ring of per-tile "MMAs complete" barriers (a power of two)
 // Eight warps expand rows: with four a tile waited for its two new rows.  ResNet-50's stem at batch 256 takes 269 us with four
 // expanders and one issuer, 213 with eight and two, 230 or more with only one of the two.
@@ -1832,7 +1832,7 @@ struct StemArgs {
     const int32_t* bias; const float* w_scales; const float* b_scales;
     float w_scale, b_scale;
     int N, H, W, C, OH, OW, OC, KH, KW, sh, sw, pt, pl;
-    int cpad, WB, slot_bytes, raw_bytes, step, Hp, Wp, tiles, tmem_cols, acc_log2;
+    int cpad, WB, slot_bytes, raw_bytes, step, Hp, Wp, tiles, lookahead, tmem_cols, acc_log2;
     int split;                                  // 4-byte pixels, even / odd output pixels as the two 64-row halves of a tile
     int zx, a_signed, b_signed, acc_big;
     Requant rq;
@@ -1989,8 +1989,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
             const int n = t / a.OH, oy = t % a.OH;
             const long long lo = (long long)n * a.Hp + (long long)oy * a.step - v0;
             if (e == 0 && i == 1) TC_TRACE(12);
-            if (i >= ST_LOOKAHEAD) {
-                const int j = i - ST_LOOKAHEAD;
+            if (i >= a.lookahead) {
+                const int j = i - a.lookahead;
                 if (!mbar_wait(&mma_done[j % ST_DONE], (uint32_t)(j / ST_DONE) & 1u, wait_limit)) { atomicExch(&g_tc_status, 1); alive = false; break; }
             }
             for (long long rv = lo > next ? lo : next; rv < lo + a.KH && alive; ++rv) {
@@ -2207,7 +2207,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) conv_stem_kernel(const __grid_c
     }
 }
 
-struct StemPlan { bool ok; int cpad, WB, slot_bytes, raw_bytes, Wp, step, Hp, split; size_t wbytes, smem; int tmem_cols, acc_log2; };
+struct StemPlan { bool ok; int cpad, WB, slot_bytes, raw_bytes, Wp, step, Hp, lookahead, split; size_t wbytes, smem; int tmem_cols, acc_log2; };
 
 static StemPlan stem_plan(const b200k_conv2d_params* p)
 {
@@ -2235,6 +2235,10 @@ static StemPlan stem_plan(const b200k_conv2d_params* p)
     // nobody writes.
     r.step = p->kh < p->stride_h ? p->kh : p->stride_h;
     r.Hp = (p->oh - 1) * r.step + p->kh;
+    // The rows of the tiles that the expanders work on at once have to fit the ring.  Tiles of one image share rows, those of
+    // different images do not: four of them take ST_SLOTS rows at most with filters of up to eight rows, or with three
+    // output rows or more (2 * 4 + 2 * 11); two of them take 22.
+    r.lookahead = p->kh > 8 && p->oh < 3 ? 2 : ST_LOOKAHEAD;
     r.wbytes = (size_t)p->kh * p->oc * r.WB;
     if (r.wbytes > 64 * 1024) return r;
     r.tmem_cols = 32;
@@ -2302,7 +2306,7 @@ static int launch_conv_stem(const b200k_conv2d_params* p, cudaStream_t stream)
     a.w_scale = p->w.scale; a.b_scale = p->bias.scale;
     a.N = p->n; a.H = p->h; a.W = p->wd; a.C = p->c; a.OH = p->oh; a.OW = p->ow; a.OC = p->oc;
     a.KH = p->kh; a.KW = p->kw; a.sh = p->stride_h; a.sw = p->stride_w; a.pt = p->pad_top; a.pl = p->pad_left;
-    a.cpad = pl.cpad; a.WB = pl.WB; a.slot_bytes = pl.slot_bytes; a.raw_bytes = pl.raw_bytes; a.step = pl.step; a.Hp = pl.Hp; a.Wp = pl.Wp;
+    a.cpad = pl.cpad; a.WB = pl.WB; a.slot_bytes = pl.slot_bytes; a.raw_bytes = pl.raw_bytes; a.step = pl.step; a.Hp = pl.Hp; a.Wp = pl.Wp; a.lookahead = pl.lookahead;
     a.split = pl.split;
     a.tiles = p->n * p->oh; a.tmem_cols = pl.tmem_cols; a.acc_log2 = pl.acc_log2;
     a.zx = p->x.zero_point;

@@ -18,6 +18,9 @@ CASES = {
     # strides above the filter's height: rows between two tiles that none reads
     "1x1_stride_2_rows": lambda: random_conv_case(9, 400, 15, 32, 3, 16, 1, 1, stride=(2, 1)), "2x2_stride_3_rows": lambda: random_conv_case(10, 400, 23, 32, 3, 16, 2, 2, stride=(3, 2), **U8X),
     "3x3_stride_4_rows": lambda: random_conv_case(11, 400, 31, 48, 1, 32, 3, 3, stride=(4, 1), act=(1, 0, 0)), "1x3_stride_4_rows": lambda: random_conv_case(12, 600, 18, 32, 2, 48, 1, 3, stride=(4, 1), pad=(1, 0, 1, 1)),
+    # tall filters with one or two output rows: tiles of different images share no rows
+    "11_rows_one_output_row": lambda: random_conv_case(13, 3000, 11, 16, 3, 16, 11, 3), "9_rows_one_output_row": lambda: random_conv_case(14, 2500, 9, 16, 4, 32, 9, 3, pad=(0, 0, 1, 1)),
+    "8_rows_one_output_row": lambda: random_conv_case(15, 2500, 8, 16, 3, 16, 8, 3, **U8X), "11_rows_stride_4_two_output_rows": lambda: random_conv_case(16, 1600, 14, 16, 3, 32, 11, 3, stride=(4, 1), pad=(1, 0, 0, 0)),
 }
 
 

@@ -24,6 +24,7 @@ class Rings:
             self.new.append(list(range(max(lo, top), lo + kh)))
             top = max(top, lo + kh)
         self.tiles, self.acc = tiles, accumulators
+        self.lookahead = 2 if kh > 8 and oh < 3 else K["ST_LOOKAHEAD"]
         warps = [self.issuer(i) for i in range(K["ST_ISSUERS"])] + [self.loader(), self.epilogue()]
         self.warps = warps + [self.expander(e) for e in range(K["ST_EXPANDERS"])]
         self.waiting = [next(w, None) for w in self.warps]          # (barrier, phase) that has to be complete
@@ -50,8 +51,8 @@ class Rings:
     def expander(self, me):
         n = 0
         for i in range(self.tiles):
-            if i >= K["ST_LOOKAHEAD"]:
-                j = i - K["ST_LOOKAHEAD"]
+            if i >= self.lookahead:
+                j = i - self.lookahead
                 yield ("done", j % K["ST_DONE"]), j // K["ST_DONE"]
             for rv in self.new[i]:
                 if rv % K["ST_EXPANDERS"] == me:
@@ -108,7 +109,8 @@ def check(kh, stride, oh, first, tiles=44, accumulators=4):
 
 # filter rows, stride, output rows per image, first output row
 @pytest.mark.parametrize("kh,stride,oh,first", [(1, 1, 50, 0), (2, 1, 7, 3), (3, 1, 50, 0), (3, 1, 5, 2), (5, 1, 50, 0), (7, 1, 9, 8), (3, 2, 50, 0), (7, 2, 50, 0),
-                                                (7, 2, 3, 1), (11, 4, 50, 0), (11, 4, 3, 2), (11, 1, 4, 0), (4, 4, 6, 0), (3, 3, 50, 0), (1, 2, 8, 0), (1, 4, 5, 3), (2, 3, 8, 1), (3, 4, 7, 0)])
+                                                (7, 2, 3, 1), (11, 4, 50, 0), (11, 4, 3, 2), (11, 1, 4, 0), (4, 4, 6, 0), (3, 3, 50, 0), (1, 2, 8, 0), (1, 4, 5, 3), (2, 3, 8, 1), (3, 4, 7, 0),
+                                                (8, 1, 1, 0), (9, 1, 1, 0), (11, 4, 1, 0), (8, 4, 2, 1), (9, 4, 2, 0), (10, 2, 2, 1), (11, 1, 2, 1), (11, 4, 2, 0)])
 @pytest.mark.parametrize("accumulators", [2, 4])
 def test_no_wait_is_overtaken(kh, stride, oh, first, accumulators):
     assert check(kh, stride, oh, first, accumulators=accumulators) is None
