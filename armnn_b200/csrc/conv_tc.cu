@@ -2565,7 +2565,7 @@ int launch_conv_tc(const b200k_conv2d_params* p, cudaStream_t stream, int kvalid
     // CTA pairs on 256 x 256 tiles: from K = 2048 on (16 slices), where the loads bound a wide tile, and with a tile for every
     // pair.  FullyConnected 4096 x 4096 x 4096 takes 55.2 us without and 48.5 with them, 512 -> 512 channels, 3 x 3, 64 x 14 x 14
     // 36.5 and 33.7; all of ResNet-50 at batch 256 2685 from 16 slices on, 2686 from 9, 2702 from 4 (K = 1024 gains nothing).
-    const bool pair = swz == 128 && !row_mode && a.nzw == 0 && !fa.res && p->selftest_us == 0 && p->oc >= 256 && (size_t)a.ncls * 256 * 4 <= 32 * 1024 &&
+    const bool pair = swz == 128 && !row_mode && a.nzw == 0 && !fa.res && p->oc >= 256 && (size_t)a.ncls * 256 * 4 <= 32 * 1024 &&
                       a.nslices >= 16 && ((p->oc + 255) / 256) * (((long long)a.ntm + 1) / 2) >= tc_pairs() && tc_pairs() > 0;
     const int bn = pair ? 256 : pick_bn(p->oc, a.ntm);
     a.ntn = (p->oc + bn - 1) / bn;

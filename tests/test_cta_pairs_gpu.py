@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from cases import S8, U8, run_case
-from q8util import random_conv_case, random_fc_case
+from q8util import Cuda, gpu_pack, random_conv_case, random_fc_case
 
 pytestmark = pytest.mark.gpu
 
@@ -18,6 +18,11 @@ CASES = {
     "conv_stride_2": lambda: random_conv_case(9, 100, 28, 28, 256, 256, 3, 3, stride=(2, 2), pad=(0, 1, 0, 1)),
     "conv_1x1_stride_2": lambda: random_conv_case(10, 100, 28, 27, 2048, 256, 1, 1, stride=(2, 2)),
     "conv_1x1": lambda: random_conv_case(11, 97, 14, 14, 2048, 272, 1, 1, act=(1, 0, 0)),
+    # 149 row tiles: the second tile of the last pair lies wholly beyond the last image
+    "conv_3x3_odd_tiles": lambda: random_conv_case(13, 97, 14, 14, 256, 256, 3, 3, pad=(1, 1, 1, 1), act=(1, 0, 0)),
+    "conv_3x3_odd_tiles_no_padding": lambda: random_conv_case(14, 132, 14, 14, 256, 256, 3, 3),
+    "conv_stride_2_odd_tiles_u8_input": lambda: random_conv_case(15, 97, 28, 28, 240, 256, 3, 3, stride=(2, 2), pad=(0, 1, 0, 1), **U8X),
+    "conv_1x1_stride_2_odd_tiles": lambda: random_conv_case(16, 97, 28, 27, 2048, 272, 1, 1, stride=(2, 2)),
     # one K-slice short of a pair's
     "fc_15_slices": lambda: random_fc_case(12, 74 * 256, 1920, 256),
 }
@@ -29,3 +34,19 @@ def test_exact(built, name):
     want, got = case.run_oracle(), case.run_gpu()
     for a, b in zip(want, got):
         assert a.shape == b.shape and np.array_equal(a, b), (name, int((np.asarray(a) != np.asarray(b)).sum()), np.asarray(a).size)
+
+
+def test_bounded_waits_give_up(built):
+    """Loads that never arrive (no load is issued at all): every wait of both CTAs runs into its limit, the launch returns and says so."""
+    from armnn_b200 import _abi, lib
+    l = lib.load_library()
+    case = random_conv_case(17, 97, 14, 14, 256, 256, 3, 3, pad=(1, 1, 1, 1))
+    mem = Cuda()
+    p, _, _ = case.params(mem, False, 2)
+    p.packed = gpu_pack(mem, p)
+    p.selftest_us = 3000
+    lib.call("conv2d_q8", p)
+    assert l.b200k_poll_status() == _abi.E_TIMEOUT
+    assert l.b200k_poll_status() == 0
+    want, got = case.run_oracle(want_acc=False)[0], case.run_gpu(want_acc=False, algo=2)[0]
+    assert np.array_equal(want, got)
