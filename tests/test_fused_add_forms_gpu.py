@@ -62,3 +62,23 @@ def _without_table(case, table):
     p.add_out.scale = scale
     lib.call("conv2d_q8", p)
     return mem.fetch(y)
+
+
+# Which of the two a launch takes: with every entry of its packed table inverted, only the arithmetic still gives the oracle's bytes.
+@pytest.mark.parametrize("shape", ["small", "many_tiles"])
+@pytest.mark.parametrize("quant", ["s8", "s8_relu", "u8", "u8_relu", "halves"])
+def test_which_form_runs(built, quant, shape):
+    dtype, y_q, other_q, out_q, relu = QUANT[quant]
+    n, h, w, c, oc = SHAPES[shape]
+    u8 = dict(x_dtype=U8, w_dtype=U8, y_dtype=U8, x_q=(0.02, 128)) if dtype == U8 else {}
+    case = random_conv_case(31, n, h, w, c, oc, 1, 1, act=(1, 0, 0) if relu else (0, 0, 0), fused_add=True, **u8)
+    case.y_q, case.add = y_q, (case.add[0], other_q, out_q)
+    mem = Cuda()
+    p, y, _ = case.params(mem, False, 2)
+    p.packed = gpu_pack(mem, p)
+    words = [t for t in mem.keep if t.data_ptr() == p.packed][0]
+    tag = int(np.flatnonzero(words.cpu().numpy() == 0x4C555431)[0])                # the table's 256 rows of 260 bytes end here
+    words[tag - 256 * 65:tag].bitwise_not_()
+    lib.call("conv2d_q8", p)
+    same = np.array_equal(case.run_oracle()[0], mem.fetch(y))
+    assert same == (quant != "halves")
