@@ -41,7 +41,7 @@ def conv_cases():
     c["grouped_c16_oc96_u8_everything"] = lambda: random_conv_case(17, 2, 28, 28, 16, 96, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8,
                                                                    per_axis=False, x_q=(0.02, 117), y_zp=0, act=(2, 6.0, 0.0),
                                                                    y_scale=0.02)
-    c["c24_oc144_u8_everything_padded_input"] = lambda: random_conv_case(18, 2, 28, 28, 24, 144, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8,
+    c["c24_oc144_u8_everything_groups_of_pixels"] = lambda: random_conv_case(18, 2, 28, 28, 24, 144, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8,
                                                                     per_axis=False, x_q=(0.02, 131), y_zp=0, act=(2, 6.0, 0.0),
                                                                     y_scale=0.02)
     c["grouped_c96_oc24_u8_everything"] = lambda: random_conv_case(19, 2, 28, 28, 96, 24, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8,

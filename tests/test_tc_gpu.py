@@ -62,9 +62,13 @@ CONV = {
                                                     fused_add=True),
     "rowwin_u8w_stem_3x3_s2_oc32": lambda: random_conv_case(267, 2, 64, 64, 3, 32, 3, 3, stride=(2, 2), pad=(0, 1, 0, 1), x_dtype=U8,
                                                             w_dtype=U8, y_dtype=U8, x_q=(0.02, 128), act=(2, 6.0, 0.0), y_zp=0),
-    # channel counts that are multiples of 8 only: zero-padded copies in scratch (input) and / or a padded output
-    "padded_c24_oc144_u8w": lambda: random_conv_case(270, 2, 28, 28, 24, 144, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8,
+    # channel counts that are multiples of 8 only: groups of pixels, or zero-padded copies in scratch (input) and / or a padded output
+    "grouped_c24_oc144_u8w": lambda: random_conv_case(270, 2, 28, 28, 24, 144, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8,
                                                      x_q=(0.02, 128), act=(2, 6.0, 0.0), y_zp=0),
+    # (these do not go by groups of pixels: 255 of them, a stride, a 3x3 filter)
+    "padded_c24_oc144_u8w_odd_pixels": lambda: random_conv_case(274, 1, 15, 17, 24, 144, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8, x_q=(0.02, 128)),
+    "padded_c24_oc144_u8w_stride2": lambda: random_conv_case(275, 2, 14, 14, 24, 144, 1, 1, stride=(2, 2), x_dtype=U8, w_dtype=U8, y_dtype=U8, x_q=(0.02, 31)),
+    "padded_c40_oc96_u8w_3x3": lambda: random_conv_case(276, 1, 14, 14, 40, 96, 3, 3, pad=(1, 1, 1, 1), x_dtype=U8, w_dtype=U8, y_dtype=U8, x_q=(0.02, 117)),
     "padded_c144_oc24_u8w": lambda: random_conv_case(271, 2, 28, 28, 144, 24, 1, 1, x_dtype=U8, w_dtype=U8, y_dtype=U8, x_q=(0.02, 111)),
     "padded_c24_oc24_s8_3x3": lambda: random_conv_case(272, 1, 14, 14, 24, 24, 3, 3, pad=(1, 1, 1, 1)),
     "padded_c40_oc72_stride2": lambda: random_conv_case(273, 2, 14, 14, 40, 72, 3, 3, stride=(2, 2), pad=(0, 1, 0, 1), act=(1, 0, 0)),
