@@ -4,6 +4,7 @@
 // dequantise to fp32, accumulate in CpuRef's (y, x) visiting order with unfused fp32 adds, divide,
 // re-quantise — so the results equal CpuRef's bit for bit (Pooling2d.cpp:142-303, Reduce.cpp:68-173 of
 // the Arm NN tree).
+#include <type_traits>
 #include "common.cuh"
 
 namespace b200k {
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(256) pool2d_kernel(const PoolArgs a)
 // general kernel.
 //
 // Two 16-bit maxima take a word's odd bytes as they lie (the even byte below only breaks ties) and its even bytes shifted up:
-// three instructions per four bytes, where a byte maximum is made of several.  A block of B x B taps is loaded before the first
+// three instructions per four bytes, where a byte maximum is made of several.  A block of BH x BW taps is loaded before the first
 // is compared; where the window ends inside a block its last tap repeats.  Bound by the loads' latency and by L2: ResNet-50's
 // 112 x 112 x 64 at batch 256, 257 MB, took 84 us with byte maxima and a load per tap and trip, 68 now.
 template <bool U8>
@@ -157,7 +158,7 @@ __device__ __forceinline__ uint32_t max16x2(uint32_t a, uint32_t b)
     return d;
 }
 
-template <bool U8, int B>
+template <bool U8, int BH, int BW>
 __global__ void __launch_bounds__(256) maxpool_same_quant_kernel(const PoolArgs a)
 {
     pdl_enter();
@@ -185,14 +186,14 @@ __global__ void __launch_bounds__(256) maxpool_same_quant_kernel(const PoolArgs 
         #pragma unroll
         for (int k = 0; k < 4; ++k) odd[k] = even[k] = lowest;
         const uint8_t* x = (const uint8_t*)a.x.data + (long long)n * a.H * a.W * a.C + c;
-        for (int iy = hstart; iy < hend; iy += B)
-            for (int ix = wstart; ix < wend; ix += B) {
-                uint4 v[B * B];
+        for (int iy = hstart; iy < hend; iy += BH)
+            for (int ix = wstart; ix < wend; ix += BW) {
+                uint4 v[BH * BW];
                 #pragma unroll
-                for (int j = 0; j < B * B; ++j)
-                    v[j] = *(const uint4*)(x + ((long long)min(iy + j / B, hend - 1) * a.W + min(ix + j % B, wend - 1)) * a.C);
+                for (int j = 0; j < BH * BW; ++j)
+                    v[j] = *(const uint4*)(x + ((long long)min(iy + j / BW, hend - 1) * a.W + min(ix + j % BW, wend - 1)) * a.C);
                 #pragma unroll
-                for (int j = 0; j < B * B; ++j) {
+                for (int j = 0; j < BH * BW; ++j) {
                     const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
                     #pragma unroll
                     for (int k = 0; k < 4; ++k) { odd[k] = max16x2<U8>(odd[k], w[k]); even[k] = max16x2<U8>(even[k], w[k] << 8); }
@@ -263,6 +264,12 @@ __global__ void __launch_bounds__(MEAN_THREADS) mean_staged_kernel(const MeanArg
     store_vec_f<VEC>(a.y, (long long)n * a.C + c, r);
 }
 
+// Taps per block along one axis of the window.  Blocks of three repeat taps in windows of one, two and four: with them for
+// every window above 2 x 2, 64 x 56 x 56 x 128 took 39.5 us at 1 x 7 (26.3 with a load per tap and trip, 25.7 now), 17.8 at
+// 1 x 4, stride 2 (11.6, 10.2), 15.0 at 4 x 4, stride 2 (14.5, 10.4), 13.4 at 3 x 2 (15.1, 11.2).  Longer ones gain from three: 7 x 7, stride 2
+// 32.3 and 27.4, 9 x 9 162 and 82.
+static int taps_per_block(int window) { return window == 1 ? 1 : (window == 2 || window == 4 ? 2 : 3); }
+
 static int pick_vec(const b200k_qtensor& x, const b200k_qtensor& y, int C)
 {
     if (!is_q8(x.dtype) || !is_q8(y.dtype)) return 1;
@@ -301,10 +308,24 @@ extern "C" int b200k_pool2d_q8(const b200k_pool2d_params* p, void* stream)
     type_range(p->x.dtype, lo, hi);
     if (vec == 16 && p->pool_type == 0 && p->x.dtype == p->y.dtype && p->x.scale == p->y.scale &&
         p->x.zero_point == p->y.zero_point && ordinary_scale(p->x.scale) && p->x.zero_point >= lo && p->x.zero_point <= hi) {
-        const bool u8 = p->x.dtype == B200K_U8, two = p->pool_h <= 2 && p->pool_w <= 2;
+        const bool u8 = p->x.dtype == B200K_U8;
         auto go = [&](auto kern) { launch_pdl(kern, dim3((unsigned)(div_up(a.total, 256))), dim3(256), 0, s, a); };
-        if (two) { if (u8) go(maxpool_same_quant_kernel<true, 2>); else go(maxpool_same_quant_kernel<false, 2>); }
-        else     { if (u8) go(maxpool_same_quant_kernel<true, 3>); else go(maxpool_same_quant_kernel<false, 3>); }
+        auto width = [&](auto bh, auto bw) {
+            constexpr int BH = decltype(bh)::value, BW = decltype(bw)::value;
+            if (u8) go(maxpool_same_quant_kernel<true, BH, BW>); else go(maxpool_same_quant_kernel<false, BH, BW>);
+        };
+        auto height = [&](auto bh) {
+            switch (taps_per_block(p->pool_w)) {
+                case 1:  width(bh, std::integral_constant<int, 1>{}); break;
+                case 2:  width(bh, std::integral_constant<int, 2>{}); break;
+                default: width(bh, std::integral_constant<int, 3>{}); break;
+            }
+        };
+        switch (taps_per_block(p->pool_h)) {
+            case 1:  height(std::integral_constant<int, 1>{}); break;
+            case 2:  height(std::integral_constant<int, 2>{}); break;
+            default: height(std::integral_constant<int, 3>{}); break;
+        }
         return check_launch("maxpool_same_quant_kernel");
     }
     if (vec == 16)     launch_pdl(pool2d_kernel<16>, dim3((unsigned)(div_up(a.total, 256))), dim3(256), 0, s, a);

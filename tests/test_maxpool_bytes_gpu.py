@@ -30,7 +30,7 @@ def _pool(dtype, n, h, w, c, ph, pw, sh, sw, pads):
 # (enough outputs for the 16-channel kernel: 148 SMs x 1024 threads x 16 channels)
 @pytest.mark.parametrize("dtype", [S8, U8])
 @pytest.mark.parametrize("ph,pw,sh,sw,pads", [(3, 3, 2, 2, (1, 0, 1, 0)), (2, 2, 2, 2, (0, 0, 0, 0)), (1, 1, 2, 2, (0, 0, 0, 0)), (2, 3, 1, 2, (1, 1, 1, 1)),
-                                              (5, 4, 2, 2, (2, 2, 1, 1)), (7, 7, 2, 3, (3, 3, 3, 3)), (2, 2, 2, 2, (3, 3, 3, 3))])
+                                              (5, 4, 2, 2, (2, 2, 1, 1)), (1, 4, 1, 2, (0, 0, 1, 1)), (1, 5, 1, 2, (0, 0, 2, 2)), (4, 1, 2, 1, (1, 1, 0, 0)), (5, 1, 2, 1, (2, 2, 0, 0)), (7, 7, 2, 3, (3, 3, 3, 3)), (2, 2, 2, 2, (3, 3, 3, 3))])
 def test_exact(built, dtype, ph, pw, sh, sw, pads):
     outputs = ((56 + pads[0] + pads[1] - ph) // sh + 1) * ((50 + pads[2] + pads[3] - pw) // sw + 1) * 4
     case = _pool(dtype, -(-148 * 1024 // outputs) + 1, 56, 50, 64, ph, pw, sh, sw, pads)
