@@ -405,8 +405,8 @@ struct Quant4 {
             unpack2(q01, q[0], q[1]); unpack2(q23, q[2], q[3]);
             unpack2(n01, n[0], n[1]); unpack2(n23, n[2], n[3]);
             // An exact half that the constant rounded towards zero goes the other way.  (Interpolation and sums of tensors whose
-            // scales are in simple ratios are full of halves: a Resize, an Add and an ArgMax of 11 MB took 32.6 us with the
-            // calls of roundf that were here, and take 29.3.)
+            // scales are in simple ratios are full of halves: a Resize, an Add and an ArgMax of 11 MB take 32.3 us with calls of
+            // roundf here, 31.9 without.  A quotient too large for the constant saturates: ordinary_quant limits the zero point.)
             #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const float h = copysignf(0.5f, q[k]);

@@ -169,7 +169,10 @@ static GroupPlan group_plan(int oc, int kh, int kw, int c)
     if (c > 16 && oc % 16 == 0 && wants_padding(oc, c)) {
         // Only the input channels are odd: groups of two or four where g OC columns fill most of their 256-wide tiles, else a
         // zero-padded copy of the (small) input.  24 -> 144 channels at 56 x 56 (56 % of a tile, 75 % of three with g = 4):
-        // MobileNet-v2 at batch 64 takes 807 us with the copy, 791 with g = 4, 793 with 8, 804 with 16.
+        // MobileNet-v2 at batch 64 takes 807 us with the copy, 791 with g = 4, 793 with 8, 804 with 16.  Of 49 pairs of channel
+        // counts (24 - 264 to 48 - 320) at 196 to 200704 pixels the copy takes up to 2.75 times as long, and nowhere less up
+        // to 50176 pixels.  At 200704 it is the faster one for 24 - 56 to 192 - 256 channels: by up to 14 % (40 -> 192: 34.4
+        // and 29.5 us), where at 50176 it is 12 - 25 % slower.
         for (g = 2; g <= 4; g *= 2)
             if ((g * c) % 16 == 0 && (long long)g * oc * 10 >= (g * oc + 255ll) / 256 * 256 * 7) break;
         // (small matrices only: the multiplications grow with g, and the tables of b200k_conv2d_q8_static have to hold them)

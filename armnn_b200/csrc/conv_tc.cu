@@ -510,9 +510,9 @@ __device__ __forceinline__ void lds_f2x2(uint32_t addr, float2& a, float2& b)   
 // The reference chain (above) is three roundings away from the real number R = ((acc - cc) m + b) / sy.  The hot path
 // evaluates q" = fma(float(acc), mq, bq) with mq = RN(m / sy) and bq = (b - cc m) / sy + zoff (zoff = the output zero
 // point, for the table also minus the type minimum) prepared per n-tile to within one rounding, so that
-//     |reference q + zoff - q"| <= E = 1.5 * 2^-24 * (4 Rmax + 3 RZmax + 2 max|b / sy| + 4 max|bq| + |zoff|)
-// for every value that can round to something inside the output range (Rmax, RZmax: the largest |R| and |R + zoff| that
-// do).  t = q" + MAGIC rounds q" to an integer n; whenever |q" - n| < 0.5 - E the reference's q lies on the same side of
+//     |reference q + zoff - q"| <= E = 1.1 * 2^-24 * ((3 + big) Rmax + (1 + big) max|b / sy| + (1 + big) (257 + max|bq|) + 2 max|bq| + |zoff| + 257)
+// for every value that can round to something inside the output range (Rmax: the largest |R| that does; |R + zoff| is at most 257
+// there; big: 1 where an accumulator can exceed 2^24, else 0).  t = q" + MAGIC rounds q" to an integer n; whenever |q" - n| < 0.5 - E the reference's q lies on the same side of
 // every rounding boundary, so n is the reference's result and the halves-away-from-zero rule cannot matter.  A group of
 // four values in which some lane sees |q" - n| >= 0.5 - E (about one group in twenty) is re-evaluated with the
 // reference arithmetic itself (epi_fix_values).  Values whose q" is huge lose the integer grid of the magic constant:
@@ -520,9 +520,9 @@ __device__ __forceinline__ void lds_f2x2(uint32_t addr, float2& a, float2& b)   
 // Where mq and bq come from.  TabFast: tables in shared memory, read with 128-bit loads that every lane of the warp
 // repeats (all lanes work on the same columns; bq: this lane's class row): four wavefronts of the shared-memory pipe per
 // four outputs and table.  TabFastP: tables in the kernel's parameter space (constant bank): the column index is the
-// same for the whole warp, so the loads are uniform loads that do not touch the shared-memory pipe at all, which is
-// what bounds the fused-Add epilogue (its table lookups live there too).  Only launches whose tables the host can
-// compute (see HostPack) and that have a single class of pixels take that form.
+// same for the whole warp, so the loads are uniform loads that do not touch the shared-memory pipe, which bounds a fused Add by
+// its table (its look-ups live there too); the Add as arithmetic takes that form where a CTA has several tiles (launch_conv_tc
+// has the figures).  Only launches whose tables the host can compute (see HostPack) and that have a single class of pixels do.
 struct TabFast {
     uint32_t mq, bq;
     __device__ __forceinline__ void load(int g, float2& m01, float2& m23, float2& b01, float2& b23) const
@@ -2341,8 +2341,8 @@ static int launch_conv_stem(const b200k_conv2d_params* p, cudaStream_t stream)
 
 // ---- host copies of a fused-Add convolution's per-channel constants ------------------------------------------------
 //
-// The fused-Add epilogue is bound by the shared-memory pipe (table lookups), so its mq / bq tables go through the
-// kernel's parameter space instead (TabFastP), which means the host has to know them.  b200k_conv2d_pack therefore
+// The mq / bq tables of a fused Add go through the kernel's parameter space where that is the faster place (see TabFastP), so the
+// host has to know them, and which form of the Add gives the entries of its table.  b200k_conv2d_pack therefore
 // reads the per-channel weight sums, scales and bias of such a layer back once (a few KB, at load time) and keeps
 // them keyed by the packed buffer's address; a launch uses them when the buffer and the four device arrays are the
 // ones that were packed, and otherwise stages its tables on the device as every other launch does.
