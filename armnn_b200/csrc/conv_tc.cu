@@ -735,8 +735,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 // two shared buffers; every epilogue warp releases it after reading its part.
 //
 // What a launch ends in is compiled in (MODE), so that none carries the others' code and registers: no fused Add; a fused Add by
-// its table or by its formula, each with the per-channel constants in shared memory or in the parameter space.
-enum { TC_PLAIN = 0, TC_LUT = 1, TC_LUT_PTAB = 2, TC_ADD = 3, TC_ADD_PTAB = 4 };
+// its table or by its formula, each with the per-channel constants in shared memory or in the parameter space; a fused Add without
+// tables (TC_EXACT).
+enum { TC_PLAIN = 0, TC_LUT = 1, TC_LUT_PTAB = 2, TC_ADD = 3, TC_ADD_PTAB = 4, TC_EXACT = 5 };
 //
 // PAIR: two CTAs of a cluster work on two neighbouring M-tiles and one n-tile as one 256 x BN MMA: each loads its own 128 rows of A
 // and half of the weight tile, the first CTA's issuer multiplies for both, each reads its own accumulators.  A wide tile's
@@ -748,7 +749,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmR,
                const __grid_constant__ TcArgs a, const __grid_constant__ std::conditional_t<MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB, TcTabs, TcNoTabs> tabs)
 {
-    constexpr bool PTAB = MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB, fused = MODE != TC_PLAIN, formula = MODE == TC_ADD || MODE == TC_ADD_PTAB;
+    constexpr bool PTAB = MODE == TC_LUT_PTAB || MODE == TC_ADD_PTAB, fused = MODE != TC_PLAIN, formula = MODE == TC_ADD || MODE == TC_ADD_PTAB, exact = MODE == TC_EXACT;
     using L = TcSmem<BN, SWZ>;
     static_assert(!PAIR || (EG == 1 && SWZ == 128), "CTA pairs: one tile per CTA in the epilogue");
     constexpr int B_BYTES = PAIR ? L::B_BYTES / 2 : L::B_BYTES;          // what this CTA loads of a slice's weight tile
@@ -875,7 +876,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int s = 0; s < a.nslices; ++s)
                     tma_load_2d(s_wst + (size_t)s * L::B_BYTES, &tmB, w_full, (int)s_tab[s].z, 0);
             }
-            if (fused && !formula && a.add_lut && prod == 0 && elect_one()) {
+            if (fused && !formula && !exact && a.add_lut && prod == 0 && elect_one()) {
                 // the fused-add table: one bulk copy (the epilogue checks its tag before using it)
                 mbar_expect_tx(lut_full, (uint32_t)TC_LUT_BYTES);
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -1060,7 +1061,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // The fused-add table arrives by a bulk copy the producer has issued.  A table is used only if it was built
         // for exactly this launch's quantisation parameters.
         bool lut_ok = false;
-        if (fused && !formula && a.add_lut) {
+        if (fused && !formula && !exact && a.add_lut) {
             if (etid == 0) {
                 uint32_t ok = 1;
                 const uint32_t* tag = (const uint32_t*)(a.add_lut + TC_LUT_BYTES);
@@ -1211,8 +1212,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
             }
         };
-        // A fused Add whose table is missing or made for other parameters: the reference arithmetic for every value, and no look-up
-        // (a launch without packed tables has no table in its shared memory either).
+        // A fused Add without packed tables has no table in its shared memory: the reference arithmetic for every value and no
+        // look-up.  In a kernel of its own: beside the look-ups, as another way through the same kernel, it made 64 -> 256
+        // channels, 56 x 56 at batch 256, with a table 161 us instead of 143.
         auto exact_chunks = [&](uint32_t* r, uint32_t tcol, int col0, uint32_t res_row, uint32_t st_row, uint32_t a_m, uint32_t a_b, uint32_t a_cc) {
             tc_ld16_wait(r);                                 // (no load in flight across the call)
             #pragma unroll 1
@@ -1279,7 +1281,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const uint32_t st_row = st_base + (uint32_t)lane * W;
                     auto chunks = [&](auto kind_tag) { unit_chunks(kind_tag, r, tacc + (uint32_t)colw, colw, res_row, st_row, a_m, a_b, a_cc, a_mq, a_bq, n0); };
                     if constexpr (formula)    chunks(std::integral_constant<int, EPI_ADD>{});
-                    else if constexpr (fused) { if (use_lut) chunks(std::integral_constant<int, EPI_LUT>{}); else exact_chunks(r, tacc + (uint32_t)colw, colw, res_row, st_row, a_m, a_b, a_cc); }
+                    else if constexpr (exact) exact_chunks(r, tacc + (uint32_t)colw, colw, res_row, st_row, a_m, a_b, a_cc);
+                    else if constexpr (fused) chunks(std::integral_constant<int, EPI_LUT>{});      // (with a table for other parameters its results are all replaced)
                     else if (kind == EPI_SAT_U8) chunks(std::integral_constant<int, EPI_SAT_U8>{});
                     else if (kind == EPI_SAT_S8) chunks(std::integral_constant<int, EPI_SAT_S8>{});
                     else chunks(std::integral_constant<int, EPI_CLAMP>{});
@@ -1713,6 +1716,7 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUten
 {
     if constexpr (EG == 1 && MODE == TC_PLAIN && !PAIR) {
         if (a.res) {
+            if (!formula && !a.add_lut) return launch_tc<BN, SWZ, EG, TC_EXACT>(tmA, tmB, tmY, tmR, a, stream);
             if (formula) return tabs ? launch_tc<BN, SWZ, EG, TC_ADD_PTAB>(tmA, tmB, tmY, tmR, a, stream, tabs) : launch_tc<BN, SWZ, EG, TC_ADD>(tmA, tmB, tmY, tmR, a, stream);
             return tabs ? launch_tc<BN, SWZ, EG, TC_LUT_PTAB>(tmA, tmB, tmY, tmR, a, stream, tabs) : launch_tc<BN, SWZ, EG, TC_LUT>(tmA, tmB, tmY, tmR, a, stream);
         }
